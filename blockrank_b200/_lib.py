@@ -20,7 +20,8 @@ EXPORTS = ("brk_version", "brk_last_error", "brk_device_check", "brk_spans_from_
            "brk_attn_fwd_workspace_bytes", "brk_attn_fwd", "brk_attn_bwd_workspace_bytes", "brk_attn_bwd",
            "brk_status_poll", "brk_selftest_bounded_wait",
            "brk_doc_scores_workspace_bytes",
-           "brk_doc_scores", "brk_doc_scores_static", "brk_raw_scores", "brk_rmsnorm", "brk_rope", "brk_silu_mul")
+           "brk_doc_scores", "brk_doc_scores_static", "brk_raw_scores",
+           "brk_raw_scores_bwd_workspace_bytes", "brk_raw_scores_bwd", "brk_rmsnorm", "brk_rope", "brk_silu_mul")
 
 
 class View(C.Structure):
@@ -92,6 +93,11 @@ def lib() -> C.CDLL:
     L.brk_doc_scores_static.argtypes = [C.POINTER(ScoreParams), C.c_void_p]
     L.brk_raw_scores.restype = C.c_int
     L.brk_raw_scores.argtypes = [C.POINTER(ScoreParams), C.c_void_p, C.c_void_p]
+    L.brk_raw_scores_bwd_workspace_bytes.restype = C.c_size_t
+    L.brk_raw_scores_bwd_workspace_bytes.argtypes = [C.POINTER(ScoreParams)]
+    L.brk_raw_scores_bwd.restype = C.c_int
+    L.brk_raw_scores_bwd.argtypes = [C.POINTER(ScoreParams), C.c_void_p, C.POINTER(View), C.POINTER(View), C.c_int32,
+                                     C.c_void_p, C.c_size_t, C.c_void_p]
     L.brk_rmsnorm.restype = C.c_int
     L.brk_rmsnorm.argtypes = [C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32,
                               C.c_float, C.c_void_p]

@@ -17,12 +17,13 @@
 #include <algorithm>
 
 #include "brk_common.cuh"
+#include "mma_bf16.cuh"
 
 namespace brk {
 
 namespace {
 
-constexpr int kT = 64;         // tokens (rows or keys) per staged tile
+constexpr int kT = kMmaTileRows;  // tokens (rows or keys) per staged tile
 constexpr int kWarps = 4;
 constexpr int kThreadsM = kWarps * 32;
 // Row-tile buffers of the dk/dv kernel: 2 = the next tile is requested before the current one is multiplied (104 KB
@@ -51,37 +52,10 @@ __device__ __forceinline__ void span_of(const BwdMmaArgs& a, int b, int m, int& 
   if (start < 0 || len < 0 || len > a.max_block_len || start > a.S - len) len = 0;  // skipped: nothing out of bounds
 }
 
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void* p) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(p);
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(s));
-}
-__device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const void* p) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(p);
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(s));
-}
-__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-  return *reinterpret_cast<uint32_t*>(&h);
-}
-
-template <int D>
-struct Tile {
-  static constexpr int kPitch = D + 8;  // elements: 16 bytes of padding per row
-  __nv_bfloat16 e[kT][kPitch];
-};
-
 // rows [row0, row0 + kT) of head `h` of a (B, heads, S, D) bf16 tensor -> tile, zero beyond `nvalid`.
 // All of a thread's loads are issued before its first store, so a tile costs one memory latency.
 template <int D>
-__device__ __forceinline__ void stage(Tile<D>& t, const View& x, int b, int h, int row0, int nvalid) {
+__device__ __forceinline__ void stage(MmaTile<D>& t, const View& x, int b, int h, int row0, int nvalid) {
   constexpr int kPer = kT * (D / 8) / kThreadsM;
   const __nv_bfloat16* base = reinterpret_cast<const __nv_bfloat16*>(x.ptr) + (int64_t)b * x.sb + (int64_t)h * x.sh;
   uint4 val[kPer];
@@ -99,25 +73,10 @@ __device__ __forceinline__ void stage(Tile<D>& t, const View& x, int b, int h, i
   }
 }
 
-__device__ __forceinline__ void cp_async16_zfill(void* smem_dst, const void* gmem_src, bool valid) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
-  const int n = valid ? 16 : 0;  // 0 source bytes: the 16 destination bytes are filled with zeros
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gmem_src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
 // the same copy as stage(), asynchronous (completion through cp.async groups): the next tile travels while the
 // current one is multiplied
 template <int D>
-__device__ __forceinline__ void stage_async(Tile<D>& t, const View& x, int b, int h, int row0, int nvalid) {
+__device__ __forceinline__ void stage_async(MmaTile<D>& t, const View& x, int b, int h, int row0, int nvalid) {
   constexpr int kPer = kT * (D / 8) / kThreadsM;
   const __nv_bfloat16* base = reinterpret_cast<const __nv_bfloat16*>(x.ptr) + (int64_t)b * x.sb + (int64_t)h * x.sh;
 #pragma unroll
@@ -131,7 +90,7 @@ __device__ __forceinline__ void stage_async(Tile<D>& t, const View& x, int b, in
 
 // A fragments (16 rows x D) of rows [r0, r0+16) of a tile: frag[ks] covers columns [16 ks, 16 ks + 16)
 template <int D>
-__device__ __forceinline__ void load_a(uint32_t (&frag)[D / 16][4], const Tile<D>& t, int r0, int lane) {
+__device__ __forceinline__ void load_a(uint32_t (&frag)[D / 16][4], const MmaTile<D>& t, int r0, int lane) {
   const int j = lane >> 3, r = lane & 7;
 #pragma unroll
   for (int ks = 0; ks < D / 16; ++ks) ldsm_x4(frag[ks], &t.e[r0 + r + (j & 1) * 8][ks * 16 + (j >> 1) * 8]);
@@ -139,7 +98,7 @@ __device__ __forceinline__ void load_a(uint32_t (&frag)[D / 16][4], const Tile<D
 
 // C[16 x 16] (two n-tiles: c[0] columns 0..7, c[1] columns 8..15) = A[16 x D] * Y[n0 .. n0+16][0 .. D)^T
 template <int D>
-__device__ __forceinline__ void mm_nt(float (&c)[2][4], const uint32_t (&a)[D / 16][4], const Tile<D>& y, int n0, int lane) {
+__device__ __forceinline__ void mm_nt(float (&c)[2][4], const uint32_t (&a)[D / 16][4], const MmaTile<D>& y, int n0, int lane) {
   const int j = lane >> 3, r = lane & 7;
 #pragma unroll
   for (int i = 0; i < 4; ++i) c[0][i] = c[1][i] = 0.f;
@@ -152,28 +111,15 @@ __device__ __forceinline__ void mm_nt(float (&c)[2][4], const uint32_t (&a)[D / 
   }
 }
 
-// acc[16 x D] += A[16 x 16] * Z[k0 .. k0+16][0 .. D)   (acc[nt] covers columns [8 nt, 8 nt + 8))
-template <int D>
-__device__ __forceinline__ void mm_nn_acc(float (&acc)[D / 8][4], const uint32_t (&a)[4], const Tile<D>& z, int k0, int lane) {
-  const int j = lane >> 3, r = lane & 7;
-#pragma unroll
-  for (int np = 0; np < D / 16; ++np) {
-    uint32_t bfr[4];
-    ldsm_x4_t(bfr, &z.e[k0 + r + (j & 1) * 8][np * 16 + (j >> 1) * 8]);
-    mma16816(acc[2 * np], a, bfr[0], bfr[1]);
-    mma16816(acc[2 * np + 1], a, bfr[2], bfr[3]);
-  }
-}
-
 // grid: x = 64-token tile of the block, y = block, z = prompt * N + head.  kLast: the launch for the last block,
 // whose rows see every key of the prompt: y = split instead, the row tile's key tiles are dealt to `ksplit` CTAs
 // and the results are added into the fp32 array dq32 (converted by attn_bwd_store_dq_last_kernel).
 template <int D, bool kLast>
 __global__ void __launch_bounds__(kThreadsM, 3) attn_bwd_dq_mma_kernel(BwdMmaArgs a) {
   extern __shared__ __align__(16) unsigned char dyn_smem[];
-  Tile<D>* const tiles = reinterpret_cast<Tile<D>*>(dyn_smem);  // [0], [1]: Q / dO first, then K / V; [2], [3]: the other K / V buffer
-  Tile<D>& t0s = tiles[0];
-  Tile<D>& t1s = tiles[1];
+  MmaTile<D>* const tiles = reinterpret_cast<MmaTile<D>*>(dyn_smem);  // [0], [1]: Q / dO first, then K / V; [2], [3]: the other K / V buffer
+  MmaTile<D>& t0s = tiles[0];
+  MmaTile<D>& t1s = tiles[1];
   __shared__ float delta_s[kT], lse_s[kT];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
   const int b = blockIdx.z / a.N, head = blockIdx.z % a.N, g = head / a.G;
@@ -280,8 +226,8 @@ __global__ void __launch_bounds__(kThreadsM, 3) attn_bwd_dq_mma_kernel(BwdMmaArg
     cp_async_wait<1>();  // all but the newest group: the current tile has landed
     __syncthreads();
     {
-      const Tile<D>& kt = tiles[2 * buf];
-      const Tile<D>& vt = tiles[2 * buf + 1];
+      const MmaTile<D>& kt = tiles[2 * buf];
+      const MmaTile<D>& vt = tiles[2 * buf + 1];
       const bool own = cur.own;
       const int k0 = cur.k0, nv = min(kT, cur.kl - cur.k0);
       // this warp's rows see keys up to (own block) token tok0 + 16 warp + 15
@@ -367,10 +313,10 @@ __global__ void __launch_bounds__(256) attn_bwd_store_dq_last_kernel(BwdMmaArgs 
 template <int D>
 __global__ void __launch_bounds__(kThreadsM, 2) attn_bwd_dkv_mma_kernel(BwdMmaArgs a) {
   extern __shared__ __align__(16) unsigned char dyn_smem[];
-  Tile<D>& ks_t = *reinterpret_cast<Tile<D>*>(dyn_smem);
-  Tile<D>& vs_t = *reinterpret_cast<Tile<D>*>(dyn_smem + sizeof(Tile<D>));
-  Tile<D>* const row_tiles = reinterpret_cast<Tile<D>*>(dyn_smem + 2 * sizeof(Tile<D>));  // [2 buf]: Q, [2 buf + 1]: dO
-  float* const row_stats = reinterpret_cast<float*>(dyn_smem + (2 + 2 * kRowBufs) * sizeof(Tile<D>));  // [buf][lse: kT | delta: kT]
+  MmaTile<D>& ks_t = *reinterpret_cast<MmaTile<D>*>(dyn_smem);
+  MmaTile<D>& vs_t = *reinterpret_cast<MmaTile<D>*>(dyn_smem + sizeof(MmaTile<D>));
+  MmaTile<D>* const row_tiles = reinterpret_cast<MmaTile<D>*>(dyn_smem + 2 * sizeof(MmaTile<D>));  // [2 buf]: Q, [2 buf + 1]: dO
+  float* const row_stats = reinterpret_cast<float*>(dyn_smem + (2 + 2 * kRowBufs) * sizeof(MmaTile<D>));  // [buf][lse: kT | delta: kT]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
   const int split = blockIdx.z % a.nsplit, bg = blockIdx.z / a.nsplit;
   const int b = bg / a.Nk, g = bg % a.Nk;
@@ -451,8 +397,8 @@ __global__ void __launch_bounds__(kThreadsM, 2) attn_bwd_dkv_mma_kernel(BwdMmaAr
     }
     __syncthreads();     // (the first time also: K and V of this CTA's keys are in place)
     {
-      const Tile<D>& qs_t = row_tiles[2 * buf];
-      const Tile<D>& gs_t = row_tiles[2 * buf + 1];
+      const MmaTile<D>& qs_t = row_tiles[2 * buf];
+      const MmaTile<D>& gs_t = row_tiles[2 * buf + 1];
       const float* lse_s = row_stats + buf * 2 * kT;
       const float* delta_s = lse_s + kT;
       const bool own = cur.own;
@@ -519,7 +465,7 @@ __global__ void __launch_bounds__(kThreadsM, 2) attn_bwd_dkv_mma_kernel(BwdMmaAr
 template <int D>
 int launch_mma(BwdMmaArgs a, cudaStream_t st) {
   const int tiles = (a.max_block_len + kT - 1) / kT;
-  const int smem_dq = 4 * (int)sizeof(Tile<D>);
+  const int smem_dq = 4 * (int)sizeof(MmaTile<D>);
   BRK_CUDA(cudaFuncSetAttribute(attn_bwd_dq_mma_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dq));
   BRK_CUDA(cudaFuncSetAttribute(attn_bwd_dq_mma_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dq));
   // the last block first: its CTAs are the long ones
@@ -536,7 +482,7 @@ int launch_mma(BwdMmaArgs a, cudaStream_t st) {
     attn_bwd_store_dq_last_kernel<D><<<std::max(blocks, 1), 256, 0, st>>>(a);
     BRK_CUDA(cudaGetLastError());
   }
-  const int smem = (2 + 2 * kRowBufs) * (int)sizeof(Tile<D>) + 2 * kRowBufs * kT * (int)sizeof(float);
+  const int smem = (2 + 2 * kRowBufs) * (int)sizeof(MmaTile<D>) + 2 * kRowBufs * kT * (int)sizeof(float);
   BRK_CUDA(cudaFuncSetAttribute(attn_bwd_dkv_mma_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   // block 0's keys are seen by every row block: many CTAs per key tile; the other blocks' keys by two at most
   a.m_base = 0;

@@ -172,6 +172,14 @@ int brk_raw_scores(const brk_score_params* p, void* out, void* stream) {
   return raw_scores_launch(*p, out, (cudaStream_t)stream);
 }
 
+size_t brk_raw_scores_bwd_workspace_bytes(const brk_score_params* p) { return p ? raw_scores_bwd_workspace(*p) : 0; }
+
+int brk_raw_scores_bwd(const brk_score_params* p, const void* d_raw, const brk_view* dq, const brk_view* dk,
+                       int32_t accumulate, void* workspace, size_t workspace_bytes, void* stream) {
+  BRK_REQUIRE(p != nullptr && dq != nullptr && dk != nullptr, BRK_E_ARG, "params / dq / dk is null");
+  return raw_scores_bwd_launch(*p, d_raw, *dq, *dk, accumulate, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
 int brk_rmsnorm(int32_t dtype, const void* x, void* residual, const void* weight, void* out, int64_t rows,
                 int32_t hidden, float eps, void* stream) {
   BRK_REQUIRE(x && weight && out, BRK_E_ARG, "null pointer");

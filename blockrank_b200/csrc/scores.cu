@@ -20,12 +20,12 @@
 //                        merges the per-document pairs into the softmax over all
 //                        document tokens, emits the per-document probability mass and
 //                        then the mean over heads and rows / temperature.
-//   raw_scores_kernel    compatibility output: raw masked logits of the last R
-//                        slots against every slot.
 #include <algorithm>
 #include <atomic>
 
 #include "brk_common.cuh"
+#include "mma_bf16.cuh"
+#include "score_args.cuh"
 
 namespace brk {
 namespace {
@@ -35,30 +35,6 @@ constexpr int kRowBatch = 8;  // signal rows accumulated per pass over a key
 constexpr int kKeyStages = 4;   // asynchronous key-row copies a lane keeps in flight in the bf16 kernel
 constexpr int kDocsPerCta = 64;  // documents one CTA of the bf16 kernel walks through, at most
 
-struct ScoreArgs {
-  View q, k;
-  const int32_t* rows;
-  const int32_t* blk_start;
-  const int32_t* blk_len;
-  float2* partial;  // [B, N, R, nd]
-  unsigned* done_bg;  // [B, Nk] document CTAs of the (prompt, KV head) that have published their partials
-  unsigned* done_b;   // [B] KV-head groups of the prompt whose masses are written; both wrap to 0 by themselves
-  float* mass;      // [B, N, R, nd] out
-  float* logits;    // [B, nd] out, optional
-  float inv_count_temp;  // 1 / (N * R * temperature)
-  int B, N, Nk, S, M, R;
-  float scale;
-};
-
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 
 __device__ __forceinline__ void merge_ml(float& m, float& l, float m2, float l2) {
   const float mn = fmaxf(m, m2);
@@ -292,14 +268,6 @@ __global__ void __launch_bounds__(kThreads) doc_partial_kernel(ScoreArgs a) {
   finalize_if_last(a, b, g);
 }
 
-__device__ __forceinline__ void mma_bf16_16x8x16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                                 uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 // bf16 version of doc_partial_kernel on warp-level MMA.  One CTA per (document, prompt, KV head);
 // a warp takes 8 keys at a time: C[16 signal rows x 8 keys] += Q[16 x 16] K^T[16 x 8] over D/16
 // steps.  Lane (q = lane/4, j = lane%4) reads 16 bytes (8 elements of d) of key q per 32 elements
@@ -391,8 +359,8 @@ __global__ void __launch_bounds__(kThreads, 4) doc_partial_mma_kernel(ScoreArgs 
         float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int st = 0; st < kSteps; ++st) {
-          mma_bf16_16x8x16(c, qa[st].x, qb[st].x, qa[st].y, qb[st].y, kf[st].x, kf[st].y);
-          mma_bf16_16x8x16(c, qa[st].z, qb[st].z, qa[st].w, qb[st].w, kf[st].z, kf[st].w);
+          mma16816(c, {qa[st].x, qb[st].x, qa[st].y, qb[st].y}, kf[st].x, kf[st].y);
+          mma16816(c, {qa[st].z, qb[st].z, qa[st].w, qb[st].w}, kf[st].z, kf[st].w);
         }
         // c[0], c[1]: row qr, keys base + 2j, 2j + 1; c[2], c[3]: row qr + 8, same keys
         const bool ok0 = base + 2 * j < len, ok1 = base + 2 * j + 1 < len;
@@ -431,94 +399,6 @@ __global__ void __launch_bounds__(kThreads, 4) doc_partial_mma_kernel(ScoreArgs 
   finalize_if_last(a, b, g);
 }
 
-// block index of a slot, or -1 for padding (blk_start is non-decreasing)
-__device__ __forceinline__ int block_of(const int32_t* bs, const int32_t* bl, int M, int s) {
-  int lo = 0, hi = M;  // first index with bs > s
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (bs[mid] <= s) lo = mid + 1; else hi = mid;
-  }
-  const int m = lo - 1;
-  return (m >= 0 && s < bs[m] + bl[m]) ? m : -1;
-}
-
-template <typename T, int D>
-__global__ void __launch_bounds__(kThreads) raw_scores_kernel(ScoreArgs a, T* __restrict__ out, float neg) {
-  extern __shared__ __align__(16) float smem[];
-  const int G = a.N / a.Nk;
-  const int GR = G * a.R;
-  float* qs = smem;                               // [GR][D], scaled and rounded like the reference's Q*scaling
-  int* qblk = reinterpret_cast<int*>(qs + GR * D);  // [R] block index of each row (-1 = padding)
-  const int b = blockIdx.y / a.Nk, g = blockIdx.y % a.Nk;
-  const int tid = threadIdx.x;
-  const int32_t* bs = a.blk_start + (size_t)b * a.M;
-  const int32_t* bl = a.blk_len + (size_t)b * a.M;
-  for (int i = tid; i < GR * D; i += kThreads) {
-    const int row = i / D, dd = i % D;
-    const int hl = row / a.R, r = row % a.R;
-    const T* qp = reinterpret_cast<const T*>(a.q.ptr) + (int64_t)b * a.q.sb + (int64_t)(g * G + hl) * a.q.sh +
-                  (int64_t)(a.S - a.R + r) * a.q.ss;
-    qs[i] = Elem<T>::round(Elem<T>::load(qp + dd) * a.scale);
-  }
-  if (tid < a.R) qblk[tid] = block_of(bs, bl, a.M, a.S - a.R + tid);
-  __syncthreads();
-  const int s = blockIdx.x * kThreads + tid;
-  if (s >= a.S) return;
-  const int kblk = block_of(bs, bl, a.M, s);
-  const T* kp = reinterpret_cast<const T*>(a.k.ptr) + (int64_t)b * a.k.sb + (int64_t)g * a.k.sh + (int64_t)s * a.k.ss;
-  for (int r0 = 0; r0 < GR; r0 += kRowBatch) {
-    const int nrows = min(kRowBatch, GR - r0);
-    float acc[kRowBatch];
-    key_dots<T, D>(kp, qs + r0 * D, nrows, acc);
-#pragma unroll
-    for (int i = 0; i < kRowBatch; ++i) {
-      if (i < nrows) {
-        const int row = r0 + i;
-        const int n = g * G + row / a.R, r = row % a.R;
-        const int qb = qblk[r], qslot = a.S - a.R + r;
-        const bool ok = qb >= 0 && kblk >= 0 &&
-                        ((kblk == qb && s <= qslot) || (qb == a.M - 1 && kblk < qb) ||
-                         (qb > 0 && qb < a.M - 1 && kblk == 0));
-        Elem<T>::store(out + (((size_t)b * a.N + n) * a.R + r) * a.S + s, ok ? acc[i] : neg);
-      }
-    }
-  }
-}
-
-ScoreArgs make_args(const brk_score_params& p) {
-  ScoreArgs a;
-  a.q = make_view(p.q);
-  a.k = make_view(p.k);
-  a.rows = p.rows;
-  a.blk_start = p.blk_start;
-  a.blk_len = p.blk_len;
-  a.partial = nullptr;
-  a.done_bg = nullptr;
-  a.done_b = nullptr;
-  a.mass = nullptr;
-  a.logits = nullptr;
-  a.inv_count_temp = 0.f;
-  a.B = p.B; a.N = p.N; a.Nk = p.Nk; a.S = p.S; a.M = p.M; a.R = p.R;
-  a.scale = p.scale;
-  return a;
-}
-
-int check(const brk_score_params& p) {
-  BRK_REQUIRE(p.q.ptr && p.k.ptr && p.blk_start && p.blk_len, BRK_E_ARG, "null pointer in score params");
-  BRK_REQUIRE(p.B > 0 && p.N > 0 && p.Nk > 0 && p.N % p.Nk == 0 && p.S > 0 && p.M >= 1, BRK_E_ARG,
-              "bad score shape B=%d N=%d Nk=%d S=%d M=%d", p.B, p.N, p.Nk, p.S, p.M);
-  BRK_REQUIRE(p.R >= 1 && p.R <= 64 && (p.N / p.Nk) * p.R <= 256, BRK_E_ARG, "R=%d out of range", p.R);
-  BRK_REQUIRE(p.D == 64 || p.D == 128, BRK_E_UNSUPPORTED, "head_dim %d not supported (64 or 128)", p.D);
-  BRK_REQUIRE(p.dtype == BRK_BF16 || p.dtype == BRK_F32, BRK_E_UNSUPPORTED, "dtype %d", p.dtype);
-  const int al = p.dtype == BRK_BF16 ? 8 : 4;
-  BRK_REQUIRE(p.q.stride_s % al == 0 && p.q.stride_h % al == 0 && p.q.stride_b % al == 0 && p.k.stride_s % al == 0 &&
-                  p.k.stride_h % al == 0 && p.k.stride_b % al == 0 && ((uintptr_t)p.q.ptr % 16 == 0) &&
-                  ((uintptr_t)p.k.ptr % 16 == 0),
-              BRK_E_ARG, "q/k rows must be 16-byte aligned");
-  BRK_REQUIRE(p.B * p.Nk <= 65535, BRK_E_UNSUPPORTED, "B*Nk too large");
-  return BRK_OK;
-}
-
 }  // namespace
 
 // scratch layout: completion counters ([B, Nk] then [B] unsigned, padded to `counter_bytes`), then the
@@ -536,14 +416,14 @@ size_t doc_scores_workspace(const brk_score_params& p) { return counter_bytes(p)
 // counters_zero: the caller guarantees that the counters are zero (they return to zero after every completed call)
 static int doc_scores_run(const brk_score_params& p, void* ws, size_t ws_bytes, size_t counter_region, bool counters_zero,
                           cudaStream_t st) {
-  int rc = check(p);
+  int rc = check_score_params(p);
   if (rc) return rc;
   BRK_REQUIRE(p.M >= 3, BRK_E_ARG, "document scores need at least one document block (M=%d)", p.M);
   BRK_REQUIRE(p.rows && p.doc_mass, BRK_E_ARG, "rows / doc_mass must be given");
   BRK_REQUIRE(ws != nullptr && ws_bytes >= counter_region + partial_bytes(p) && ((uintptr_t)ws & 7) == 0, BRK_E_WORKSPACE,
               "workspace %zu < %zu bytes (or not 8-byte aligned)", ws_bytes, counter_region + partial_bytes(p));
   BRK_REQUIRE(p.temperature > 0.f, BRK_E_ARG, "temperature must be positive");
-  ScoreArgs a = make_args(p);
+  ScoreArgs a = make_score_args(p);
   a.done_bg = reinterpret_cast<unsigned*>(ws);
   a.done_b = a.done_bg + (size_t)p.B * p.Nk;
   a.partial = reinterpret_cast<float2*>(static_cast<unsigned char*>(ws) + counter_region);
@@ -598,7 +478,7 @@ static __device__ __align__(256) unsigned char g_static_scratch[BRK_STATIC_SCRAT
 constexpr size_t kStaticCounterBytes = 16384;  // room for 4096 counters: B * (Nk + 1) <= 4096
 
 int doc_scores_static_launch(const brk_score_params& p, cudaStream_t st) {
-  int rc = check(p);  // argument errors are reported as such, before the size test
+  int rc = check_score_params(p);  // argument errors are reported as such, before the size test
   if (rc) return rc;
   BRK_REQUIRE(p.M >= 3, BRK_E_ARG, "document scores need at least one document block (M=%d)", p.M);
   // the counters keep a fixed place at the front of the array whatever the problem size, so that the zeros
@@ -628,33 +508,6 @@ int doc_scores_static_launch(const brk_score_params& p, cudaStream_t st) {
   // every (prompt, head, row, document) pair is overwritten by the partial kernels before the finalizing CTA
   // reads it, and the counters are back at zero, so nothing left by an earlier call has to be cleared
   return doc_scores_run(p, ptr, (size_t)BRK_STATIC_SCRATCH_BYTES, kStaticCounterBytes, true, st);
-}
-
-int raw_scores_launch(const brk_score_params& p, void* out, cudaStream_t st) {
-  int rc = check(p);
-  if (rc) return rc;
-  BRK_REQUIRE(out != nullptr, BRK_E_ARG, "out is null");
-  BRK_REQUIRE(p.R <= p.S, BRK_E_ARG, "R=%d exceeds S=%d", p.R, p.S);
-  ScoreArgs a = make_args(p);
-  const int G = p.N / p.Nk;
-  dim3 grid((p.S + kThreads - 1) / kThreads, p.B * p.Nk);
-  const size_t sm = (size_t)G * p.R * p.D * 4 + p.R * sizeof(int);
-  auto launch = [&](auto kern, auto* o, float neg) -> int {
-    // (the kernels also hold a few KB of static shared memory, which counts against the same 48 KB default)
-    if (sm + 8192 > 48 * 1024) BRK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    kern<<<grid, kThreads, sm, st>>>(a, o, neg);
-    BRK_CUDA(cudaGetLastError());
-    return BRK_OK;
-  };
-  // 0.7 * lowest finite value of the dtype, computed the way the reference does (python float -> dtype)
-  if (p.dtype == BRK_BF16) {
-    const float neg = 0.7f * -3.3895313892515355e38f;
-    return p.D == 128 ? launch(raw_scores_kernel<__nv_bfloat16, 128>, (__nv_bfloat16*)out, neg)
-                      : launch(raw_scores_kernel<__nv_bfloat16, 64>, (__nv_bfloat16*)out, neg);
-  }
-  const float neg = (float)(0.7 * -3.4028234663852886e38);
-  return p.D == 128 ? launch(raw_scores_kernel<float, 128>, (float*)out, neg)
-                    : launch(raw_scores_kernel<float, 64>, (float*)out, neg);
 }
 
 }  // namespace brk

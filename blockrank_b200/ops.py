@@ -236,6 +236,36 @@ def raw_scores(q: torch.Tensor, k: torch.Tensor, blk_start: torch.Tensor, blk_le
     return out
 
 
+def raw_scores_bwd(q: torch.Tensor, k: torch.Tensor, d_raw: torch.Tensor, blk_start: torch.Tensor, blk_len: torch.Tensor,
+                   scale: float, dq: Optional[torch.Tensor] = None, dk: Optional[torch.Tensor] = None):
+    """Gradient of :func:`raw_scores`: d_raw (B,N,R,S) -> (dq (B,N,S,D), dk (B,Nk,S,D)).
+
+    With dq and dk given (both, e.g. what :func:`attention_bwd` returned) it is added to them in place; otherwise new
+    tensors are returned, dq zero outside the last R rows."""
+    _need_cuda(q, k, d_raw, dq, dk)
+    B, N, S, D = q.shape
+    Nk, R = k.shape[1], d_raw.shape[2]
+    if d_raw.shape != (B, N, R, S) or d_raw.dtype != q.dtype:
+        raise ValueError(f"d_raw must be ({B}, {N}, R, {S}) {q.dtype}, got {tuple(d_raw.shape)} {d_raw.dtype}")
+    add = dq is not None
+    if add != (dk is not None):
+        raise ValueError("give both dq and dk, or neither")
+    if not add:
+        dq = torch.zeros(B, S, N, D, dtype=q.dtype, device=q.device).permute(0, 2, 1, 3)
+        dk = torch.empty(B, S, Nk, D, dtype=q.dtype, device=q.device).permute(0, 2, 1, 3)
+    d_raw, bs, bl = d_raw.contiguous(), blk_start.contiguous(), blk_len.contiguous()
+    p = _score_params(q, k, bs, bl, scale, R)
+    vq, vk = _view(dq), _view(dk)
+    L = _lib.lib()
+    with torch.cuda.device(q.device):
+        nbytes = L.brk_raw_scores_bwd_workspace_bytes(C.byref(p))
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+        _lib.check(L.brk_raw_scores_bwd(C.byref(p), d_raw.data_ptr(), C.byref(vq), C.byref(vk), int(add), ws.data_ptr(),
+                                        nbytes, _stream(q)), "brk_raw_scores_bwd")
+    _count(2)
+    return dq, dk
+
+
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, residual: Optional[torch.Tensor] = None,
             out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """RMSNorm over the last dim.  With ``residual`` given: residual += x (in place), norm of the sum."""

@@ -221,6 +221,17 @@ BRK_API int brk_doc_scores_static(const brk_score_params* p, void* stream);
  * Uses q, k, scale, blk_* of brk_score_params; rows/doc_mass/logits ignored. */
 BRK_API int brk_raw_scores(const brk_score_params* p, void* out, void* stream);
 
+/* Gradient of brk_raw_scores (what autograd derives from the reference's raw-score return; the mask addend is constant,
+ * so d_raw reaches every position): with d_raw[B, N, R, S] in `dtype`,
+ *   dk[b, g, s] (+)= scale * sum over the group's heads and the last R rows of d_raw * q,  every slot s
+ *   dq[b, n, S-R+r] (+)= scale * sum over s of d_raw * k
+ * dq (B, N, S, D) and dk (B, Nk, S, D) are views in `dtype`.  accumulate != 0: added to what dq / dk hold (the gradients
+ * of the attention output); 0: dk and the last R rows of dq are overwritten, other rows of dq are not touched.
+ * workspace: brk_raw_scores_bwd_workspace_bytes() bytes of device scratch, 16-byte aligned. */
+BRK_API size_t brk_raw_scores_bwd_workspace_bytes(const brk_score_params* p);
+BRK_API int brk_raw_scores_bwd(const brk_score_params* p, const void* d_raw, const brk_view* dq, const brk_view* dk,
+                               int32_t accumulate, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Runner helpers (the model code around the attention call; the reference
  * relies on transformers' modeling_mistral.py for these). All row-major. */
 /* out = weight * (x * rsqrt(mean(x^2) + eps)); if residual != NULL first

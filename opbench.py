@@ -278,7 +278,7 @@ def backward_bench(a, ops, ref_loader, q, k, v, mask, start, ln, scale, H, S, pr
         try:
             qg, kg, vg = (t.detach().clone().requires_grad_(True) for t in (q, k, v))
             if name == "ours":
-                run = lambda: _AttentionFn.apply(qg, kg, vg, start, ln, scale, H, 0, _lib.ALGO_AUTO)
+                run = lambda: _AttentionFn.apply(qg, kg, vg, start, ln, scale, H, 0, _lib.ALGO_AUTO, None, None)
             else:
                 if not ref_loader.available():
                     raise RuntimeError(ref_loader.why_unavailable())

@@ -181,3 +181,41 @@ def test_fused_doc_scores_refuse_autograd():
         cuda_blockrank_attention_forward(Layer(), q, k, v, cuda_blockrank_attention_mask(attention_mask=mask.to(dev)),
                                          0.125, layers_to_return_scores=[0], blockrank_doc_scores=True,
                                          signal_rows=torch.tensor([[22, 23]]))
+
+
+@pytest.mark.parametrize("N,Nk,D,M,H,R,dtype", [
+    (8, 2, 128, 5, 48, 16, torch.bfloat16),    # 64 (head, row) pairs, slots not a multiple of the 64-slot tile
+    (4, 4, 64, 3, 8, 8, torch.bfloat16),       # window = H, 8 pairs, fewer slots than one tile
+    (4, 2, 128, 7, 16, 16, torch.bfloat16),    # 32 pairs
+    (16, 2, 64, 4, 32, 16, torch.bfloat16),    # 128 pairs: two passes
+    (2, 1, 128, 3, 9, 5, torch.bfloat16),      # odd S (27), odd R
+    (8, 2, 128, 5, 48, 16, torch.float32),
+    (16, 2, 64, 3, 9, 9, torch.float32),       # 72 pairs, odd S
+])
+def test_raw_scores_and_gradient(N, Nk, D, M, H, R, dtype):
+    """Raw logits and their gradient (added to given gradients, and on their own) against fp64 products."""
+    from blockrank_b200 import ops
+    g = torch.Generator().manual_seed(N * D + M)
+    B, S, scale = 2, M * H, D ** -0.5
+    lens = torch.randint(1, H + 1, (B, M), generator=g).tolist()
+    mask = _mask(lens, H)
+    rb = lambda *s: torch.randn(*s, generator=g).to(dtype).cuda()
+    q, k, d_raw = rb(B, N, S, D), rb(B, Nk, S, D), rb(B, N, R, S)
+    dq0, dk0 = rb(B, N, S, D), rb(B, Nk, S, D)
+    start, ln = ops.spans_from_mask(mask.cuda())
+    raw = ops.raw_scores(q, k, start, ln, scale, R).double().cpu()
+    ql, kx = (q[:, :, S - R:] * scale).double().cpu(), k.double().cpu().repeat_interleave(N // Nk, 1)
+    ref = ql @ kx.transpose(-1, -2)
+    ok = orc.allowed_pairs(mask)[:, None, S - R:].expand(B, N, R, S)
+    tol = 1e-2 if dtype == torch.bfloat16 else 1e-5
+    assert (raw[~ok] < -1e37).all()
+    assert (raw - ref)[ok].norm() <= tol * ref[ok].norm()
+    gd = d_raw.double().cpu() * scale
+    rq = torch.zeros(B, N, S, D, dtype=torch.float64)
+    rq[:, :, S - R:] = gd @ kx
+    rk = (gd.transpose(-1, -2) @ q[:, :, S - R:].double().cpu()).view(B, Nk, N // Nk, S, D).sum(2)
+    for given in (False, True):
+        dq, dk = ops.raw_scores_bwd(q, k, d_raw, start, ln, scale, *((dq0.clone(), dk0.clone()) if given else ()))
+        for got, r, base in ((dq, rq, dq0), (dk, rk, dk0)):
+            r = r + base.double().cpu() if given else r
+            assert (got.double().cpu() - r).norm() <= tol * r.norm()
