@@ -82,22 +82,26 @@ namespace {
 constexpr int BM = 128;  // query rows (token, head) per row tile
 constexpr int BN = 64;   // keys per slot (one TMA box)
 constexpr int BT = 128;  // keys per MMA tile (two slots)
-constexpr int HD = 128;  // head dim
 constexpr int kSlots = 5;        // 64-key K/V slots in shared memory
 constexpr int kMaxGroup = 4;  // consecutive blocks of one (prompt, KV head) per work item, at most
 constexpr int kThreads = 352;
-constexpr uint32_t kQBytes = 2 * BM * 128;       // one Q tile: two 64-wide halves of D
-constexpr uint32_t kSlotHalf = BN * 128;         // K (or V) of one slot, one 64-wide half of D
-constexpr uint32_t kPoolHalf = kSlots * kSlotHalf;  // all slots of one half of D, contiguous: key k at k * 128 B
-constexpr uint32_t kSlotBytes = 4 * kSlotHalf;   // K + V of one slot
-constexpr uint32_t kOffQ = 0;
-constexpr uint32_t kOffK = kOffQ + 2 * kQBytes;
-constexpr uint32_t kOffV = kOffK + 2 * kPoolHalf;
-constexpr uint32_t kOffBar = kOffV + 2 * kPoolHalf;
+constexpr uint32_t kSlotHalf = BN * 128;         // K (or V) of one slot, one 64-wide chunk of head_dim
+constexpr uint32_t kPoolHalf = kSlots * kSlotHalf;  // all slots of one chunk, contiguous: key k at k * 128 B
 constexpr int kJobRing = 4;                      // published jobs in flight per chain
-constexpr uint32_t kOffJobs = kOffBar + 512;     // 2 x kJobRing records of 16 ints
-constexpr uint32_t kSmemBytes = kOffJobs + 2 * kJobRing * 64 + 1024;  // + slack for the 1024-byte round-up
-static_assert(kSmemBytes <= 232448, "shared memory per CTA");
+// Shared-memory layout for head_dim HD (64 or 128): tiles are stored as HD / 64 chunks of 128-byte rows.
+template <int HD>
+struct Geo {
+  static constexpr uint32_t kChunks = HD / 64;
+  static constexpr uint32_t kQBytes = kChunks * BM * 128;  // one Q tile
+  static constexpr uint32_t kSlotBytes = 2 * kChunks * kSlotHalf;  // K + V of one slot
+  static constexpr uint32_t kOffQ = 0;
+  static constexpr uint32_t kOffK = kOffQ + 2 * kQBytes;
+  static constexpr uint32_t kOffV = kOffK + kChunks * kPoolHalf;
+  static constexpr uint32_t kOffBar = kOffV + kChunks * kPoolHalf;
+  static constexpr uint32_t kOffJobs = kOffBar + 512;     // 2 x kJobRing records of 16 ints
+  static constexpr uint32_t kSmemBytes = kOffJobs + 2 * kJobRing * 64 + 1024;  // + slack for the 1024-byte round-up
+  static_assert(kSmemBytes <= 232448, "shared memory per CTA");
+};
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kChainCols = 256;  // per chain: S [0,128) (P over its first 64 columns), then O [128,256)
 constexpr uint32_t kColO = 128;
@@ -340,9 +344,13 @@ __device__ __forceinline__ Pair decode_pair(const TcArgs& a, int b, int g, int m
 // (tiles are dealt 0,1,1,0,0,1,1,0,...)
 __device__ __forceinline__ int deal_chain(int i) { return ((i & 3) == 0 || (i & 3) == 3) ? 0 : 1; }
 
+template <int HD>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, const TcArgs a) {
+  using L = Geo<HD>;
+  constexpr uint32_t kOffQ = L::kOffQ, kOffK = L::kOffK, kOffV = L::kOffV, kOffBar = L::kOffBar, kOffJobs = L::kOffJobs;
+  constexpr uint32_t kQBytes = L::kQBytes, kSlotBytes = L::kSlotBytes;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   if (a.hdr[1] != 0) return;  // malformed block spans (found by the prologue kernel): write nothing
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -470,9 +478,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     auto load_slot = [&](int s, int bs, int g, int b, int lo) {
       const uint32_t kd = sbase + kOffK + (uint32_t)s * kSlotHalf, vd = sbase + kOffV + (uint32_t)s * kSlotHalf;
       ptx::tma_load_4d(kd, &tmK, bar(kKVFull + bs), 0, g, lo, b);
-      ptx::tma_load_4d(kd + kPoolHalf, &tmK, bar(kKVFull + bs), 64, g, lo, b);
       ptx::tma_load_4d(vd, &tmV, bar(kKVFull + bs), 0, g, lo, b);
-      ptx::tma_load_4d(vd + kPoolHalf, &tmV, bar(kKVFull + bs), 64, g, lo, b);
+      if (HD == 128) {
+        ptx::tma_load_4d(kd + kPoolHalf, &tmK, bar(kKVFull + bs), 64, g, lo, b);
+        ptx::tma_load_4d(vd + kPoolHalf, &tmV, bar(kKVFull + bs), 64, g, lo, b);
+      }
     };
 
     // ---- streamed pair: both chains walk the same 128-key tiles through a two-deep ring (slots 0-1, 2-3) ----
@@ -712,7 +722,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         const uint32_t dst = sbase + kOffQ + (uint32_t)x * kQBytes;
         ptx::mbar_expect_tx(bar(kQFull + x), kQBytes);
         ptx::tma_load_4d(dst, &tmQ, bar(kQFull + x), 0, jb.g * G, jb.start + jb.t0, jb.b);
-        ptx::tma_load_4d(dst + BM * 128, &tmQ, bar(kQFull + x), 64, jb.g * G, jb.start + jb.t0, jb.b);
+        if (HD == 128) ptx::tma_load_4d(dst + BM * 128, &tmQ, bar(kQFull + x), 64, jb.g * G, jb.start + jb.t0, jb.b);
       }
       ++q_issued;
     };
@@ -1080,6 +1090,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 }
 
 // Merge the key-chunk partials of the query block: one warp per (prompt, head, query token).
+template <int HD>
 __global__ void __launch_bounds__(128) attn_combine_kernel(TcArgs a) {
   if (a.hdr[1] != 0) return;
   const int lane = threadIdx.x & 31;
@@ -1092,6 +1103,7 @@ __global__ void __launch_bounds__(128) attn_combine_kernel(TcArgs a) {
   const int start = a.blk_start[(size_t)b * a.M + a.M - 1], len = a.blk_len[(size_t)b * a.M + a.M - 1];
   if (tok >= len) return;
   const float2* ml = a.part_ml + w * a.n_split;
+  const int col = (lane * 4) & (HD - 1);  // (head_dim 64: the upper half of the warp repeats the lower one's work)
   float mx = -INFINITY;
   for (int c = 0; c < a.n_split; ++c) mx = fmaxf(mx, ml[c].x);
   const float ref = (mx == -INFINITY) ? 0.f : mx;
@@ -1101,7 +1113,7 @@ __global__ void __launch_bounds__(128) attn_combine_kernel(TcArgs a) {
     const float2 x = ml[c];
     if (x.y > 0.f) {  // chunks that saw no key carry no output
       const float wgt = exp2f(x.x - ref);
-      const float4 o = *reinterpret_cast<const float4*>(a.part_o + (w * a.n_split + c) * HD + lane * 4);
+      const float4 o = *reinterpret_cast<const float4*>(a.part_o + (w * a.n_split + c) * HD + col);
       acc.x = fmaf(o.x, wgt, acc.x); acc.y = fmaf(o.y, wgt, acc.y);
       acc.z = fmaf(o.z, wgt, acc.z); acc.w = fmaf(o.w, wgt, acc.w);
       l = fmaf(x.y, wgt, l);
@@ -1109,8 +1121,8 @@ __global__ void __launch_bounds__(128) attn_combine_kernel(TcArgs a) {
   }
   const float inv = l > 0.f ? 1.f / l : 0.f;
   __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.o.ptr) + (int64_t)b * a.o.sb + (int64_t)(start + tok) * a.o.ss +
-                       (int64_t)n * a.o.sh + lane * 4;
-  store4(dst, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
+                       (int64_t)n * a.o.sh + col;
+  if (lane * 4 < HD) store4(dst, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
   if (a.lse != nullptr && lane == 0) a.lse[((int64_t)b * a.N + n) * a.S + start + tok] = (ref + log2f(l)) * 0.6931471805599453f;
 }
 
@@ -1189,12 +1201,11 @@ size_t attn_tc_workspace(const brk_attn_params& p) {
   const int ns = tc_splits(p);
   if (ns <= 1) return kWsHeader;  // work counter and span verdict
   const size_t rows = (size_t)p.B * p.N * query_rows(p) * ns;
-  return kWsHeader + rows * HD * sizeof(float) + rows * sizeof(float2);
+  return kWsHeader + rows * p.D * sizeof(float) + rows * sizeof(float2);
 }
 
-int attn_tc_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStream_t st) {
-  BRK_REQUIRE(p.dtype == BRK_BF16 && p.D == HD, BRK_E_UNSUPPORTED,
-              "tcgen05 attention needs bf16 and head_dim 128 (dtype %d, head_dim %d)", p.dtype, p.D);
+template <int HD>
+static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStream_t st) {
   const int G = p.N / p.Nk;
   BRK_REQUIRE(G == 1 || G == 2 || G == 4 || G == 8, BRK_E_UNSUPPORTED, "tcgen05 attention needs N/Nk in {1,2,4,8}, got %d", G);
   BRK_REQUIRE(p.scale > 0.f, BRK_E_ARG, "softmax scale must be positive");
@@ -1219,7 +1230,8 @@ int attn_tc_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStre
   BRK_CUDA(cudaGetDevice(&dev));
   BRK_REQUIRE(dev >= 0 && dev < 64, BRK_E_UNSUPPORTED, "device ordinal %d out of range", dev);
   if (!configured[dev]) {
-    BRK_CUDA(cudaFuncSetAttribute(attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+    BRK_CUDA(cudaFuncSetAttribute(attn_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)Geo<HD>::kSmemBytes));
     sms[dev] = sm_count();
     BRK_REQUIRE(sms[dev] > 0, BRK_E_CUDA, "could not read the SM count");
     configured[dev] = true;
@@ -1262,14 +1274,20 @@ int attn_tc_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStre
   a.part_ml = ns > 1 ? reinterpret_cast<float2*>(part + rows * HD) : nullptr;
   if ((rc = attn_prologue_launch(p, reinterpret_cast<int*>(ws), a.part_ml, ns > 1 ? (int64_t)rows : 0, st))) return rc;
   const int grid = (int)(total_items < sms[dev] ? total_items : sms[dev]);
-  attn_tc_kernel<<<grid, kThreads, kSmemBytes, st>>>(tq, tk, tv, a);
+  attn_tc_kernel<HD><<<grid, kThreads, Geo<HD>::kSmemBytes, st>>>(tq, tk, tv, a);
   BRK_CUDA(cudaGetLastError());
   if (ns > 1) {
     const int64_t warps = (int64_t)p.B * p.N * lq;
-    attn_combine_kernel<<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(a);
+    attn_combine_kernel<HD><<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(a);
     BRK_CUDA(cudaGetLastError());
   }
   return BRK_OK;
+}
+
+int attn_tc_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStream_t st) {
+  BRK_REQUIRE(p.dtype == BRK_BF16 && (p.D == 64 || p.D == 128), BRK_E_UNSUPPORTED,
+              "tcgen05 attention needs bf16 and head_dim 64 or 128 (dtype %d, head_dim %d)", p.dtype, p.D);
+  return p.D == 128 ? attn_tc_run<128>(p, ws, ws_bytes, st) : attn_tc_run<64>(p, ws, ws_bytes, st);
 }
 
 }  // namespace brk

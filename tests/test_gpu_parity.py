@@ -113,6 +113,24 @@ def test_attention_tc_vs_oracle(case):
     assert out.float().cpu()[~rows].abs().sum().item() == 0
 
 
+@pytest.mark.parametrize("case", [  # B, N, Nk, M, H, seed: every group size; one block, streamed blocks, key chunks of the query block
+    (2, 4, 2, 5, 32, 41), (1, 4, 4, 4, 96, 42), (2, 8, 2, 12, 160, 43), (1, 8, 1, 3, 40, 44), (2, 4, 2, 1, 128, 45),
+    (1, 16, 8, 30, 120, 46), (1, 4, 2, 3, 1024, 47), (1, 2, 2, 2, 16, 48)])
+def test_attention_tc_head_dim_64_vs_oracle(case):
+    B, N, Nk, M, H, seed = case
+    D = 64
+    lens = H_.random_lens(B, M, H, seed)
+    mask = H_.ragged_mask(B, M, H, lens)
+    q, k, v = H_.qkv(B, N, Nk, M * H, D, seed + 100, torch.bfloat16)
+    out, lse = _run_attn(q, k, v, mask, D ** -0.5, TC, lse=True)
+    ref, ref_lse = orc.attention_dense(q, k, v, mask, D ** -0.5)
+    rows = mask.reshape(B, -1)
+    assert (out.float().cpu() - ref.float())[rows].abs().max().item() < 2e-2
+    lrows = rows[:, None, :].expand(B, N, M * H)
+    assert (lse.cpu() - ref_lse.float())[lrows].abs().max().item() < 2e-3
+    assert out.float().cpu()[~rows].abs().sum().item() == 0
+
+
 @pytest.mark.parametrize("algo", [SIMT, TC])
 def test_attention_large_logit_range(algo):
     """Logits spread over tens of units (queries scaled up): the running maximum jumps by more than the
