@@ -1,7 +1,8 @@
-"""ctypes binding of libblockrank_b200.so (the C ABI in include/blockrank_b200.h).
+"""Bindings of libblockrank_b200.so (the C ABI in include/blockrank_b200.h): ``lib()`` is the library itself through
+ctypes, ``host()`` the extension module that calls it with PyTorch tensors (csrc/torch_host.cpp).
 
-There is no fallback: if the shared library is missing or a call fails, an
-exception is raised.  Build the library with ``python -m blockrank_b200.build``.
+There is no fallback: if a shared library is missing or a call fails, an
+exception is raised.  Build both with ``python -m blockrank_b200.build``.
 """
 from __future__ import annotations
 
@@ -21,7 +22,8 @@ EXPORTS = ("brk_version", "brk_last_error", "brk_device_check", "brk_spans_from_
            "brk_status_poll", "brk_selftest_bounded_wait",
            "brk_doc_scores_workspace_bytes",
            "brk_doc_scores", "brk_doc_scores_static", "brk_raw_scores",
-           "brk_raw_scores_bwd_workspace_bytes", "brk_raw_scores_bwd", "brk_rmsnorm", "brk_rope", "brk_silu_mul")
+           "brk_raw_scores_bwd_workspace_bytes", "brk_raw_scores_bwd", "brk_signal_rows", "brk_rmsnorm",
+           "brk_rope", "brk_silu_mul")
 
 
 class View(C.Structure):
@@ -108,6 +110,24 @@ def lib() -> C.CDLL:
     L.brk_silu_mul.argtypes = [C.c_int32, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_void_p]
     _lib = L
     return L
+
+
+_host = None
+
+
+def host():
+    """The extension module between PyTorch tensors and the library, loaded once; same ImportError as :func:`lib`."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise ImportError(f"{PKG}/_host.so is missing or does not load ({e}): run `python -m blockrank_b200.build`") from e
+        import torch
+        module.set_error_classes(BlockRankLibraryError, torch.OutOfMemoryError)
+        _host = module
+    return _host
 
 
 def check(rc: int, what: str) -> None:

@@ -39,6 +39,11 @@ class BlockSpans(torch.Tensor):
     unknown) and ``grid_h`` (the H of the reference's (M, H) grid it was derived from, None for a padding-free
     layout)."""
 
+    def __getitem__(self, item):
+        """Plain tensors: the halves are read on every call, and subclass dispatch would cost more than the slice."""
+        with torch._C.DisableTorchFunctionSubclass():
+            return super().__getitem__(item)
+
     @staticmethod
     def make(start: torch.Tensor, length: torch.Tensor, max_block_len: int, grid_h: Optional[int] = None,
              max_query_len: int = 0) -> "BlockSpans":
@@ -68,35 +73,6 @@ def cuda_blockrank_attention_mask(*args, attention_mask: Optional[torch.Tensor] 
     return BlockSpans.make(start, length, attention_mask.shape[-1], grid_h=attention_mask.shape[-1])
 
 
-class _AttentionFn(torch.autograd.Function):
-    """BlockRank attention with its backward (``brk_attn_bwd``).  With ``num_last`` given it also returns the raw logits
-    of the last R slots, (B,N,R,S) = scale * q[:, :, S-R:] k^T + a constant mask addend (std:219-233, 256-262): the
-    addend is constant, so their gradient flows to q and k at every position (``brk_raw_scores_bwd``, which adds
-    into the gradients of the attention output instead of leaving two pairs of tensors for autograd to sum)."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, start, length, scale, max_block_len, max_query_len, algo, num_last, grid_h):
-        ctx.set_materialize_grads(False)
-        out, lse = ops.attention(q, k, v, start, length, scale, max_block_len, return_lse=True, algo=algo,
-                                 max_query_len=max_query_len)
-        ctx.save_for_backward(q, k, v, out, lse, start, length)
-        ctx.scale, ctx.max_block_len = float(scale), int(max_block_len)
-        if num_last is None:
-            return out
-        return out, ops.raw_scores(q, k, start, length, scale, num_last, grid_h=grid_h)
-
-    @staticmethod
-    def backward(ctx, d_out, d_raw=None):
-        q, k, v, out, lse, start, length = ctx.saved_tensors
-        dq = dk = dv = None
-        if d_out is not None:
-            dq, dk, dv = ops.attention_bwd(q, k, v, out, d_out.to(out.dtype), lse, start, length, ctx.scale,
-                                           ctx.max_block_len)
-        if d_raw is not None:
-            dq, dk = ops.raw_scores_bwd(q, k, d_raw.to(q.dtype), start, length, ctx.scale, dq, dk)
-        return dq, dk, dv, None, None, None, None, None, None, None, None
-
-
 def _wants_scores(module, kwargs) -> bool:
     # same precedence as std:244-254
     layers = kwargs.get("layers_to_return_scores", None)
@@ -124,35 +100,29 @@ def cuda_blockrank_attention_forward(module, query, key, value, attention_mask, 
         if attention_mask is None:
             raise ValueError("BlockRank attention requires block spans (got attention_mask=None)")
         attention_mask = cuda_blockrank_attention_mask(attention_mask=attention_mask, **kwargs)
-    train = torch.is_grad_enabled() and (query.requires_grad or key.requires_grad or value.requires_grad)
     if dropout and getattr(module, "training", False):
         warnings.warn("cuda_blockrank attention ignores attention dropout")
     spans = attention_mask
-    start, length = spans[0], spans[1]
     algo = kwargs.get("blockrank_algo", _lib.ALGO_AUTO)
-    num_last, grid_h = kwargs.get("num_last_queries", 16), getattr(spans, "grid_h", None)
-    max_query_len = getattr(spans, "max_query_len", 0)
-    wants = start.shape[-1] > 1 and _wants_scores(module, kwargs)
-    fused = wants and kwargs.get("blockrank_doc_scores", False)
-    if fused and train:
-        raise NotImplementedError("blockrank_doc_scores=True is inference-only; train on the raw scores "
-                                  "(compute_auxiliary_attention_loss differentiates them)")
-    if train:
-        res = _AttentionFn.apply(query, key, value, start, length, scaling, spans.max_block_len, max_query_len, algo,
-                                 num_last if wants else None, grid_h)
-        return res if wants else (res, None)
-    out = ops.attention(query, key, value, start, length, scaling, spans.max_block_len, algo=algo,
-                        max_query_len=max_query_len)
+    num_last, grid_h = -1, -1  # no raw logits; no grid
     scores = None
-    if fused:
-        rows = kwargs.get("signal_rows")
-        if rows is None:
-            raise ValueError("blockrank_doc_scores=True needs signal_rows (B, R) slot indices")
-        scores, _ = ops.doc_scores(query, key, start, length, rows.to(device=query.device, dtype=torch.int32),
-                                   scaling, kwargs.get("temperature", 0.05))
-    elif wants:
-        scores = ops.raw_scores(query, key, start, length, scaling, num_last, grid_h=grid_h)
-    return out, scores
+    if _wants_scores(module, kwargs) and spans.shape[-1] > 1:
+        if kwargs.get("blockrank_doc_scores", False):
+            if torch.is_grad_enabled() and (query.requires_grad or key.requires_grad or value.requires_grad):
+                raise NotImplementedError("blockrank_doc_scores=True is inference-only; train on the raw scores "
+                                          "(compute_auxiliary_attention_loss differentiates them)")
+            rows = kwargs.get("signal_rows")
+            if rows is None:
+                raise ValueError("blockrank_doc_scores=True needs signal_rows (B, R) slot indices")
+            scores, _ = ops.doc_scores(query, key, spans[0], spans[1], rows.to(device=query.device, dtype=torch.int32),
+                                       scaling, kwargs.get("temperature", 0.05))
+        else:
+            num_last = max(0, int(kwargs.get("num_last_queries", 16)))
+            h = getattr(spans, "grid_h", None)
+            grid_h = -1 if h is None else int(h)
+    out, raw = _lib.host().attention_forward(query, key, value, spans, scaling, spans.max_block_len,
+                                             getattr(spans, "max_query_len", 0), algo, num_last, grid_h)
+    return out, raw if scores is None else scores
 
 
 def register_cuda_blockrank_attention(name: str = ATTN_NAME) -> str:

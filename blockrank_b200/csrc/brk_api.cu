@@ -147,6 +147,10 @@ int brk_status_poll(int32_t* status, void* stream) {
               "overlapping its predecessor): the attention call wrote nothing");
     return BRK_E_ARG;
   }
+  if (v == kStatusBadRows) {
+    set_error("a signal row lies outside the prompt's slots [0, S)");
+    return BRK_E_ARG;
+  }
   set_error("a bounded device-side wait gave up (code %d: %s); the outputs of that call are incomplete", v,
             v == kStatusSelfTest ? "self-test" : v < 20 ? "TMA warp" : v < 30 ? "MMA warp" : v < 40 ? "softmax warp" : "job ring");
   return BRK_E_TIMEOUT;
@@ -200,6 +204,17 @@ int brk_rope(int32_t dtype, void* q, int64_t q_row_stride, int32_t N, void* k, i
   BRK_REQUIRE((q == nullptr || (((uintptr_t)q & 15) == 0 && q_row_stride % 8 == 0)) && (k == nullptr || (((uintptr_t)k & 15) == 0 && k_row_stride % 8 == 0)), BRK_E_ARG, "rope rows must be 16-byte aligned");
   BRK_REQUIRE(T * (D / 16) / 256 < (1ll << 31), BRK_E_ARG, "rope problem too large");
   return rope_launch(dtype, q, q_row_stride, N, k, k_row_stride, Nk, D, pos, inv_freq, T, (cudaStream_t)stream);
+}
+
+int brk_signal_rows(int32_t dtype, const void* x, int32_t hidden, const int32_t* pos, const int32_t* rows, int32_t B, int32_t S,
+                    int32_t R, void* x_out, int32_t* pos_out, int32_t* local, int32_t* status, void* stream) {
+  BRK_REQUIRE(x && pos && rows && x_out && pos_out && local, BRK_E_ARG, "null pointer");
+  BRK_REQUIRE(dtype == BRK_BF16 || dtype == BRK_F32, BRK_E_UNSUPPORTED, "dtype %d", dtype);
+  BRK_REQUIRE(B > 0 && S > 0 && R > 0 && (int64_t)B * R < (1ll << 31) && hidden > 0 && hidden % 8 == 0, BRK_E_ARG,
+              "bad signal_rows shape B=%d S=%d R=%d hidden=%d", B, S, R, hidden);
+  BRK_REQUIRE((((uintptr_t)x | (uintptr_t)x_out) & 15) == 0, BRK_E_ARG, "signal_rows buffers must be 16-byte aligned");
+  return signal_rows_launch(x, hidden * (dtype == BRK_BF16 ? 2 : 4), pos, rows, B, S, R, x_out, pos_out, local, status,
+                            (cudaStream_t)stream);
 }
 
 int brk_silu_mul(int32_t dtype, const void* gate_up, void* out, int64_t rows, int32_t inter, void* stream) {

@@ -100,9 +100,11 @@ inline View make_view(const brk_view& v) { return View{(char*)v.ptr, v.stride_b,
 // Every attention call gets a 256-byte header at the start of its workspace: [0] the work counter of the
 // tensor-core kernel, [1] the verdict of the span check (non-zero: malformed, the kernels write nothing).
 constexpr size_t kWsHeader = 256;
-// Values of the caller's status word: 10..49 name the bounded wait that gave up, 50 malformed block spans,
+// Values of the caller's status word: 10..49 name the bounded wait that gave up, 50 malformed block spans, 51 a
+// signal row outside the prompt,
 // 90 the self-test's wait.
 constexpr int kStatusBadSpans = 50;
+constexpr int kStatusBadRows = 51;
 constexpr int kStatusSelfTest = 90;
 
 // kernel launchers implemented in the .cu files
@@ -131,5 +133,7 @@ int rmsnorm_launch(int dtype, const void* x, void* residual, const void* w, void
                    float eps, cudaStream_t st);
 int rope_launch(int dtype, void* q, int64_t q_rs, int N, void* k, int64_t k_rs, int Nk, int D, const int32_t* pos,
                 const float* inv_freq, int64_t T, cudaStream_t st);
+int signal_rows_launch(const void* x, int row_bytes, const int32_t* pos, const int32_t* rows, int B, int S, int R, void* x_out,
+                       int32_t* pos_out, int32_t* local, int32_t* status, cudaStream_t st);
 int silu_mul_launch(int dtype, const void* gu, void* out, int64_t rows, int inter, cudaStream_t st);
 }  // namespace brk

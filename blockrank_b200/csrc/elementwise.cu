@@ -176,7 +176,33 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const T* __restrict__ gu,
   for (int v = 0; v < kVec; v += 8) store8(out + r * inter + c + v, *reinterpret_cast<float (*)[8]>(&o[v]));
 }
 
+// One CTA per signal row: its normalised activations, its position, and its index among the prompt's signal rows.  A row
+// outside [0, S) sets the status word and reads slot 0.
+__global__ void __launch_bounds__(128) signal_rows_kernel(const uint4* __restrict__ x, int row16, const int32_t* __restrict__ pos,
+                                                          const int32_t* __restrict__ rows, int S, int R,
+                                                          uint4* __restrict__ x_out, int32_t* __restrict__ pos_out,
+                                                          int32_t* __restrict__ local, int32_t* status) {
+  const int i = blockIdx.x, b = i / R;
+  int slot = rows[i];
+  const bool ok = slot >= 0 && slot < S;
+  if (!ok) slot = 0;
+  const int64_t t = (int64_t)b * S + slot;
+  for (int c = threadIdx.x; c < row16; c += blockDim.x) x_out[(int64_t)i * row16 + c] = x[t * row16 + c];
+  if (threadIdx.x == 0) {
+    pos_out[i] = pos[t];
+    local[i] = i % R;
+    if (!ok && status) atomicCAS(status, 0, kStatusBadRows);
+  }
+}
+
 }  // namespace
+
+int signal_rows_launch(const void* x, int row_bytes, const int32_t* pos, const int32_t* rows, int B, int S, int R, void* x_out,
+                       int32_t* pos_out, int32_t* local, int32_t* status, cudaStream_t st) {
+  signal_rows_kernel<<<B * R, 128, 0, st>>>((const uint4*)x, row_bytes / 16, pos, rows, S, R, (uint4*)x_out, pos_out, local, status);
+  BRK_CUDA(cudaGetLastError());
+  return BRK_OK;
+}
 
 int spans_launch(const uint8_t* mask, int B, int M, int H, int32_t* start, int32_t* len, cudaStream_t st) {
   const int total = B * M;

@@ -1,0 +1,576 @@
+// Native host path between PyTorch tensors and the C ABI (include/blockrank_b200.h).
+//
+// One call of the Python package is one call into this module: argument checks, output and scratch allocation
+// (PyTorch's caching allocator, current stream), parameter structs, the C-ABI calls and -- for the registered
+// attention function under autograd and for the early-exit ranker -- the sequence of such calls.  Written in Python the
+// same steps cost 40-60 us per attention call, more than its kernels take on a short prompt.
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/extension.h>
+
+#include <atomic>
+#include <mutex>
+#include <optional>
+#include <string>
+#include <tuple>
+#include <vector>
+
+#include "../../include/blockrank_b200.h"
+
+namespace {
+
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+// ---- errors -----------------------------------------------------------------------------------
+// Raised as blockrank_b200's BlockRankLibraryError; argument errors are ValueErrors, CPU tensors RuntimeErrors.
+struct LibError : std::runtime_error {
+  using std::runtime_error::runtime_error;
+};
+PyObject *g_lib_error = nullptr, *g_oom_error = nullptr;  // BlockRankLibraryError, torch.OutOfMemoryError
+
+#define BRK_VALUE(cond, ...)                                                  \
+  do {                                                                        \
+    if (!(cond)) C10_THROW_ERROR(ValueError, c10::str(__VA_ARGS__));          \
+  } while (0)
+
+const char* code_name(int rc) {
+  switch (rc) {
+    case -1: return "BRK_E_ARG";
+    case -2: return "BRK_E_UNSUPPORTED";
+    case -3: return "BRK_E_WORKSPACE";
+    case -4: return "BRK_E_CUDA";
+    case -5: return "BRK_E_DEVICE";
+    case -6: return "BRK_E_TIMEOUT";
+    default: return "error";
+  }
+}
+void check(int rc, const char* what) {
+  if (rc == 0) return;
+  const std::string msg = c10::str(what, ": ", code_name(rc), ": ", brk_last_error());
+  if (rc >= -3 && rc <= -1) C10_THROW_ERROR(ValueError, msg);
+  throw LibError(msg);
+}
+
+void need_cuda(std::initializer_list<const Tensor*> ts) {
+  for (const Tensor* t : ts)
+    if (t != nullptr && t->defined())
+      TORCH_CHECK(t->is_cuda(), "blockrank_b200 kernels run on CUDA tensors only (there is no CPU path)");
+}
+const Tensor* opt(const OptTensor& t) { return t.has_value() ? &*t : nullptr; }
+
+std::atomic<int64_t> g_launches{0};  // kernels launched through this module
+void count(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+
+// ---- parameter building -----------------------------------------------------------------------
+int dtype_code(const Tensor& t) {
+  if (t.scalar_type() == at::kBFloat16) return BRK_BF16;
+  if (t.scalar_type() == at::kFloat) return BRK_F32;
+  C10_THROW_ERROR(ValueError, c10::str("blockrank_b200 supports bfloat16 and float32, got ", t.scalar_type()));
+}
+void* stream_of(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+
+// (B, heads, S, D) tensor (any strides, innermost contiguous) -> brk_view
+brk_view view_of(const Tensor& t) {
+  BRK_VALUE(t.dim() == 4 && t.stride(3) == 1, "expected a (B, heads, S, D) tensor with contiguous head_dim");
+  brk_view v;
+  v.ptr = t.data_ptr();
+  v.stride_b = t.stride(0);
+  v.stride_h = t.stride(1);
+  v.stride_s = t.stride(2);
+  return v;
+}
+// (B, S, heads, D) tensor -> the same view
+brk_view view_bshd(const Tensor& t) {
+  BRK_VALUE(t.dim() == 4 && t.stride(3) == 1, "expected a (B, heads, S, D) tensor with contiguous head_dim");
+  brk_view v;
+  v.ptr = t.data_ptr();
+  v.stride_b = t.stride(0);
+  v.stride_h = t.stride(2);
+  v.stride_s = t.stride(1);
+  return v;
+}
+Tensor empty_bshd(const Tensor& like, int64_t B, int64_t S, int64_t heads, int64_t D) {
+  return at::empty({B, S, heads, D}, like.options().requires_grad(false));
+}
+Tensor scratch(size_t bytes, const Tensor& like) {
+  return at::empty({(int64_t)bytes}, like.options().dtype(at::kByte).requires_grad(false));
+}
+
+// One int32 status word per device, zeroed when created.  Every attention call passes it; the kernels set it (first
+// event wins) when a bounded wait gives up or the block spans are malformed.
+Tensor status_word(int device) {
+  static std::mutex mu;
+  static auto* words = new std::vector<Tensor>();  // (never destroyed: the CUDA context may be gone at exit)
+  std::lock_guard<std::mutex> lock(mu);
+  if ((int)words->size() <= device) words->resize(device + 1);
+  Tensor& t = (*words)[device];
+  if (!t.defined()) t = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
+  return t;
+}
+
+std::tuple<Tensor, Tensor> spans_from_mask(const Tensor& mask) {
+  need_cuda({&mask});
+  BRK_VALUE(mask.dim() == 3, "block mask must be (B, M, H)");
+  c10::cuda::CUDAGuard guard(mask.device());
+  Tensor m8 = mask.scalar_type() == at::kBool ? mask.contiguous().view(at::kByte) : mask.ne(0).to(at::kByte).contiguous();
+  const auto opts = m8.options().dtype(at::kInt);
+  Tensor start = at::empty({m8.size(0), m8.size(1)}, opts), len = at::empty({m8.size(0), m8.size(1)}, opts);
+  check(brk_spans_from_mask((const uint8_t*)m8.data_ptr(), (int)m8.size(0), (int)m8.size(1), (int)m8.size(2),
+                            (int32_t*)start.data_ptr(), (int32_t*)len.data_ptr(), stream_of(m8)),
+        "brk_spans_from_mask");
+  count(1);
+  return {start, len};
+}
+
+// ---- attention --------------------------------------------------------------------------------
+std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& blk_start,
+                                     const Tensor& blk_len, double scale, int64_t max_block_len, const OptTensor& out_in,
+                                     bool return_lse, int64_t algo, int64_t max_query_len, const OptTensor& lse_in) {
+  need_cuda({&q, &k, &v, &blk_start, &blk_len});
+  BRK_VALUE(q.dim() == 4 && k.dim() == 4 && v.dim() == 4, "expected (B, heads, S, D) tensors");
+  const int64_t B = q.size(0), N = q.size(1), S = q.size(2), D = q.size(3), Nk = k.size(1);
+  BRK_VALUE(k.size(0) == B && k.size(2) == S && k.size(3) == D && v.sizes() == k.sizes(), "shape mismatch q", q.sizes(), " k",
+            k.sizes(), " v", v.sizes());
+  BRK_VALUE(k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(), "q, k, v must share a dtype");
+  BRK_VALUE(blk_start.scalar_type() == at::kInt && blk_len.scalar_type() == at::kInt && blk_start.sizes() == blk_len.sizes(),
+            "blk_start / blk_len must be int32 tensors of the same (B, M) shape");
+  c10::cuda::CUDAGuard guard(q.device());
+  Tensor out = out_in.has_value() ? *out_in : empty_bshd(q, B, S, N, D);
+  Tensor lse = lse_in.has_value() ? *lse_in
+               : return_lse       ? at::empty({B, N, S}, q.options().dtype(at::kFloat).requires_grad(false))
+                                  : Tensor();
+  const Tensor bs = blk_start.contiguous(), bl = blk_len.contiguous();
+  brk_attn_params p{};
+  p.dtype = dtype_code(q);
+  p.algo = (int32_t)algo;
+  p.B = (int32_t)B; p.N = (int32_t)N; p.Nk = (int32_t)Nk; p.D = (int32_t)D; p.S = (int32_t)S;
+  p.M = (int32_t)bs.size(-1);
+  p.max_block_len = (int32_t)max_block_len;
+  p.max_query_len = (int32_t)max_query_len;
+  p.scale = (float)scale;
+  p.q = view_of(q); p.k = view_of(k); p.v = view_of(v);
+  p.o = view_bshd(out);
+  p.lse = lse.defined() ? (float*)lse.data_ptr() : nullptr;
+  p.blk_start = (const int32_t*)bs.data_ptr();
+  p.blk_len = (const int32_t*)bl.data_ptr();
+  p.status = (int32_t*)status_word(q.get_device()).data_ptr();
+  const size_t nbytes = brk_attn_fwd_workspace_bytes(&p);
+  Tensor ws = scratch(nbytes, q);
+  check(brk_attn_fwd(&p, ws.data_ptr(), nbytes, stream_of(q)), "brk_attn_fwd");
+  // span check / reset kernel + main kernel [+ merge of the key-chunked query block on the tensor-core path]
+  count(nbytes > 256 ? 3 : 2);
+  return {out, lse};
+}
+
+std::tuple<Tensor, Tensor, Tensor> attention_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out,
+                                                 const Tensor& d_out_in, const Tensor& lse_in, const Tensor& blk_start,
+                                                 const Tensor& blk_len, double scale, int64_t max_block_len) {
+  need_cuda({&q, &k, &v, &out, &d_out_in, &lse_in, &blk_start, &blk_len});
+  BRK_VALUE(q.dim() == 4 && k.dim() == 4, "expected (B, heads, S, D) tensors");
+  const int64_t B = q.size(0), N = q.size(1), S = q.size(2), D = q.size(3), Nk = k.size(1);
+  BRK_VALUE(out.sizes() == at::IntArrayRef({B, S, N, D}) && d_out_in.sizes() == out.sizes(), "out / d_out must be (B,S,N,D) = ",
+            at::IntArrayRef({B, S, N, D}), ", got ", out.sizes(), " / ", d_out_in.sizes());
+  BRK_VALUE(lse_in.sizes() == at::IntArrayRef({B, N, S}) && lse_in.scalar_type() == at::kFloat,
+            "lse must be the forward's fp32 (B, N, S) tensor");
+  for (const Tensor* t : {&k, &v, &out, &d_out_in})
+    BRK_VALUE(t->scalar_type() == q.scalar_type(), "q, k, v, out, d_out must share a dtype");
+  c10::cuda::CUDAGuard guard(q.device());
+  const Tensor d_out = d_out_in.contiguous(), lse = lse_in.contiguous();  // (autograd may hand over expanded or transposed gradients)
+  Tensor dq = empty_bshd(q, B, S, N, D).permute({0, 2, 1, 3});
+  Tensor dk = empty_bshd(q, B, S, Nk, D).permute({0, 2, 1, 3});
+  Tensor dv = empty_bshd(q, B, S, Nk, D).permute({0, 2, 1, 3});
+  const Tensor bs = blk_start.contiguous(), bl = blk_len.contiguous();
+  brk_attn_bwd_params p{};
+  p.dtype = dtype_code(q);
+  p.B = (int32_t)B; p.N = (int32_t)N; p.Nk = (int32_t)Nk; p.D = (int32_t)D; p.S = (int32_t)S;
+  p.M = (int32_t)bs.size(-1);
+  p.max_block_len = (int32_t)max_block_len;
+  p.scale = (float)scale;
+  p.q = view_of(q); p.k = view_of(k); p.v = view_of(v);
+  p.o = view_bshd(out); p.d_o = view_bshd(d_out);
+  p.lse = (const float*)lse.data_ptr();
+  p.blk_start = (const int32_t*)bs.data_ptr();
+  p.blk_len = (const int32_t*)bl.data_ptr();
+  p.dq = view_of(dq); p.dk = view_of(dk); p.dv = view_of(dv);
+  const size_t nbytes = brk_attn_bwd_workspace_bytes(&p);
+  Tensor ws = scratch(nbytes, q);
+  check(brk_attn_bwd(&p, ws.data_ptr(), nbytes, stream_of(q)), "brk_attn_bwd");
+  count(3);  // dq (+ delta), dk/dv accumulation, conversion of the accumulators
+  return {dq, dk, dv};
+}
+
+// ---- scores -----------------------------------------------------------------------------------
+brk_score_params score_params(const Tensor& q, const Tensor& k, const Tensor& bs, const Tensor& bl, double scale, int64_t R,
+                              double temperature) {
+  brk_score_params p{};
+  p.dtype = dtype_code(q);
+  p.B = (int32_t)q.size(0); p.N = (int32_t)q.size(1); p.Nk = (int32_t)k.size(1); p.D = (int32_t)q.size(3);
+  p.S = (int32_t)q.size(2);
+  p.M = (int32_t)bs.size(-1);
+  p.R = (int32_t)R;
+  p.scale = (float)scale;
+  p.temperature = (float)temperature;
+  p.q = view_of(q);
+  p.k = view_of(k);
+  p.blk_start = (const int32_t*)bs.data_ptr();
+  p.blk_len = (const int32_t*)bl.data_ptr();
+  return p;
+}
+
+std::tuple<Tensor, Tensor> doc_scores(const Tensor& q, const Tensor& k, const Tensor& blk_start, const Tensor& blk_len,
+                                      const Tensor& rows_in, double scale, double temperature) {
+  need_cuda({&q, &k, &blk_start, &blk_len, &rows_in});
+  BRK_VALUE(rows_in.scalar_type() == at::kInt && rows_in.dim() == 2, "rows must be int32 (B, R)");
+  BRK_VALUE(q.dim() == 4 && k.dim() == 4, "expected (B, heads, S, D) tensors");
+  c10::cuda::CUDAGuard guard(q.device());
+  const Tensor bs = blk_start.contiguous(), bl = blk_len.contiguous(), rows = rows_in.contiguous();
+  brk_score_params p = score_params(q, k, bs, bl, scale, rows.size(1), temperature);
+  p.S = (int32_t)q.size(2);
+  const int64_t nd = p.M > 2 ? p.M - 2 : 0;
+  const auto f32 = q.options().dtype(at::kFloat).requires_grad(false);
+  Tensor mass = at::empty({q.size(0), q.size(1), rows.size(1), nd}, f32), logits = at::empty({q.size(0), nd}, f32);
+  p.rows = (const int32_t*)rows.data_ptr();
+  p.doc_mass = (float*)mass.data_ptr();
+  p.logits = (float*)logits.data_ptr();
+  const size_t nbytes = brk_doc_scores_workspace_bytes(&p);
+  Tensor ws = scratch(nbytes > 8 ? nbytes : 8, q);
+  check(brk_doc_scores(&p, ws.data_ptr(), nbytes, stream_of(q)), "brk_doc_scores");
+  count(1);  // per-document partials; the CTA that completes a prompt also writes its masses and logits
+  return {mass, logits};
+}
+
+// grid_h < 0: no grid (padding-free layout)
+Tensor raw_scores(const Tensor& q, const Tensor& k, const Tensor& blk_start, const Tensor& blk_len, double scale,
+                  int64_t num_last, int64_t grid_h) {
+  need_cuda({&q, &k, &blk_start, &blk_len});
+  BRK_VALUE(q.dim() == 4 && k.dim() == 4, "expected (B, heads, S, D) tensors");
+  const int64_t B = q.size(0), N = q.size(1), S = q.size(2);
+  const int64_t R = std::min(num_last, grid_h < 0 ? S : grid_h);
+  c10::cuda::CUDAGuard guard(q.device());
+  const Tensor bs = blk_start.contiguous(), bl = blk_len.contiguous();
+  brk_score_params p = score_params(q, k, bs, bl, scale, R, 0.05);
+  Tensor out = at::empty({B, N, R, S}, q.options().requires_grad(false));
+  check(brk_raw_scores(&p, out.data_ptr(), stream_of(q)), "brk_raw_scores");
+  count(1);
+  return out;
+}
+
+std::tuple<Tensor, Tensor> raw_scores_bwd(const Tensor& q, const Tensor& k, const Tensor& d_raw_in, const Tensor& blk_start,
+                                          const Tensor& blk_len, double scale, const OptTensor& dq_in, const OptTensor& dk_in) {
+  need_cuda({&q, &k, &d_raw_in, opt(dq_in), opt(dk_in)});
+  BRK_VALUE(q.dim() == 4 && k.dim() == 4 && d_raw_in.dim() == 4, "expected (B, heads, S, D) tensors");
+  const int64_t B = q.size(0), N = q.size(1), S = q.size(2), D = q.size(3), Nk = k.size(1), R = d_raw_in.size(2);
+  BRK_VALUE(d_raw_in.sizes() == at::IntArrayRef({B, N, R, S}) && d_raw_in.scalar_type() == q.scalar_type(), "d_raw must be (", B,
+            ", ", N, ", R, ", S, ") ", q.scalar_type(), ", got ", d_raw_in.sizes(), " ", d_raw_in.scalar_type());
+  const bool add = dq_in.has_value();
+  BRK_VALUE(add == dk_in.has_value(), "give both dq and dk, or neither");
+  c10::cuda::CUDAGuard guard(q.device());
+  Tensor dq = add ? *dq_in : at::zeros({B, S, N, D}, q.options().requires_grad(false)).permute({0, 2, 1, 3});
+  Tensor dk = add ? *dk_in : empty_bshd(q, B, S, Nk, D).permute({0, 2, 1, 3});
+  const Tensor d_raw = d_raw_in.contiguous(), bs = blk_start.contiguous(), bl = blk_len.contiguous();
+  brk_score_params p = score_params(q, k, bs, bl, scale, R, 0.05);
+  const brk_view vq = view_of(dq), vk = view_of(dk);
+  const size_t nbytes = brk_raw_scores_bwd_workspace_bytes(&p);
+  Tensor ws = scratch(nbytes, q);
+  check(brk_raw_scores_bwd(&p, d_raw.data_ptr(), &vq, &vk, add ? 1 : 0, ws.data_ptr(), nbytes, stream_of(q)),
+        "brk_raw_scores_bwd");
+  count(2);
+  return {dq, dk};
+}
+
+// ---- autograd ---------------------------------------------------------------------------------
+// An error of the library raised in a backward thread keeps its Python type.
+[[noreturn]] void rethrow_as_python(const LibError& e) {
+  pybind11::gil_scoped_acquire gil;
+  PyErr_SetString(g_lib_error, e.what());
+  python_error err;
+  err.persist();
+  throw err;
+}
+
+// BlockRank attention with its backward (brk_attn_bwd).  With num_last >= 0 it also returns the raw logits of the last R
+// slots, (B,N,R,S) = scale * q[:, :, S-R:] k^T + a constant mask addend (std:219-233, 256-262): the addend is constant,
+// so their gradient flows to q and k at every position (brk_raw_scores_bwd, which adds into the gradients of the
+// attention output instead of leaving two pairs of tensors for autograd to sum).
+struct AttentionFn : torch::autograd::Function<AttentionFn> {
+  using Ctx = torch::autograd::AutogradContext;
+  using List = torch::autograd::variable_list;
+
+  static List forward(Ctx* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& start, const Tensor& length,
+                      double scale, int64_t max_block_len, int64_t max_query_len, int64_t algo, int64_t num_last,
+                      int64_t grid_h) {
+    ctx->set_materialize_grads(false);
+    auto [out, lse] = attention(q, k, v, start, length, scale, max_block_len, std::nullopt, true, algo, max_query_len,
+                                std::nullopt);
+    ctx->save_for_backward({q, k, v, out, lse, start, length});
+    ctx->saved_data["scale"] = scale;
+    ctx->saved_data["max_block_len"] = max_block_len;
+    if (num_last < 0) return {out};
+    return {out, raw_scores(q, k, start, length, scale, num_last, grid_h)};
+  }
+
+  static List backward(Ctx* ctx, List grads) {
+    try {
+      const auto saved = ctx->get_saved_variables();
+      const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &out = saved[3], &lse = saved[4], &start = saved[5],
+                   &length = saved[6];
+      const double scale = ctx->saved_data["scale"].toDouble();
+      const int64_t max_block_len = ctx->saved_data["max_block_len"].toInt();
+      Tensor dq, dk, dv;
+      if (grads[0].defined())
+        std::tie(dq, dk, dv) = attention_bwd(q, k, v, out, grads[0].to(out.scalar_type()), lse, start, length, scale, max_block_len);
+      if (grads.size() > 1 && grads[1].defined()) {
+        const bool add = dq.defined();
+        std::tie(dq, dk) = raw_scores_bwd(q, k, grads[1].to(q.scalar_type()), start, length, scale,
+                                          add ? OptTensor(dq) : std::nullopt, add ? OptTensor(dk) : std::nullopt);
+      }
+      return {dq, dk, dv, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    } catch (const LibError& e) {
+      rethrow_as_python(e);
+    }
+  }
+};
+
+// num_last < 0: no raw logits.  spans: int32 (2, B, M) [starts; lengths].  Returns (out, raw or None).
+std::tuple<Tensor, OptTensor> attention_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& spans,
+                                                double scale, int64_t max_block_len, int64_t max_query_len, int64_t algo,
+                                                int64_t num_last, int64_t grid_h) {
+  BRK_VALUE(spans.dim() == 3 && spans.size(0) == 2, "block spans must be an int32 (2, B, M) tensor");
+  const Tensor start = spans.select(0, 0), length = spans.select(0, 1);
+  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) {
+    auto res = AttentionFn::apply(q, k, v, start, length, scale, max_block_len, max_query_len, algo, num_last, grid_h);
+    return {res[0], num_last < 0 ? OptTensor() : OptTensor(res[1])};
+  }
+  Tensor out = std::get<0>(attention(q, k, v, start, length, scale, max_block_len, std::nullopt, false, algo, max_query_len,
+                                     std::nullopt));
+  if (num_last < 0) return {out, std::nullopt};
+  return {out, raw_scores(q, k, start, length, scale, num_last, grid_h)};
+}
+
+// ---- runner helpers ---------------------------------------------------------------------------
+Tensor rmsnorm(const Tensor& x, const Tensor& weight, double eps, const OptTensor& residual, const OptTensor& out_in) {
+  need_cuda({&x, &weight, opt(residual)});
+  BRK_VALUE(x.is_contiguous() && (!residual.has_value() || residual->is_contiguous()), "rmsnorm expects contiguous rows");
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t hidden = x.size(-1), rows = hidden > 0 ? x.numel() / hidden : 0;
+  Tensor out = out_in.has_value() ? *out_in : at::empty_like(x);
+  check(brk_rmsnorm(dtype_code(x), x.data_ptr(), residual.has_value() ? residual->data_ptr() : nullptr, weight.data_ptr(),
+                    out.data_ptr(), rows, (int32_t)hidden, (float)eps, stream_of(x)),
+        "brk_rmsnorm");
+  count(1);
+  return out;
+}
+
+void rope_(const OptTensor& q, const OptTensor& k, const Tensor& pos, const Tensor& inv_freq) {
+  if (!q.has_value() && !k.has_value()) return;
+  const Tensor& ref = q.has_value() ? *q : *k;
+  need_cuda({&ref, &pos, &inv_freq});
+  BRK_VALUE(ref.dim() == 3, "rope_ expects (T, heads, D) views with contiguous heads");
+  const int64_t T = ref.size(0), D = ref.size(2);
+  for (const Tensor* t : {opt(q), opt(k)})
+    if (t != nullptr)
+      BRK_VALUE(t->dim() == 3 && t->size(0) == T && t->size(2) == D && t->stride(2) == 1 && t->stride(1) == D,
+                "rope_ expects (T, heads, D) views with contiguous heads");
+  BRK_VALUE(pos.scalar_type() == at::kInt && inv_freq.scalar_type() == at::kFloat && pos.numel() == T && pos.is_contiguous(),
+            "pos must be contiguous int32 (T,) and inv_freq float32");
+  c10::cuda::CUDAGuard guard(ref.device());
+  check(brk_rope(dtype_code(ref), q.has_value() ? q->data_ptr() : nullptr, q.has_value() ? q->stride(0) : 0,
+                 q.has_value() ? (int32_t)q->size(1) : 0, k.has_value() ? k->data_ptr() : nullptr,
+                 k.has_value() ? k->stride(0) : 0, k.has_value() ? (int32_t)k->size(1) : 0, (int32_t)D,
+                 (const int32_t*)pos.data_ptr(), (const float*)inv_freq.data_ptr(), T, stream_of(ref)),
+        "brk_rope");
+  count(1);
+}
+
+Tensor silu_mul(const Tensor& gate_up, const OptTensor& out_in) {
+  need_cuda({&gate_up});
+  BRK_VALUE(gate_up.is_contiguous(), "silu_mul expects a contiguous (rows, 2*I) tensor");
+  c10::cuda::CUDAGuard guard(gate_up.device());
+  const int64_t inter = gate_up.size(-1) / 2, rows = inter > 0 ? gate_up.numel() / (2 * inter) : 0;
+  Tensor out;
+  if (out_in.has_value()) {
+    out = *out_in;
+  } else {
+    auto shape = gate_up.sizes().vec();
+    shape.back() = inter;
+    out = at::empty(shape, gate_up.options());
+  }
+  check(brk_silu_mul(dtype_code(gate_up), gate_up.data_ptr(), out.data_ptr(), rows, (int32_t)inter, stream_of(gate_up)),
+        "brk_silu_mul");
+  count(1);
+  return out;
+}
+
+// ---- early-exit ranker --------------------------------------------------------------------------
+// PyTorch's GEMMs with the autograd layers of its dispatcher left out: nothing here is ever differentiated.
+struct NoAutograd {
+  at::NoGradGuard no_grad;
+  at::AutoDispatchBelowADInplaceOrView below_autograd;
+};
+
+
+// input norm, fused QKV projection, RoPE on q and k in place: (T, (N + 2 Nk) D)
+Tensor layer_qkv(const Tensor& h, const Tensor& ln1, const Tensor& wqkv, const Tensor& pos, const Tensor& inv_freq, int64_t N,
+                 int64_t Nk, int64_t D, double eps) {
+  NoAutograd guard;
+  Tensor qkv = at::mm(rmsnorm(h, ln1, eps, std::nullopt, std::nullopt), wqkv.t());
+  const int64_t T = qkv.size(0), row = qkv.stride(0), at0 = qkv.storage_offset();
+  rope_(qkv.as_strided({T, N, D}, {row, D, 1}, at0), qkv.as_strided({T, Nk, D}, {row, D, 1}, at0 + N * D), pos, inv_freq);
+  return qkv;
+}
+
+Tensor layer_attention(const Tensor& qkv, const Tensor& blk_start, const Tensor& blk_len, int64_t B, int64_t S, int64_t N,
+                       int64_t Nk, int64_t D, int64_t max_block_len, int64_t max_query_len, int64_t algo) {
+  NoAutograd guard;
+  const int64_t row = qkv.stride(0), at0 = qkv.storage_offset();
+  auto heads = [&](int64_t n, int64_t first) {
+    return qkv.as_strided({B, n, S, D}, {S * row, D, row, 1}, at0 + first * D);
+  };
+  return std::get<0>(attention(heads(N, 0), heads(Nk, N), heads(Nk, N + Nk), blk_start, blk_len, 1.0 / std::sqrt((double)D),
+                               max_block_len, std::nullopt, false, algo, max_query_len, std::nullopt));
+}
+
+// h += o_proj(attn); h += down_proj(silu(gate) * up) of its norm.  Both residual additions happen in the epilogue of the
+// GEMM that produces the branch (C = C + A B, added in fp32 before the rounding).
+void layer_rest(Tensor& h, const Tensor& attn, const Tensor& wo, const Tensor& ln2, const Tensor& wgu, const Tensor& wd,
+                double eps) {
+  NoAutograd guard;
+  h.addmm_(attn.view({h.size(0), wo.size(1)}), wo.t());
+  const Tensor x = rmsnorm(h, ln2, eps, std::nullopt, std::nullopt);
+  h.addmm_(silu_mul(at::mm(x, wgu.t()), std::nullopt), wd.t());
+}
+
+// layers: {ln1, wqkv, wo, ln2, wgu, wd} of every layer in front of the scoring layer.  ids (B, S), pos int32 (B S,).
+Tensor hidden_states(const Tensor& embed, const Tensor& ids, const std::vector<std::vector<Tensor>>& layers, const Tensor& pos,
+                     const Tensor& inv_freq, const Tensor& blk_start, const Tensor& blk_len, int64_t max_block_len,
+                     int64_t max_query_len, int64_t N, int64_t Nk, int64_t D, double eps, int64_t algo) {
+  NoAutograd guard;
+  c10::cuda::CUDAGuard device(embed.device());
+  const int64_t B = ids.size(0), S = ids.size(1);
+  Tensor h = at::embedding(embed, ids.reshape({B * S}));
+  for (const auto& L : layers) {
+    const Tensor attn = layer_attention(layer_qkv(h, L.at(0), L.at(1), pos, inv_freq, N, Nk, D, eps), blk_start, blk_len, B, S,
+                                        N, Nk, D, max_block_len, max_query_len, algo);
+    layer_rest(h, attn, L.at(2), L.at(3), L.at(4), L.at(5), eps);
+  }
+  return h;
+}
+
+// The scoring layer up to the score epilogue: keys of every token, queries of the signal rows, both rotated; and the
+// index of each query row inside q.  Returns (q (B,N,R,D), k (B,Nk,S,D), rows int32 (B,R)).
+std::tuple<Tensor, Tensor, Tensor> score_qk(const Tensor& h, const Tensor& pos, const Tensor& signal_rows, const Tensor& ln1,
+                                            const Tensor& wq, const Tensor& wk, const Tensor& inv_freq, int64_t N, int64_t Nk,
+                                            int64_t D, double eps) {
+  NoAutograd guard;
+  c10::cuda::CUDAGuard device(h.device());
+  need_cuda({&h, &pos, &signal_rows});
+  BRK_VALUE(signal_rows.scalar_type() == at::kInt && signal_rows.dim() == 2 && pos.scalar_type() == at::kInt && pos.is_contiguous(),
+            "signal_rows must be int32 (B, R) and positions contiguous int32");
+  const int64_t B = signal_rows.size(0), R = signal_rows.size(1), T = h.size(0), S = T / B;
+  const Tensor x = rmsnorm(h, ln1, eps, std::nullopt, std::nullopt), rows = signal_rows.contiguous();
+  Tensor k = at::mm(x, wk.t());
+  Tensor xs = at::empty({B * R, x.size(1)}, x.options()), ps = at::empty({B * R}, pos.options()), local = at::empty({B, R}, pos.options());
+  check(brk_signal_rows(dtype_code(x), x.data_ptr(), (int32_t)x.size(1), (const int32_t*)pos.data_ptr(),
+                        (const int32_t*)rows.data_ptr(), (int32_t)B, (int32_t)S, (int32_t)R, xs.data_ptr(),
+                        (int32_t*)ps.data_ptr(), (int32_t*)local.data_ptr(), (int32_t*)status_word(x.get_device()).data_ptr(),
+                        stream_of(x)),
+        "brk_signal_rows");
+  count(1);
+  Tensor q = at::mm(xs, wq.t());
+  rope_(q.view({B * R, N, D}), std::nullopt, ps, inv_freq);
+  rope_(std::nullopt, k.view({T, Nk, D}), pos, inv_freq);
+  return {q.view({B, R, N, D}).permute({0, 2, 1, 3}), k.view({B, S, Nk, D}).permute({0, 2, 1, 3}), local};
+}
+
+// Host tensors of a batch -> device: (ids, positions int32, start, length, signal rows), and the longest query block.
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, int64_t> upload(const Tensor& ids, const Tensor& pos, const Tensor& spans,
+                                                                   const Tensor& rows, const c10::Device& device) {
+  NoAutograd guard;
+  BRK_VALUE(spans.dim() == 3 && spans.size(0) == 2 && spans.scalar_type() == at::kInt, "block_spans must be int32 (2, B, M)");
+  const Tensor d_ids = ids.to(device, ids.scalar_type(), true), d_pos = pos.to(device, pos.scalar_type(), true).to(at::kInt);
+  const Tensor d_spans = spans.to(device, spans.scalar_type(), true), d_rows = rows.to(device, rows.scalar_type(), true);
+  const Tensor q_len = spans.select(0, 1).select(1, spans.size(2) - 1);
+  int64_t longest = 0;
+  if (q_len.is_cpu()) {
+    for (int64_t b = 0; b < q_len.size(0); ++b)
+      longest = std::max<int64_t>(longest, static_cast<const int32_t*>(q_len.data_ptr())[b * q_len.stride(0)]);
+  } else {
+    longest = q_len.max().item().toLong();
+  }
+  return {d_ids, d_pos, d_spans.select(0, 0), d_spans.select(0, 1), d_rows, longest};
+}
+
+// Scores and the indices of the k best documents -> host, with one synchronisation, after which a problem a kernel
+// reported is raised.
+std::tuple<Tensor, Tensor> download(const Tensor& logits_in, int64_t k) {
+  NoAutograd guard;
+  c10::cuda::CUDAGuard device(logits_in.device());
+  const Tensor logits = logits_in.contiguous();
+  const Tensor top = std::get<1>(at::topk(logits, std::min(k, logits.size(-1)), -1));
+  const Tensor word = status_word(logits.get_device());
+  const auto stream = at::cuda::getCurrentCUDAStream(logits.get_device());
+  const size_t nl = logits.nbytes(), nt = top.nbytes(), at_top = (nl + 15) & ~(size_t)15, at_word = at_top + ((nt + 15) & ~(size_t)15);
+  Tensor stage = at::empty({(int64_t)(at_word + 16)}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
+  char* const base = static_cast<char*>(stage.data_ptr());
+  C10_CUDA_CHECK(cudaMemcpyAsync(base, logits.data_ptr(), nl, cudaMemcpyDeviceToHost, stream));
+  C10_CUDA_CHECK(cudaMemcpyAsync(base + at_top, top.data_ptr(), nt, cudaMemcpyDeviceToHost, stream));
+  C10_CUDA_CHECK(cudaMemcpyAsync(base + at_word, word.data_ptr(), 4, cudaMemcpyDeviceToHost, stream));
+  {
+    pybind11::gil_scoped_release release;
+    C10_CUDA_CHECK(cudaStreamSynchronize(stream));
+  }
+  Tensor h_logits = at::empty(logits.sizes(), logits.options().device(at::kCPU)), h_top = at::empty(top.sizes(), top.options().device(at::kCPU));
+  memcpy(h_logits.data_ptr(), base, nl);
+  memcpy(h_top.data_ptr(), base + at_top, nt);
+  int32_t code;
+  memcpy(&code, base + at_word, 4);
+  if (code != 0) check(brk_status_poll((int32_t*)word.data_ptr(), stream.stream()), "brk_status_poll");
+  return {h_logits, h_top};
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  namespace py = pybind11;
+  py::register_exception_translator([](std::exception_ptr p) {
+    try {
+      if (p) std::rethrow_exception(p);
+    } catch (const LibError& e) {
+      PyErr_SetString(g_lib_error, e.what());
+    } catch (const c10::OutOfMemoryError& e) {
+      PyErr_SetString(g_oom_error, e.what_without_backtrace());
+    } catch (const c10::ValueError& e) {
+      PyErr_SetString(PyExc_ValueError, e.what_without_backtrace());
+    } catch (const c10::IndexError& e) {
+      PyErr_SetString(PyExc_IndexError, e.what_without_backtrace());
+    } catch (const c10::Error& e) {
+      PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+    }
+  });
+  m.def("set_error_classes", [](py::object lib, py::object oom) {
+    g_lib_error = lib.release().ptr();
+    g_oom_error = oom.release().ptr();
+  });
+  m.def("launch_count", [] { return g_launches.load(); });
+  m.def("status_word", &status_word);
+  m.def("spans_from_mask", &spans_from_mask);
+  m.def("attention", &attention);
+  m.def("attention_bwd", &attention_bwd);
+  m.def("attention_forward", &attention_forward);
+  m.def("doc_scores", &doc_scores);
+  m.def("raw_scores", &raw_scores);
+  m.def("raw_scores_bwd", &raw_scores_bwd);
+  m.def("rmsnorm", &rmsnorm);
+  m.def("rope_", &rope_);
+  m.def("silu_mul", &silu_mul);
+  m.def("layer_qkv", &layer_qkv);
+  m.def("layer_attention", &layer_attention);
+  m.def("layer_rest", &layer_rest);
+  m.def("hidden_states", &hidden_states);
+  m.def("score_qk", &score_qk);
+  m.def("upload", &upload);
+  m.def("download", &download);
+}

@@ -47,6 +47,9 @@ class RankerConfig:
                             num_attention_heads=4, num_key_value_heads=2, head_dim=64, score_layer=score_layer)
 
 
+_LAYER_WEIGHTS = ("ln1", "wqkv", "wo", "ln2", "wgu", "wd")  # of a full layer
+
+
 @dataclass
 class _CapturedScore:
     graph: "torch.cuda.CUDAGraph"
@@ -125,36 +128,28 @@ class MistralPrefillRanker:
         Both residual additions happen in the epilogue of the GEMM that produces the branch
         (``h.addmm_``: C = C + A·B, added in fp32 before the rounding), so the branch output is never
         written to memory and the RMSNorm that follows reads one tensor instead of two."""
-        c = self.cfg
+        c, L, host = self.cfg, self.layers[i], _lib.host()
         N, Nk, D = c.num_attention_heads, c.num_key_value_heads, c.head_dim
-        qd, kd = N * D, Nk * D
-        T = B * S
-        L = self.layers[i]
-        x = ops.rmsnorm(h, L["ln1"], c.rms_norm_eps)
-        qkv = torch.matmul(x, L["wqkv"].t())                         # (T, qd + 2 kd)
-        q3 = qkv[:, :qd].view(T, N, D)
-        k3 = qkv[:, qd:qd + kd].view(T, Nk, D)
-        ops.rope_(q3, k3, pos, self.inv_freq)
-        q4 = qkv[:, :qd].view(B, S, N, D).permute(0, 2, 1, 3)
-        k4 = qkv[:, qd:qd + kd].view(B, S, Nk, D).permute(0, 2, 1, 3)
-        v4 = qkv[:, qd + kd:].view(B, S, Nk, D).permute(0, 2, 1, 3)
+        qkv = host.layer_qkv(h, L["ln1"], L["wqkv"], pos, self.inv_freq, N, Nk, D, c.rms_norm_eps)
         ev = self._tick("attn")
-        attn = ops.attention(q4, k4, v4, blk_start, blk_len, D ** -0.5, max_block_len, algo=self.algo,
-                             max_query_len=max_query_len)
+        attn = host.layer_attention(qkv, blk_start, blk_len, B, S, N, Nk, D, max_block_len, max_query_len, self.algo)
         self._tock(ev)
-        h.addmm_(attn.view(T, qd), L["wo"].t())                      # h += o_proj(attn)
-        x = ops.rmsnorm(h, L["ln2"], c.rms_norm_eps)
-        act = ops.silu_mul(torch.matmul(x, L["wgu"].t()))
-        h.addmm_(act, L["wd"].t())                                   # h += down_proj(act)
+        host.layer_rest(h, attn, L["wo"], L["ln2"], L["wgu"], L["wd"], c.rms_norm_eps)
         return h
 
     @torch.no_grad()
     def hidden_before_score_layer(self, input_ids, position_ids, blk_start, blk_len, max_block_len, max_query_len=0):
         """Run layers 0..l*-1; returns the residual stream entering layer l*, shape (B*S, hidden)."""
         B, S = input_ids.shape
+        c = self.cfg
         pos = position_ids.reshape(B * S).to(torch.int32)
+        if self.events is None:  # the layers in one native call
+            return _lib.host().hidden_states(
+                self.embed, input_ids, [[L[n] for n in _LAYER_WEIGHTS] for L in self.layers[:c.score_layer]], pos, self.inv_freq,
+                blk_start, blk_len, max_block_len, max_query_len, c.num_attention_heads, c.num_key_value_heads, c.head_dim,
+                c.rms_norm_eps, self.algo)
         h = torch.embedding(self.embed, input_ids.reshape(B * S))
-        for i in range(self.cfg.score_layer):
+        for i in range(c.score_layer):
             self.decoder_layer(i, h, pos, B, S, blk_start, blk_len, max_block_len, max_query_len)
         return h
 
@@ -175,24 +170,12 @@ class MistralPrefillRanker:
         """The scoring layer's share of the work, from the residual stream ``h`` (B*S, hidden) entering it:
         input RMSNorm, ``k_proj`` of every token, ``q_proj`` of the signal rows, RoPE, fused score epilogue."""
         c = self.cfg
-        B, S = position_ids.shape
-        N, Nk, D = c.num_attention_heads, c.num_key_value_heads, c.head_dim
-        R = signal_rows.shape[1]
         L = self.layers[c.score_layer]
-        x = ops.rmsnorm(h, L["ln1"], c.rms_norm_eps)
-        T = B * S
-        pos = position_ids.reshape(T).to(torch.int32)
-        k = torch.matmul(x, L["wk"].t()).view(T, Nk, D)
-        flat_rows = (signal_rows.to(torch.int64) + torch.arange(B, device=x.device)[:, None] * S).reshape(-1)
-        q = torch.matmul(x.index_select(0, flat_rows), L["wq"].t()).view(B * R, N, D)
-        # RoPE: keys of every token, queries of the signal rows only
-        ops.rope_(q, None, pos.index_select(0, flat_rows), self.inv_freq)
-        ops.rope_(None, k, pos, self.inv_freq)
-        q4 = q.view(B, R, N, D).permute(0, 2, 1, 3)
-        k4 = k.view(B, S, Nk, D).permute(0, 2, 1, 3)
-        local_rows = torch.arange(R, device=x.device, dtype=torch.int32).expand(B, R).contiguous()
+        pos = position_ids.reshape(-1).to(torch.int32)
+        q, k, rows = _lib.host().score_qk(h, pos, signal_rows.to(torch.int32), L["ln1"], L["wq"], L["wk"], self.inv_freq,
+                                          c.num_attention_heads, c.num_key_value_heads, c.head_dim, c.rms_norm_eps)
         ev = self._tick("score")
-        mass, logits = ops.doc_scores(q4, k4, blk_start, blk_len, local_rows, D ** -0.5, c.temperature)
+        mass, logits = ops.doc_scores(q, k, blk_start, blk_len, rows, c.head_dim ** -0.5, c.temperature)
         self._tock(ev)
         return logits, mass
 
@@ -246,18 +229,12 @@ class MistralPrefillRanker:
         """End-to-end call on HOST tensors: ``batch`` holds pinned ``input_ids``/``position_ids`` (B, S) int64,
         ``block_spans`` int32 (2, B, M), ``signal_rows`` int32 (B, R) and ``max_block_len``.  Copies them to the
         device, scores, and returns (logits, top-k document indices) on the host."""
-        dev = self.device
-        ids = batch["input_ids"].to(dev, non_blocking=True)
-        pos = batch["position_ids"].to(dev, non_blocking=True)
-        spans = batch["block_spans"].to(dev, non_blocking=True)
-        rows = batch["signal_rows"].to(dev, non_blocking=True)
+        ids, pos, start, length, rows, max_query_len = _lib.host().upload(
+            batch["input_ids"], batch["position_ids"], batch["block_spans"], batch["signal_rows"], self.device)
         run = self.score_graphed if self.use_graphs else self.score
-        mql = int(batch["block_spans"][1, :, -1].max())  # host tensor: no synchronisation
-        logits, _ = run(ids, pos, spans[0], spans[1], int(batch["max_block_len"]), rows, mql)
-        top = torch.topk(logits, k=min(k, logits.shape[-1]), dim=-1).indices
-        out = logits.cpu(), top.cpu()
-        ops.check_status(dev)  # raises if a kernel reported malformed spans or a wait that gave up
-        return out
+        logits, _ = run(ids, pos, start, length, int(batch["max_block_len"]), rows, max_query_len)
+        # (raises if a kernel reported malformed spans or a wait that gave up)
+        return _lib.host().download(logits, k)
 
     def weight_bytes(self) -> int:
         n = self.embed.numel() * self.embed.element_size()

@@ -242,6 +242,11 @@ BRK_API int brk_rmsnorm(int32_t dtype, const void* x, void* residual, const void
  * in elements), angle = pos[t] * inv_freq[i].  q may be NULL when N == 0, k when Nk == 0. */
 BRK_API int brk_rope(int32_t dtype, void* q, int64_t q_row_stride, int32_t N, void* k, int64_t k_row_stride,
              int32_t Nk, int32_t D, const int32_t* pos, const float* inv_freq, int64_t T, void* stream);
+/* The signal rows of every prompt: x_out[b R + r] = x[b S + rows[b, r]] (rows of `hidden` elements), the same for the
+ * positions, and local[b, r] = r (the slot of each row in the gathered tensor).  A row outside [0, S) sets `status` (may be
+ * NULL; see brk_status_poll). */
+BRK_API int brk_signal_rows(int32_t dtype, const void* x, int32_t hidden, const int32_t* pos, const int32_t* rows, int32_t B,
+                            int32_t S, int32_t R, void* x_out, int32_t* pos_out, int32_t* local, int32_t* status, void* stream);
 /* out[r, c] = silu(gate_up[r, c]) * gate_up[r, inter + c]. */
 BRK_API int brk_silu_mul(int32_t dtype, const void* gate_up, void* out, int64_t rows, int32_t inter, void* stream);
 

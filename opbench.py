@@ -268,8 +268,8 @@ def model_bench(a, ops, ref_loader, mask, H, S, prompts, bl):
 def backward_bench(a, ops, ref_loader, q, k, v, mask, start, ln, scale, H, S, prompts, bl, flops, valid):
     """Forward + backward of the attention op under autograd: this library (tcgen05 forward, CUDA-core backward)
     beside autograd over the reference's eager and SDPA functions, same tensors, gradients compared."""
-    from blockrank_b200.attention import _AttentionFn
-    from blockrank_b200 import _lib
+    from blockrank_b200 import BlockSpans, cuda_blockrank_attention_forward
+    spans = BlockSpans.make(start, ln, H)
     g = torch.Generator(device=q.device).manual_seed(4)
     d_out = (torch.randn(prompts, S, N, D, generator=g, device=q.device) * valid[:, :, None, None]).bfloat16()
     impls = ["ours", "eager_ref", "sdpa_ref"] if a.impl == "all" else a.impl.split(",")
@@ -278,7 +278,7 @@ def backward_bench(a, ops, ref_loader, q, k, v, mask, start, ln, scale, H, S, pr
         try:
             qg, kg, vg = (t.detach().clone().requires_grad_(True) for t in (q, k, v))
             if name == "ours":
-                run = lambda: _AttentionFn.apply(qg, kg, vg, start, ln, scale, H, 0, _lib.ALGO_AUTO, None, None)
+                run = lambda: cuda_blockrank_attention_forward(None, qg, kg, vg, spans, scale)[0]
             else:
                 if not ref_loader.available():
                     raise RuntimeError(ref_loader.why_unavailable())
