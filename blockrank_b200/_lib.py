@@ -42,7 +42,8 @@ class AttnBwdParams(C.Structure):
     _fields_ = [("dtype", C.c_int32), ("B", C.c_int32), ("N", C.c_int32), ("Nk", C.c_int32), ("D", C.c_int32),
                 ("S", C.c_int32), ("M", C.c_int32), ("max_block_len", C.c_int32), ("scale", C.c_float),
                 ("q", View), ("k", View), ("v", View), ("o", View), ("d_o", View), ("lse", C.c_void_p),
-                ("blk_start", C.c_void_p), ("blk_len", C.c_void_p), ("dq", View), ("dk", View), ("dv", View)]
+                ("blk_start", C.c_void_p), ("blk_len", C.c_void_p), ("dq", View), ("dk", View), ("dv", View),
+                ("status", C.c_void_p)]
 
 
 class ScoreParams(C.Structure):

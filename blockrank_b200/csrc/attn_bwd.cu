@@ -317,7 +317,9 @@ int launch_all(const BwdArgs& a, cudaStream_t st) {
 size_t dq_last_bytes(const brk_attn_bwd_params& p) {
   return p.dtype == BRK_BF16 ? (size_t)p.B * p.N * p.max_block_len * p.D * sizeof(float) : 0;
 }
-size_t attn_bwd_workspace(const brk_attn_bwd_params& p) { return delta_bytes(p) + 2 * acc_bytes(p) + dq_last_bytes(p); }
+size_t attn_bwd_workspace(const brk_attn_bwd_params& p) {
+  return delta_bytes(p) + 2 * acc_bytes(p) + dq_last_bytes(p) + (attn_bwd_tc_supported(p) ? attn_bwd_tc_extra_bytes(p) : 0);
+}
 
 int attn_bwd_launch(const brk_attn_bwd_params& p, void* ws, size_t ws_bytes, cudaStream_t st) {
   BRK_REQUIRE(ws != nullptr && ws_bytes >= attn_bwd_workspace(p) && ((uintptr_t)ws & 15) == 0, BRK_E_WORKSPACE,
@@ -335,6 +337,10 @@ int attn_bwd_launch(const brk_attn_bwd_params& p, void* ws, size_t ws_bytes, cud
   a.nsplit = p.M > 2 ? std::min(p.M, 64) : 1;  // block 0 is seen by every row block: its key tiles need many CTAs
   a.scale = p.scale;
   a.scale_log2 = p.scale * 1.4426950408889634f;
+  if (attn_bwd_tc_supported(p)) {
+    unsigned char* const dq32 = w + delta_bytes(p) + 2 * acc_bytes(p);
+    return attn_bwd_tc_launch(p, a.delta, a.dk32, reinterpret_cast<float*>(dq32), dq32 + dq_last_bytes(p), st);
+  }
   BRK_CUDA(cudaMemsetAsync(w + delta_bytes(p), 0, 2 * acc_bytes(p) + dq_last_bytes(p), st));
   if (p.dtype == BRK_BF16) {
     // bf16: the tensor-core kernels compute dq and the accumulators; the conversion kernel is shared

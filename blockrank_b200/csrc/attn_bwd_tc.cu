@@ -1,0 +1,739 @@
+// BlockRank attention backward on the sm_100a tensor cores (tcgen05 + TMEM), bf16, head_dim 64 or 128.
+//
+// A work item is one block of one (prompt, KV head): the keys are the block's own ones, for a document with the prefix
+// block's in front, in tiles of 128; the rows are the block's own query tokens (all G heads of the group, 128 / G tokens
+// x G heads per row tile) and then the query block's rows, which see the block's own keys.  So every key of a document
+// and every row of a document meets all its partners inside one item:
+//
+//   dV, dK of own keys     accumulate in tensor memory over the key tile's row tiles and are stored once, in bf16
+//   dK, dV of the prefix   get one fp32 reduction per document item (red.global.add)
+//   dQ of own rows         is the sum over the item's key tiles: two at most for documents up to 128 tokens plus prefix;
+//                          a partial sum waits in fp32 in a scratch of the CTA, laid out for coalesced access by the
+//                          thread that wrote it
+//   dQ of the query block  fp32 reductions (every item contributes)
+//
+// Per (key tile, row tile) pair, all five products on tcgen05, keys down the 128 TMEM lanes:
+//   S^T = K Q^T      dP^T = V dO^T      P^T = 2^(S^T scale - lse)     dS^T = P^T (dP^T - delta)
+//   dV += P^T dO (P^T read from tensor memory)    dK += dS^T Q    dQ = dS K   (dS^T in shared memory serves both: K-major
+//                                                 for dK, MN-major for dQ)
+//
+// Roles (320 threads, one CTA per SM, items claimed from a global counter):
+//   warps 0-7  the element-wise part: warp w owns lanes 32 (w % 4) and the row-tile columns (or head_dim half) w / 4;
+//              they also load K / V (cp.async, zero beyond the list, so any prefix length packs against any document),
+//              drain dQ, dK, dV
+//   warp 8     MMA issue
+//   warp 9     claims items, loads Q / dO by TMA two row tiles deep, and the columns' lse and delta
+//
+// Order of the tensor pipe: dP(i) | dV(i) S(i+1) | dK(i) dQ(i), so that the exponentials of tile i + 1 run beside
+// dK(i) / dQ(i) and the dS of tile i beside dV(i) / S(i+1).  Tensor memory (head_dim 128, all 512 columns): S / P 128,
+// dP / dQ 128, dV 128, dK 128.
+#include <cuda.h>
+
+#include <algorithm>
+
+#include "brk_common.cuh"
+#include "mma_bf16.cuh"
+#include "tc_ptx.cuh"
+
+namespace brk {
+
+namespace {
+
+constexpr int kTile = 128;  // keys per key tile, rows per row tile
+constexpr int kComputeThreads = 256;
+constexpr int kThreads = 320;
+constexpr uint32_t kChunk = kTile * 128;  // 128 rows of 64 bf16: one 64-wide chunk of a tile
+constexpr uint32_t kWaitBudget = 1u << 18;
+constexpr int kMaxRowTiles = 16;  // per block: bounds the dQ scratch of a CTA (64 KB per tile at head_dim 128)
+
+template <int HD>
+struct Geo {
+  static constexpr uint32_t kTileBytes = (HD / 64) * kChunk;
+  static constexpr uint32_t kOffK = 0;
+  static constexpr uint32_t kOffV = kOffK + kTileBytes;
+  static constexpr uint32_t kOffQ = kOffV + kTileBytes;        // two stages of [Q | dO]
+  static constexpr uint32_t kOffDs = kOffQ + 4 * kTileBytes;
+  static constexpr uint32_t kOffCol = kOffDs + 2 * kChunk;     // two stages of [-lse log2 e | delta], 128 floats each
+  static constexpr uint32_t kOffBar = kOffCol + 2 * 2 * kTile * 4;
+  static constexpr uint32_t kSmem = kOffBar + 256;
+  static_assert(kSmem <= 232448, "shared memory per CTA");
+};
+constexpr uint32_t kColS = 0, kColDp = 128, kColDv = 256, kColDk = 384;
+
+enum {
+  kQFull = 0,    // +stage  Q, dO landed and the columns' lse / delta written (expect_tx arrival + 1)
+  kQFree = 2,    // +stage  dK has read the stage
+  kSFull = 4,
+  kDpFull = 5,
+  kPFull = 6,    // P^T in tensor memory (8 warps)
+  kDsFull = 7,   // dS^T in shared memory, dP consumed (8 warps)
+  kDqFull = 8,
+  kDqFree = 9,   // dQ drained (8 warps)
+  kAccFull = 10, // every product of the key tile complete
+  kKvFull = 11,  // K, V of the key tile in shared memory, the accumulators drained (8 warps)
+  kTail = 12,    // the rows beyond the block zeroed in a partial row tile (8 warps)
+  kItemFull = 13,  // +slot
+  kItemFree = 15,  // +slot (8 compute warps + MMA warp)
+  kNumBars = 17
+};
+static_assert(kNumBars * 8 + 16 <= 256, "barrier area");  // + TMEM base, two item slots
+
+struct BwdTcArgs {
+  View q, k, v, o, d_o, dq, dk, dv;
+  const float* lse;
+  float* delta;     // [B, N, S]
+  float* pre;       // prefix accumulators: dK then dV, [B, Nk, max_block_len, D] each; nullptr: block 0 stored directly
+  float* dq32;      // [B, N, max_block_len, D]: dQ of the last block's rows
+  float* part;      // [CTA][row tile][16 (HD / 128)][256 threads] float4: dQ of rows whose keys span several tiles
+  int* counter;
+  int32_t* status;
+  const int32_t* blk_start;
+  const int32_t* blk_len;
+  int B, N, Nk, S, M, G, g_shift, max_block_len, row_tiles, total_items;
+  float scale, scale_log2;
+};
+
+__device__ __forceinline__ void span_of(const BwdTcArgs& a, int b, int m, int& start, int& len) {
+  start = a.blk_start[(size_t)b * a.M + m];
+  len = a.blk_len[(size_t)b * a.M + m];
+  if (start < 0 || len < 0 || len > a.max_block_len || start > a.S - len) len = 0;  // skipped: nothing out of bounds
+}
+
+__device__ __forceinline__ void red4(float* p, float x, float y, float z, float w) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+
+struct Item {
+  int b, g, m;
+  int start, len;    // the block
+  int s0, l0;        // prefix keys in front of the own ones (l0 = 0: none)
+  int qs, ql;        // query-block rows that see the own keys (ql = 0: none)
+  int n_kt, R, RQ;   // key tiles, own row tiles, query row tiles
+};
+
+__device__ __forceinline__ Item decode(const BwdTcArgs& a, int idx) {
+  Item it;
+  const int nbg = a.B * a.Nk, bg = idx % nbg;
+  it.m = idx / nbg;
+  it.b = bg / a.Nk;
+  it.g = bg % a.Nk;
+  span_of(a, it.b, it.m, it.start, it.len);
+  it.s0 = it.l0 = it.qs = it.ql = 0;
+  if (it.m > 0 && it.m < a.M - 1) span_of(a, it.b, 0, it.s0, it.l0);
+  if (it.m < a.M - 1) span_of(a, it.b, a.M - 1, it.qs, it.ql);
+  const int tok = kTile >> a.g_shift;
+  it.n_kt = it.len > 0 ? (it.l0 + it.len + kTile - 1) / kTile : 0;
+  it.R = (it.len + tok - 1) / tok;
+  it.RQ = (it.ql + tok - 1) / tok;
+  return it;
+}
+
+// Row tiles of key tile kt: own tiles r0 .. R-1, then query tiles 0 .. nq-1.
+struct RowList {
+  int r0, n_own, n;
+};
+__device__ __forceinline__ RowList rows_of(const BwdTcArgs& a, const Item& it, int kt) {
+  RowList l;
+  l.r0 = max(0, kt * kTile - it.l0) >> (7 - a.g_shift);  // first tile with a token at or behind the key tile's first own key
+  l.n_own = it.R - l.r0;
+  l.n = l.n_own + ((kt + 1) * kTile > it.l0 ? it.RQ : 0);
+  return l;
+}
+struct RowTile {
+  bool own;
+  int t0, nrow, slot;  // first token inside the block, valid rows, first token slot
+  int r;               // own: row tile number
+};
+__device__ __forceinline__ RowTile row_tile(const BwdTcArgs& a, const Item& it, const RowList& l, int i) {
+  RowTile t;
+  t.own = i < l.n_own;
+  t.r = t.own ? l.r0 + i : i - l.n_own;
+  t.t0 = t.r * (kTile >> a.g_shift);
+  t.slot = (t.own ? it.start : it.qs) + t.t0;
+  t.nrow = min(kTile, ((t.own ? it.len : it.ql) - t.t0) << a.g_shift);
+  return t;
+}
+
+template <int HD>
+__global__ void __launch_bounds__(kThreads, 1)
+attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG, const BwdTcArgs a) {
+  using L = Geo<HD>;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t sbase = ptx::smem_u32(smem);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  auto bar = [&](int i) { return sbase + L::kOffBar + (uint32_t)i * 8u; };
+  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kOffBar + kNumBars * 8);
+  int* const item_slot = reinterpret_cast<int*>(smem + L::kOffBar + kNumBars * 8 + 4);
+  if (tid == 0) {
+    for (int i = 0; i < kNumBars; ++i) {
+      uint32_t cnt = 1u;
+      if (i == kPFull || i == kDsFull || i == kDqFree || i == kKvFull || i == kTail) cnt = 8u;
+      if (i == kQFull || i == kQFull + 1) cnt = 2u;
+      if (i >= kItemFree) cnt = 9u;
+      ptx::mbar_init(bar(i), cnt);
+    }
+    ptx::fence_barrier_init();
+    ptx::prefetch_tmap(&tmQ);
+    ptx::prefetch_tmap(&tmG);
+  }
+  __syncwarp();
+  if (warp == 0) {
+    ptx::tmem_alloc(ptx::smem_u32(tmem_slot), 512);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  bool failed = false;
+  auto wait = [&](int i, uint32_t parity, int code) {
+    if (failed) return;
+    // (inlined: 64 probabilities are live across some of these waits)
+    for (uint32_t n = 0; n < kWaitBudget; ++n)
+      if (ptx::mbar_try(bar(i), parity & 1u)) return;
+    failed = true;
+    if (a.status) atomicCAS(a.status, 0, code);
+  };
+  uint32_t n_items = 0;
+  // next item of this CTA, or -1 (consumers: warps 0-8)
+  auto next_item = [&]() {
+    const uint32_t slot = n_items & 1u;
+    wait(kItemFull + slot, n_items >> 1, 40);
+    int idx = item_slot[slot];
+    if (__any_sync(0xffffffffu, failed)) idx = -1;
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive(bar(kItemFree + slot));
+    ++n_items;
+    return idx;
+  };
+
+  if (warp == 9) {
+    // =============================== loader ======================================================
+    uint32_t tile = 0, pub = 0;
+    const bool leader = lane == 0;
+    auto claim = [&]() {
+      int v = 0;
+      if (leader) v = atomicAdd(a.counter, 1);
+      v = __shfl_sync(0xffffffffu, v, 0);
+      return v < a.total_items ? v : -1;
+    };
+    for (;;) {
+      const int idx = claim();
+      if (pub >= 2) wait(kItemFree + (pub & 1u), (pub >> 1) - 1, 60);
+      if (leader) {
+        item_slot[pub & 1u] = idx;
+        ptx::mbar_arrive(bar(kItemFull + (pub & 1u)));
+      }
+      ++pub;
+      if (idx < 0 || __any_sync(0xffffffffu, failed)) break;
+      const Item it = decode(a, idx);
+      for (int kt = 0; kt < it.n_kt; ++kt) {
+        const RowList rows = rows_of(a, it, kt);
+        for (int i = 0; i < rows.n; ++i, ++tile) {
+          const RowTile t = row_tile(a, it, rows, i);
+          const uint32_t st = tile & 1u;
+          if (tile >= 2) wait(kQFree + st, (tile >> 1) - 1, 61);
+          if (leader) {
+            const uint32_t q = sbase + L::kOffQ + st * 2 * L::kTileBytes, g = q + L::kTileBytes;
+            ptx::mbar_expect_tx(bar(kQFull + st), 2 * L::kTileBytes);
+#pragma unroll
+            for (int c = 0; c < HD / 64; ++c) {
+              ptx::tma_load_4d(q + c * kChunk, &tmQ, bar(kQFull + st), 64 * c, it.g * a.G, t.slot, it.b);
+              ptx::tma_load_4d(g + c * kChunk, &tmG, bar(kQFull + st), 64 * c, it.g * a.G, t.slot, it.b);
+            }
+          }
+          float* const col = reinterpret_cast<float*>(smem + L::kOffCol) + st * 2 * kTile;
+#pragma unroll
+          for (int j = 0; j < kTile / 32; ++j) {
+            const int c = lane + 32 * j;
+            float nl = -INFINITY, dl = 0.f;  // beyond the block: P = 0
+            if (c < t.nrow) {
+              const size_t id = ((size_t)it.b * a.N + it.g * a.G + (c & (a.G - 1))) * a.S + t.slot + (c >> a.g_shift);
+              nl = a.lse[id] * -1.4426950408889634f;
+              dl = a.delta[id];
+            }
+            col[c] = nl;
+            col[kTile + c] = dl;
+          }
+          __syncwarp();
+          if (leader) ptx::mbar_arrive(bar(kQFull + st));
+        }
+      }
+    }
+  } else if (warp == 8) {
+    // =============================== MMA issue ===================================================
+    const bool leader = lane == 0;
+    uint32_t tile = 0, kts = 0, tails = 0;
+    const uint32_t id_dkv = ptx::idesc_bf16(kTile, HD, 0, 1);  // dV, dK: A K-major, B (dO / Q) MN-major
+    const uint32_t id_dq = ptx::idesc_bf16(kTile, HD, 1, 1);   // dQ: A (dS) and B (K) MN-major
+    const uint64_t k_k = ptx::smem_desc_sw128(sbase + L::kOffK, 16, 1024), v_k = ptx::smem_desc_sw128(sbase + L::kOffV, 16, 1024);
+    const uint64_t k_mn = ptx::smem_desc_sw128(sbase + L::kOffK, kChunk, 1024);
+    const uint64_t ds_k = ptx::smem_desc_sw128(sbase + L::kOffDs, 16, 1024), ds_mn = ptx::smem_desc_sw128(sbase + L::kOffDs, kChunk, 1024);
+    const uint64_t q_k = ptx::smem_desc_sw128(sbase + L::kOffQ, 16, 1024), q_mn = ptx::smem_desc_sw128(sbase + L::kOffQ, kChunk, 1024);
+    constexpr uint32_t kStage = (2 * L::kTileBytes) >> 4, kOfG = L::kTileBytes >> 4;
+    // contraction over head_dim: both operands K-major, [128 rows][64] chunks
+    auto nt = [&](uint32_t d, uint64_t da, uint64_t db, uint32_t boff, int n16) {
+      const uint32_t idesc = ptx::idesc_bf16(kTile, 0, 0, 0) | ((uint32_t)n16 << 18);
+#pragma unroll
+      for (int ks = 0; ks < HD / 16; ++ks) {
+        const uint32_t off = (uint32_t)(ks >> 2) * (kChunk >> 4) + (uint32_t)(ks & 3) * 2;
+        ptx::mma_ss_lohi(d, (uint32_t)da + off, (uint32_t)(da >> 32), (uint32_t)db + boff + off, (uint32_t)(db >> 32), idesc, ks > 0);
+      }
+    };
+    for (;;) {
+      const int idx = next_item();
+      if (idx < 0) break;
+      const Item it = decode(a, idx);
+      for (int kt = 0; kt < it.n_kt; ++kt, ++kts) {
+        const RowList rows = rows_of(a, it, kt);
+        const int keys16 = (min(kTile, it.l0 + it.len - kt * kTile) + 15) >> 4;
+        wait(kKvFull, kts, 62);
+        auto issue_s = [&](uint32_t no, int i) {  // S^T of row tile i (tile number no)
+          const RowTile t = row_tile(a, it, rows, i);
+          wait(kQFull + (no & 1u), no >> 1, 63);
+          if (t.nrow < kTile) wait(kTail, tails++, 64);
+          ptx::tc_fence_after_sync();
+          if (leader) {
+            nt(tmem + kColS, k_k, q_k, (no & 1u) * kStage, (t.nrow + 15) >> 4);
+            ptx::mma_commit(bar(kSFull));
+          }
+        };
+        for (int i = 0; i < rows.n; ++i, ++tile) {
+          const RowTile t = row_tile(a, it, rows, i);
+          const uint32_t so = (tile & 1u) * kStage;
+          const int r16 = (t.nrow + 15) >> 4;
+          if (i == 0) issue_s(tile, 0);
+          if (tile > 0) wait(kDqFree, tile - 1, 65);  // dQ of the previous tile has left these columns
+          ptx::tc_fence_after_sync();
+          if (leader) {
+            nt(tmem + kColDp, v_k, q_k, so + kOfG, r16);
+            ptx::mma_commit(bar(kDpFull));
+          }
+          wait(kPFull, tile, 66);
+          ptx::tc_fence_after_sync();
+          if (leader) {  // dV += P^T dO: each warp group wrote its 64 columns of P over the first half of its columns of S
+            for (int ks = 0; ks < r16; ++ks)
+              ptx::mma_ts_lohi(tmem + kColDv, tmem + kColS + (uint32_t)(ks >> 2) * 64 + (uint32_t)(ks & 3) * 8,
+                               (uint32_t)q_mn + so + kOfG + (uint32_t)ks * 128, (uint32_t)(q_mn >> 32), id_dkv, (i > 0 || ks > 0) ? 1u : 0u);
+          }
+          __syncwarp();
+          if (i + 1 < rows.n) issue_s(tile + 1, i + 1);  // (behind dV, which reads P out of the same columns)
+          wait(kDsFull, tile, 67);
+          ptx::tc_fence_after_sync();
+          if (leader) {
+            for (int ks = 0; ks < r16; ++ks)
+              ptx::mma_ss_lohi(tmem + kColDk, (uint32_t)ds_k + (uint32_t)(ks >> 2) * (kChunk >> 4) + (uint32_t)(ks & 3) * 2,
+                               (uint32_t)(ds_k >> 32), (uint32_t)q_mn + so + (uint32_t)ks * 128, (uint32_t)(q_mn >> 32), id_dkv,
+                               (i > 0 || ks > 0) ? 1u : 0u);
+            ptx::mma_commit(bar(kQFree + (tile & 1u)));
+            for (int ks = 0; ks < keys16; ++ks)
+              ptx::mma_ss_lohi(tmem + kColDp, (uint32_t)ds_mn + (uint32_t)ks * 128, (uint32_t)(ds_mn >> 32),
+                               (uint32_t)k_mn + (uint32_t)ks * 128, (uint32_t)(k_mn >> 32), id_dq, ks > 0);
+            ptx::mma_commit(bar(kDqFull));
+            if (i + 1 == rows.n) ptx::mma_commit(bar(kAccFull));
+          }
+          __syncwarp();
+        }
+      }
+    }
+  } else {
+    // =============================== element-wise part, loads of K / V, outputs ===================
+    const int wg = warp >> 2, row = tid & 127;
+    const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    uint32_t tile = 0, kts = 0;
+    constexpr int kHalf = HD / 2;  // columns of dQ a thread drains
+    auto arrive = [&](int i) {
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(bar(i));
+    };
+
+    // K and V of list positions [128 kt, 128 kt + 128) -> shared memory, zero beyond the list
+    auto load_kv = [&](const Item& it, int kt) {
+      constexpr int kPieces = HD / 8;
+      const __nv_bfloat16* kb = reinterpret_cast<const __nv_bfloat16*>(a.k.ptr) + (int64_t)it.b * a.k.sb + (int64_t)it.g * a.k.sh;
+      const __nv_bfloat16* vb = reinterpret_cast<const __nv_bfloat16*>(a.v.ptr) + (int64_t)it.b * a.v.sb + (int64_t)it.g * a.v.sh;
+#pragma unroll 4
+      for (int i = tid; i < kTile * kPieces; i += kComputeThreads) {
+        const int r = i / kPieces, c = i % kPieces, j = kt * kTile + r;
+        const bool ok = j < it.l0 + it.len;
+        const int slot = !ok ? it.start : j < it.l0 ? it.s0 + j : it.start + j - it.l0;
+        const uint32_t off = (uint32_t)(c >> 3) * kChunk + (uint32_t)r * 128u + (uint32_t)(((c & 7) ^ (r & 7)) << 4);
+        cp_async16_zfill(smem + L::kOffK + off, kb + (int64_t)slot * a.k.ss + c * 8, ok);
+        cp_async16_zfill(smem + L::kOffV + off, vb + (int64_t)slot * a.v.ss + c * 8, ok);
+      }
+      cp_async_commit();
+    };
+
+    // dV (warps 0-3) or dK (warps 4-7) of one key tile: thread = key
+    auto drain_acc = [&](const Item& it, int kt) {
+      const int j = kt * kTile + row;
+      const bool valid = j < it.l0 + it.len;
+      const float f = wg ? a.scale : 1.f;
+      const bool prefix = a.pre != nullptr && (it.m == 0 || j < it.l0);
+      const View& out = wg ? a.dk : a.dv;
+      float* const acc = a.pre + ((size_t)(wg ? 0 : 1) * a.B * a.Nk + (size_t)it.b * a.Nk + it.g) * a.max_block_len * HD + (size_t)j * HD;
+      __nv_bfloat16* const dst = reinterpret_cast<__nv_bfloat16*>(out.ptr) + (int64_t)it.b * out.sb + (int64_t)it.g * out.sh +
+                                 (int64_t)(it.start + j - it.l0) * out.ss;
+#pragma unroll 1
+      for (int c0 = 0; c0 < HD; c0 += 32) {
+        uint32_t x[32];
+        __syncwarp();
+        ptx::tmem_ld32(lanes + (wg ? kColDk : kColDv) + (uint32_t)c0, x);
+        ptx::tmem_wait_ld(x);
+        if (!valid) continue;
+        if (prefix) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            red4(acc + c0 + i, __uint_as_float(x[i]) * f, __uint_as_float(x[i + 1]) * f, __uint_as_float(x[i + 2]) * f,
+                 __uint_as_float(x[i + 3]) * f);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; i += 8)
+            *reinterpret_cast<uint4*>(dst + c0 + i) =
+                make_uint4(pack_bf16(__uint_as_float(x[i]) * f, __uint_as_float(x[i + 1]) * f),
+                           pack_bf16(__uint_as_float(x[i + 2]) * f, __uint_as_float(x[i + 3]) * f),
+                           pack_bf16(__uint_as_float(x[i + 4]) * f, __uint_as_float(x[i + 5]) * f),
+                           pack_bf16(__uint_as_float(x[i + 6]) * f, __uint_as_float(x[i + 7]) * f));
+        }
+      }
+    };
+
+    // dQ of one (key tile, row tile) pair: thread = row, columns [wg HD / 2, + HD / 2)
+    auto drain_dq = [&](const Item& it, int kt, const RowTile& t) {
+      const int tok = t.t0 + (row >> a.g_shift), head = it.g * a.G + (row & (a.G - 1));
+      const bool valid = row < t.nrow;
+      const bool sum32 = a.M > 1 && (!t.own || it.m == a.M - 1);  // rows of the query block
+      // own rows: the key tiles that see this row tile are 0 .. last
+      const int last = t.own ? (it.l0 + min(it.len, t.t0 + (kTile >> a.g_shift)) - 1) / kTile : 0;
+      float* const d32 = a.dq32 + (((size_t)it.b * a.N + head) * a.max_block_len + tok) * HD + wg * kHalf;
+      float4* const part = reinterpret_cast<float4*>(a.part) +
+                           ((size_t)blockIdx.x * a.row_tiles + t.r) * (HD / 8) * kComputeThreads + tid;
+      __nv_bfloat16* const dst = reinterpret_cast<__nv_bfloat16*>(a.dq.ptr) + (int64_t)it.b * a.dq.sb + (int64_t)head * a.dq.sh +
+                                 (int64_t)(it.start + tok) * a.dq.ss + wg * kHalf;
+      const float f = a.scale;
+#pragma unroll 1
+      for (int c0 = 0; c0 < kHalf; c0 += 32) {
+        uint32_t x[32];
+        __syncwarp();
+        ptx::tmem_ld32(lanes + kColDp + (uint32_t)(wg * kHalf + c0), x);
+        ptx::tmem_wait_ld(x);
+        if (c0 + 32 >= kHalf) {  // out of tensor memory: the next tile's dP may overwrite it
+          ptx::tc_fence_before_sync();
+          arrive(kDqFree);
+        }
+        if (!valid) continue;
+        if (sum32) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            red4(d32 + c0 + i, __uint_as_float(x[i]) * f, __uint_as_float(x[i + 1]) * f, __uint_as_float(x[i + 2]) * f,
+                 __uint_as_float(x[i + 3]) * f);
+          continue;
+        }
+        if (kt > 0) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float4 y = part[(size_t)(c0 / 4 + i) * kComputeThreads];
+            x[4 * i] = __float_as_uint(__uint_as_float(x[4 * i]) + y.x);
+            x[4 * i + 1] = __float_as_uint(__uint_as_float(x[4 * i + 1]) + y.y);
+            x[4 * i + 2] = __float_as_uint(__uint_as_float(x[4 * i + 2]) + y.z);
+            x[4 * i + 3] = __float_as_uint(__uint_as_float(x[4 * i + 3]) + y.w);
+          }
+        }
+        if (kt < last) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            part[(size_t)(c0 / 4 + i) * kComputeThreads] =
+                make_float4(__uint_as_float(x[4 * i]), __uint_as_float(x[4 * i + 1]), __uint_as_float(x[4 * i + 2]),
+                            __uint_as_float(x[4 * i + 3]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; i += 8)
+            *reinterpret_cast<uint4*>(dst + c0 + i) =
+                make_uint4(pack_bf16(__uint_as_float(x[i]) * f, __uint_as_float(x[i + 1]) * f),
+                           pack_bf16(__uint_as_float(x[i + 2]) * f, __uint_as_float(x[i + 3]) * f),
+                           pack_bf16(__uint_as_float(x[i + 4]) * f, __uint_as_float(x[i + 5]) * f),
+                           pack_bf16(__uint_as_float(x[i + 6]) * f, __uint_as_float(x[i + 7]) * f));
+        }
+      }
+    };
+
+    Item prev{};
+    int prev_kt = -1;
+    for (;;) {
+      const int idx = next_item();
+      if (idx < 0) break;
+      const Item it = decode(a, idx);
+      for (int kt = 0; kt < it.n_kt; ++kt, ++kts) {
+        if (prev_kt >= 0) wait(kAccFull, kts - 1, 70);  // every product of the previous key tile is complete
+        load_kv(it, kt);
+        if (prev_kt >= 0) {
+          ptx::tc_fence_after_sync();
+          drain_acc(prev, prev_kt);
+          ptx::tc_fence_before_sync();
+        }
+        prev = it;
+        prev_kt = kt;
+        cp_async_wait<0>();
+        ptx::fence_proxy_async_smem();
+        arrive(kKvFull);
+        const RowList rows = rows_of(a, it, kt);
+        const int j = kt * kTile + row;  // this thread's key: list position
+        for (int i = 0; i < rows.n; ++i, ++tile) {
+          const RowTile t = row_tile(a, it, rows, i);
+          const uint32_t st = tile & 1u;
+          wait(kQFull + st, tile >> 1, 71);
+          if (t.nrow < kTile) {  // rows beyond the block hold other tokens: zero them, whatever they are
+            const int per = kTile - t.nrow;
+#pragma unroll
+            for (int c = 0; c < 2 * (HD / 64); ++c) {
+              uint4* const z = reinterpret_cast<uint4*>(smem + L::kOffQ + st * 2 * L::kTileBytes + c * kChunk) + t.nrow * 8;
+              for (int x = tid; x < per * 8; x += kComputeThreads) z[x] = make_uint4(0, 0, 0, 0);
+            }
+            ptx::fence_proxy_async_smem();
+            arrive(kTail);
+          }
+          const float* const col = reinterpret_cast<const float*>(smem + L::kOffCol) + st * 2 * kTile + wg * 64;
+          // Row-tile columns below cmin do not see this key: causality inside the block; the prefix is not the query
+          // rows' business here; positions beyond the list are no keys.
+          int cmin = t.own ? (j - it.l0 - t.t0) * a.G : (j < it.l0 ? kTile : 0);
+          if (j >= it.l0 + it.len) cmin = kTile;
+          cmin -= wg * 64;
+
+          wait(kSFull, tile, 72);
+          ptx::tc_fence_after_sync();
+          __syncwarp();
+          float p[64];
+          {
+            uint32_t s[64];
+            ptx::tmem_ld32(lanes + kColS + (uint32_t)wg * 64, *reinterpret_cast<uint32_t (*)[32]>(&s[0]));
+            ptx::tmem_ld32(lanes + kColS + (uint32_t)wg * 64 + 32, *reinterpret_cast<uint32_t (*)[32]>(&s[32]));
+            ptx::tmem_wait_ld(s);
+#pragma unroll
+            for (int c = 0; c < 64; c += 4) {
+              const float4 nl = *reinterpret_cast<const float4*>(col + c);
+              p[c] = ptx::ex2(fmaf(__uint_as_float(s[c]), a.scale_log2, nl.x));
+              p[c + 1] = ptx::ex2(fmaf(__uint_as_float(s[c + 1]), a.scale_log2, nl.y));
+              p[c + 2] = ptx::ex2(fmaf(__uint_as_float(s[c + 2]), a.scale_log2, nl.z));
+              p[c + 3] = ptx::ex2(fmaf(__uint_as_float(s[c + 3]), a.scale_log2, nl.w));
+            }
+          }
+          if (__any_sync(0xffffffffu, cmin > 0)) {
+#pragma unroll
+            for (int c = 0; c < 64; ++c) p[c] = c < cmin ? 0.f : p[c];
+          }
+          {
+            uint32_t pk[32];
+#pragma unroll
+            for (int c = 0; c < 32; ++c) pk[c] = pack_bf16(p[2 * c], p[2 * c + 1]);
+            ptx::tmem_st32(lanes + kColS + (uint32_t)wg * 64, pk);
+            ptx::tmem_wait_st();
+          }
+          ptx::tc_fence_before_sync();
+          arrive(kPFull);
+
+          if (i > 0) {
+            wait(kDqFull, tile - 1, 73);
+            ptx::tc_fence_after_sync();
+            drain_dq(it, kt, row_tile(a, it, rows, i - 1));
+          }
+          wait(kDpFull, tile, 74);
+          ptx::tc_fence_after_sync();
+          __syncwarp();
+          uint8_t* const ds_row = smem + L::kOffDs + wg * kChunk + row * 128;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t x[32];
+            ptx::tmem_ld32(lanes + kColDp + (uint32_t)(wg * 64 + h * 32), x);
+            ptx::tmem_wait_ld(x);
+#pragma unroll
+            for (int c = 0; c < 32; c += 8) {
+              const float4 d0 = *reinterpret_cast<const float4*>(col + kTile + h * 32 + c);
+              const float4 d1 = *reinterpret_cast<const float4*>(col + kTile + h * 32 + c + 4);
+              const float* pp = &p[h * 32 + c];
+              uint4 w;
+              w.x = pack_bf16(pp[0] * (__uint_as_float(x[c]) - d0.x), pp[1] * (__uint_as_float(x[c + 1]) - d0.y));
+              w.y = pack_bf16(pp[2] * (__uint_as_float(x[c + 2]) - d0.z), pp[3] * (__uint_as_float(x[c + 3]) - d0.w));
+              w.z = pack_bf16(pp[4] * (__uint_as_float(x[c + 4]) - d1.x), pp[5] * (__uint_as_float(x[c + 5]) - d1.y));
+              w.w = pack_bf16(pp[6] * (__uint_as_float(x[c + 6]) - d1.z), pp[7] * (__uint_as_float(x[c + 7]) - d1.w));
+              *reinterpret_cast<uint4*>(ds_row + (((h * 4 + (c >> 3)) ^ (row & 7)) << 4)) = w;
+            }
+          }
+          ptx::fence_proxy_async_smem();
+          ptx::tc_fence_before_sync();
+          arrive(kDsFull);
+        }
+        wait(kDqFull, tile - 1, 73);
+        ptx::tc_fence_after_sync();
+        drain_dq(it, kt, row_tile(a, it, rows, rows.n - 1));
+      }
+    }
+    if (prev_kt >= 0) {
+      wait(kAccFull, kts - 1, 75);
+      ptx::tc_fence_after_sync();
+      drain_acc(prev, prev_kt);
+    }
+  }
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 0) ptx::tmem_dealloc(tmem, 512);
+}
+
+__device__ __forceinline__ bool slot_in_block(const BwdTcArgs& a, int b, int s) {
+  int lo = 0, hi = a.M;  // first block that starts behind s (blk_start is non-decreasing)
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (a.blk_start[(size_t)b * a.M + mid] <= s) lo = mid + 1; else hi = mid;
+  }
+  if (lo == 0) return false;
+  int start, len;
+  span_of(a, b, lo - 1, start, len);
+  return s < start + len;
+}
+
+// delta = rowsum(dO * O): one warp per 32 slots of one (prompt, head), HD / 8 lanes per row.  The same warps write the
+// zeros of the slots outside every block; all threads clear the accumulators and the item counter.  Bound by memory:
+// reads O and dO once.
+template <int HD>
+__global__ void __launch_bounds__(256) attn_bwd_tc_prep_kernel(BwdTcArgs a, float4* zero, int64_t n_zero) {
+  const int64_t gid = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  for (int64_t i = gid; i < n_zero; i += (int64_t)gridDim.x * 256) zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (gid == 0) *a.counter = 0;
+  const int lane = threadIdx.x & 31;
+  const int groups = (a.S + 31) / 32;
+  const int64_t w = gid >> 5;
+  if (w >= (int64_t)a.B * groups * a.N) return;
+  const int n = (int)(w % a.N), grp = (int)((w / a.N) % groups), b = (int)(w / ((int64_t)a.N * groups));
+  const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(a.d_o.ptr) + (int64_t)b * a.d_o.sb + (int64_t)n * a.d_o.sh;
+  const __nv_bfloat16* op = reinterpret_cast<const __nv_bfloat16*>(a.o.ptr) + (int64_t)b * a.o.sb + (int64_t)n * a.o.sh;
+  constexpr int kLanes = HD / 8, kRows = 32 / kLanes;  // lanes per row, rows per pass
+  const int sub = lane / kLanes, c = (lane % kLanes) * 8;
+  float mine = 0.f;
+#pragma unroll 4
+  for (int r = 0; r < 32; r += kRows) {
+    const int s = grp * 32 + r + sub;
+    float d = 0.f;
+    if (s < a.S) {
+      float x[8], y[8];
+      load8(gp + (int64_t)s * a.d_o.ss + c, x);
+      load8(op + (int64_t)s * a.o.ss + c, y);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) d = fmaf(x[i], y[i], d);
+    }
+#pragma unroll
+    for (int off = kLanes / 2; off > 0; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+      const float v = __shfl_sync(0xffffffffu, d, k * kLanes);
+      if (lane == r + k) mine = v;
+    }
+  }
+  const int s = grp * 32 + lane;
+  if (s < a.S) a.delta[((size_t)b * a.N + n) * a.S + s] = mine;
+  unsigned gap = __ballot_sync(0xffffffffu, s < a.S && !slot_in_block(a, b, s));
+  for (; gap; gap &= gap - 1) {
+    const int z = grp * 32 + __ffs((int)gap) - 1;
+    auto clear = [&](const View& t) {
+      __nv_bfloat16* p = reinterpret_cast<__nv_bfloat16*>(t.ptr) + (int64_t)b * t.sb + (int64_t)n * t.sh + (int64_t)z * t.ss;
+      if (lane < kLanes) *reinterpret_cast<uint4*>(p + lane * 8) = make_uint4(0, 0, 0, 0);
+    };
+    clear(a.dq);
+    if (n < a.Nk) {
+      clear(a.dk);
+      clear(a.dv);
+    }
+  }
+}
+
+// fp32 sums -> bf16: dQ of the last block's rows, dK and dV of the prefix.  One thread per 8 elements.
+template <int HD>
+__global__ void __launch_bounds__(256) attn_bwd_tc_finish_kernel(BwdTcArgs a) {
+  const int64_t nq = (int64_t)a.B * a.N * a.max_block_len * (HD / 8), np = a.pre ? (int64_t)a.B * a.Nk * a.max_block_len * (HD / 8) : 0;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < nq + 2 * np; i += (int64_t)gridDim.x * 256) {
+    const bool q = i < nq;
+    const int64_t x = q ? i : (i - nq) % np;
+    const bool dv = !q && i - nq >= np;
+    const int heads = q ? a.N : a.Nk;
+    const int c = (int)(x % (HD / 8)) * 8, tok = (int)(x / (HD / 8) % a.max_block_len);
+    const int64_t bh = x / ((int64_t)(HD / 8) * a.max_block_len);
+    const int h = (int)(bh % heads), b = (int)(bh / heads);
+    int start, len;
+    span_of(a, b, q ? a.M - 1 : 0, start, len);
+    if (tok >= len) continue;
+    float v[8];
+    load8((q ? a.dq32 : a.pre + (dv ? np * 8 : 0)) + x * 8, v);
+    const View& t = q ? a.dq : dv ? a.dv : a.dk;
+    store8(reinterpret_cast<__nv_bfloat16*>(t.ptr) + (int64_t)b * t.sb + (int64_t)h * t.sh + (int64_t)(start + tok) * t.ss + c, v);
+  }
+}
+
+int row_tiles(const brk_attn_bwd_params& p) { return (p.max_block_len * (p.N / p.Nk) + kTile - 1) / kTile; }
+// Rows whose keys can span several key tiles need the fp32 dQ scratch.
+bool needs_part(const brk_attn_bwd_params& p) { return (int64_t)(p.M > 2 ? 2 : 1) * p.max_block_len > kTile; }
+size_t part_bytes(const brk_attn_bwd_params& p) {
+  return needs_part(p) ? (size_t)std::max(1, sm_count()) * row_tiles(p) * kTile * p.D * sizeof(float) : 0;
+}
+
+template <int HD>
+int launch(const brk_attn_bwd_params& p, BwdTcArgs a, float4* zero, int64_t n_zero, cudaStream_t st) {
+  const int tok = kTile / a.G;
+  CUtensorMap tq, tg;
+  int rc;
+  if ((rc = make_tmap_bf16(&tq, p.q.ptr, HD, p.N, p.S, p.B, p.q.stride_h, p.q.stride_s, p.q.stride_b, a.G, tok))) return rc;
+  if ((rc = make_tmap_bf16(&tg, p.d_o.ptr, HD, p.N, p.S, p.B, p.d_o.stride_h, p.d_o.stride_s, p.d_o.stride_b, a.G, tok))) return rc;
+  const int64_t warps = (int64_t)p.B * ((p.S + 31) / 32) * p.N;
+  attn_bwd_tc_prep_kernel<HD><<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(a, zero, n_zero);
+  BRK_CUDA(cudaGetLastError());
+  BRK_CUDA(cudaFuncSetAttribute(attn_bwd_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Geo<HD>::kSmem));
+  const int sms = sm_count();
+  BRK_REQUIRE(sms > 0, BRK_E_CUDA, "could not read the SM count");
+  attn_bwd_tc_kernel<HD><<<std::min(sms, a.total_items), kThreads, Geo<HD>::kSmem, st>>>(tq, tg, a);
+  BRK_CUDA(cudaGetLastError());
+  if (p.M > 1) {
+    const int64_t n = (int64_t)p.B * (p.N + (a.pre ? 2 * p.Nk : 0)) * p.max_block_len * (HD / 8);
+    attn_bwd_tc_finish_kernel<HD><<<(unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8), 256, 0, st>>>(a);
+    BRK_CUDA(cudaGetLastError());
+  }
+  return BRK_OK;
+}
+
+}  // namespace
+
+// bf16 with a group size that divides a row tile, and blocks short enough for the dQ scratch of a CTA (512 tokens at four
+// heads per KV head).  Longer blocks go to the warp-level kernels, which split a block over CTAs.
+bool attn_bwd_tc_supported(const brk_attn_bwd_params& p) {
+  const int G = p.Nk > 0 ? p.N / p.Nk : 0;
+  return p.dtype == BRK_BF16 && (p.D == 64 || p.D == 128) && (G == 1 || G == 2 || G == 4 || G == 8) && row_tiles(p) <= kMaxRowTiles;
+}
+size_t attn_bwd_tc_extra_bytes(const brk_attn_bwd_params& p) { return p.M > 2 || part_bytes(p) > 0 ? 256 + part_bytes(p) : 0; }
+
+// ws32: the two [B, Nk, S, D] accumulators of the warp-level kernels (used for the prefix sums here), then dq32; extra: the
+// bytes of attn_bwd_tc_extra_bytes (the item counter goes into the unused accumulators when there are none)
+int attn_bwd_tc_launch(const brk_attn_bwd_params& p, float* delta, float* ws32, float* dq32, void* extra, cudaStream_t st) {
+  BwdTcArgs a{};
+  a.q = make_view(p.q); a.k = make_view(p.k); a.v = make_view(p.v); a.o = make_view(p.o); a.d_o = make_view(p.d_o);
+  a.dq = make_view(p.dq); a.dk = make_view(p.dk); a.dv = make_view(p.dv);
+  a.lse = p.lse;
+  a.delta = delta;
+  a.blk_start = p.blk_start; a.blk_len = p.blk_len;
+  a.status = p.status;
+  a.B = p.B; a.N = p.N; a.Nk = p.Nk; a.S = p.S; a.M = p.M; a.G = p.N / p.Nk; a.max_block_len = p.max_block_len;
+  while ((1 << a.g_shift) < a.G) ++a.g_shift;
+  a.row_tiles = row_tiles(p);
+  BRK_REQUIRE((int64_t)p.B * p.Nk * p.M < (1ll << 31), BRK_E_UNSUPPORTED, "too many work items");
+  a.total_items = p.B * p.Nk * p.M;
+  a.scale = p.scale;
+  a.scale_log2 = p.scale * 1.4426950408889634f;
+  // With two blocks or fewer no document adds to the prefix's dK / dV: block 0's own item stores them.
+  const int64_t n_pre = p.M > 2 ? 2ll * p.B * p.Nk * p.max_block_len * p.D : 0, n_q = p.M > 1 ? (int64_t)p.B * p.N * p.max_block_len * p.D : 0;
+  // The prefix sums sit at the end of the accumulators, directly in front of dq32: one range to clear.
+  a.pre = n_pre ? dq32 - n_pre : nullptr;
+  a.dq32 = dq32;
+  unsigned char* const x = static_cast<unsigned char*>(extra);
+  const bool has_extra = attn_bwd_tc_extra_bytes(p) > 0;
+  a.counter = has_extra ? reinterpret_cast<int*>(x) : reinterpret_cast<int*>(ws32);
+  a.part = part_bytes(p) ? reinterpret_cast<float*>(x + 256) : nullptr;
+  float4* const zero = reinterpret_cast<float4*>(dq32 - n_pre);
+  return p.D == 128 ? launch<128>(p, a, zero, (n_pre + n_q) / 4, st) : launch<64>(p, a, zero, (n_pre + n_q) / 4, st);
+}
+
+}  // namespace brk

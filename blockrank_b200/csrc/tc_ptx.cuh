@@ -28,7 +28,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 }
 // Bounded wait on a phase parity. Returns false if the budget ran out.  Out of line: the kernels wait in
 // dozens of places and an inlined copy of the loop at each of them is pure instruction-cache pressure.
-__device__ __noinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t budget = (1u << 22)) {
+static __device__ __noinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t budget = (1u << 22)) {
   for (uint32_t it = 0; it < budget; ++it) {
     uint32_t done;
     asm volatile(
@@ -41,6 +41,19 @@ __device__ __noinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t b
     if (done) return true;
   }
   return false;
+}
+
+// One suspending attempt (the hardware bounds it), for waits written in line.
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
 }
 
 // Non-blocking test of a phase parity.

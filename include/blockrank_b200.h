@@ -126,7 +126,7 @@ BRK_API int brk_attn_fwd(const brk_attn_params* p, void* workspace, size_t works
  * auxiliary-loss trainer (src/blockrank/trainer.py:51-107).
  * Inputs are the forward's q, k, v, its output o and its lse ([B, N, S], natural log) and the gradient d_o of o
  * (same layout as o).  Outputs dq (like q), dk and dv (like k, v; summed over the query heads of each KV group);
- * slots outside every block get zero gradients.  bf16: warp-level tensor-core MMA (fp32 accumulation);
+ * slots outside every block get zero gradients.  bf16: tcgen05 (fp32 accumulation; warp-level MMA for blocks of more than 16 row tiles of 128 / (N / Nk) tokens);
  * fp32: CUDA cores (there N / Nk must divide 64). */
 typedef struct brk_attn_bwd_params {
   int32_t dtype;          /* BRK_BF16 or BRK_F32 (q, k, v, o, d_o, dq, dk, dv share it) */
@@ -138,6 +138,7 @@ typedef struct brk_attn_bwd_params {
   const int32_t* blk_start;
   const int32_t* blk_len;
   brk_view dq, dk, dv;    /* written through their strides; dk, dv: (B, Nk, S, D) views */
+  int32_t* status;        /* optional device word (bf16: a bounded wait that gave up); see brk_status_poll */
 } brk_attn_bwd_params;
 
 /* fp32 scratch: the rows' dot(d_o, o), the dk / dv accumulators and (bf16) the last block's dq; cleared by the call */

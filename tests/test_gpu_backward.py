@@ -128,6 +128,22 @@ def test_attention_backward_bf16(name, lens, H, N, Nk, D):
             assert t.float().cpu().permute(0, 2, 1, 3)[pad].abs().max() == 0
 
 
+TC_EDGES = [  # name, block lengths per prompt, H, N, Nk, D: tile edges of the tcgen05 backward and every group size
+    ("keys_end_on_a_tile", [[64, 64, 192, 128, 32], [128, 1, 0, 127, 129]], 192, 4, 1, 128),
+    ("prefix_fills_a_tile", [[130, 126, 3, 250, 70]], 256, 4, 1, 128),
+    ("empty_prefix_and_query", [[0, 33, 90, 40, 0]], 96, 4, 1, 64),
+    ("group_8", [[17, 100, 45, 16, 31]], 104, 8, 1, 64),
+    ("group_1", [[40, 129, 200, 5, 60]], 200, 2, 2, 64),
+    ("two_long_blocks", [[200, 150]], 200, 4, 2, 128),
+    ("longer_than_the_scratch", [[30, 600, 40]], 600, 4, 1, 64),  # more than 16 row tiles: the warp-level kernels
+]
+
+
+@pytest.mark.parametrize("name,lens,H,N,Nk,D", TC_EDGES, ids=[c[0] for c in TC_EDGES])
+def test_attention_backward_bf16_tile_edges(name, lens, H, N, Nk, D):
+    test_attention_backward_bf16(name, lens, H, N, Nk, D)
+
+
 def test_registered_function_trains_attention_and_raw_scores():
     """The registered attention function under autograd: gradients of a loss over the attention output and
     the raw last-rows scores (what compute_auxiliary_attention_loss consumes) match fp64 autograd."""
