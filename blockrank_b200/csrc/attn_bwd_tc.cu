@@ -262,7 +262,6 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
   } else if (warp == 8) {
     // =============================== MMA issue ===================================================
-    const bool leader = lane == 0;
     uint32_t tile = 0, kts = 0, tails = 0;
     const uint32_t id_dkv = ptx::idesc_bf16(kTile, HD, 0, 1);  // dV, dK: A K-major, B (dO / Q) MN-major
     const uint32_t id_dq = ptx::idesc_bf16(kTile, HD, 1, 1);   // dQ: A (dS) and B (K) MN-major
@@ -293,7 +292,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           wait(kQFull + (no & 1u), no >> 1, 63);
           if (t.nrow < kTile) wait(kTail, tails++, 64);
           ptx::tc_fence_after_sync();
-          if (leader) {
+          if (ptx::elect_one()) {
             nt(tmem + kColS, k_k, q_k, (no & 1u) * kStage, (t.nrow + 15) >> 4);
             ptx::mma_commit(bar(kSFull));
           }
@@ -305,13 +304,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           if (i == 0) issue_s(tile, 0);
           if (tile > 0) wait(kDqFree, tile - 1, 65);  // dQ of the previous tile has left these columns
           ptx::tc_fence_after_sync();
-          if (leader) {
+          if (ptx::elect_one()) {
             nt(tmem + kColDp, v_k, q_k, so + kOfG, r16);
             ptx::mma_commit(bar(kDpFull));
           }
           wait(kPFull, tile, 66);
           ptx::tc_fence_after_sync();
-          if (leader) {  // dV += P^T dO: each warp group wrote its 64 columns of P over the first half of its columns of S
+          if (ptx::elect_one()) {  // dV += P^T dO: each warp group wrote its 64 columns of P over the first half of its columns of S
             for (int ks = 0; ks < r16; ++ks)
               ptx::mma_ts_lohi(tmem + kColDv, tmem + kColS + (uint32_t)(ks >> 2) * 64 + (uint32_t)(ks & 3) * 8,
                                (uint32_t)q_mn + so + kOfG + (uint32_t)ks * 128, (uint32_t)(q_mn >> 32), id_dkv, (i > 0 || ks > 0) ? 1u : 0u);
@@ -320,7 +319,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           if (i + 1 < rows.n) issue_s(tile + 1, i + 1);  // (behind dV, which reads P out of the same columns)
           wait(kDsFull, tile, 67);
           ptx::tc_fence_after_sync();
-          if (leader) {
+          if (ptx::elect_one()) {
             for (int ks = 0; ks < r16; ++ks)
               ptx::mma_ss_lohi(tmem + kColDk, (uint32_t)ds_k + (uint32_t)(ks >> 2) * (kChunk >> 4) + (uint32_t)(ks & 3) * 2,
                                (uint32_t)(ds_k >> 32), (uint32_t)q_mn + so + (uint32_t)ks * 128, (uint32_t)(q_mn >> 32), id_dkv,

@@ -667,7 +667,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // MMAs of the thread that executes it).  The two chains' issuers never wait for each other;
     // they only meet in the kKVFree barriers (two arrivals hand a slot back to the TMA warp).
     const int x = warp - 9;
-    const bool leader = lane == 0;
     uint32_t q_uses = 0, p_seen = 0, jobs_done = 0;
     uint32_t full_par = 0;  // bit s: parity of the next kKVFull+s phase this warp has not consumed yet
     int blk_waited = 0;     // resident block: slots [0, blk_waited) have landed
@@ -688,7 +687,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       const uint32_t idesc = idesc_qk0 | ((uint32_t)((keys + 15) >> 4) << 18);  // N/8 at bit 17, N a multiple of 16
       const uint32_t a_lo = (uint32_t)q_desc0, a_hi = (uint32_t)(q_desc0 >> 32);
       const uint32_t b_lo = (uint32_t)k_desc0 + (uint32_t)slot * (kSlotHalf >> 4), b_hi = (uint32_t)(k_desc0 >> 32);
-      if (leader) {
+      if (ptx::elect_one()) {
 #pragma unroll 1
         for (int ks = 0; ks < HD / 16; ++ks) {
           const uint32_t aoff = (uint32_t)(ks >> 2) * ((BM * 128) >> 4) + (uint32_t)(ks & 3) * 2;
@@ -703,7 +702,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     auto issue_pv = [&](int slot, int keys, bool first) {
       const uint32_t b_lo = (uint32_t)v_desc0 + (uint32_t)slot * (kSlotHalf >> 4), b_hi = (uint32_t)(v_desc0 >> 32);
       const int ksteps = (keys + 15) >> 4;
-      if (leader) {
+      if (ptx::elect_one()) {
 #pragma unroll 1
         for (int ks = 0; ks < BT / 16; ++ks)
           if (ks < ksteps)
@@ -729,7 +728,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     uint32_t q_issued = 0;
     auto request_q = [&](const Job& jb) {
       if (q_issued > 0) wait(kQFree + x, q_issued - 1, 28 + x);  // every Q K^T of the previous job has read the buffer
-      if (leader) {
+      if (ptx::elect_one()) {
         const uint32_t dst = sbase + kOffQ + (uint32_t)x * kQBytes;
         ptx::mbar_expect_tx(bar(kQFull + x), kQBytes);
         ptx::tma_load_4d(dst, &tmQ, bar(kQFull + x), 0, jb.g * G, jb.start + jb.t0, jb.b);
@@ -813,7 +812,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         const int rel_lo = it.aux & 0xff, rel_hi = (it.aux >> 8) & 0xff;
         ensure(rel_hi);
         for (int s = rel_lo; s < rel_hi; ++s)
-          if (leader) ptx::mma_commit(bar(kKVFree + s));
+          if (ptx::elect_one()) ptx::mma_commit(bar(kKVFree + s));
       } else {
         // ---- streamed pair: tile t sits in ring position (tile0 + t) & 1 = pool slots 0-1 or 2-3 ----
         const int Ti = it.aux;  // tiles of the item; this chain computes on the first T of them
@@ -838,12 +837,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             if (t == 0 && jobs_done > 0) wait(kOFree + x, jobs_done - 1, 26 + x);
               ptx::tc_fence_after_sync();
             issue_pv(slot, keys_of(t), t == 0);
-            if (leader) ptx::mma_commit(bar(kKVFree + slot));
+            if (ptx::elect_one()) ptx::mma_commit(bar(kKVFree + slot));
             if (t + 1 < T) issue_qk(2 * ((it.tile0 + t + 1) & 1), keys_of(t + 1), t + 2 == T);
               if (t + 2 == T) request_next_q(job_no);  // the job's last Q K^T is in the pipe
           } else {
             need_kv(t);  // not visible to this chain: consume the phase, then hand the tile back
-            if (leader) ptx::mma_commit(bar(kKVFree + slot));
+            if (ptx::elect_one()) ptx::mma_commit(bar(kKVFree + slot));
           }
         }
         if (T > 0) ++jobs_done;

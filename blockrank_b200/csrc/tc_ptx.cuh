@@ -132,6 +132,21 @@ __device__ __forceinline__ void st_global_v8(void* p, const uint32_t (&w)[8]) {
                : "memory");
 }
 
+// True in exactly one lane of a converged warp, always the same one.  Unlike `lane == 0` the compiler knows that a single
+// lane runs what it guards, so the operands of tcgen05.mma go to uniform registers directly instead of through a loop
+// over the active lanes.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p)
+      :
+      : "memory");
+  return p != 0;
+}
+
 // ---- fences ---------------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
