@@ -20,7 +20,8 @@ LIB = os.path.join(PKG, "libblockrank_b200.so")
 HOST_LIB = os.path.join(PKG, "_host.so")
 HOST_SOURCE = os.path.join(CSRC, "torch_host.cpp")
 HEADER = os.path.join(os.path.dirname(PKG), "include", "blockrank_b200.h")
-SOURCES = ["brk_api.cu", "attn_simt.cu", "attn_tc.cu", "attn_bwd.cu", "attn_bwd_mma.cu", "attn_bwd_tc.cu", "scores.cu",
+SOURCES = ["brk_api.cu", "attn_simt.cu", "attn_f32.cu", "attn_tc.cu", "attn_bwd.cu", "attn_bwd_mma.cu", "attn_bwd_tc.cu", "attn_bwd_f32.cu",
+           "scores.cu",
            "raw_scores.cu", "elementwise.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "--expt-relaxed-constexpr"]

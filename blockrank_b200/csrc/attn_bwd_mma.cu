@@ -1,5 +1,5 @@
 // BlockRank attention backward for bf16 on warp-level tensor-core MMA (mma.sync m16n8k16, fp32 accumulate).
-// Same mathematics and the same two-kernel split as attn_bwd.cu (which stays the fp32 path):
+// The path of blocks too long for a work item of attn_bwd_tc.cu:
 //
 //   attn_bwd_dq_mma_kernel   a CTA owns 64 query tokens of one (prompt, head, block); each of its four warps
 //                            keeps the A fragments of 16 rows of Q and dO in registers and walks through the
@@ -9,7 +9,7 @@
 //                            memory, 16 keys per warp, and walks through the rows that see them, 64 tokens of
 //                            one head staged at a time: S^T = K Q^T, dP^T = V dO^T, dV += P^T dO,
 //                            dK += dS^T Q.  Row blocks are dealt to `nsplit` CTAs, which add their fp32
-//                            results into the accumulators with atomics (attn_bwd.cu's layout and store kernel).
+//                            results into the accumulators with atomics; attn_bwd_store_kernel converts them.
 //
 // Operands reach the MMAs through ldmatrix from shared-memory tiles whose rows are padded by 16 bytes
 // (conflict-free); a product that is the left operand of the next MMA (P^T, dS, dS^T) goes from accumulator
@@ -31,7 +31,7 @@ constexpr int kThreadsM = kWarps * 32;
 constexpr int kRowBufs = 2;
 
 struct BwdMmaArgs {
-  View q, k, v, o, d_o, dq;
+  View q, k, v, o, d_o, dq, dk, dv;
   const float* lse;
   float* delta;   // [B, N, S]
   float* dk32;    // [B, Nk, S, D]
@@ -462,6 +462,23 @@ __global__ void __launch_bounds__(kThreadsM, 2) attn_bwd_dkv_mma_kernel(BwdMmaAr
   }
 }
 
+// fp32 accumulators [B, Nk, S, D] -> dk, dv (slots outside every block hold zeros)
+__global__ void __launch_bounds__(256) attn_bwd_store_kernel(BwdMmaArgs a, int D) {
+  const int64_t n4 = (int64_t)a.B * a.Nk * a.S * (D / 4);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
+    const int d4 = (int)(i % (D / 4));
+    const int64_t row = i / (D / 4);
+    const int s = (int)(row % a.S);
+    const int g = (int)((row / a.S) % a.Nk), b = (int)(row / ((int64_t)a.S * a.Nk));
+    auto put = [&](const View& t, const float* src) {
+      store4(reinterpret_cast<__nv_bfloat16*>(t.ptr) + (int64_t)b * t.sb + (int64_t)g * t.sh + (int64_t)s * t.ss + d4 * 4,
+             load4(src + row * D + d4 * 4));
+    };
+    put(a.dk, a.dk32);
+    put(a.dv, a.dv32);
+  }
+}
+
 template <int D>
 int launch_mma(BwdMmaArgs a, cudaStream_t st) {
   const int tiles = (a.max_block_len + kT - 1) / kT;
@@ -495,18 +512,20 @@ int launch_mma(BwdMmaArgs a, cudaStream_t st) {
     attn_bwd_dkv_mma_kernel<D><<<dim3(tiles, a.M - 1, a.B * a.Nk * a.nsplit), kThreadsM, smem, st>>>(a);
     BRK_CUDA(cudaGetLastError());
   }
+  const int64_t n4 = (int64_t)a.B * a.Nk * a.S * (D / 4);
+  attn_bwd_store_kernel<<<(unsigned)std::min<int64_t>((n4 + 255) / 256, 148 * 16), 256, 0, st>>>(a, D);
+  BRK_CUDA(cudaGetLastError());
   return BRK_OK;
 }
 
 }  // namespace
 
-// dq (and delta) and the fp32 dk / dv accumulators for bf16 tensors; the caller clears the accumulators
-// before and converts them afterwards.
+// The caller clears the accumulators dk32, dv32 and dq32 before.
 int attn_bwd_mma_launch(const brk_attn_bwd_params& p, float* delta, float* dk32, float* dv32, float* dq32,
                         cudaStream_t st) {
   BwdMmaArgs a;
   a.q = make_view(p.q); a.k = make_view(p.k); a.v = make_view(p.v); a.o = make_view(p.o); a.d_o = make_view(p.d_o);
-  a.dq = make_view(p.dq);
+  a.dq = make_view(p.dq); a.dk = make_view(p.dk); a.dv = make_view(p.dv);
   a.lse = p.lse; a.delta = delta; a.dk32 = dk32; a.dv32 = dv32; a.dq32 = dq32;
   a.blk_start = p.blk_start; a.blk_len = p.blk_len;
   a.B = p.B; a.N = p.N; a.Nk = p.Nk; a.S = p.S; a.M = p.M; a.G = p.N / p.Nk; a.max_block_len = p.max_block_len;

@@ -1,8 +1,7 @@
-// BlockRank attention forward on CUDA cores (fp32 accumulate).
+// BlockRank attention forward for bf16 tensors on CUDA cores (fp32 accumulate).
 //
-// This is the exact-arithmetic kernel of the library: it serves fp32 models
-// (tensor cores would drop to tf32) and any head_dim / group size the tcgen05
-// kernel does not cover.  One CTA owns (prompt, block, KV head, tile of query
+// The explicitly chosen alternative to the tcgen05 kernel, and the path of softmax
+// scales that are not positive.  One CTA owns (prompt, block, KV head, tile of query
 // tokens) and all query heads of that KV group, so K/V rows are staged in
 // shared memory once per group (no repeat_kv).  Each query row is held by four
 // threads, each owning a quarter of head_dim; keys are visited only inside the
@@ -207,13 +206,8 @@ int attn_simt_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaSt
   a.B = p.B; a.N = p.N; a.Nk = p.Nk; a.S = p.S; a.M = p.M;
   a.scale_log2 = p.scale * 1.4426950408889634f;
   BRK_REQUIRE(p.B * p.Nk <= 65535 && p.M <= 65535, BRK_E_UNSUPPORTED, "grid too large: B*Nk=%d M=%d", p.B * p.Nk, p.M);
-  if (p.dtype == BRK_F32) {
-    if (p.D == 64) return launch_g<float, 64>(p, a, st);
-    if (p.D == 128) return launch_g<float, 128>(p, a, st);
-  } else {
-    if (p.D == 64) return launch_g<__nv_bfloat16, 64>(p, a, st);
-    if (p.D == 128) return launch_g<__nv_bfloat16, 128>(p, a, st);
-  }
+  if (p.D == 64) return launch_g<__nv_bfloat16, 64>(p, a, st);
+  if (p.D == 128) return launch_g<__nv_bfloat16, 128>(p, a, st);
   set_error("SIMT attention supports head_dim 64 or 128, got %d", p.D);
   return BRK_E_UNSUPPORTED;
 }

@@ -41,6 +41,7 @@
 
 #include <type_traits>
 
+#include "attn_combine.cuh"
 #include "brk_common.cuh"
 #include "tc_ptx.cuh"
 
@@ -1099,43 +1100,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   if (warp == 0) ptx::tmem_dealloc(tmem, kTmemCols);
 }
 
-// Merge the key-chunk partials of the query block: one warp per (prompt, head, query token).
-template <int HD>
-__global__ void __launch_bounds__(128) attn_combine_kernel(TcArgs a) {
-  if (a.hdr[1] != 0) return;
-  const int lane = threadIdx.x & 31;
-  const int64_t w = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-  const int64_t total = (int64_t)a.B * a.N * a.lq_max;
-  if (w >= total) return;
-  const int tok = (int)(w % a.lq_max);
-  const int n = (int)((w / a.lq_max) % a.N);
-  const int b = (int)(w / ((int64_t)a.lq_max * a.N));
-  const int start = a.blk_start[(size_t)b * a.M + a.M - 1], len = a.blk_len[(size_t)b * a.M + a.M - 1];
-  if (tok >= len) return;
-  const float2* ml = a.part_ml + w * a.n_split;
-  const int col = (lane * 4) & (HD - 1);  // (head_dim 64: the upper half of the warp repeats the lower one's work)
-  float mx = -INFINITY;
-  for (int c = 0; c < a.n_split; ++c) mx = fmaxf(mx, ml[c].x);
-  const float ref = (mx == -INFINITY) ? 0.f : mx;
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  float l = 0.f;
-  for (int c = 0; c < a.n_split; ++c) {
-    const float2 x = ml[c];
-    if (x.y > 0.f) {  // chunks that saw no key carry no output
-      const float wgt = exp2f(x.x - ref);
-      const float4 o = *reinterpret_cast<const float4*>(a.part_o + (w * a.n_split + c) * HD + col);
-      acc.x = fmaf(o.x, wgt, acc.x); acc.y = fmaf(o.y, wgt, acc.y);
-      acc.z = fmaf(o.z, wgt, acc.z); acc.w = fmaf(o.w, wgt, acc.w);
-      l = fmaf(x.y, wgt, l);
-    }
-  }
-  const float inv = l > 0.f ? 1.f / l : 0.f;
-  __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.o.ptr) + (int64_t)b * a.o.sb + (int64_t)(start + tok) * a.o.ss +
-                       (int64_t)n * a.o.sh + col;
-  if (lane * 4 < HD) store4(dst, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
-  if (a.lse != nullptr && lane == 0) a.lse[((int64_t)b * a.N + n) * a.S + start + tok] = (ref + log2f(l)) * 0.6931471805599453f;
-}
-
 }  // namespace
 
 // The give-up path of the kernels' bounded waits, exercised without a fault: one thread waits, with a small
@@ -1201,10 +1165,6 @@ static int tc_splits(const brk_attn_params& p) {
   if (p.M < 2) return 1;
   int n = (p.S + 1023) / 1024;
   return n < 1 ? 1 : (n > 32 ? 32 : n);
-}
-
-static int query_rows(const brk_attn_params& p) {
-  return (p.max_query_len > 0 && p.max_query_len < p.max_block_len) ? p.max_query_len : p.max_block_len;
 }
 
 size_t attn_tc_workspace(const brk_attn_params& p) {
@@ -1287,9 +1247,8 @@ static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cuda
   attn_tc_kernel<HD><<<grid, kThreads, Geo<HD>::kSmemBytes, st>>>(tq, tk, tv, a);
   BRK_CUDA(cudaGetLastError());
   if (ns > 1) {
-    const int64_t warps = (int64_t)p.B * p.N * lq;
-    attn_combine_kernel<HD><<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(a);
-    BRK_CUDA(cudaGetLastError());
+    const CombineArgs c{a.o, a.lse, a.blk_start, a.blk_len, a.hdr, p.B, p.N, p.S, p.M, lq, ns, a.part_o, a.part_ml};
+    return attn_combine_launch<__nv_bfloat16, HD>(c, st);
   }
   return BRK_OK;
 }

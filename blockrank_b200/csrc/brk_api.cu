@@ -89,13 +89,15 @@ int brk_spans_from_mask(const uint8_t* mask, int32_t B, int32_t M, int32_t H, in
 
 size_t brk_attn_fwd_workspace_bytes(const brk_attn_params* p) {
   if (p == nullptr) return 0;
-  return resolve_algo(p) == BRK_ALGO_TC ? attn_tc_workspace(*p) : kWsHeader;
+  if (resolve_algo(p) == BRK_ALGO_TC) return attn_tc_workspace(*p);
+  return p->dtype == BRK_F32 ? attn_f32_workspace(*p) : kWsHeader;
 }
 
 int brk_attn_fwd(const brk_attn_params* p, void* workspace, size_t workspace_bytes, void* stream) {
   int rc = check_attn(p);
   if (rc) return rc;
   const int algo = resolve_algo(p);
+  if (algo == BRK_ALGO_SIMT && p->dtype == BRK_F32) return attn_f32_launch(*p, workspace, workspace_bytes, (cudaStream_t)stream);
   if (algo == BRK_ALGO_SIMT) return attn_simt_launch(*p, workspace, workspace_bytes, (cudaStream_t)stream);
   if (algo == BRK_ALGO_TC) return attn_tc_launch(*p, workspace, workspace_bytes, (cudaStream_t)stream);
   set_error("unknown attention algorithm %d", p->algo);

@@ -112,9 +112,16 @@ int attn_prologue_launch(const brk_attn_params& p, int* hdr, float2* ml, int64_t
 int attn_simt_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStream_t st);
 int selftest_wait_launch(int32_t* status, uint32_t budget, cudaStream_t st);
 int attn_tc_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStream_t st);
+size_t attn_f32_workspace(const brk_attn_params& p);
+int attn_f32_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStream_t st);
+// bound on the last block's length
+inline int query_rows(const brk_attn_params& p) {
+  return (p.max_query_len > 0 && p.max_query_len < p.max_block_len) ? p.max_query_len : p.max_block_len;
+}
 size_t attn_tc_workspace(const brk_attn_params& p);
 size_t attn_bwd_workspace(const brk_attn_bwd_params& p);
 int attn_bwd_launch(const brk_attn_bwd_params& p, void* ws, size_t ws_bytes, cudaStream_t st);
+int attn_bwd_f32_launch(const brk_attn_bwd_params& p, float* delta, cudaStream_t st);
 bool attn_bwd_tc_supported(const brk_attn_bwd_params& p);
 size_t attn_bwd_tc_extra_bytes(const brk_attn_bwd_params& p);
 int attn_bwd_tc_launch(const brk_attn_bwd_params& p, float* delta, float* ws32, float* dq32, void* extra, cudaStream_t st);
