@@ -6,11 +6,13 @@
 // and every row of a document meets all its partners inside one item:
 //
 //   dV, dK of own keys     accumulate in tensor memory over the key tile's row tiles and are stored once, in bf16
-//   dK, dV of the prefix   get one fp32 reduction per document item (red.global.add)
+//   dK, dV of the prefix   get one fp32 reduction per document item
 //   dQ of own rows         is the sum over the item's key tiles: two at most for documents up to 128 tokens plus prefix;
 //                          a partial sum waits in fp32 in a scratch of the CTA, laid out for coalesced access by the
 //                          thread that wrote it
 //   dQ of the query block  fp32 reductions (every item contributes)
+//
+// Outputs leave through shared memory by TMA (store or fp32 add), 32 rows per warp.
 //
 // Per (key tile, row tile) pair, all five products on tcgen05, keys down the 128 TMEM lanes:
 //   S^T = K Q^T      dP^T = V dO^T      P^T = 2^(S^T scale - lse)     dS^T = P^T (dP^T - delta)
@@ -84,7 +86,7 @@ struct BwdTcArgs {
   float* delta;     // [B, N, S]
   float* pre;       // prefix accumulators: dK then dV, [B, Nk, max_block_len, D] each; nullptr: block 0 stored directly
   float* dq32;      // [B, N, max_block_len, D]: dQ of the last block's rows
-  float* part;      // [CTA][row tile][16 (HD / 128)][256 threads] float4: dQ of rows whose keys span several tiles
+  float* part;      // [CTA][row tile][16][128 HD / 64 threads] float4: dQ of rows whose keys span several tiles
   int* counter;
   int32_t* status;
   const int32_t* blk_start;
@@ -97,10 +99,6 @@ __device__ __forceinline__ void span_of(const BwdTcArgs& a, int b, int m, int& s
   start = a.blk_start[(size_t)b * a.M + m];
   len = a.blk_len[(size_t)b * a.M + m];
   if (start < 0 || len < 0 || len > a.max_block_len || start > a.S - len) len = 0;  // skipped: nothing out of bounds
-}
-
-__device__ __forceinline__ void red4(float* p, float x, float y, float z, float w) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
 
 struct Item {
@@ -154,9 +152,15 @@ __device__ __forceinline__ RowTile row_tile(const BwdTcArgs& a, const Item& it, 
   return t;
 }
 
+// Inputs by row tile; outputs by warp (32 rows or keys).
+struct Maps {
+  CUtensorMap q, g;        // Q, dO: box {64, G, 128 / G}
+  CUtensorMap dq, dk, dv;  // boxes {64, G, 32 / G}, {64, 1, 32}
+  CUtensorMap dq32, pre;   // fp32 sums: boxes {32, G, 32 / G}, {32, 1, 32}
+};
+
 template <int HD>
-__global__ void __launch_bounds__(kThreads, 1)
-attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmG, const BwdTcArgs a) {
+__global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_constant__ Maps maps, const BwdTcArgs a) {
   using L = Geo<HD>;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = ptx::smem_u32(smem);
@@ -173,8 +177,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       ptx::mbar_init(bar(i), cnt);
     }
     ptx::fence_barrier_init();
-    ptx::prefetch_tmap(&tmQ);
-    ptx::prefetch_tmap(&tmG);
+    ptx::prefetch_tmap(&maps.q);
+    ptx::prefetch_tmap(&maps.g);
   }
   __syncwarp();
   if (warp == 0) {
@@ -238,8 +242,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             ptx::mbar_expect_tx(bar(kQFull + st), 2 * L::kTileBytes);
 #pragma unroll
             for (int c = 0; c < HD / 64; ++c) {
-              ptx::tma_load_4d(q + c * kChunk, &tmQ, bar(kQFull + st), 64 * c, it.g * a.G, t.slot, it.b);
-              ptx::tma_load_4d(g + c * kChunk, &tmG, bar(kQFull + st), 64 * c, it.g * a.G, t.slot, it.b);
+              ptx::tma_load_4d(q + c * kChunk, &maps.q, bar(kQFull + st), 64 * c, it.g * a.G, t.slot, it.b);
+              ptx::tma_load_4d(g + c * kChunk, &maps.g, bar(kQFull + st), 64 * c, it.g * a.G, t.slot, it.b);
             }
           }
           float* const col = reinterpret_cast<float*>(smem + L::kOffCol) + st * 2 * kTile;
@@ -340,7 +344,29 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int wg = warp >> 2, row = tid & 127;
     const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     uint32_t tile = 0, kts = 0;
-    constexpr int kHalf = HD / 2;  // columns of dQ a thread drains
+    constexpr int kPartThreads = 128 * (HD / 64);  // threads that drain dQ: 64 columns each
+    // This warp's 4 KB of the dS buffer, 32 rows of 128 bytes: outputs pass through it between the last product that reads
+    // dS and the next dS, so that they leave as whole rows by TMA.  (A thread owns a row: stored directly, an instruction
+    // touched 32 lines, and these stores took more time than the products.)
+    const uint32_t slab = sbase + L::kOffDs + (uint32_t)wg * kChunk + (uint32_t)(warp & 3) * 4096u;
+    uint8_t* const slab_row = smem + L::kOffDs + wg * kChunk + row * 128;
+    auto put = [&](int piece, uint4 w) { *reinterpret_cast<uint4*>(slab_row + ((piece ^ (row & 7)) << 4)) = w; };
+    auto slab_free = [&]() {  // the warp's earlier transfers have read it
+      if (lane == 0) ptx::bulk_wait_read();
+      __syncwarp();
+    };
+    auto put_f32 = [&](const uint32_t (&x)[32], float f) {  // 32 columns
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        put(i, make_uint4(__float_as_uint(__uint_as_float(x[4 * i]) * f), __float_as_uint(__uint_as_float(x[4 * i + 1]) * f),
+                          __float_as_uint(__uint_as_float(x[4 * i + 2]) * f), __float_as_uint(__uint_as_float(x[4 * i + 3]) * f)));
+    };
+    auto pack8 = [&](const uint32_t (&x)[32], int i, float f) {
+      return make_uint4(pack_bf16(__uint_as_float(x[i]) * f, __uint_as_float(x[i + 1]) * f),
+                        pack_bf16(__uint_as_float(x[i + 2]) * f, __uint_as_float(x[i + 3]) * f),
+                        pack_bf16(__uint_as_float(x[i + 4]) * f, __uint_as_float(x[i + 5]) * f),
+                        pack_bf16(__uint_as_float(x[i + 6]) * f, __uint_as_float(x[i + 7]) * f));
+    };
     auto arrive = [&](int i) {
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(bar(i));
@@ -365,12 +391,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
     // dV (warps 0-3) or dK (warps 4-7) of one key tile: thread = key
     auto drain_acc = [&](const Item& it, int kt) {
-      const int j = kt * kTile + row;
-      const bool valid = j < it.l0 + it.len;
+      const int j = kt * kTile + row, jw = kt * kTile + (warp & 3) * 32;  // this key, the warp's first
+      const int n_list = it.l0 + it.len;
       const float f = wg ? a.scale : 1.f;
-      const bool prefix = a.pre != nullptr && (it.m == 0 || j < it.l0);
+      const int pre_end = a.pre == nullptr ? 0 : it.m == 0 ? it.len : it.l0;  // keys whose sums other items share
+      const bool whole = jw >= pre_end && jw + 32 <= n_list;                  // 32 own keys
+      const bool mine = j >= pre_end && j < n_list;
       const View& out = wg ? a.dk : a.dv;
-      float* const acc = a.pre + ((size_t)(wg ? 0 : 1) * a.B * a.Nk + (size_t)it.b * a.Nk + it.g) * a.max_block_len * HD + (size_t)j * HD;
       __nv_bfloat16* const dst = reinterpret_cast<__nv_bfloat16*>(out.ptr) + (int64_t)it.b * out.sb + (int64_t)it.g * out.sh +
                                  (int64_t)(it.start + j - it.l0) * out.ss;
 #pragma unroll 1
@@ -379,59 +406,77 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         __syncwarp();
         ptx::tmem_ld32(lanes + (wg ? kColDk : kColDv) + (uint32_t)c0, x);
         ptx::tmem_wait_ld(x);
-        if (!valid) continue;
-        if (prefix) {
+        if (jw < pre_end) {  // (rows beyond the prefix go to rows of the sums that nothing reads)
+          slab_free();
+          put_f32(x, f);
+          ptx::fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            ptx::tma_add_4d(&maps.pre, slab, c0, ((wg ? 0 : a.B) + it.b) * a.Nk + it.g, jw, 0);
+            ptx::bulk_commit();
+          }
+        }
+        if (whole) {
+          if ((c0 & 32) == 0) slab_free();
 #pragma unroll
-          for (int i = 0; i < 32; i += 4)
-            red4(acc + c0 + i, __uint_as_float(x[i]) * f, __uint_as_float(x[i + 1]) * f, __uint_as_float(x[i + 2]) * f,
-                 __uint_as_float(x[i + 3]) * f);
-        } else {
+          for (int i = 0; i < 32; i += 8) put(((c0 & 32) + i) >> 3, pack8(x, i, f));
+          if (c0 & 32) {
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              ptx::tma_store_4d(wg ? &maps.dk : &maps.dv, slab, c0 - 32, it.g, it.start + jw - it.l0, it.b);
+              ptx::bulk_commit();
+            }
+          }
+        } else if (mine) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 8)
-            *reinterpret_cast<uint4*>(dst + c0 + i) =
-                make_uint4(pack_bf16(__uint_as_float(x[i]) * f, __uint_as_float(x[i + 1]) * f),
-                           pack_bf16(__uint_as_float(x[i + 2]) * f, __uint_as_float(x[i + 3]) * f),
-                           pack_bf16(__uint_as_float(x[i + 4]) * f, __uint_as_float(x[i + 5]) * f),
-                           pack_bf16(__uint_as_float(x[i + 6]) * f, __uint_as_float(x[i + 7]) * f));
+          for (int i = 0; i < 32; i += 8) *reinterpret_cast<uint4*>(dst + c0 + i) = pack8(x, i, f);
         }
       }
     };
 
-    // dQ of one (key tile, row tile) pair: thread = row, columns [wg HD / 2, + HD / 2)
+    // dQ of one (key tile, row tile) pair: thread = row, columns [64 wg, + 64) (head_dim 64: warps 0-3 only)
     auto drain_dq = [&](const Item& it, int kt, const RowTile& t) {
+      if (wg * 64 >= HD) {
+        arrive(kDqFree);
+        return;
+      }
       const int tok = t.t0 + (row >> a.g_shift), head = it.g * a.G + (row & (a.G - 1));
+      const int row_w = (warp & 3) * 32, tok_w = t.t0 + (row_w >> a.g_shift);  // the warp's first row
       const bool valid = row < t.nrow;
       const bool sum32 = a.M > 1 && (!t.own || it.m == a.M - 1);  // rows of the query block
       // own rows: the key tiles that see this row tile are 0 .. last
       const int last = t.own ? (it.l0 + min(it.len, t.t0 + (kTile >> a.g_shift)) - 1) / kTile : 0;
-      float* const d32 = a.dq32 + (((size_t)it.b * a.N + head) * a.max_block_len + tok) * HD + wg * kHalf;
-      float4* const part = reinterpret_cast<float4*>(a.part) +
-                           ((size_t)blockIdx.x * a.row_tiles + t.r) * (HD / 8) * kComputeThreads + tid;
+      float4* const part = reinterpret_cast<float4*>(a.part) + ((size_t)blockIdx.x * a.row_tiles + t.r) * 16 * kPartThreads + tid;
       __nv_bfloat16* const dst = reinterpret_cast<__nv_bfloat16*>(a.dq.ptr) + (int64_t)it.b * a.dq.sb + (int64_t)head * a.dq.sh +
-                                 (int64_t)(it.start + tok) * a.dq.ss + wg * kHalf;
+                                 (int64_t)(it.start + tok) * a.dq.ss + wg * 64;
       const float f = a.scale;
 #pragma unroll 1
-      for (int c0 = 0; c0 < kHalf; c0 += 32) {
+      for (int c0 = 0; c0 < 64; c0 += 32) {
         uint32_t x[32];
         __syncwarp();
-        ptx::tmem_ld32(lanes + kColDp + (uint32_t)(wg * kHalf + c0), x);
+        ptx::tmem_ld32(lanes + kColDp + (uint32_t)(wg * 64 + c0), x);
         ptx::tmem_wait_ld(x);
-        if (c0 + 32 >= kHalf) {  // out of tensor memory: the next tile's dP may overwrite it
+        if (c0 > 0) {  // out of tensor memory: the next tile's dP may overwrite it
           ptx::tc_fence_before_sync();
           arrive(kDqFree);
         }
-        if (!valid) continue;
-        if (sum32) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 4)
-            red4(d32 + c0 + i, __uint_as_float(x[i]) * f, __uint_as_float(x[i + 1]) * f, __uint_as_float(x[i + 2]) * f,
-                 __uint_as_float(x[i + 3]) * f);
+        if (row_w >= t.nrow) continue;
+        if (sum32) {  // (rows beyond the block go to rows of the sums that nothing reads)
+          slab_free();
+          put_f32(x, f);
+          ptx::fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            ptx::tma_add_4d(&maps.dq32, slab, wg * 64 + c0, it.g * a.G, tok_w, it.b);
+            ptx::bulk_commit();
+          }
           continue;
         }
         if (kt > 0) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            const float4 y = part[(size_t)(c0 / 4 + i) * kComputeThreads];
+            const float4 y = part[(size_t)(c0 / 4 + i) * kPartThreads];
             x[4 * i] = __float_as_uint(__uint_as_float(x[4 * i]) + y.x);
             x[4 * i + 1] = __float_as_uint(__uint_as_float(x[4 * i + 1]) + y.y);
             x[4 * i + 2] = __float_as_uint(__uint_as_float(x[4 * i + 2]) + y.z);
@@ -441,17 +486,24 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (kt < last) {
 #pragma unroll
           for (int i = 0; i < 8; ++i)
-            part[(size_t)(c0 / 4 + i) * kComputeThreads] =
+            part[(size_t)(c0 / 4 + i) * kPartThreads] =
                 make_float4(__uint_as_float(x[4 * i]), __uint_as_float(x[4 * i + 1]), __uint_as_float(x[4 * i + 2]),
                             __uint_as_float(x[4 * i + 3]));
-        } else {
+        } else if (row_w + 32 <= t.nrow) {
+          if (c0 == 0) slab_free();
 #pragma unroll
-          for (int i = 0; i < 32; i += 8)
-            *reinterpret_cast<uint4*>(dst + c0 + i) =
-                make_uint4(pack_bf16(__uint_as_float(x[i]) * f, __uint_as_float(x[i + 1]) * f),
-                           pack_bf16(__uint_as_float(x[i + 2]) * f, __uint_as_float(x[i + 3]) * f),
-                           pack_bf16(__uint_as_float(x[i + 4]) * f, __uint_as_float(x[i + 5]) * f),
-                           pack_bf16(__uint_as_float(x[i + 6]) * f, __uint_as_float(x[i + 7]) * f));
+          for (int i = 0; i < 32; i += 8) put((c0 + i) >> 3, pack8(x, i, f));
+          if (c0 > 0) {
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              ptx::tma_store_4d(&maps.dq, slab, wg * 64, it.g * a.G, it.start + tok_w, it.b);
+              ptx::bulk_commit();
+            }
+          }
+        } else if (valid) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) *reinterpret_cast<uint4*>(dst + c0 + i) = pack8(x, i, f);
         }
       }
     };
@@ -538,7 +590,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           wait(kDpFull, tile, 74);
           ptx::tc_fence_after_sync();
           __syncwarp();
-          uint8_t* const ds_row = smem + L::kOffDs + wg * kChunk + row * 128;
+          slab_free();
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             uint32_t x[32];
@@ -554,7 +606,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
               w.y = pack_bf16(pp[2] * (__uint_as_float(x[c + 2]) - d0.z), pp[3] * (__uint_as_float(x[c + 3]) - d0.w));
               w.z = pack_bf16(pp[4] * (__uint_as_float(x[c + 4]) - d1.x), pp[5] * (__uint_as_float(x[c + 5]) - d1.y));
               w.w = pack_bf16(pp[6] * (__uint_as_float(x[c + 6]) - d1.z), pp[7] * (__uint_as_float(x[c + 7]) - d1.w));
-              *reinterpret_cast<uint4*>(ds_row + (((h * 4 + (c >> 3)) ^ (row & 7)) << 4)) = w;
+              put(h * 4 + (c >> 3), w);
             }
           }
           ptx::fence_proxy_async_smem();
@@ -571,6 +623,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       ptx::tc_fence_after_sync();
       drain_acc(prev, prev_kt);
     }
+    if (lane == 0) ptx::bulk_wait();
   }
   ptx::tc_fence_before_sync();
   __syncthreads();
@@ -606,12 +659,14 @@ __global__ void __launch_bounds__(256) attn_bwd_tc_prep_kernel(BwdTcArgs a, floa
   const __nv_bfloat16* op = reinterpret_cast<const __nv_bfloat16*>(a.o.ptr) + (int64_t)b * a.o.sb + (int64_t)n * a.o.sh;
   constexpr int kLanes = HD / 8, kRows = 32 / kLanes;  // lanes per row, rows per pass
   const int sub = lane / kLanes, c = (lane % kLanes) * 8;
+  const int own = grp * 32 + lane;
+  const unsigned live = __ballot_sync(0xffffffffu, own < a.S && slot_in_block(a, b, own));  // the others are not read
   float mine = 0.f;
 #pragma unroll 4
   for (int r = 0; r < 32; r += kRows) {
     const int s = grp * 32 + r + sub;
     float d = 0.f;
-    if (s < a.S) {
+    if ((live >> (r + sub)) & 1u) {
       float x[8], y[8];
       load8(gp + (int64_t)s * a.d_o.ss + c, x);
       load8(op + (int64_t)s * a.o.ss + c, y);
@@ -626,9 +681,8 @@ __global__ void __launch_bounds__(256) attn_bwd_tc_prep_kernel(BwdTcArgs a, floa
       if (lane == r + k) mine = v;
     }
   }
-  const int s = grp * 32 + lane;
-  if (s < a.S) a.delta[((size_t)b * a.N + n) * a.S + s] = mine;
-  unsigned gap = __ballot_sync(0xffffffffu, s < a.S && !slot_in_block(a, b, s));
+  if (own < a.S) a.delta[((size_t)b * a.N + n) * a.S + own] = mine;
+  unsigned gap = ~live & __ballot_sync(0xffffffffu, own < a.S);
   for (; gap; gap &= gap - 1) {
     const int z = grp * 32 + __ffs((int)gap) - 1;
     auto clear = [&](const View& t) {
@@ -674,18 +728,26 @@ size_t part_bytes(const brk_attn_bwd_params& p) {
 
 template <int HD>
 int launch(const brk_attn_bwd_params& p, BwdTcArgs a, float4* zero, int64_t n_zero, cudaStream_t st) {
-  const int tok = kTile / a.G;
-  CUtensorMap tq, tg;
+  const int tok = kTile / a.G, tok_w = std::max(1, 32 / a.G);
+  Maps t;
+  auto map = [&](CUtensorMap& m, const brk_view& v, int heads, int box_h, int box_s) {
+    return make_tmap_bf16(&m, v.ptr, HD, heads, p.S, p.B, v.stride_h, v.stride_s, v.stride_b, box_h, box_s);
+  };
   int rc;
-  if ((rc = make_tmap_bf16(&tq, p.q.ptr, HD, p.N, p.S, p.B, p.q.stride_h, p.q.stride_s, p.q.stride_b, a.G, tok))) return rc;
-  if ((rc = make_tmap_bf16(&tg, p.d_o.ptr, HD, p.N, p.S, p.B, p.d_o.stride_h, p.d_o.stride_s, p.d_o.stride_b, a.G, tok))) return rc;
+  if ((rc = map(t.q, p.q, p.N, a.G, tok)) || (rc = map(t.g, p.d_o, p.N, a.G, tok)) || (rc = map(t.dq, p.dq, p.N, a.G, tok_w)) ||
+      (rc = map(t.dk, p.dk, p.Nk, 1, 32)) || (rc = map(t.dv, p.dv, p.Nk, 1, 32)))
+    return rc;
+  const int64_t mbl = p.max_block_len;
+  if ((rc = make_tmap_f32(&t.dq32, a.dq32, HD, p.N, p.max_block_len, p.B, mbl * HD, HD, (int64_t)p.N * mbl * HD, a.G, tok_w))) return rc;
+  t.pre = t.dq32;
+  if (a.pre && (rc = make_tmap_f32(&t.pre, a.pre, HD, 2 * p.B * p.Nk, p.max_block_len, 1, mbl * HD, HD, 0, 1, 32))) return rc;
   const int64_t warps = (int64_t)p.B * ((p.S + 31) / 32) * p.N;
   attn_bwd_tc_prep_kernel<HD><<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(a, zero, n_zero);
   BRK_CUDA(cudaGetLastError());
   BRK_CUDA(cudaFuncSetAttribute(attn_bwd_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Geo<HD>::kSmem));
   const int sms = sm_count();
   BRK_REQUIRE(sms > 0, BRK_E_CUDA, "could not read the SM count");
-  attn_bwd_tc_kernel<HD><<<std::min(sms, a.total_items), kThreads, Geo<HD>::kSmem, st>>>(tq, tg, a);
+  attn_bwd_tc_kernel<HD><<<std::min(sms, a.total_items), kThreads, Geo<HD>::kSmem, st>>>(t, a);
   BRK_CUDA(cudaGetLastError());
   if (p.M > 1) {
     const int64_t n = (int64_t)p.B * (p.N + (a.pre ? 2 * p.Nk : 0)) * p.max_block_len * (HD / 8);

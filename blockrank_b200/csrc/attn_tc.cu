@@ -60,17 +60,17 @@ EncodeTiledFn get_encode_tiled() {
   return fn;
 }
 
-int make_tmap_bf16(CUtensorMap* out, const void* ptr, int D, int heads, int S, int B, int64_t stride_h,
-                   int64_t stride_s, int64_t stride_b, int box_h, int box_s) {
+static int make_tmap(CUtensorMap* out, CUtensorMapDataType type, int bytes, const void* ptr, int D, int heads, int S, int B,
+                     int64_t stride_h, int64_t stride_s, int64_t stride_b, int box_h, int box_s) {
   EncodeTiledFn enc = get_encode_tiled();
   BRK_REQUIRE(enc != nullptr, BRK_E_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   if (B == 1) stride_b = (int64_t)S * stride_s;  // a size-1 dim may carry any stride
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)heads, (cuuint64_t)S, (cuuint64_t)B};
-  cuuint64_t strides[3] = {(cuuint64_t)stride_h * 2, (cuuint64_t)stride_s * 2, (cuuint64_t)stride_b * 2};
-  cuuint32_t box[4] = {64, (cuuint32_t)box_h, (cuuint32_t)box_s, 1};
+  cuuint64_t strides[3] = {(cuuint64_t)stride_h * bytes, (cuuint64_t)stride_s * bytes, (cuuint64_t)stride_b * bytes};
+  cuuint32_t box[4] = {(cuuint32_t)(128 / bytes), (cuuint32_t)box_h, (cuuint32_t)box_s, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   auto encode = [&] {
-    return enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, strides, box, estr,
+    return enc(out, type, 4, const_cast<void*>(ptr), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   };
@@ -84,9 +84,19 @@ int make_tmap_bf16(CUtensorMap* out, const void* ptr, int D, int heads, int S, i
     r = encode();
   }
   BRK_REQUIRE(r == CUDA_SUCCESS, BRK_E_CUDA,
-              "cuTensorMapEncodeTiled failed (%d): dims {%d,%d,%d,%d} strides {%lld,%lld,%lld} box {64,%d,%d,1}", (int)r,
-              D, heads, S, B, (long long)stride_h, (long long)stride_s, (long long)stride_b, box_h, box_s);
+              "cuTensorMapEncodeTiled failed (%d): dims {%d,%d,%d,%d} strides {%lld,%lld,%lld} box {%d,%d,%d,1}", (int)r,
+              D, heads, S, B, (long long)stride_h, (long long)stride_s, (long long)stride_b, 128 / bytes, box_h,
+              box_s);
   return BRK_OK;
+}
+
+int make_tmap_bf16(CUtensorMap* out, const void* ptr, int D, int heads, int S, int B, int64_t stride_h, int64_t stride_s,
+                   int64_t stride_b, int box_h, int box_s) {
+  return make_tmap(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr, D, heads, S, B, stride_h, stride_s, stride_b, box_h, box_s);
+}
+int make_tmap_f32(CUtensorMap* out, const void* ptr, int D, int heads, int S, int B, int64_t stride_h, int64_t stride_s,
+                  int64_t stride_b, int box_h, int box_s) {
+  return make_tmap(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, ptr, D, heads, S, B, stride_h, stride_s, stride_b, box_h, box_s);
 }
 
 namespace {
