@@ -19,16 +19,19 @@
 //   dV += P^T dO (P^T read from tensor memory)    dK += dS^T Q    dQ = dS K   (dS^T in shared memory serves both: K-major
 //                                                 for dK, MN-major for dQ)
 //
-// Roles (320 threads, one CTA per SM, items claimed from a global counter):
-//   warps 0-7  the element-wise part: warp w owns lanes 32 (w % 4) and the row-tile columns (or head_dim half) w / 4;
-//              they also load K / V (cp.async, zero beyond the list, so any prefix length packs against any document),
-//              drain dQ, dK, dV
-//   warp 8     MMA issue
-//   warp 9     claims items, loads Q / dO by TMA two row tiles deep, and the columns' lse and delta
+// Roles (512 threads, one CTA per SM, items claimed from a global counter, longest blocks first):
+//   warps 0-7   element-wise part: warp w owns lanes 32 (w % 4) and the row-tile columns 64 (w / 4) + {0..63}
+//   warps 8-11  outputs: dQ after every pair, dV and dK after every key tile, from tensor memory through shared memory to
+//               TMA, beside the element-wise part of the next pair
+//   warp 12     MMA issue
+//   warp 13     claims items, loads Q (two stages) and dO (one) by TMA and the columns' lse and delta
+//   warps 14-15 load K / V (cp.async, zero beyond the list, so any prefix length packs against any document) and zero the
+//               rows of a partial row tile that lie beyond its block
 //
-// Order of the tensor pipe: dP(i) | dV(i) S(i+1) | dK(i) dQ(i), so that the exponentials of tile i + 1 run beside
-// dK(i) / dQ(i) and the dS of tile i beside dV(i) / S(i+1).  Tensor memory (head_dim 128, all 512 columns): S / P 128,
-// dP / dQ 128, dV 128, dK 128.
+// Order of the tensor pipe: dP(i) | dV(i) S(i+1) | dK(i) dQ(i): the exponentials of tile i + 1 run beside dK(i) / dQ(i) and
+// the dS of tile i beside dV(i) / S(i+1).  Tensor memory (head_dim 128, all 512 columns): S / P 128, dP / dQ 128, dV 128,
+// dK 128; dQ shares dP's columns, so the way dQ(i) -> read out -> dP(i+1) -> dS(i+1) is the kernel's cycle, and that is
+// why the reading has warps of its own.
 #include <cuda.h>
 
 #include <algorithm>
@@ -42,8 +45,7 @@ namespace brk {
 namespace {
 
 constexpr int kTile = 128;  // keys per key tile, rows per row tile
-constexpr int kComputeThreads = 256;
-constexpr int kThreads = 320;
+constexpr int kThreads = 512;
 constexpr uint32_t kChunk = kTile * 128;  // 128 rows of 64 bf16: one 64-wide chunk of a tile
 constexpr uint32_t kWaitBudget = 1u << 18;
 constexpr int kMaxRowTiles = 16;  // per block: bounds the dQ scratch of a CTA (64 KB per tile at head_dim 128)
@@ -53,9 +55,11 @@ struct Geo {
   static constexpr uint32_t kTileBytes = (HD / 64) * kChunk;
   static constexpr uint32_t kOffK = 0;
   static constexpr uint32_t kOffV = kOffK + kTileBytes;
-  static constexpr uint32_t kOffQ = kOffV + kTileBytes;        // two stages of [Q | dO]
-  static constexpr uint32_t kOffDs = kOffQ + 4 * kTileBytes;
-  static constexpr uint32_t kOffCol = kOffDs + 2 * kChunk;     // two stages of [-lse log2 e | delta], 128 floats each
+  static constexpr uint32_t kOffQ = kOffV + kTileBytes;  // two stages
+  static constexpr uint32_t kOffG = kOffQ + 2 * kTileBytes;
+  static constexpr uint32_t kOffDs = kOffG + kTileBytes;
+  static constexpr uint32_t kOffOut = kOffDs + 2 * kChunk;   // output staging: two slabs of 4 KB for each of warps 8-11
+  static constexpr uint32_t kOffCol = kOffOut + 8 * 4096;    // two stages of [-lse log2 e | delta], 128 floats each
   static constexpr uint32_t kOffBar = kOffCol + 2 * 2 * kTile * 4;
   static constexpr uint32_t kSmem = kOffBar + 256;
   static_assert(kSmem <= 232448, "shared memory per CTA");
@@ -63,20 +67,24 @@ struct Geo {
 constexpr uint32_t kColS = 0, kColDp = 128, kColDv = 256, kColDk = 384;
 
 enum {
-  kQFull = 0,    // +stage  Q, dO landed and the columns' lse / delta written (expect_tx arrival + 1)
-  kQFree = 2,    // +stage  dK has read the stage
-  kSFull = 4,
-  kDpFull = 5,
-  kPFull = 6,    // P^T in tensor memory (8 warps)
-  kDsFull = 7,   // dS^T in shared memory, dP consumed (8 warps)
-  kDqFull = 8,
-  kDqFree = 9,   // dQ drained (8 warps)
-  kAccFull = 10, // every product of the key tile complete
-  kKvFull = 11,  // K, V of the key tile in shared memory, the accumulators drained (8 warps)
-  kTail = 12,    // the rows beyond the block zeroed in a partial row tile (8 warps)
-  kItemFull = 13,  // +slot
-  kItemFree = 15,  // +slot (8 compute warps + MMA warp)
-  kNumBars = 17
+  kQFull = 0,    // +stage  Q landed and the columns' lse / delta written (expect_tx arrival + 1)
+  kQFree = 2,    // +stage  dK has read the stage (commit + 2 warps)
+  kGFull = 4,    // dO landed
+  kGFree = 5,    // dV has read it (commit + 2 warps)
+  kQTail = 6,    // the rows beyond the block zeroed in a partial Q / dO tile (2 warps)
+  kGTail = 7,
+  kSFull = 8,
+  kDpFull = 9,
+  kPFull = 10,   // P^T in tensor memory (8 warps)
+  kDsFull = 11,  // dS^T in shared memory, dP consumed (8 warps)
+  kDqFull = 12,
+  kDqFree = 13,  // dQ read out (4 warps)
+  kAccFull = 14, // every product of the key tile complete
+  kAccFree = 15, // dV, dK read out (4 warps)
+  kKvFull = 16,  // K, V of the key tile in shared memory (2 warps)
+  kItemFull = 17,  // +slot
+  kItemFree = 19,  // +slot (15 consuming warps)
+  kNumBars = 21
 };
 static_assert(kNumBars * 8 + 16 <= 256, "barrier area");  // + TMEM base, two item slots
 
@@ -86,8 +94,9 @@ struct BwdTcArgs {
   float* delta;     // [B, N, S]
   float* pre;       // prefix accumulators: dK then dV, [B, Nk, max_block_len, D] each; nullptr: block 0 stored directly
   float* dq32;      // [B, N, max_block_len, D]: dQ of the last block's rows
-  float* part;      // [CTA][row tile][16][128 HD / 64 threads] float4: dQ of rows whose keys span several tiles
+  float* part;      // [CTA][row tile][HD / 4][128 threads] float4: dQ of rows whose keys span several tiles
   int* counter;
+  int* order;       // (prompt, block) pairs, longest block first; nullptr: as they come
   int32_t* status;
   const int32_t* blk_start;
   const int32_t* blk_len;
@@ -111,10 +120,10 @@ struct Item {
 
 __device__ __forceinline__ Item decode(const BwdTcArgs& a, int idx) {
   Item it;
-  const int nbg = a.B * a.Nk, bg = idx % nbg;
-  it.m = idx / nbg;
-  it.b = bg / a.Nk;
-  it.g = bg % a.Nk;
+  const int bm = a.order ? a.order[idx / a.Nk] : idx / a.Nk;
+  it.b = bm / a.M;
+  it.m = bm % a.M;
+  it.g = idx % a.Nk;
   span_of(a, it.b, it.m, it.start, it.len);
   it.s0 = it.l0 = it.qs = it.ql = 0;
   if (it.m > 0 && it.m < a.M - 1) span_of(a, it.b, 0, it.s0, it.l0);
@@ -171,9 +180,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
   if (tid == 0) {
     for (int i = 0; i < kNumBars; ++i) {
       uint32_t cnt = 1u;
-      if (i == kPFull || i == kDsFull || i == kDqFree || i == kKvFull || i == kTail) cnt = 8u;
-      if (i == kQFull || i == kQFull + 1) cnt = 2u;
-      if (i >= kItemFree) cnt = 9u;
+      if (i == kPFull || i == kDsFull) cnt = 8u;
+      if (i == kDqFree || i == kAccFree) cnt = 4u;
+      if (i == kQFull || i == kQFull + 1 || i == kQTail || i == kGTail || i == kKvFull) cnt = 2u;
+      if (i == kQFree || i == kQFree + 1 || i == kGFree) cnt = 3u;
+      if (i >= kItemFree) cnt = 15u;
       ptx::mbar_init(bar(i), cnt);
     }
     ptx::fence_barrier_init();
@@ -198,161 +209,233 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
     failed = true;
     if (a.status) atomicCAS(a.status, 0, code);
   };
+  auto arrive = [&](int i) {
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive(bar(i));
+  };
   uint32_t n_items = 0;
-  // next item of this CTA, or -1 (consumers: warps 0-8)
+  // next item of this CTA, or -1 (every warp but the loader)
   auto next_item = [&]() {
     const uint32_t slot = n_items & 1u;
-    wait(kItemFull + slot, n_items >> 1, 40);
+    wait(kItemFull + slot, n_items >> 1, 60);
     int idx = item_slot[slot];
     if (__any_sync(0xffffffffu, failed)) idx = -1;
-    __syncwarp();
-    if (lane == 0) ptx::mbar_arrive(bar(kItemFree + slot));
+    arrive(kItemFree + slot);
     ++n_items;
     return idx;
   };
 
-  if (warp == 9) {
-    // =============================== loader ======================================================
-    uint32_t tile = 0, pub = 0;
-    const bool leader = lane == 0;
-    auto claim = [&]() {
-      int v = 0;
-      if (leader) v = atomicAdd(a.counter, 1);
-      v = __shfl_sync(0xffffffffu, v, 0);
-      return v < a.total_items ? v : -1;
-    };
-    for (;;) {
-      const int idx = claim();
-      if (pub >= 2) wait(kItemFree + (pub & 1u), (pub >> 1) - 1, 60);
-      if (leader) {
-        item_slot[pub & 1u] = idx;
-        ptx::mbar_arrive(bar(kItemFull + (pub & 1u)));
+  // Registers: 512 x 128 at launch = 256 x 160 + 128 x 120 + 128 x 72.
+  if (warp >= 12) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    if (warp == 13) {
+      // =============================== loader ====================================================
+      uint32_t tile = 0, pub = 0;
+      const bool leader = lane == 0;
+      for (;;) {
+        int idx = 0;
+        if (leader) idx = atomicAdd(a.counter, 1);
+        idx = __shfl_sync(0xffffffffu, idx, 0);
+        if (idx >= a.total_items) idx = -1;
+        if (pub >= 2) wait(kItemFree + (pub & 1u), (pub >> 1) - 1, 61);
+        if (leader) {
+          item_slot[pub & 1u] = idx;
+          ptx::mbar_arrive(bar(kItemFull + (pub & 1u)));
+        }
+        ++pub;
+        if (idx < 0 || __any_sync(0xffffffffu, failed)) break;
+        const Item it = decode(a, idx);
+        for (int kt = 0; kt < it.n_kt; ++kt) {
+          const RowList rows = rows_of(a, it, kt);
+          for (int i = 0; i < rows.n; ++i, ++tile) {
+            const RowTile t = row_tile(a, it, rows, i);
+            const uint32_t st = tile & 1u;
+            if (tile >= 2) wait(kQFree + st, (tile >> 1) - 1, 62);
+            if (leader) {
+              const uint32_t q = sbase + L::kOffQ + st * L::kTileBytes;
+              ptx::mbar_expect_tx(bar(kQFull + st), L::kTileBytes);
+#pragma unroll
+              for (int c = 0; c < HD / 64; ++c)
+                ptx::tma_load_4d(q + c * kChunk, &maps.q, bar(kQFull + st), 64 * c, it.g * a.G, t.slot, it.b);
+            }
+            float* const col = reinterpret_cast<float*>(smem + L::kOffCol) + st * 2 * kTile;
+#pragma unroll
+            for (int j = 0; j < kTile / 32; ++j) {
+              const int c = lane + 32 * j;
+              float nl = -INFINITY, dl = 0.f;  // beyond the block: P = 0
+              if (c < t.nrow) {
+                const size_t id = ((size_t)it.b * a.N + it.g * a.G + (c & (a.G - 1))) * a.S + t.slot + (c >> a.g_shift);
+                nl = a.lse[id] * -1.4426950408889634f;
+                dl = a.delta[id];
+              }
+              col[c] = nl;
+              col[kTile + c] = dl;
+            }
+            arrive(kQFull + st);
+            if (tile >= 1) wait(kGFree, tile - 1, 63);
+            if (leader) {
+              ptx::mbar_expect_tx(bar(kGFull), L::kTileBytes);
+#pragma unroll
+              for (int c = 0; c < HD / 64; ++c)
+                ptx::tma_load_4d(sbase + L::kOffG + c * kChunk, &maps.g, bar(kGFull), 64 * c, it.g * a.G, t.slot, it.b);
+            }
+          }
+        }
       }
-      ++pub;
-      if (idx < 0 || __any_sync(0xffffffffu, failed)) break;
-      const Item it = decode(a, idx);
-      for (int kt = 0; kt < it.n_kt; ++kt) {
-        const RowList rows = rows_of(a, it, kt);
-        for (int i = 0; i < rows.n; ++i, ++tile) {
-          const RowTile t = row_tile(a, it, rows, i);
-          const uint32_t st = tile & 1u;
-          if (tile >= 2) wait(kQFree + st, (tile >> 1) - 1, 61);
-          if (leader) {
-            const uint32_t q = sbase + L::kOffQ + st * 2 * L::kTileBytes, g = q + L::kTileBytes;
-            ptx::mbar_expect_tx(bar(kQFull + st), 2 * L::kTileBytes);
+    } else if (warp == 12) {
+      // =============================== MMA issue =================================================
+      uint32_t tile = 0, kts = 0, q_tails = 0, g_tails = 0;
+      const uint32_t id_dkv = ptx::idesc_bf16(kTile, HD, 0, 1);  // dV, dK: A K-major, B (dO / Q) MN-major
+      const uint32_t id_dq = ptx::idesc_bf16(kTile, HD, 1, 1);   // dQ: A (dS) and B (K) MN-major
+      const uint64_t k_k = ptx::smem_desc_sw128(sbase + L::kOffK, 16, 1024), v_k = ptx::smem_desc_sw128(sbase + L::kOffV, 16, 1024);
+      const uint64_t k_mn = ptx::smem_desc_sw128(sbase + L::kOffK, kChunk, 1024);
+      const uint64_t ds_k = ptx::smem_desc_sw128(sbase + L::kOffDs, 16, 1024), ds_mn = ptx::smem_desc_sw128(sbase + L::kOffDs, kChunk, 1024);
+      const uint64_t q_k = ptx::smem_desc_sw128(sbase + L::kOffQ, 16, 1024), q_mn = ptx::smem_desc_sw128(sbase + L::kOffQ, kChunk, 1024);
+      const uint64_t g_k = ptx::smem_desc_sw128(sbase + L::kOffG, 16, 1024), g_mn = ptx::smem_desc_sw128(sbase + L::kOffG, kChunk, 1024);
+      constexpr uint32_t kStage = L::kTileBytes >> 4;
+      // contraction over head_dim: both operands K-major, [128 rows][64] chunks
+      auto nt = [&](uint32_t d, uint64_t da, uint64_t db, uint32_t boff, int n16) {
+        const uint32_t idesc = ptx::idesc_bf16(kTile, 0, 0, 0) | ((uint32_t)n16 << 18);
 #pragma unroll
-            for (int c = 0; c < HD / 64; ++c) {
-              ptx::tma_load_4d(q + c * kChunk, &maps.q, bar(kQFull + st), 64 * c, it.g * a.G, t.slot, it.b);
-              ptx::tma_load_4d(g + c * kChunk, &maps.g, bar(kQFull + st), 64 * c, it.g * a.G, t.slot, it.b);
+        for (int ks = 0; ks < HD / 16; ++ks) {
+          const uint32_t off = (uint32_t)(ks >> 2) * (kChunk >> 4) + (uint32_t)(ks & 3) * 2;
+          ptx::mma_ss_lohi(d, (uint32_t)da + off, (uint32_t)(da >> 32), (uint32_t)db + boff + off, (uint32_t)(db >> 32), idesc, ks > 0);
+        }
+      };
+      for (;;) {
+        const int idx = next_item();
+        if (idx < 0) break;
+        const Item it = decode(a, idx);
+        for (int kt = 0; kt < it.n_kt; ++kt, ++kts) {
+          const RowList rows = rows_of(a, it, kt);
+          const int keys16 = (min(kTile, it.l0 + it.len - kt * kTile) + 15) >> 4;
+          wait(kKvFull, kts, 64);
+          auto issue_s = [&](uint32_t no, int i) {  // S^T of row tile i (tile number no)
+            const RowTile t = row_tile(a, it, rows, i);
+            wait(kQFull + (no & 1u), no >> 1, 65);
+            if (t.nrow < kTile) wait(kQTail, q_tails++, 66);
+            ptx::tc_fence_after_sync();
+            if (ptx::elect_one()) {
+              nt(tmem + kColS, k_k, q_k, (no & 1u) * kStage, (t.nrow + 15) >> 4);
+              ptx::mma_commit(bar(kSFull));
             }
+          };
+          for (int i = 0; i < rows.n; ++i, ++tile) {
+            const RowTile t = row_tile(a, it, rows, i);
+            const uint32_t so = (tile & 1u) * kStage;
+            const int r16 = (t.nrow + 15) >> 4;
+            if (i == 0) issue_s(tile, 0);
+            wait(kGFull, tile, 67);
+            if (t.nrow < kTile) wait(kGTail, g_tails++, 68);
+            if (tile > 0) wait(kDqFree, tile - 1, 69);  // dQ of the previous tile has left these columns
+            ptx::tc_fence_after_sync();
+            if (ptx::elect_one()) {
+              nt(tmem + kColDp, v_k, g_k, 0, r16);
+              ptx::mma_commit(bar(kDpFull));
+            }
+            wait(kPFull, tile, 70);
+            if (i == 0 && kts > 0) wait(kAccFree, kts - 1, 71);  // dV and dK of the previous key tile have been read out
+            ptx::tc_fence_after_sync();
+            if (ptx::elect_one()) {  // dV += P^T dO: each warp group wrote its 64 columns of P over the first half of its columns of S
+              for (int ks = 0; ks < r16; ++ks)
+                ptx::mma_ts_lohi(tmem + kColDv, tmem + kColS + (uint32_t)(ks >> 2) * 64 + (uint32_t)(ks & 3) * 8,
+                                 (uint32_t)g_mn + (uint32_t)ks * 128, (uint32_t)(g_mn >> 32), id_dkv, (i > 0 || ks > 0) ? 1u : 0u);
+              ptx::mma_commit(bar(kGFree));
+            }
+            __syncwarp();
+            if (i + 1 < rows.n) issue_s(tile + 1, i + 1);  // (behind dV, which reads P out of the same columns)
+            wait(kDsFull, tile, 72);
+            ptx::tc_fence_after_sync();
+            if (ptx::elect_one()) {
+              for (int ks = 0; ks < r16; ++ks)
+                ptx::mma_ss_lohi(tmem + kColDk, (uint32_t)ds_k + (uint32_t)(ks >> 2) * (kChunk >> 4) + (uint32_t)(ks & 3) * 2,
+                                 (uint32_t)(ds_k >> 32), (uint32_t)q_mn + so + (uint32_t)ks * 128, (uint32_t)(q_mn >> 32), id_dkv,
+                                 (i > 0 || ks > 0) ? 1u : 0u);
+              ptx::mma_commit(bar(kQFree + (tile & 1u)));
+              for (int ks = 0; ks < keys16; ++ks)
+                ptx::mma_ss_lohi(tmem + kColDp, (uint32_t)ds_mn + (uint32_t)ks * 128, (uint32_t)(ds_mn >> 32),
+                                 (uint32_t)k_mn + (uint32_t)ks * 128, (uint32_t)(k_mn >> 32), id_dq, ks > 0);
+              ptx::mma_commit(bar(kDqFull));
+              if (i + 1 == rows.n) ptx::mma_commit(bar(kAccFull));
+            }
+            __syncwarp();
           }
-          float* const col = reinterpret_cast<float*>(smem + L::kOffCol) + st * 2 * kTile;
+        }
+      }
+    } else {
+      // =============================== K / V, partial row tiles ==================================
+      const int t64 = tid - 14 * 32;
+      uint32_t tile = 0, kts = 0;
+      auto zero_rows = [&](uint32_t off, int nrow) {  // rows [nrow, 128) of a tile: other tokens' values, whatever they are
 #pragma unroll
-          for (int j = 0; j < kTile / 32; ++j) {
-            const int c = lane + 32 * j;
-            float nl = -INFINITY, dl = 0.f;  // beyond the block: P = 0
-            if (c < t.nrow) {
-              const size_t id = ((size_t)it.b * a.N + it.g * a.G + (c & (a.G - 1))) * a.S + t.slot + (c >> a.g_shift);
-              nl = a.lse[id] * -1.4426950408889634f;
-              dl = a.delta[id];
-            }
-            col[c] = nl;
-            col[kTile + c] = dl;
+        for (int c = 0; c < HD / 64; ++c) {
+          uint4* const z = reinterpret_cast<uint4*>(smem + off + c * kChunk) + nrow * 8;
+          for (int x = t64; x < (kTile - nrow) * 8; x += 64) z[x] = make_uint4(0, 0, 0, 0);
+        }
+        ptx::fence_proxy_async_smem();
+      };
+      for (;;) {
+        const int idx = next_item();
+        if (idx < 0) break;
+        const Item it = decode(a, idx);
+        const __nv_bfloat16* kb = reinterpret_cast<const __nv_bfloat16*>(a.k.ptr) + (int64_t)it.b * a.k.sb + (int64_t)it.g * a.k.sh;
+        const __nv_bfloat16* vb = reinterpret_cast<const __nv_bfloat16*>(a.v.ptr) + (int64_t)it.b * a.v.sb + (int64_t)it.g * a.v.sh;
+        for (int kt = 0; kt < it.n_kt; ++kt, ++kts) {
+          if (kts > 0) wait(kAccFull, kts - 1, 73);  // every product of the previous key tile is complete
+          constexpr int kPieces = HD / 8;
+          const int c = t64 % kPieces;
+#pragma unroll 8
+          for (int r = t64 / kPieces; r < kTile; r += 64 / kPieces) {
+            const int j = kt * kTile + r;
+            const bool ok = j < it.l0 + it.len;
+            const int slot = !ok ? it.start : j < it.l0 ? it.s0 + j : it.start + j - it.l0;
+            const uint32_t off = (uint32_t)(c >> 3) * kChunk + (uint32_t)r * 128u + (uint32_t)(((c & 7) ^ (r & 7)) << 4);
+            cp_async16_zfill(smem + L::kOffK + off, kb + (int64_t)slot * a.k.ss + c * 8, ok);
+            cp_async16_zfill(smem + L::kOffV + off, vb + (int64_t)slot * a.v.ss + c * 8, ok);
           }
-          __syncwarp();
-          if (leader) ptx::mbar_arrive(bar(kQFull + st));
+          cp_async_commit();
+          cp_async_wait<0>();
+          ptx::fence_proxy_async_smem();
+          arrive(kKvFull);
+          const RowList rows = rows_of(a, it, kt);
+          for (int i = 0; i < rows.n; ++i, ++tile) {
+            // (these warps see every tile, whole ones too: a parity wait must not skip phases)
+            const RowTile t = row_tile(a, it, rows, i);
+            wait(kQFull + (tile & 1u), tile >> 1, 74);
+            if (t.nrow < kTile) {
+              zero_rows(L::kOffQ + (tile & 1u) * L::kTileBytes, t.nrow);
+              arrive(kQTail);
+            }
+            arrive(kQFree + (tile & 1u));
+            wait(kGFull, tile, 75);
+            if (t.nrow < kTile) {
+              zero_rows(L::kOffG, t.nrow);
+              arrive(kGTail);
+            }
+            arrive(kGFree);
+          }
         }
       }
     }
-  } else if (warp == 8) {
-    // =============================== MMA issue ===================================================
-    uint32_t tile = 0, kts = 0, tails = 0;
-    const uint32_t id_dkv = ptx::idesc_bf16(kTile, HD, 0, 1);  // dV, dK: A K-major, B (dO / Q) MN-major
-    const uint32_t id_dq = ptx::idesc_bf16(kTile, HD, 1, 1);   // dQ: A (dS) and B (K) MN-major
-    const uint64_t k_k = ptx::smem_desc_sw128(sbase + L::kOffK, 16, 1024), v_k = ptx::smem_desc_sw128(sbase + L::kOffV, 16, 1024);
-    const uint64_t k_mn = ptx::smem_desc_sw128(sbase + L::kOffK, kChunk, 1024);
-    const uint64_t ds_k = ptx::smem_desc_sw128(sbase + L::kOffDs, 16, 1024), ds_mn = ptx::smem_desc_sw128(sbase + L::kOffDs, kChunk, 1024);
-    const uint64_t q_k = ptx::smem_desc_sw128(sbase + L::kOffQ, 16, 1024), q_mn = ptx::smem_desc_sw128(sbase + L::kOffQ, kChunk, 1024);
-    constexpr uint32_t kStage = (2 * L::kTileBytes) >> 4, kOfG = L::kTileBytes >> 4;
-    // contraction over head_dim: both operands K-major, [128 rows][64] chunks
-    auto nt = [&](uint32_t d, uint64_t da, uint64_t db, uint32_t boff, int n16) {
-      const uint32_t idesc = ptx::idesc_bf16(kTile, 0, 0, 0) | ((uint32_t)n16 << 18);
-#pragma unroll
-      for (int ks = 0; ks < HD / 16; ++ks) {
-        const uint32_t off = (uint32_t)(ks >> 2) * (kChunk >> 4) + (uint32_t)(ks & 3) * 2;
-        ptx::mma_ss_lohi(d, (uint32_t)da + off, (uint32_t)(da >> 32), (uint32_t)db + boff + off, (uint32_t)(db >> 32), idesc, ks > 0);
-      }
-    };
-    for (;;) {
-      const int idx = next_item();
-      if (idx < 0) break;
-      const Item it = decode(a, idx);
-      for (int kt = 0; kt < it.n_kt; ++kt, ++kts) {
-        const RowList rows = rows_of(a, it, kt);
-        const int keys16 = (min(kTile, it.l0 + it.len - kt * kTile) + 15) >> 4;
-        wait(kKvFull, kts, 62);
-        auto issue_s = [&](uint32_t no, int i) {  // S^T of row tile i (tile number no)
-          const RowTile t = row_tile(a, it, rows, i);
-          wait(kQFull + (no & 1u), no >> 1, 63);
-          if (t.nrow < kTile) wait(kTail, tails++, 64);
-          ptx::tc_fence_after_sync();
-          if (ptx::elect_one()) {
-            nt(tmem + kColS, k_k, q_k, (no & 1u) * kStage, (t.nrow + 15) >> 4);
-            ptx::mma_commit(bar(kSFull));
-          }
-        };
-        for (int i = 0; i < rows.n; ++i, ++tile) {
-          const RowTile t = row_tile(a, it, rows, i);
-          const uint32_t so = (tile & 1u) * kStage;
-          const int r16 = (t.nrow + 15) >> 4;
-          if (i == 0) issue_s(tile, 0);
-          if (tile > 0) wait(kDqFree, tile - 1, 65);  // dQ of the previous tile has left these columns
-          ptx::tc_fence_after_sync();
-          if (ptx::elect_one()) {
-            nt(tmem + kColDp, v_k, q_k, so + kOfG, r16);
-            ptx::mma_commit(bar(kDpFull));
-          }
-          wait(kPFull, tile, 66);
-          ptx::tc_fence_after_sync();
-          if (ptx::elect_one()) {  // dV += P^T dO: each warp group wrote its 64 columns of P over the first half of its columns of S
-            for (int ks = 0; ks < r16; ++ks)
-              ptx::mma_ts_lohi(tmem + kColDv, tmem + kColS + (uint32_t)(ks >> 2) * 64 + (uint32_t)(ks & 3) * 8,
-                               (uint32_t)q_mn + so + kOfG + (uint32_t)ks * 128, (uint32_t)(q_mn >> 32), id_dkv, (i > 0 || ks > 0) ? 1u : 0u);
-          }
-          __syncwarp();
-          if (i + 1 < rows.n) issue_s(tile + 1, i + 1);  // (behind dV, which reads P out of the same columns)
-          wait(kDsFull, tile, 67);
-          ptx::tc_fence_after_sync();
-          if (ptx::elect_one()) {
-            for (int ks = 0; ks < r16; ++ks)
-              ptx::mma_ss_lohi(tmem + kColDk, (uint32_t)ds_k + (uint32_t)(ks >> 2) * (kChunk >> 4) + (uint32_t)(ks & 3) * 2,
-                               (uint32_t)(ds_k >> 32), (uint32_t)q_mn + so + (uint32_t)ks * 128, (uint32_t)(q_mn >> 32), id_dkv,
-                               (i > 0 || ks > 0) ? 1u : 0u);
-            ptx::mma_commit(bar(kQFree + (tile & 1u)));
-            for (int ks = 0; ks < keys16; ++ks)
-              ptx::mma_ss_lohi(tmem + kColDp, (uint32_t)ds_mn + (uint32_t)ks * 128, (uint32_t)(ds_mn >> 32),
-                               (uint32_t)k_mn + (uint32_t)ks * 128, (uint32_t)(k_mn >> 32), id_dq, ks > 0);
-            ptx::mma_commit(bar(kDqFull));
-            if (i + 1 == rows.n) ptx::mma_commit(bar(kAccFull));
-          }
-          __syncwarp();
-        }
-      }
-    }
-  } else {
-    // =============================== element-wise part, loads of K / V, outputs ===================
-    const int wg = warp >> 2, row = tid & 127;
+  } else if (warp >= 8) {
+    // =============================== outputs =====================================================
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 120;");
+    const int row = tid & 127;
     const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    uint32_t tile = 0, kts = 0;
-    constexpr int kPartThreads = 128 * (HD / 64);  // threads that drain dQ: 64 columns each
-    // This warp's 4 KB of the dS buffer, 32 rows of 128 bytes: outputs pass through it between the last product that reads
-    // dS and the next dS, so that they leave as whole rows by TMA.  (A thread owns a row: stored directly, an instruction
-    // touched 32 lines, and these stores took more time than the products.)
-    const uint32_t slab = sbase + L::kOffDs + (uint32_t)wg * kChunk + (uint32_t)(warp & 3) * 4096u;
-    uint8_t* const slab_row = smem + L::kOffDs + wg * kChunk + row * 128;
-    auto put = [&](int piece, uint4 w) { *reinterpret_cast<uint4*>(slab_row + ((piece ^ (row & 7)) << 4)) = w; };
-    auto slab_free = [&]() {  // the warp's earlier transfers have read it
-      if (lane == 0) ptx::bulk_wait_read();
+    uint32_t tile = 0, kts = 0, fills = 0;
+    // 32 rows of 128 bytes pass through one of the warp's two 4 KB slabs, so that they leave as whole rows by TMA.  (A thread
+    // owns a row: stored directly, one instruction touches 32 lines.)
+    const uint32_t slab0 = sbase + L::kOffOut + (uint32_t)(warp & 3) * 8192u;
+    auto slab = [&]() { return slab0 + (fills & 1u) * 4096u; };
+    auto put = [&](int piece, uint4 w) {
+      *reinterpret_cast<uint4*>(smem + (slab() - sbase) + lane * 128 + ((piece ^ (lane & 7)) << 4)) = w;
+    };
+    auto begin_fill = [&]() {  // the slab's previous transfer has read it
+      if (lane == 0) ptx::bulk_wait_read_but_one();
+      __syncwarp();
+    };
+    auto end_fill = [&]() {  // fill visible to the TMA; the caller issues from lane 0
+      ptx::fence_proxy_async_smem();
       __syncwarp();
     };
     auto put_f32 = [&](const uint32_t (&x)[32], float f) {  // 32 columns
@@ -367,197 +450,183 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
                         pack_bf16(__uint_as_float(x[i + 4]) * f, __uint_as_float(x[i + 5]) * f),
                         pack_bf16(__uint_as_float(x[i + 6]) * f, __uint_as_float(x[i + 7]) * f));
     };
-    auto arrive = [&](int i) {
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(bar(i));
-    };
 
-    // K and V of list positions [128 kt, 128 kt + 128) -> shared memory, zero beyond the list
-    auto load_kv = [&](const Item& it, int kt) {
-      constexpr int kPieces = HD / 8;
-      const __nv_bfloat16* kb = reinterpret_cast<const __nv_bfloat16*>(a.k.ptr) + (int64_t)it.b * a.k.sb + (int64_t)it.g * a.k.sh;
-      const __nv_bfloat16* vb = reinterpret_cast<const __nv_bfloat16*>(a.v.ptr) + (int64_t)it.b * a.v.sb + (int64_t)it.g * a.v.sh;
-#pragma unroll 4
-      for (int i = tid; i < kTile * kPieces; i += kComputeThreads) {
-        const int r = i / kPieces, c = i % kPieces, j = kt * kTile + r;
-        const bool ok = j < it.l0 + it.len;
-        const int slot = !ok ? it.start : j < it.l0 ? it.s0 + j : it.start + j - it.l0;
-        const uint32_t off = (uint32_t)(c >> 3) * kChunk + (uint32_t)r * 128u + (uint32_t)(((c & 7) ^ (r & 7)) << 4);
-        cp_async16_zfill(smem + L::kOffK + off, kb + (int64_t)slot * a.k.ss + c * 8, ok);
-        cp_async16_zfill(smem + L::kOffV + off, vb + (int64_t)slot * a.v.ss + c * 8, ok);
-      }
-      cp_async_commit();
-    };
-
-    // dV (warps 0-3) or dK (warps 4-7) of one key tile: thread = key
+    // dV, then dK of a key tile: thread = key
     auto drain_acc = [&](const Item& it, int kt) {
       const int j = kt * kTile + row, jw = kt * kTile + (warp & 3) * 32;  // this key, the warp's first
       const int n_list = it.l0 + it.len;
-      const float f = wg ? a.scale : 1.f;
       const int pre_end = a.pre == nullptr ? 0 : it.m == 0 ? it.len : it.l0;  // keys whose sums other items share
       const bool whole = jw >= pre_end && jw + 32 <= n_list;                  // 32 own keys
       const bool mine = j >= pre_end && j < n_list;
-      const View& out = wg ? a.dk : a.dv;
-      __nv_bfloat16* const dst = reinterpret_cast<__nv_bfloat16*>(out.ptr) + (int64_t)it.b * out.sb + (int64_t)it.g * out.sh +
-                                 (int64_t)(it.start + j - it.l0) * out.ss;
 #pragma unroll 1
-      for (int c0 = 0; c0 < HD; c0 += 32) {
-        uint32_t x[32];
+      for (int x = 0; x < 2 * HD; x += 32) {
+        const bool is_k = x >= HD;
+        const int c0 = x & (HD - 1);
+        const float f = is_k ? a.scale : 1.f;
+        uint32_t v[32];
         __syncwarp();
-        ptx::tmem_ld32(lanes + (wg ? kColDk : kColDv) + (uint32_t)c0, x);
-        ptx::tmem_wait_ld(x);
+        ptx::tmem_ld32(lanes + (is_k ? kColDk : kColDv) + (uint32_t)c0, v);
+        ptx::tmem_wait_ld(v);
+        if (x + 32 == 2 * HD) {
+          ptx::tc_fence_before_sync();
+          arrive(kAccFree);
+        }
         if (jw < pre_end) {  // (rows beyond the prefix go to rows of the sums that nothing reads)
-          slab_free();
-          put_f32(x, f);
-          ptx::fence_proxy_async_smem();
-          __syncwarp();
+          begin_fill();
+          put_f32(v, f);
+          end_fill();
           if (lane == 0) {
-            ptx::tma_add_4d(&maps.pre, slab, c0, ((wg ? 0 : a.B) + it.b) * a.Nk + it.g, jw, 0);
+            ptx::tma_add_4d(&maps.pre, slab(), c0, ((is_k ? 0 : a.B) + it.b) * a.Nk + it.g, jw, 0);
             ptx::bulk_commit();
           }
+          ++fills;
         }
         if (whole) {
-          if ((c0 & 32) == 0) slab_free();
+          if ((c0 & 32) == 0) begin_fill();
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) put(((c0 & 32) + i) >> 3, pack8(x, i, f));
+          for (int i = 0; i < 32; i += 8) put(((c0 & 32) + i) >> 3, pack8(v, i, f));
           if (c0 & 32) {
-            ptx::fence_proxy_async_smem();
-            __syncwarp();
+            end_fill();
             if (lane == 0) {
-              ptx::tma_store_4d(wg ? &maps.dk : &maps.dv, slab, c0 - 32, it.g, it.start + jw - it.l0, it.b);
+              ptx::tma_store_4d(is_k ? &maps.dk : &maps.dv, slab(), c0 - 32, it.g, it.start + jw - it.l0, it.b);
               ptx::bulk_commit();
             }
+            ++fills;
           }
         } else if (mine) {
+          const View& out = is_k ? a.dk : a.dv;
+          __nv_bfloat16* const dst = reinterpret_cast<__nv_bfloat16*>(out.ptr) + (int64_t)it.b * out.sb + (int64_t)it.g * out.sh +
+                                     (int64_t)(it.start + j - it.l0) * out.ss + c0;
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) *reinterpret_cast<uint4*>(dst + c0 + i) = pack8(x, i, f);
+          for (int i = 0; i < 32; i += 8) *reinterpret_cast<uint4*>(dst + i) = pack8(v, i, f);
         }
       }
     };
 
-    // dQ of one (key tile, row tile) pair: thread = row, columns [64 wg, + 64) (head_dim 64: warps 0-3 only)
-    auto drain_dq = [&](const Item& it, int kt, const RowTile& t) {
-      if (wg * 64 >= HD) {
-        arrive(kDqFree);
-        return;
-      }
-      const int tok = t.t0 + (row >> a.g_shift), head = it.g * a.G + (row & (a.G - 1));
-      const int row_w = (warp & 3) * 32, tok_w = t.t0 + (row_w >> a.g_shift);  // the warp's first row
-      const bool valid = row < t.nrow;
-      const bool sum32 = a.M > 1 && (!t.own || it.m == a.M - 1);  // rows of the query block
-      // own rows: the key tiles that see this row tile are 0 .. last
-      const int last = t.own ? (it.l0 + min(it.len, t.t0 + (kTile >> a.g_shift)) - 1) / kTile : 0;
-      float4* const part = reinterpret_cast<float4*>(a.part) + ((size_t)blockIdx.x * a.row_tiles + t.r) * 16 * kPartThreads + tid;
-      __nv_bfloat16* const dst = reinterpret_cast<__nv_bfloat16*>(a.dq.ptr) + (int64_t)it.b * a.dq.sb + (int64_t)head * a.dq.sh +
-                                 (int64_t)(it.start + tok) * a.dq.ss + wg * 64;
-      const float f = a.scale;
-#pragma unroll 1
-      for (int c0 = 0; c0 < 64; c0 += 32) {
-        uint32_t x[32];
-        __syncwarp();
-        ptx::tmem_ld32(lanes + kColDp + (uint32_t)(wg * 64 + c0), x);
-        ptx::tmem_wait_ld(x);
-        if (c0 > 0) {  // out of tensor memory: the next tile's dP may overwrite it
-          ptx::tc_fence_before_sync();
-          arrive(kDqFree);
-        }
-        if (row_w >= t.nrow) continue;
-        if (sum32) {  // (rows beyond the block go to rows of the sums that nothing reads)
-          slab_free();
-          put_f32(x, f);
-          ptx::fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            ptx::tma_add_4d(&maps.dq32, slab, wg * 64 + c0, it.g * a.G, tok_w, it.b);
-            ptx::bulk_commit();
-          }
-          continue;
-        }
-        if (kt > 0) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float4 y = part[(size_t)(c0 / 4 + i) * kPartThreads];
-            x[4 * i] = __float_as_uint(__uint_as_float(x[4 * i]) + y.x);
-            x[4 * i + 1] = __float_as_uint(__uint_as_float(x[4 * i + 1]) + y.y);
-            x[4 * i + 2] = __float_as_uint(__uint_as_float(x[4 * i + 2]) + y.z);
-            x[4 * i + 3] = __float_as_uint(__uint_as_float(x[4 * i + 3]) + y.w);
-          }
-        }
-        if (kt < last) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            part[(size_t)(c0 / 4 + i) * kPartThreads] =
-                make_float4(__uint_as_float(x[4 * i]), __uint_as_float(x[4 * i + 1]), __uint_as_float(x[4 * i + 2]),
-                            __uint_as_float(x[4 * i + 3]));
-        } else if (row_w + 32 <= t.nrow) {
-          if (c0 == 0) slab_free();
-#pragma unroll
-          for (int i = 0; i < 32; i += 8) put((c0 + i) >> 3, pack8(x, i, f));
-          if (c0 > 0) {
-            ptx::fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              ptx::tma_store_4d(&maps.dq, slab, wg * 64, it.g * a.G, it.start + tok_w, it.b);
-              ptx::bulk_commit();
-            }
-          }
-        } else if (valid) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 8) *reinterpret_cast<uint4*>(dst + c0 + i) = pack8(x, i, f);
-        }
-      }
-    };
-
-    Item prev{};
-    int prev_kt = -1;
     for (;;) {
       const int idx = next_item();
       if (idx < 0) break;
       const Item it = decode(a, idx);
       for (int kt = 0; kt < it.n_kt; ++kt, ++kts) {
-        if (prev_kt >= 0) wait(kAccFull, kts - 1, 70);  // every product of the previous key tile is complete
-        load_kv(it, kt);
-        if (prev_kt >= 0) {
+        const RowList rows = rows_of(a, it, kt);
+        for (int i = 0; i < rows.n; ++i, ++tile) {
+          // dQ: thread = row
+          const RowTile t = row_tile(a, it, rows, i);
+          const int row_w = (warp & 3) * 32, tok_w = t.t0 + (row_w >> a.g_shift);  // the warp's first row
+          const bool sum32 = a.M > 1 && (!t.own || it.m == a.M - 1);               // rows of the query block
+          // own rows: the key tiles that see this row tile are 0 .. last
+          const int last = t.own ? (it.l0 + min(it.len, t.t0 + (kTile >> a.g_shift)) - 1) / kTile : 0;
+          float4* const part = reinterpret_cast<float4*>(a.part) + ((size_t)blockIdx.x * a.row_tiles + t.r) * (HD / 4) * 128 + row;
+          const bool take = !sum32 && kt > 0, leave = !sum32 && kt < last;
+          float4 y[2][8];  // the partial sum so far, fetched ahead of the product
+          auto fetch = [&](int ch) {
+            if (take) {
+#pragma unroll
+              for (int q = 0; q < 8; ++q) y[ch & 1][q] = part[(size_t)(ch * 8 + q) * 128];
+            }
+          };
+          fetch(0);
+          fetch(1);
+          wait(kDqFull, tile, 76);
           ptx::tc_fence_after_sync();
-          drain_acc(prev, prev_kt);
-          ptx::tc_fence_before_sync();
+          const float f = a.scale;
+#pragma unroll
+          for (int ch = 0; ch < HD / 32; ++ch) {
+            uint32_t v[32];
+            __syncwarp();
+            ptx::tmem_ld32(lanes + kColDp + (uint32_t)ch * 32, v);
+            ptx::tmem_wait_ld(v);
+            if (ch + 1 == HD / 32) {  // out of tensor memory: the next tile's dP may overwrite it
+              ptx::tc_fence_before_sync();
+              arrive(kDqFree);
+            }
+            if (row_w >= t.nrow) continue;
+            if (sum32) {  // (rows beyond the block go to rows of the sums that nothing reads)
+              begin_fill();
+              put_f32(v, f);
+              end_fill();
+              if (lane == 0) {
+                ptx::tma_add_4d(&maps.dq32, slab(), ch * 32, it.g * a.G, tok_w, it.b);
+                ptx::bulk_commit();
+              }
+              ++fills;
+              continue;
+            }
+            if (take) {
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                const float4 z = y[ch & 1][q];
+                v[4 * q] = __float_as_uint(__uint_as_float(v[4 * q]) + z.x);
+                v[4 * q + 1] = __float_as_uint(__uint_as_float(v[4 * q + 1]) + z.y);
+                v[4 * q + 2] = __float_as_uint(__uint_as_float(v[4 * q + 2]) + z.z);
+                v[4 * q + 3] = __float_as_uint(__uint_as_float(v[4 * q + 3]) + z.w);
+              }
+              if (ch + 2 < HD / 32) fetch(ch + 2);
+            }
+            if (leave) {
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                part[(size_t)(ch * 8 + q) * 128] = make_float4(__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]),
+                                                               __uint_as_float(v[4 * q + 2]), __uint_as_float(v[4 * q + 3]));
+            } else if (row_w + 32 <= t.nrow) {
+              if ((ch & 1) == 0) begin_fill();
+#pragma unroll
+              for (int q = 0; q < 32; q += 8) put((ch & 1) * 4 + (q >> 3), pack8(v, q, f));
+              if (ch & 1) {
+                end_fill();
+                if (lane == 0) {
+                  ptx::tma_store_4d(&maps.dq, slab(), (ch - 1) * 32, it.g * a.G, it.start + tok_w, it.b);
+                  ptx::bulk_commit();
+                }
+                ++fills;
+              }
+            } else if (row < t.nrow) {
+              __nv_bfloat16* const dst = reinterpret_cast<__nv_bfloat16*>(a.dq.ptr) + (int64_t)it.b * a.dq.sb +
+                                         (int64_t)(it.g * a.G + (row & (a.G - 1))) * a.dq.sh +
+                                         (int64_t)(t.slot + (row >> a.g_shift)) * a.dq.ss + ch * 32;
+#pragma unroll
+              for (int q = 0; q < 32; q += 8) *reinterpret_cast<uint4*>(dst + q) = pack8(v, q, f);
+            }
+          }
         }
-        prev = it;
-        prev_kt = kt;
-        cp_async_wait<0>();
-        ptx::fence_proxy_async_smem();
-        arrive(kKvFull);
+        wait(kAccFull, kts, 77);
+        ptx::tc_fence_after_sync();
+        drain_acc(it, kt);
+      }
+    }
+    if (lane == 0) ptx::bulk_wait();
+  } else {
+    // =============================== element-wise part ===========================================
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
+    const int wg = warp >> 2, row = tid & 127;
+    const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)wg * 64;
+    uint8_t* const ds_row = smem + L::kOffDs + wg * kChunk + row * 128;
+    uint32_t tile = 0;
+    for (;;) {
+      const int idx = next_item();
+      if (idx < 0) break;
+      const Item it = decode(a, idx);
+      for (int kt = 0; kt < it.n_kt; ++kt) {
         const RowList rows = rows_of(a, it, kt);
         const int j = kt * kTile + row;  // this thread's key: list position
         for (int i = 0; i < rows.n; ++i, ++tile) {
           const RowTile t = row_tile(a, it, rows, i);
           const uint32_t st = tile & 1u;
-          wait(kQFull + st, tile >> 1, 71);
-          if (t.nrow < kTile) {  // rows beyond the block hold other tokens: zero them, whatever they are
-            const int per = kTile - t.nrow;
-#pragma unroll
-            for (int c = 0; c < 2 * (HD / 64); ++c) {
-              uint4* const z = reinterpret_cast<uint4*>(smem + L::kOffQ + st * 2 * L::kTileBytes + c * kChunk) + t.nrow * 8;
-              for (int x = tid; x < per * 8; x += kComputeThreads) z[x] = make_uint4(0, 0, 0, 0);
-            }
-            ptx::fence_proxy_async_smem();
-            arrive(kTail);
-          }
           const float* const col = reinterpret_cast<const float*>(smem + L::kOffCol) + st * 2 * kTile + wg * 64;
           // Row-tile columns below cmin do not see this key: causality inside the block; the prefix is not the query
           // rows' business here; positions beyond the list are no keys.
           int cmin = t.own ? (j - it.l0 - t.t0) * a.G : (j < it.l0 ? kTile : 0);
           if (j >= it.l0 + it.len) cmin = kTile;
           cmin -= wg * 64;
-
-          wait(kSFull, tile, 72);
+          wait(kQFull + st, tile >> 1, 78);
+          wait(kSFull, tile, 79);
           ptx::tc_fence_after_sync();
           __syncwarp();
           float p[64];
           {
             uint32_t s[64];
-            ptx::tmem_ld32(lanes + kColS + (uint32_t)wg * 64, *reinterpret_cast<uint32_t (*)[32]>(&s[0]));
-            ptx::tmem_ld32(lanes + kColS + (uint32_t)wg * 64 + 32, *reinterpret_cast<uint32_t (*)[32]>(&s[32]));
+            ptx::tmem_ld32(lanes + kColS, *reinterpret_cast<uint32_t (*)[32]>(&s[0]));
+            ptx::tmem_ld32(lanes + kColS + 32, *reinterpret_cast<uint32_t (*)[32]>(&s[32]));
             ptx::tmem_wait_ld(s);
 #pragma unroll
             for (int c = 0; c < 64; c += 4) {
@@ -576,25 +645,19 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
             uint32_t pk[32];
 #pragma unroll
             for (int c = 0; c < 32; ++c) pk[c] = pack_bf16(p[2 * c], p[2 * c + 1]);
-            ptx::tmem_st32(lanes + kColS + (uint32_t)wg * 64, pk);
+            ptx::tmem_st32(lanes + kColS, pk);
             ptx::tmem_wait_st();
           }
           ptx::tc_fence_before_sync();
           arrive(kPFull);
 
-          if (i > 0) {
-            wait(kDqFull, tile - 1, 73);
-            ptx::tc_fence_after_sync();
-            drain_dq(it, kt, row_tile(a, it, rows, i - 1));
-          }
-          wait(kDpFull, tile, 74);
+          wait(kDpFull, tile, 80);  // (dP follows the reading of dQ, so every product that reads dS is complete too)
           ptx::tc_fence_after_sync();
           __syncwarp();
-          slab_free();
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             uint32_t x[32];
-            ptx::tmem_ld32(lanes + kColDp + (uint32_t)(wg * 64 + h * 32), x);
+            ptx::tmem_ld32(lanes + kColDp + (uint32_t)h * 32, x);
             ptx::tmem_wait_ld(x);
 #pragma unroll
             for (int c = 0; c < 32; c += 8) {
@@ -606,24 +669,15 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
               w.y = pack_bf16(pp[2] * (__uint_as_float(x[c + 2]) - d0.z), pp[3] * (__uint_as_float(x[c + 3]) - d0.w));
               w.z = pack_bf16(pp[4] * (__uint_as_float(x[c + 4]) - d1.x), pp[5] * (__uint_as_float(x[c + 5]) - d1.y));
               w.w = pack_bf16(pp[6] * (__uint_as_float(x[c + 6]) - d1.z), pp[7] * (__uint_as_float(x[c + 7]) - d1.w));
-              put(h * 4 + (c >> 3), w);
+              *reinterpret_cast<uint4*>(ds_row + (((h * 4 + (c >> 3)) ^ (row & 7)) << 4)) = w;
             }
           }
           ptx::fence_proxy_async_smem();
           ptx::tc_fence_before_sync();
           arrive(kDsFull);
         }
-        wait(kDqFull, tile - 1, 73);
-        ptx::tc_fence_after_sync();
-        drain_dq(it, kt, row_tile(a, it, rows, rows.n - 1));
       }
     }
-    if (prev_kt >= 0) {
-      wait(kAccFull, kts - 1, 75);
-      ptx::tc_fence_after_sync();
-      drain_acc(prev, prev_kt);
-    }
-    if (lane == 0) ptx::bulk_wait();
   }
   ptx::tc_fence_before_sync();
   __syncthreads();
@@ -644,11 +698,36 @@ __device__ __forceinline__ bool slot_in_block(const BwdTcArgs& a, int b, int s) 
 
 // delta = rowsum(dO * O): one warp per 32 slots of one (prompt, head), HD / 8 lanes per row.  The same warps write the
 // zeros of the slots outside every block; all threads clear the accumulators and the item counter.  Bound by memory:
-// reads O and dO once.
+// reads O and dO once.  The last block orders the items.
 template <int HD>
 __global__ void __launch_bounds__(256) attn_bwd_tc_prep_kernel(BwdTcArgs a, float4* zero, int64_t n_zero) {
+  if (a.order && blockIdx.x == gridDim.x - 1) {
+    // (prompt, block) pairs by length, longest first (counting sort, one bucket per 8 tokens up to 512)
+    __shared__ int first[64];
+    const int n = a.B * a.M;
+    auto bucket = [&](int i) {
+      int start, len;
+      span_of(a, i / a.M, i % a.M, start, len);
+      return 63 - min(63, (len + 7) >> 3);
+    };
+    if (threadIdx.x < 64) first[threadIdx.x] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += 256) atomicAdd(&first[bucket(i)], 1);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int sum = 0;
+      for (int i = 0; i < 64; ++i) {
+        const int c = first[i];
+        first[i] = sum;
+        sum += c;
+      }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += 256) a.order[atomicAdd(&first[bucket(i)], 1)] = i;
+    return;
+  }
   const int64_t gid = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  for (int64_t i = gid; i < n_zero; i += (int64_t)gridDim.x * 256) zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int64_t i = gid; i < n_zero; i += (int64_t)(gridDim.x - (a.order ? 1 : 0)) * 256) zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   if (gid == 0) *a.counter = 0;
   const int lane = threadIdx.x & 31;
   const int groups = (a.S + 31) / 32;
@@ -742,7 +821,7 @@ int launch(const brk_attn_bwd_params& p, BwdTcArgs a, float4* zero, int64_t n_ze
   t.pre = t.dq32;
   if (a.pre && (rc = make_tmap_f32(&t.pre, a.pre, HD, 2 * p.B * p.Nk, p.max_block_len, 1, mbl * HD, HD, 0, 1, 32))) return rc;
   const int64_t warps = (int64_t)p.B * ((p.S + 31) / 32) * p.N;
-  attn_bwd_tc_prep_kernel<HD><<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(a, zero, n_zero);
+  attn_bwd_tc_prep_kernel<HD><<<(unsigned)((warps + 7) / 8 + (a.order ? 1 : 0)), 256, 0, st>>>(a, zero, n_zero);
   BRK_CUDA(cudaGetLastError());
   BRK_CUDA(cudaFuncSetAttribute(attn_bwd_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Geo<HD>::kSmem));
   const int sms = sm_count();
@@ -765,7 +844,9 @@ bool attn_bwd_tc_supported(const brk_attn_bwd_params& p) {
   const int G = p.Nk > 0 ? p.N / p.Nk : 0;
   return p.dtype == BRK_BF16 && (p.D == 64 || p.D == 128) && (G == 1 || G == 2 || G == 4 || G == 8) && row_tiles(p) <= kMaxRowTiles;
 }
-size_t attn_bwd_tc_extra_bytes(const brk_attn_bwd_params& p) { return p.M > 2 || part_bytes(p) > 0 ? 256 + part_bytes(p) : 0; }
+// item counter and item order, then the dQ scratch
+static size_t head_bytes(const brk_attn_bwd_params& p) { return (256 + (size_t)p.B * p.M * sizeof(int) + 255) & ~(size_t)255; }
+size_t attn_bwd_tc_extra_bytes(const brk_attn_bwd_params& p) { return p.M > 2 || part_bytes(p) > 0 ? head_bytes(p) + part_bytes(p) : 0; }
 
 // ws32: the two [B, Nk, S, D] accumulators of the warp-level kernels (used for the prefix sums here), then dq32; extra: the
 // bytes of attn_bwd_tc_extra_bytes (the item counter goes into the unused accumulators when there are none)
@@ -792,7 +873,8 @@ int attn_bwd_tc_launch(const brk_attn_bwd_params& p, float* delta, float* ws32, 
   unsigned char* const x = static_cast<unsigned char*>(extra);
   const bool has_extra = attn_bwd_tc_extra_bytes(p) > 0;
   a.counter = has_extra ? reinterpret_cast<int*>(x) : reinterpret_cast<int*>(ws32);
-  a.part = part_bytes(p) ? reinterpret_cast<float*>(x + 256) : nullptr;
+  a.order = has_extra && p.M > 2 ? reinterpret_cast<int*>(x + 256) : nullptr;
+  a.part = part_bytes(p) ? reinterpret_cast<float*>(x + head_bytes(p)) : nullptr;
   float4* const zero = reinterpret_cast<float4*>(dq32 - n_pre);
   return p.D == 128 ? launch<128>(p, a, zero, (n_pre + n_q) / 4, st) : launch<64>(p, a, zero, (n_pre + n_q) / 4, st);
 }
