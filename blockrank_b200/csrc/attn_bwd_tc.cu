@@ -20,15 +20,15 @@
 //                                                 for dK, MN-major for dQ)
 //
 // Roles (512 threads, one CTA per SM, items claimed from a global counter, longest blocks first):
-//   warps 0-7   element-wise part: warp w owns lanes 32 (w % 4) and the row-tile columns 64 (w / 4) + {0..63}
+//   warps 0-7   element-wise part: warp w owns lanes 32 (w % 4) and the row-tile columns 64 (w / 4) + {0..63}; between key
+//               tiles they load K / V (cp.async, zero beyond the list, so any prefix length packs against any document)
 //   warps 8-11  outputs: dQ after every pair, dV and dK after every key tile, from tensor memory through shared memory to
 //               TMA, beside the element-wise part of the next pair
 //   warp 12     MMA issue
 //   warp 13     claims items, loads Q (two stages) and dO (one) by TMA and the columns' lse and delta
-//   warps 14-15 load K / V (cp.async, zero beyond the list, so any prefix length packs against any document) and zero the
-//               rows of a partial row tile that lie beyond its block
+//   warps 14-15 zero the rows of a partial row tile that lie beyond its block
 //
-// Order of the tensor pipe: dP(i) | dV(i) S(i+1) | dK(i) dQ(i): the exponentials of tile i + 1 run beside dK(i) / dQ(i) and
+// Order of the tensor pipe: dP(i) | dV(i) S(i+1) | dQ(i) dK(i): the exponentials of tile i + 1 run beside dQ(i) / dK(i) and
 // the dS of tile i beside dV(i) / S(i+1).  Tensor memory (head_dim 128, all 512 columns): S / P 128, dP / dQ 128, dV 128,
 // dK 128; dQ shares dP's columns, so the way dQ(i) -> read out -> dP(i+1) -> dS(i+1) is the kernel's cycle, and that is
 // why the reading has warps of its own.
@@ -69,22 +69,23 @@ constexpr uint32_t kColS = 0, kColDp = 128, kColDv = 256, kColDk = 384;
 enum {
   kQFull = 0,    // +stage  Q landed and the columns' lse / delta written (expect_tx arrival + 1)
   kQFree = 2,    // +stage  dK has read the stage (commit + 2 warps)
-  kGFull = 4,    // dO landed
-  kGFree = 5,    // dV has read it (commit + 2 warps)
-  kQTail = 6,    // the rows beyond the block zeroed in a partial Q / dO tile (2 warps)
-  kGTail = 7,
-  kSFull = 8,
-  kDpFull = 9,
-  kPFull = 10,   // P^T in tensor memory (8 warps)
-  kDsFull = 11,  // dS^T in shared memory, dP consumed (8 warps)
-  kDqFull = 12,
-  kDqFree = 13,  // dQ read out (4 warps)
-  kAccFull = 14, // every product of the key tile complete
-  kAccFree = 15, // dV, dK read out (4 warps)
-  kKvFull = 16,  // K, V of the key tile in shared memory (2 warps)
-  kItemFull = 17,  // +slot
-  kItemFree = 19,  // +slot (15 consuming warps)
-  kNumBars = 21
+  kQTail = 4,    // +stage  the rows beyond the block zeroed in a partial Q tile (2 warps).  Per stage: with one barrier the
+                 //         two tiles behind a key tile's end could both arrive before the first was waited for
+  kGFull = 6,    // dO landed
+  kGFree = 7,    // dV has read it (commit + 2 warps)
+  kGTail = 8,    // as kQTail
+  kSFull = 9,
+  kDpFull = 10,
+  kPFull = 11,   // P^T in tensor memory (8 warps)
+  kDsFull = 12,  // dS^T in shared memory, dP consumed (8 warps)
+  kDqFull = 13,
+  kDqFree = 14,  // dQ read out (4 warps)
+  kAccFull = 15, // every product of the key tile complete
+  kAccFree = 16, // dV, dK read out (4 warps)
+  kKvFull = 17,  // K, V of the key tile in shared memory (8 warps)
+  kItemFull = 18,  // +slot
+  kItemFree = 20,  // +slot (15 consuming warps)
+  kNumBars = 22
 };
 static_assert(kNumBars * 8 + 16 <= 256, "barrier area");  // + TMEM base, two item slots
 
@@ -180,9 +181,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
   if (tid == 0) {
     for (int i = 0; i < kNumBars; ++i) {
       uint32_t cnt = 1u;
-      if (i == kPFull || i == kDsFull) cnt = 8u;
+      if (i == kPFull || i == kDsFull || i == kKvFull) cnt = 8u;
       if (i == kDqFree || i == kAccFree) cnt = 4u;
-      if (i == kQFull || i == kQFull + 1 || i == kQTail || i == kGTail || i == kKvFull) cnt = 2u;
+      if (i == kQFull || i == kQFull + 1 || i == kQTail || i == kQTail + 1 || i == kGTail) cnt = 2u;
       if (i == kQFree || i == kQFree + 1 || i == kGFree) cnt = 3u;
       if (i >= kItemFree) cnt = 15u;
       ptx::mbar_init(bar(i), cnt);
@@ -225,9 +226,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
     return idx;
   };
 
-  // Registers: 512 x 128 at launch = 256 x 160 + 128 x 120 + 128 x 72.
+  // Registers: 512 x 128 at launch = 256 x 136 + 128 x 176 + 128 x 64.
   if (warp >= 12) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     if (warp == 13) {
       // =============================== loader ====================================================
       uint32_t tile = 0, pub = 0;
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
       }
     } else if (warp == 12) {
       // =============================== MMA issue =================================================
-      uint32_t tile = 0, kts = 0, q_tails = 0, g_tails = 0;
+      uint32_t tile = 0, kts = 0, q_tails0 = 0, q_tails1 = 0, g_tails = 0;
       const uint32_t id_dkv = ptx::idesc_bf16(kTile, HD, 0, 1);  // dV, dK: A K-major, B (dO / Q) MN-major
       const uint32_t id_dq = ptx::idesc_bf16(kTile, HD, 1, 1);   // dQ: A (dS) and B (K) MN-major
       const uint64_t k_k = ptx::smem_desc_sw128(sbase + L::kOffK, 16, 1024), v_k = ptx::smem_desc_sw128(sbase + L::kOffV, 16, 1024);
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
           auto issue_s = [&](uint32_t no, int i) {  // S^T of row tile i (tile number no)
             const RowTile t = row_tile(a, it, rows, i);
             wait(kQFull + (no & 1u), no >> 1, 65);
-            if (t.nrow < kTile) wait(kQTail, q_tails++, 66);
+            if (t.nrow < kTile) wait(kQTail + (no & 1u), (no & 1u) ? q_tails1++ : q_tails0++, 66);
             ptx::tc_fence_after_sync();
             if (ptx::elect_one()) {
               nt(tmem + kColS, k_k, q_k, (no & 1u) * kStage, (t.nrow + 15) >> 4);
@@ -347,15 +348,15 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
             wait(kDsFull, tile, 72);
             ptx::tc_fence_after_sync();
             if (ptx::elect_one()) {
+              for (int ks = 0; ks < keys16; ++ks)  // dQ first: the next dP waits until it has been read out
+                ptx::mma_ss_lohi(tmem + kColDp, (uint32_t)ds_mn + (uint32_t)ks * 128, (uint32_t)(ds_mn >> 32),
+                                 (uint32_t)k_mn + (uint32_t)ks * 128, (uint32_t)(k_mn >> 32), id_dq, ks > 0);
+              ptx::mma_commit(bar(kDqFull));
               for (int ks = 0; ks < r16; ++ks)
                 ptx::mma_ss_lohi(tmem + kColDk, (uint32_t)ds_k + (uint32_t)(ks >> 2) * (kChunk >> 4) + (uint32_t)(ks & 3) * 2,
                                  (uint32_t)(ds_k >> 32), (uint32_t)q_mn + so + (uint32_t)ks * 128, (uint32_t)(q_mn >> 32), id_dkv,
                                  (i > 0 || ks > 0) ? 1u : 0u);
               ptx::mma_commit(bar(kQFree + (tile & 1u)));
-              for (int ks = 0; ks < keys16; ++ks)
-                ptx::mma_ss_lohi(tmem + kColDp, (uint32_t)ds_mn + (uint32_t)ks * 128, (uint32_t)(ds_mn >> 32),
-                                 (uint32_t)k_mn + (uint32_t)ks * 128, (uint32_t)(k_mn >> 32), id_dq, ks > 0);
-              ptx::mma_commit(bar(kDqFull));
               if (i + 1 == rows.n) ptx::mma_commit(bar(kAccFull));
             }
             __syncwarp();
@@ -363,9 +364,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
         }
       }
     } else {
-      // =============================== K / V, partial row tiles ==================================
+      // =============================== partial row tiles =========================================
       const int t64 = tid - 14 * 32;
-      uint32_t tile = 0, kts = 0;
+      uint32_t tile = 0;
       auto zero_rows = [&](uint32_t off, int nrow) {  // rows [nrow, 128) of a tile: other tokens' values, whatever they are
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c) {
@@ -378,25 +379,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
         const int idx = next_item();
         if (idx < 0) break;
         const Item it = decode(a, idx);
-        const __nv_bfloat16* kb = reinterpret_cast<const __nv_bfloat16*>(a.k.ptr) + (int64_t)it.b * a.k.sb + (int64_t)it.g * a.k.sh;
-        const __nv_bfloat16* vb = reinterpret_cast<const __nv_bfloat16*>(a.v.ptr) + (int64_t)it.b * a.v.sb + (int64_t)it.g * a.v.sh;
-        for (int kt = 0; kt < it.n_kt; ++kt, ++kts) {
-          if (kts > 0) wait(kAccFull, kts - 1, 73);  // every product of the previous key tile is complete
-          constexpr int kPieces = HD / 8;
-          const int c = t64 % kPieces;
-#pragma unroll 8
-          for (int r = t64 / kPieces; r < kTile; r += 64 / kPieces) {
-            const int j = kt * kTile + r;
-            const bool ok = j < it.l0 + it.len;
-            const int slot = !ok ? it.start : j < it.l0 ? it.s0 + j : it.start + j - it.l0;
-            const uint32_t off = (uint32_t)(c >> 3) * kChunk + (uint32_t)r * 128u + (uint32_t)(((c & 7) ^ (r & 7)) << 4);
-            cp_async16_zfill(smem + L::kOffK + off, kb + (int64_t)slot * a.k.ss + c * 8, ok);
-            cp_async16_zfill(smem + L::kOffV + off, vb + (int64_t)slot * a.v.ss + c * 8, ok);
-          }
-          cp_async_commit();
-          cp_async_wait<0>();
-          ptx::fence_proxy_async_smem();
-          arrive(kKvFull);
+        for (int kt = 0; kt < it.n_kt; ++kt) {
           const RowList rows = rows_of(a, it, kt);
           for (int i = 0; i < rows.n; ++i, ++tile) {
             // (these warps see every tile, whole ones too: a parity wait must not skip phases)
@@ -404,7 +387,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
             wait(kQFull + (tile & 1u), tile >> 1, 74);
             if (t.nrow < kTile) {
               zero_rows(L::kOffQ + (tile & 1u) * L::kTileBytes, t.nrow);
-              arrive(kQTail);
+              arrive(kQTail + (tile & 1u));
             }
             arrive(kQFree + (tile & 1u));
             wait(kGFull, tile, 75);
@@ -419,7 +402,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
     }
   } else if (warp >= 8) {
     // =============================== outputs =====================================================
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 120;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 176;");
     const int row = tid & 127;
     const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     uint32_t tile = 0, kts = 0, fills = 0;
@@ -517,30 +500,32 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
           // own rows: the key tiles that see this row tile are 0 .. last
           const int last = t.own ? (it.l0 + min(it.len, t.t0 + (kTile >> a.g_shift)) - 1) / kTile : 0;
           float4* const part = reinterpret_cast<float4*>(a.part) + ((size_t)blockIdx.x * a.row_tiles + t.r) * (HD / 4) * 128 + row;
-          const bool take = !sum32 && kt > 0, leave = !sum32 && kt < last;
-          float4 y[2][8];  // the partial sum so far, fetched ahead of the product
-          auto fetch = [&](int ch) {
-            if (take) {
+          const bool take = !sum32 && kt > 0 && row_w < t.nrow, leave = !sum32 && kt < last;
+          float all[HD / 32][32] = {};
+          if (take) {  // the partial sum so far: on its way while the product is computed
 #pragma unroll
-              for (int q = 0; q < 8; ++q) y[ch & 1][q] = part[(size_t)(ch * 8 + q) * 128];
-            }
-          };
-          fetch(0);
-          fetch(1);
+            for (int ch = 0; ch < HD / 32; ++ch)
+#pragma unroll
+              for (int q = 0; q < 8; ++q) *reinterpret_cast<float4*>(&all[ch][4 * q]) = part[(size_t)(ch * 8 + q) * 128];
+          }
           wait(kDqFull, tile, 76);
           ptx::tc_fence_after_sync();
+          __syncwarp();
+#pragma unroll
+          for (int ch = 0; ch < HD / 32; ++ch) {
+            uint32_t x[32];
+            ptx::tmem_ld32(lanes + kColDp + (uint32_t)ch * 32, x);
+            ptx::tmem_wait_ld(x);
+#pragma unroll
+            for (int q = 0; q < 32; ++q) all[ch][q] += __uint_as_float(x[q]);
+          }
+          ptx::tc_fence_before_sync();
+          arrive(kDqFree);  // out of tensor memory: the next tile's dP may overwrite it
+          if (row_w >= t.nrow) continue;
           const float f = a.scale;
 #pragma unroll
           for (int ch = 0; ch < HD / 32; ++ch) {
-            uint32_t v[32];
-            __syncwarp();
-            ptx::tmem_ld32(lanes + kColDp + (uint32_t)ch * 32, v);
-            ptx::tmem_wait_ld(v);
-            if (ch + 1 == HD / 32) {  // out of tensor memory: the next tile's dP may overwrite it
-              ptx::tc_fence_before_sync();
-              arrive(kDqFree);
-            }
-            if (row_w >= t.nrow) continue;
+            uint32_t (&v)[32] = *reinterpret_cast<uint32_t (*)[32]>(&all[ch]);
             if (sum32) {  // (rows beyond the block go to rows of the sums that nothing reads)
               begin_fill();
               put_f32(v, f);
@@ -551,17 +536,6 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
               }
               ++fills;
               continue;
-            }
-            if (take) {
-#pragma unroll
-              for (int q = 0; q < 8; ++q) {
-                const float4 z = y[ch & 1][q];
-                v[4 * q] = __float_as_uint(__uint_as_float(v[4 * q]) + z.x);
-                v[4 * q + 1] = __float_as_uint(__uint_as_float(v[4 * q + 1]) + z.y);
-                v[4 * q + 2] = __float_as_uint(__uint_as_float(v[4 * q + 2]) + z.z);
-                v[4 * q + 3] = __float_as_uint(__uint_as_float(v[4 * q + 3]) + z.w);
-              }
-              if (ch + 2 < HD / 32) fetch(ch + 2);
             }
             if (leave) {
 #pragma unroll
@@ -597,16 +571,37 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
     if (lane == 0) ptx::bulk_wait();
   } else {
     // =============================== element-wise part ===========================================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 136;");
     const int wg = warp >> 2, row = tid & 127;
     const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)wg * 64;
     uint8_t* const ds_row = smem + L::kOffDs + wg * kChunk + row * 128;
-    uint32_t tile = 0;
+    uint32_t tile = 0, kts = 0;
+    // one of K / V of list positions [128 kt, 128 kt + 128) -> shared memory
+    auto load = [&](const View& x, uint32_t to, const Item& it, int kt) {
+      constexpr int kPieces = HD / 8, kStep = 256 / kPieces;
+      const int c = tid % kPieces;
+      const __nv_bfloat16* const base = reinterpret_cast<const __nv_bfloat16*>(x.ptr) + (int64_t)it.b * x.sb + (int64_t)it.g * x.sh + c * 8;
+#pragma unroll
+      for (int r0 = 0; r0 < kTile; r0 += kStep) {
+        const int r = r0 + tid / kPieces, j = kt * kTile + r;
+        const bool ok = j < it.l0 + it.len;
+        const int slot = !ok ? it.start : j < it.l0 ? it.s0 + j : it.start + j - it.l0;
+        cp_async16_zfill(smem + to + (uint32_t)(c >> 3) * kChunk + (uint32_t)r * 128u + (uint32_t)(((c & 7) ^ (r & 7)) << 4),
+                         base + (int64_t)slot * x.ss, ok);
+      }
+      cp_async_commit();
+    };
     for (;;) {
       const int idx = next_item();
       if (idx < 0) break;
       const Item it = decode(a, idx);
-      for (int kt = 0; kt < it.n_kt; ++kt) {
+      for (int kt = 0; kt < it.n_kt; ++kt, ++kts) {
+        load(a.v, L::kOffV, it, kt);  // (the last dP of the previous key tile is complete: its dS has been computed)
+        if (kts > 0) wait(kAccFull, kts - 1, 73);  // every product of the previous key tile is complete
+        load(a.k, L::kOffK, it, kt);
+        cp_async_wait<0>();
+        ptx::fence_proxy_async_smem();
+        arrive(kKvFull);
         const RowList rows = rows_of(a, it, kt);
         const int j = kt * kTile + row;  // this thread's key: list position
         for (int i = 0; i < rows.n; ++i, ++tile) {
