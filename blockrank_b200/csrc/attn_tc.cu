@@ -5,7 +5,7 @@
 // (128/G consecutive query tokens x the G query heads that share a KV head, so one K/V tile
 // serves the whole GQA group and a Q tile is one 3-D TMA box of the [B,S,N,D] tensor), a
 // 256-column half of tensor memory (S 128 columns, O 128 columns), a Q buffer, four softmax
-// warps and its own MMA-issuing warp.  Chains are fed with "jobs" (one row tile against a list
+// warps, four output warps and its own MMA-issuing warp.  Chains are fed with "jobs" (one row tile against a list
 // of 64-key slots) through per-chain record rings and never wait for one another, so one
 // chain's MMAs run while the other chain's softmax threads work.
 //
@@ -24,17 +24,21 @@
 //     long to be resident): the two chains take the two row tiles of a pair and walk the same
 //     128-key tiles through a two-deep ring.
 //
-// Roles (352 threads):
-//   warps 0-3 / 4-7  softmax + output of chain 0 / 1 (thread = row = TMEM lane)
-//   warp 8           TMA producer: claims and decodes items, publishes jobs, loads K/V
-//   warps 9 / 10     MMA issuer of chain 0 / 1: S = Q K^T (both operands K-major, 128B swizzle)
-//                    and O += P V (P read from tensor memory, V as the MN-major B operand); it also
-//                    requests its chain's Q tiles by TMA (it knows when the Q buffer is free)
+// Roles (640 threads; 61,440 registers at launch, moved to the softmax warps by setmaxnreg):
+//   warps 0-3 / 4-7    softmax of chain 0 / 1 (thread = row = TMEM lane); they leave (max, sum) of each finished row
+//   warps 8-11 / 12-15 output of chain 0 / 1: O out of tensor memory, normalised, stored, while the softmax warps are at
+//                      the next row tile.  (With the softmax warps storing O themselves a row tile cost them 3-5 k cycles
+//                      more: 4 prompts of 100 documents 509 us, now 479; one prompt of 5 documents 29.4, now 20.5.)
+//   warp 16            TMA producer: claims and decodes items, publishes jobs, loads K/V
+//   warps 17 / 18      MMA issuer of chain 0 / 1: S = Q K^T (both operands K-major, 128B swizzle)
+//                      and O += P V (P read from tensor memory, V as the MN-major B operand); it also
+//                      requests its chain's Q tiles by TMA (it knows when the Q buffer is free)
+//   warp 19            zeros in the output's padding slots
 // Softmax is base-2, online, with a lazy rescale (O is only touched when the running max grows
 // by more than 2^8).  P (bf16, two keys per 32-bit column) overwrites the first half of the S
 // tile it was computed from.
 //
-// Shared memory 226 KB: Q 2x32 KB, K pool 80 KB, V pool 80 KB, barriers, job records.
+// Shared memory 227 KB: Q 2x32 KB, K pool 80 KB, V pool 80 KB, barriers, job records, row statistics.
 // No cluster multicast anywhere.  Every mbarrier wait is bounded; on expiry the thread records
 // a code in the caller's status word, stops waiting and runs to the normal exit.
 #include <cuda.h>
@@ -106,7 +110,7 @@ constexpr int BN = 64;   // keys per slot (one TMA box)
 constexpr int BT = 128;  // keys per MMA tile (two slots)
 constexpr int kSlots = 5;        // 64-key K/V slots in shared memory
 constexpr int kMaxGroup = 4;  // consecutive blocks of one (prompt, KV head) per work item, at most
-constexpr int kThreads = 352;
+constexpr int kThreads = 640;
 constexpr uint32_t kSlotHalf = BN * 128;         // K (or V) of one slot, one 64-wide chunk of head_dim
 constexpr uint32_t kPoolHalf = kSlots * kSlotHalf;  // all slots of one chunk, contiguous: key k at k * 128 B
 constexpr int kJobRing = 4;                      // published jobs in flight per chain
@@ -121,7 +125,8 @@ struct Geo {
   static constexpr uint32_t kOffV = kOffK + kChunks * kPoolHalf;
   static constexpr uint32_t kOffBar = kOffV + kChunks * kPoolHalf;
   static constexpr uint32_t kOffJobs = kOffBar + 512;     // 2 x kJobRing records of 16 ints
-  static constexpr uint32_t kSmemBytes = kOffJobs + 2 * kJobRing * 64 + 1024;  // + slack for the 1024-byte round-up
+  static constexpr uint32_t kOffStat = kOffJobs + 2 * kJobRing * 64;  // (max, sum) of each row of a chain's finished tile
+  static constexpr uint32_t kSmemBytes = kOffStat + 2 * BM * 8;
   static_assert(kSmemBytes <= 232448, "shared memory per CTA");
 };
 constexpr uint32_t kTmemCols = 512;
@@ -144,12 +149,14 @@ enum {
   kSFull = 4,    // +chain  MMA -> softmax: S tile complete
   kPFull = 6,    // +chain  softmax -> MMA: P written to tensor memory, S consumed (4 warp arrivals)
   kPVDone = 8,   // +chain  MMA -> softmax: P V of a tile complete
-  kOFree = 10,   // +chain  softmax -> MMA: O read out of TMEM (4 warp arrivals)
+  kOFree = 10,   // +chain  output -> MMA, softmax: O read out of TMEM, row statistics read (4 warp arrivals)
   kKVFull = 12,              // +slot  TMA -> MMA warps: K and V of the slot (or of the tile that starts there) landed
   kKVFree = kKVFull + kSlots,  // +slot  both MMA warps -> TMA: no MMA still reads the slot (2 arrivals)
   kJobFull = kKVFree + kSlots,            // +chain*kJobRing+i  TMA warp -> MMA warp, softmax warps: record written
-  kJobFree = kJobFull + 2 * kJobRing,     // +chain*kJobRing+i  MMA warp + 4 softmax warps -> TMA warp (5 arrivals)
-  kNumBars = kJobFree + 2 * kJobRing
+  kJobFree = kJobFull + 2 * kJobRing,     // +chain*kJobRing+i  MMA, 4 softmax, 4 output warps -> TMA warp (9 arrivals)
+  kOFull = kJobFree + 2 * kJobRing,       // +chain  MMA -> output: the job's last P V complete
+  kStat = kOFull + 2,                     // +chain  softmax -> output: row statistics written (4 warp arrivals)
+  kNumBars = kStat + 2
 };
 static_assert(kNumBars * 8 + 8 <= 512, "barrier area");  // + the TMEM base address
 
@@ -371,47 +378,17 @@ __global__ void __launch_bounds__(kThreads, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, const TcArgs a) {
   using L = Geo<HD>;
-  constexpr uint32_t kOffQ = L::kOffQ, kOffK = L::kOffK, kOffV = L::kOffV, kOffBar = L::kOffBar, kOffJobs = L::kOffJobs;
+  constexpr uint32_t kOffQ = L::kOffQ, kOffK = L::kOffK, kOffV = L::kOffV, kOffBar = L::kOffBar, kOffJobs = L::kOffJobs,
+                     kOffStat = L::kOffStat;
   constexpr uint32_t kQBytes = L::kQBytes, kSlotBytes = L::kSlotBytes;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   if (a.hdr[1] != 0) return;  // malformed block spans (found by the prologue kernel): write nothing
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = a.G;
 
-  // ---- padding slots of the output are written as zeros (gaps in front of / behind blocks) ----
-  {
-    const int per_row = a.N * (HD / 8);
-    auto zero_rows = [&](int b, int lo, int hi) {
-      __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(a.o.ptr) + (int64_t)b * a.o.sb;
-      for (int i = tid; i < (hi - lo) * per_row; i += kThreads) {
-        const int s = lo + i / per_row, rem = i % per_row;
-        *reinterpret_cast<uint4*>(ob + (int64_t)s * a.o.ss + (int64_t)(rem / (HD / 8)) * a.o.sh + (rem % (HD / 8)) * 8) =
-            make_uint4(0, 0, 0, 0);
-      }
-    };
-    // the gap in front of a block (at most a block's padding): one CTA each
-    for (int gi = blockIdx.x; gi < a.B * a.M; gi += gridDim.x) {
-      const int b = gi / a.M, m = gi % a.M;
-      const int32_t* bs = a.blk_start + (size_t)b * a.M;
-      const int32_t* bl = a.blk_len + (size_t)b * a.M;
-      zero_rows(b, (m == 0) ? 0 : bs[m - 1] + bl[m - 1], bs[m]);
-    }
-    // The gap behind the last block holds thousands of rows when a batch is padded to its longest prompt (one
-    // CTA writing all of it took longer than the rest of the kernel): every CTA takes a slice of it.
-    for (int b = 0; b < a.B; ++b) {
-      const int lo = a.blk_start[(size_t)b * a.M + a.M - 1] + a.blk_len[(size_t)b * a.M + a.M - 1];
-      const int rows = a.S - lo;
-      if (rows <= 0) continue;
-      const int per = (rows + (int)gridDim.x - 1) / (int)gridDim.x;
-      const int slot = (int)((blockIdx.x + (unsigned)b) % gridDim.x);
-      zero_rows(b, lo + min(rows, slot * per), lo + min(rows, (slot + 1) * per));
-    }
-  }
-
   // ---- shared memory carve-up, barriers, TMEM ---------------------------------------------------
-  const uint32_t raw = ptx::smem_u32(smem_raw);
-  const uint32_t sbase = (raw + 1023u) & ~1023u;
-  uint8_t* smem = smem_raw + (sbase - raw);
+  uint8_t* const smem = smem_raw;  // (no static shared memory: the array starts at offset 1024 of the window or a multiple)
+  const uint32_t sbase = ptx::smem_u32(smem_raw);
   const uint32_t sBar = sbase + kOffBar;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffBar + kNumBars * 8);
   auto bar = [&](int i) { return sBar + (uint32_t)i * 8u; };
@@ -420,9 +397,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   if (tid == 0) {
     for (int i = 0; i < kNumBars; ++i) {
       uint32_t cnt = 1u;
-      if ((i >= kPFull && i < kPFull + 2) || (i >= kOFree && i < kOFree + 2)) cnt = 4u;  // one arrival per softmax warp
+      if ((i >= kPFull && i < kPFull + 2) || (i >= kOFree && i < kOFree + 2) || i >= kStat) cnt = 4u;  // one per warp
       if (i >= kKVFree && i < kKVFree + kSlots) cnt = 2u;                                 // one per MMA warp
-      if (i >= kJobFree) cnt = 5u;                                                        // MMA warp + four softmax warps
+      if (i >= kJobFree && i < kOFull) cnt = 9u;                                          // MMA, softmax, output warps
       ptx::mbar_init(bar(i), cnt);
     }
     ptx::fence_barrier_init();
@@ -442,10 +419,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
   auto wait = [&](int i, uint32_t parity, int code) {
     if (failed) return;
-    if (!ptx::mbar_wait(bar(i), parity & 1u, kWaitBudget)) {
-      failed = true;
-      if (a.status) atomicCAS(a.status, 0, code);
-    }
+#pragma unroll 1
+    for (uint32_t n = 0; n < kWaitBudget; ++n)
+      if (ptx::mbar_try(bar(i), parity & 1u)) return;
+    failed = true;
+    if (a.status) atomicCAS(a.status, 0, code);
   };
 
   int* const job_ring = reinterpret_cast<int*>(smem + kOffJobs);
@@ -461,7 +439,38 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     return it;
   };
 
-  if (warp == 8) {
+  // Registers: 640 x 96 at launch = 256 x 144 (softmax) + 256 x 64 (output) + 128 x 64 (the rest).
+  if (warp >= 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+  if (warp == 19) {
+    // ============== padding slots of the output are written as zeros (gaps in front of / behind blocks) ==============
+    // (by a warp of its own beside the attention: in front of it, a long ragged grid's 98 MB of zeros were 20 us alone)
+    const int per_row = a.N * (HD / 8);
+    auto zero_rows = [&](int b, int lo, int hi) {
+      __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(a.o.ptr) + (int64_t)b * a.o.sb;
+      for (int s = lo; s < hi; ++s)
+        for (int i = lane; i < per_row; i += 32)
+          *reinterpret_cast<uint4*>(ob + (int64_t)s * a.o.ss + (int64_t)(i / (HD / 8)) * a.o.sh + (i % (HD / 8)) * 8) =
+              make_uint4(0, 0, 0, 0);
+    };
+    // a gap in front of a block: a quarter of it per CTA
+    for (int gi = blockIdx.x; gi < a.B * a.M * 4; gi += gridDim.x) {
+      const int bm = gi >> 2, part = gi & 3, b = bm / a.M, m = bm % a.M;
+      const int32_t* bs = a.blk_start + (size_t)b * a.M;
+      const int32_t* bl = a.blk_len + (size_t)b * a.M;
+      const int lo = m == 0 ? 0 : bs[m - 1] + bl[m - 1], n = bs[m] - lo;
+      zero_rows(b, lo + n * part / 4, lo + n * (part + 1) / 4);
+    }
+    // The gap behind the last block holds thousands of rows when a batch is padded to its longest prompt: every CTA
+    // takes a slice of it.
+    for (int b = 0; b < a.B; ++b) {
+      const int lo = a.blk_start[(size_t)b * a.M + a.M - 1] + a.blk_len[(size_t)b * a.M + a.M - 1];
+      const int rows = a.S - lo;
+      if (rows <= 0) continue;
+      const int per = (rows + (int)gridDim.x - 1) / (int)gridDim.x;
+      const int slot = (int)((blockIdx.x + (unsigned)b) % gridDim.x);
+      zero_rows(b, lo + min(rows, slot * per), lo + min(rows, (slot + 1) * per));
+    }
+  } else if (warp == 16) {
     // =============================== TMA producer ===============================================
     // The whole warp runs the control flow (so addresses and counters stay warp-uniform); one lane
     // issues the copies.
@@ -636,9 +645,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     auto claim = [&]() {
       int v = 0;
       if (leader) v = atomicAdd(a.work_counter, 1);
-      return __shfl_sync(0xffffffffu, v, 0);
+      return (int)gridDim.x + __shfl_sync(0xffffffffu, v, 0);
     };
-    int idx = claim(), idx_next = claim();
+    int idx = blockIdx.x, idx_next = claim();  // (the first item needs no counter: the prologue starts it at 0 = item gridDim.x)
     ItemRaw raw_next = load_item(a, idx, lane);
     for (; idx < a.total_items; idx = idx_next, idx_next = claim()) {
       const ItemRaw raw = raw_next;
@@ -672,12 +681,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     stop.flags = kFStop;
     publish(0, stop);
     publish(1, stop);
-  } else if (warp == 9 || warp == 10) {
+  } else if (warp == 17 || warp == 18) {
     // =============================== MMA issuer of chain x ======================================
     // Whole-warp control flow, one issuing lane (always the same one: tcgen05.commit tracks the
     // MMAs of the thread that executes it).  The two chains' issuers never wait for each other;
     // they only meet in the kKVFree barriers (two arrivals hand a slot back to the TMA warp).
-    const int x = warp - 9;
+    const int x = warp - 17;
     uint32_t q_uses = 0, p_seen = 0, jobs_done = 0;
     uint32_t full_par = 0;  // bit s: parity of the next kKVFull+s phase this warp has not consumed yet
     int blk_waited = 0;     // resident block: slots [0, blk_waited) have landed
@@ -710,7 +719,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       }
     };
     // O (+)= P V over `keys` keys starting at pool slot `slot`; P sits over the first 64 columns of S
-    auto issue_pv = [&](int slot, int keys, bool first) {
+    auto issue_pv = [&](int slot, int keys, bool first, bool last) {
       const uint32_t b_lo = (uint32_t)v_desc0 + (uint32_t)slot * (kSlotHalf >> 4), b_hi = (uint32_t)(v_desc0 >> 32);
       const int ksteps = (keys + 15) >> 4;
       if (ptx::elect_one()) {
@@ -720,6 +729,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             ptx::mma_ts_lohi(tm_o, tm_s + (uint32_t)ks * 8, b_lo + (uint32_t)ks * ((16 * 128) >> 4), b_hi, idesc_pv,
                              (!first || ks > 0) ? 1u : 0u);
         ptx::mma_commit(bar(kPVDone + x));
+        if (last) ptx::mma_commit(bar(kOFull + x));
       }
     };
     // keys of a job's last 128-key tile (every earlier tile spans 128 keys: a short context slot inside a
@@ -804,7 +814,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
               }
             }
               ptx::tc_fence_after_sync();
-            issue_pv(2 * t, keys_of(t), t == 0);
+            issue_pv(2 * t, keys_of(t), t == 0, t + 1 == T);
             // the chain's next S tile: queued behind the P V that reads P out of the same columns
             if (t + 1 < T) issue_qk(2 * t + 2, keys_of(t + 1), t + 2 == T);
             if (chain_on) {
@@ -847,7 +857,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             ++p_seen;
             if (t == 0 && jobs_done > 0) wait(kOFree + x, jobs_done - 1, 26 + x);
               ptx::tc_fence_after_sync();
-            issue_pv(slot, keys_of(t), t == 0);
+            issue_pv(slot, keys_of(t), t == 0, t + 1 == T);
             if (ptx::elect_one()) ptx::mma_commit(bar(kKVFree + slot));
             if (t + 1 < T) issue_qk(2 * ((it.tile0 + t + 1) & 1), keys_of(t + 1), t + 2 == T);
               if (t + 2 == T) request_next_q(job_no);  // the job's last Q K^T is in the pipe
@@ -859,12 +869,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         if (T > 0) ++jobs_done;
       }
     }
-  } else {
-    // =============================== softmax + output, chain x ==================================
+  } else if (warp < 8) {
+    // =============================== softmax, chain x ===========================================
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
     const int x = warp >> 2;
     const int r = tid & 127;  // row of the tile = TMEM lane
     const uint32_t tmem_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)x * kChainCols;
-    uint32_t s_seen = 0, pv_seen = 0;
+    uint32_t s_seen = 0, pv_seen = 0, tiles_done = 0;
+    float2* const stat = reinterpret_cast<float2*>(smem + kOffStat) + x * BM;
 
     for (uint32_t job_no = 0;; ++job_no) {
       const Job it = next_job(x, job_no);
@@ -874,12 +886,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       const int32_t* bs = a.blk_start + (size_t)it.b * a.M;
       const int32_t* bl = a.blk_len + (size_t)it.b * a.M;
       const int tok = it.t0 + (r >> a.g_shift);
-      const int n = it.g * G + (r & (G - 1));
-      const bool active = tok < it.len;
       const bool ctx_check = (flags & kFCtxCheck) != 0;  // the query block's context contains padding slots
       float m_run = -INFINITY, l_run = 0.f;
       const int n_mine = it.n;
-      const bool split = (flags & kFSplit) != 0;
       const int t_mine = (n_mine + 1) >> 1;
 
       for (int t = 0; t < t_mine; ++t) {
@@ -1027,30 +1036,54 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         if (lane == 0) ptx::mbar_arrive(bar(kPFull + x));
       }
 
-      // ---- output of the item ----
-      wait(kPVDone + x, pv_seen, 34 + x);  // last P V of the item
-      ++pv_seen;
-      ptx::tc_fence_after_sync();
+      ++pv_seen;  // (the output warps wait for the job's last P V)
+      if (tiles_done > 0) wait(kOFree + x, tiles_done - 1, 36 + x);  // the previous tile's statistics have been read
+      ++tiles_done;
+      stat[r] = make_float2(m_run, l_run);
       __syncwarp();
-      // O leaves tensor memory in four 32-column chunks, software-pipelined: the load of the next
-      // chunk is in flight while the current one is converted and stored.
-      uint32_t obuf[2][32];
-      ptx::tmem_ld32(tmem_lane + kColO, obuf[0]);
+      if (lane == 0) ptx::mbar_arrive(bar(kStat + x));
+    }
+  } else if (warp < 16) {
+    // =============================== output, chain x ============================================
+    // O leaves tensor memory and is stored while the chain's softmax warps are at the next row tile already.
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    const int x = (warp >> 2) - 2;
+    const int r = tid & 127;  // row of the tile = TMEM lane
+    const uint32_t tmem_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)x * kChainCols + kColO;
+    const float2* const stat = reinterpret_cast<const float2*>(smem + kOffStat) + x * BM;
+    uint32_t done = 0;
+    for (uint32_t job_no = 0;; ++job_no) {
+      const Job it = next_job(x, job_no);
+      if (it.flags & kFStop) break;
+      if (it.n == 0) continue;
+      const int tok = it.t0 + (r >> a.g_shift);
+      const int n = it.g * G + (r & (G - 1));
+      const bool active = tok < it.len;
+      const bool split = (it.flags & kFSplit) != 0;
+      wait(kStat + x, done, 38 + x);
+      const float2 ml = stat[r];
+      const float m_run = ml.x, l_run = ml.y;
+      wait(kOFull + x, done, 34 + x);
+      ++done;
+      ptx::tc_fence_after_sync();
+      auto chunk = [&](int ch, uint32_t (&orow)[32]) {
+        __syncwarp();
+        ptx::tmem_ld32(tmem_lane + (uint32_t)ch * 32, orow);
+        ptx::tmem_wait_ld(orow);
+        if (ch + 1 == HD / 32) {  // O is out of TMEM: the next job's first P V may overwrite it
+          ptx::tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(bar(kOFree + x));
+        }
+      };
       if (split) {
         // un-normalised partial (O, max, sum) of this key chunk; merged by attn_combine_kernel
         const bool wr = active && tok < a.lq_max;
         const int64_t prow = (((int64_t)it.b * a.N + n) * a.lq_max + tok) * a.n_split + it.chunk;
-#pragma unroll
+#pragma unroll 1
         for (int ch = 0; ch < HD / 32; ++ch) {
-          uint32_t (&orow)[32] = obuf[ch & 1];
-          ptx::tmem_wait_ld(orow);
-          if (ch + 1 < HD / 32) {
-            ptx::tmem_ld32(tmem_lane + kColO + (uint32_t)(ch + 1) * 32, obuf[(ch + 1) & 1]);
-          } else {  // O is out of TMEM: the next item's first P V may overwrite it
-            ptx::tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(bar(kOFree + x));
-          }
+          uint32_t orow[32];
+          chunk(ch, orow);
           if (wr) {
             float4* dst = reinterpret_cast<float4*>(a.part_o + prow * HD + ch * 32);
 #pragma unroll
@@ -1062,22 +1095,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         if (wr) a.part_ml[prow] = make_float2(m_run, l_run);
       } else {
         // O / l -> bf16, stored straight from registers: each thread owns one 256-byte output row
-        // and writes it as eight 32-byte (full-sector) stores, or sixteen 16-byte ones if the
-        // output is only 16-byte aligned.
+        // and writes it as 32-byte (full-sector) stores, or 16-byte ones if the output is only 16-byte aligned.
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
         __nv_bfloat16* out_row = reinterpret_cast<__nv_bfloat16*>(a.o.ptr) + (int64_t)it.b * a.o.sb +
                                  (int64_t)(it.start + tok) * a.o.ss + (int64_t)n * a.o.sh;
-#pragma unroll
+#pragma unroll 1
         for (int ch = 0; ch < HD / 32; ++ch) {
-          uint32_t (&orow)[32] = obuf[ch & 1];
-          ptx::tmem_wait_ld(orow);
-          if (ch + 1 < HD / 32) {
-            ptx::tmem_ld32(tmem_lane + kColO + (uint32_t)(ch + 1) * 32, obuf[(ch + 1) & 1]);
-          } else {  // O is out of TMEM: the next item's first P V may overwrite it
-            ptx::tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(bar(kOFree + x));
-          }
+          uint32_t orow[32];
+          chunk(ch, orow);
           if (active) {
 #pragma unroll
             for (int q8 = 0; q8 < 2; ++q8) {
