@@ -150,7 +150,9 @@ enum {
   kPFull = 6,    // +chain  softmax -> MMA: P written to tensor memory, S consumed (4 warp arrivals)
   kPVDone = 8,   // +chain  MMA -> softmax: P V of a tile complete
   kOFree = 10,   // +chain  output -> MMA, softmax: O read out of TMEM, row statistics read (4 warp arrivals)
-  kKVFull = 12,              // +slot  TMA -> MMA warps: K and V of the slot (or of the tile that starts there) landed
+  kKVFull = 12,              // +slot  TMA -> MMA warps: K and V of the slot landed.  Streamed tiles (slots 2i, 2i + 1):
+                             //        K on the first slot's barrier, V on the second's, because K can be handed back when its
+                             //        Q K^T is done, a softmax pass before V
   kKVFree = kKVFull + kSlots,  // +slot  both MMA warps -> TMA: no MMA still reads the slot (2 arrivals)
   kJobFull = kKVFree + kSlots,            // +chain*kJobRing+i  TMA warp -> MMA warp, softmax warps: record written
   kJobFree = kJobFull + 2 * kJobRing,     // +chain*kJobRing+i  MMA, 4 softmax, 4 output warps -> TMA warp (9 arrivals)
@@ -439,8 +441,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     return it;
   };
 
-  // Registers: 640 x 96 at launch = 256 x 144 (softmax) + 256 x 64 (output) + 128 x 64 (the rest).
-  if (warp >= 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+  // Registers: 640 x 96 at launch = 256 x 136 (softmax) + 256 x 64 (output) + 128 x 80 (the rest).
+  if (warp >= 16) asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
   if (warp == 19) {
     // ============== padding slots of the output are written as zeros (gaps in front of / behind blocks) ==============
     // (by a warp of its own beside the attention: in front of it, a long ragged grid's 98 MB of zeros were 20 us alone)
@@ -505,15 +507,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         mode = m;
       }
     };
-    // K and V of 64 keys starting at token slot `lo` -> pool slot s, completion on barrier `bs`
-    auto load_slot = [&](int s, int bs, int g, int b, int lo) {
-      const uint32_t kd = sbase + kOffK + (uint32_t)s * kSlotHalf, vd = sbase + kOffV + (uint32_t)s * kSlotHalf;
-      ptx::tma_load_4d(kd, &tmK, bar(kKVFull + bs), 0, g, lo, b);
-      ptx::tma_load_4d(vd, &tmV, bar(kKVFull + bs), 0, g, lo, b);
-      if (HD == 128) {
-        ptx::tma_load_4d(kd + kPoolHalf, &tmK, bar(kKVFull + bs), 64, g, lo, b);
-        ptx::tma_load_4d(vd + kPoolHalf, &tmV, bar(kKVFull + bs), 64, g, lo, b);
-      }
+    // K (v = 0) or V (v = 1) of 64 keys starting at token slot `lo` -> pool slot s, completion on barrier `bs`
+    auto load_slot = [&](int v, int s, int bs, int g, int b, int lo) {
+      const uint32_t dst = sbase + (v ? kOffV : kOffK) + (uint32_t)s * kSlotHalf;
+      const CUtensorMap* const tm = v ? &tmV : &tmK;
+      ptx::tma_load_4d(dst, tm, bar(kKVFull + bs), 0, g, lo, b);
+      if (HD == 128) ptx::tma_load_4d(dst + kPoolHalf, tm, bar(kKVFull + bs), 64, g, lo, b);
     };
 
     // ---- streamed pair: both chains walk the same 128-key tiles through a two-deep ring (slots 0-1, 2-3) ----
@@ -539,18 +538,20 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       publish(1, it);
       for (int t = 0; t < T; ++t) {
         const int tb = (int)((stream_tiles + (uint32_t)t) & 1u);
-        drain(2 * tb);
-        drain(2 * tb + 1);
         const int nslots = min(2, pr.n_slots - 2 * t);
-        if (leader) {
-          ptx::mbar_expect_tx(bar(kKVFull + 2 * tb), (uint32_t)nslots * kSlotBytes);
-          for (int h = 0; h < nslots; ++h) {
-            int nk, own_off; bool own;
-            const int lo = tile_lo(it, 2 * t + h, nk, own, own_off);
-            load_slot(2 * tb + h, 2 * tb, g, b, lo);
+#pragma unroll 1
+        for (int v = 0; v < 2; ++v) {
+          drain(2 * tb + v);
+          if (leader) {
+            ptx::mbar_expect_tx(bar(kKVFull + 2 * tb + v), (uint32_t)nslots * (kSlotBytes / 2));
+            for (int h = 0; h < nslots; ++h) {
+              int nk, own_off; bool own;
+              const int lo = tile_lo(it, 2 * t + h, nk, own, own_off);
+              load_slot(v, 2 * tb + h, 2 * tb + v, g, b, lo);
+            }
           }
+          out_mask |= 1u << (2 * tb + v);
         }
-        out_mask |= 1u << (2 * tb);
       }
       stream_tiles += (uint32_t)T;
     };
@@ -578,7 +579,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           const int lo = s < n_ctx ? s0 + s * BN : start + (s - n_ctx) * BN;
           if (leader) {
             ptx::mbar_expect_tx(bar(kKVFull + s), kSlotBytes);
-            load_slot(s, s, g, b, lo);
+            load_slot(0, s, s, g, b, lo);
+            load_slot(1, s, s, g, b, lo);
           }
           out_mask |= 1u << s;
         }
@@ -647,8 +649,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       if (leader) v = atomicAdd(a.work_counter, 1);
       return (int)gridDim.x + __shfl_sync(0xffffffffu, v, 0);
     };
-    int idx = blockIdx.x, idx_next = claim();  // (the first item needs no counter: the prologue starts it at 0 = item gridDim.x)
+    int idx = blockIdx.x;  // the first item needs no counter: its 0 is item gridDim.x
     ItemRaw raw_next = load_item(a, idx, lane);
+    int idx_next = claim();
     for (; idx < a.total_items; idx = idx_next, idx_next = claim()) {
       const ItemRaw raw = raw_next;
       raw_next = load_item(a, idx_next, lane);  // in flight while this item is processed
@@ -837,33 +840,39 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       } else {
         // ---- streamed pair: tile t sits in ring position (tile0 + t) & 1 = pool slots 0-1 or 2-3 ----
         const int Ti = it.aux;  // tiles of the item; this chain computes on the first T of them
-        int kv_waited = -1;
-        auto need_kv = [&](int t) {
-          if (kv_waited >= t) return;
-          wait_full(2 * ((it.tile0 + t) & 1));
-          kv_waited = t;
+        auto pos = [&](int t) { return 2 * ((it.tile0 + t) & 1); };
+        auto free_kv = [&](int i) {
+          if (ptx::elect_one()) ptx::mma_commit(bar(kKVFree + i));
+          __syncwarp();
+        };
+        auto stream_qk = [&](int t) {
+          issue_qk(pos(t), keys_of(t), t + 1 == T);
+          free_kv(pos(t));
         };
         if (T > 0) {
-          need_kv(0);
+          wait_full(pos(0));
           ptx::tc_fence_after_sync();
-          issue_qk(2 * (it.tile0 & 1), keys_of(0), T == 1);
+          stream_qk(0);
           if (T == 1) request_next_q(job_no);
         }
-        for (int t = 0; t < Ti; ++t) {
-          const int slot = 2 * ((it.tile0 + t) & 1);
-          if (t < T) {
-            if (t + 1 < T) need_kv(t + 1);  // (its ring position was handed back after P V of tile t-1)
-            wait(kPFull + x, p_seen, 24 + x);
-            ++p_seen;
-            if (t == 0 && jobs_done > 0) wait(kOFree + x, jobs_done - 1, 26 + x);
-              ptx::tc_fence_after_sync();
-            issue_pv(slot, keys_of(t), t == 0, t + 1 == T);
-            if (ptx::elect_one()) ptx::mma_commit(bar(kKVFree + slot));
-            if (t + 1 < T) issue_qk(2 * ((it.tile0 + t + 1) & 1), keys_of(t + 1), t + 2 == T);
-              if (t + 2 == T) request_next_q(job_no);  // the job's last Q K^T is in the pipe
-          } else {
-            need_kv(t);  // not visible to this chain: consume the phase, then hand the tile back
-            if (ptx::elect_one()) ptx::mma_commit(bar(kKVFree + slot));
+        for (int t = 0; t < T; ++t) {
+          // (waited for beside the softmax: between P's arrival and the products a wait costs its round trip even when the
+          // tile has landed)
+          wait_full(pos(t) + 1);
+          if (t + 1 < T) wait_full(pos(t + 1));
+          wait(kPFull + x, p_seen, 24 + x);
+          ++p_seen;
+          if (t == 0 && jobs_done > 0) wait(kOFree + x, jobs_done - 1, 26 + x);
+          ptx::tc_fence_after_sync();
+          issue_pv(pos(t), keys_of(t), t == 0, t + 1 == T);
+          free_kv(pos(t) + 1);
+          if (t + 1 < T) stream_qk(t + 1);
+          if (t + 2 == T) request_next_q(job_no);  // the job's last Q K^T is in the pipe
+        }
+        for (int t = T; t < Ti; ++t) {  // not visible to this chain: consume the phases, hand the tile back
+          for (int v = 0; v < 2; ++v) {
+            wait_full(pos(t) + v);
+            free_kv(pos(t) + v);
           }
         }
         if (T > 0) ++jobs_done;
@@ -871,7 +880,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     }
   } else if (warp < 8) {
     // =============================== softmax, chain x ===========================================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 136;");
     const int x = warp >> 2;
     const int r = tid & 127;  // row of the tile = TMEM lane
     const uint32_t tmem_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)x * kChainCols;
