@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f32_kernel(F32Args a) {
   constexpr int kKsFloats = kKeys * (kPitch > kPitchP ? kPitch : kPitchP);
   float* const vs = ks + kKsFloats;           // [64][D]
   __shared__ int s_slot[kKeys];               // slot of each key of the tile, -1: none
+  ptx::grid_dependency_wait();
   if (a.hdr[1] != 0) return;
   const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
   const bool query = (int)blockIdx.x < a.n_query;
@@ -286,9 +287,8 @@ int launch(const brk_attn_params& p, const F32Args& a, cudaStream_t st) {
   BRK_CUDA(cudaFuncSetAttribute(attn_f32_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int64_t ctas = a.n_query + (int64_t)p.B * p.Nk * (p.M - 1) * a.tiles;
   BRK_REQUIRE(ctas < (1ll << 31), BRK_E_UNSUPPORTED, "grid too large: B*Nk=%d M=%d", p.B * p.Nk, p.M);
-  attn_f32_kernel<D><<<(unsigned)ctas, kThreads, smem, st>>>(a);
-  BRK_CUDA(cudaGetLastError());
-  if (a.n_chunk == 1) return BRK_OK;
+  const int rc = launch_dependent(attn_f32_kernel<D>, dim3((unsigned)ctas), dim3(kThreads), smem, st, a);
+  if (rc || a.n_chunk == 1) return rc;
   CombineArgs c{a.o, a.lse, a.blk_start, a.blk_len, a.hdr, p.B, p.N, p.S, p.M, a.lq, a.n_chunk, a.part_o, a.part_ml};
   return attn_combine_launch<float, D>(c, st);
 }

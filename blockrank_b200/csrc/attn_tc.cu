@@ -201,10 +201,22 @@ struct TcArgs {
   int o_align32;    // output rows are 32-byte aligned (enables 32-byte stores)
   int sec1, total_items;
   FastDiv div_sec1, div_nbg, div_nk;  // by nbg*n_split, nbg, Nk
+  int max_block_len, max_query_len;
+  int one_wave;       // every CTA has one item: no counter, and the kernel checks the spans itself (no prologue kernel)
   int* work_counter;  // next unclaimed index of the work list (zeroed before the launch)
   float* part_o;    // [B, N, lq_max, n_split, 128] un-normalised partial outputs
   float2* part_ml;  // [B, N, lq_max, n_split] (running max in log2 units, sum)
 };
+
+// Is span j of the (B, M) arrays inside [0, S), no longer than allowed, and behind its predecessor?
+__device__ __forceinline__ bool span_ok(const int32_t* blk_start, const int32_t* blk_len, int j, int M, int S, int max_block_len,
+                                        int max_query_len) {
+  const int m = j % M, s = blk_start[j], l = blk_len[j];
+  bool ok = s >= 0 && l >= 0 && l <= max_block_len && s <= S - l;
+  if (ok && m > 0) ok = blk_start[j - 1] >= 0 && blk_len[j - 1] >= 0 && blk_start[j - 1] <= s - blk_len[j - 1];
+  if (ok && m == M - 1 && max_query_len > 0) ok = l <= max_query_len;
+  return ok;
+}
 
 // One row tile against a list of 64-key slots: what a chain works on.
 constexpr int kFSplit = 1, kFCtxCheck = 2, kFStop = 4, kFDoc = 8, kFFirst = 16, kFKeep = 32;
@@ -384,7 +396,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                      kOffStat = L::kOffStat;
   constexpr uint32_t kQBytes = L::kQBytes, kSlotBytes = L::kSlotBytes;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  if (a.hdr[1] != 0) return;  // malformed block spans (found by the prologue kernel): write nothing
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = a.G;
 
@@ -418,6 +429,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  ptx::grid_dependency_wait();  // (the set-up above runs beside the prologue kernel)
+  bool malformed;
+  if (a.one_wave) {
+    bool bad = false;
+    for (int j = tid; j < a.B * a.M; j += kThreads)
+      bad |= !span_ok(a.blk_start, a.blk_len, j, a.M, a.S, a.max_block_len, a.max_query_len);
+    malformed = __syncthreads_or(bad);
+    if (malformed && tid == 0 && a.status) atomicCAS(a.status, 0, kStatusBadSpans);
+  } else {
+    malformed = a.hdr[1] != 0;
+  }
+  if (malformed) {  // write nothing
+    if (warp == 0) ptx::tmem_dealloc(tmem, kTmemCols);
+    return;
+  }
 
   auto wait = [&](int i, uint32_t parity, int code) {
     if (failed) return;
@@ -645,6 +671,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // run two items ahead and the block spans of a claimed item one item ahead, so neither the
     // atomic nor the loads are waited for.
     auto claim = [&]() {
+      if (a.one_wave) return a.total_items;
       int v = 0;
       if (leader) v = atomicAdd(a.work_counter, 1);
       return (int)gridDim.x + __shfl_sync(0xffffffffu, v, 0);
@@ -1180,11 +1207,7 @@ __global__ void attn_prologue_kernel(const int32_t* __restrict__ blk_start, cons
   }
   __syncthreads();
   for (int j = threadIdx.x; j < B * M; j += blockDim.x) {
-    const int m = j % M;
-    const int s = blk_start[j], l = blk_len[j];
-    bool ok = s >= 0 && l >= 0 && l <= max_block_len && s <= S - l;
-    if (ok && m > 0) ok = blk_start[j - 1] >= 0 && blk_len[j - 1] >= 0 && blk_start[j - 1] <= s - blk_len[j - 1];
-    if (ok && m == M - 1 && max_query_len > 0) ok = l <= max_query_len;
+    const bool ok = span_ok(blk_start, blk_len, j, M, S, max_block_len, max_query_len);
     if (!ok) bad = 1;  // benign race: every writer stores the same value
   }
   __syncthreads();
@@ -1286,10 +1309,14 @@ static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cuda
   a.work_counter = reinterpret_cast<int*>(ws);
   a.part_o = ns > 1 ? part : nullptr;
   a.part_ml = ns > 1 ? reinterpret_cast<float2*>(part + rows * HD) : nullptr;
-  if ((rc = attn_prologue_launch(p, reinterpret_cast<int*>(ws), a.part_ml, ns > 1 ? (int64_t)rows : 0, st))) return rc;
+  // A call whose items all start at once needs neither the counter nor the partials' reset: its CTAs check the spans
+  // themselves.  (One prompt of 5 documents: the prologue kernel and the gap behind it were 4 of 20 us.)
+  a.max_block_len = p.max_block_len;
+  a.max_query_len = p.max_query_len;
+  a.one_wave = ns == 1 && total_items <= sms[dev];
+  if (!a.one_wave && (rc = attn_prologue_launch(p, reinterpret_cast<int*>(ws), a.part_ml, ns > 1 ? (int64_t)rows : 0, st))) return rc;
   const int grid = (int)(total_items < sms[dev] ? total_items : sms[dev]);
-  attn_tc_kernel<HD><<<grid, kThreads, Geo<HD>::kSmemBytes, st>>>(tq, tk, tv, a);
-  BRK_CUDA(cudaGetLastError());
+  if ((rc = launch_dependent(attn_tc_kernel<HD>, dim3(grid), dim3(kThreads), Geo<HD>::kSmemBytes, st, tq, tk, tv, a))) return rc;
   if (ns > 1) {
     const CombineArgs c{a.o, a.lse, a.blk_start, a.blk_len, a.hdr, p.B, p.N, p.S, p.M, lq, ns, a.part_o, a.part_ml};
     return attn_combine_launch<__nv_bfloat16, HD>(c, st);

@@ -91,6 +91,24 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&v)[8]) {
   *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// Launch that may start before the preceding kernel of the stream has finished (its blocks become resident while that one
+// drains); the kernel must execute ptx::grid_dependency_wait() before it touches memory.
+template <typename K, typename... A>
+int launch_dependent(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  BRK_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  return BRK_OK;
+}
+
 struct View {
   char* ptr;
   int64_t sb, sh, ss;
