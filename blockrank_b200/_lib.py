@@ -22,7 +22,7 @@ EXPORTS = ("brk_version", "brk_last_error", "brk_device_check", "brk_spans_from_
            "brk_status_poll", "brk_selftest_bounded_wait",
            "brk_doc_scores_workspace_bytes",
            "brk_doc_scores", "brk_doc_scores_static", "brk_raw_scores",
-           "brk_raw_scores_bwd_workspace_bytes", "brk_raw_scores_bwd", "brk_signal_rows", "brk_rmsnorm",
+           "brk_raw_scores_bwd_workspace_bytes", "brk_raw_scores_bwd", "brk_signal_rows", "brk_rank_pack", "brk_rmsnorm",
            "brk_rope", "brk_silu_mul")
 
 

@@ -208,6 +208,14 @@ int brk_rope(int32_t dtype, void* q, int64_t q_row_stride, int32_t N, void* k, i
   return rope_launch(dtype, q, q_row_stride, N, k, k_row_stride, Nk, D, pos, inv_freq, T, (cudaStream_t)stream);
 }
 
+int brk_rank_pack(const float* logits, int32_t B, int32_t nd, int32_t k, float* logits_out, int64_t* top_out,
+                  const int32_t* status, int32_t* status_out, void* stream) {
+  BRK_REQUIRE(logits && logits_out && top_out && status && status_out, BRK_E_ARG, "null pointer");
+  BRK_REQUIRE(B > 0 && nd > 0 && nd <= BRK_RANK_PACK_DOCS && k > 0 && k <= nd, BRK_E_ARG, "bad rank_pack shape B=%d nd=%d k=%d", B,
+              nd, k);
+  return rank_pack_launch(logits, B, nd, k, logits_out, top_out, status, status_out, (cudaStream_t)stream);
+}
+
 int brk_signal_rows(int32_t dtype, const void* x, int32_t hidden, const int32_t* pos, const int32_t* rows, int32_t B, int32_t S,
                     int32_t R, void* x_out, int32_t* pos_out, int32_t* local, int32_t* status, void* stream) {
   BRK_REQUIRE(x && pos && rows && x_out && pos_out && local, BRK_E_ARG, "null pointer");

@@ -161,6 +161,9 @@ int rmsnorm_launch(int dtype, const void* x, void* residual, const void* w, void
                    float eps, cudaStream_t st);
 int rope_launch(int dtype, void* q, int64_t q_rs, int N, void* k, int64_t k_rs, int Nk, int D, const int32_t* pos,
                 const float* inv_freq, int64_t T, cudaStream_t st);
+constexpr int kRankPackDocs = BRK_RANK_PACK_DOCS;
+int rank_pack_launch(const float* logits, int B, int nd, int k, float* out, int64_t* top, const int32_t* status,
+                     int32_t* status_out, cudaStream_t st);
 int signal_rows_launch(const void* x, int row_bytes, const int32_t* pos, const int32_t* rows, int B, int S, int R, void* x_out,
                        int32_t* pos_out, int32_t* local, int32_t* status, cudaStream_t st);
 int silu_mul_launch(int dtype, const void* gu, void* out, int64_t rows, int inter, cudaStream_t st);

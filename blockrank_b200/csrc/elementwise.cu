@@ -2,6 +2,8 @@
 // mask, RMSNorm (optionally fused with the residual add), rotate-half RoPE and
 // SiLU(gate) * up.  Rounding points follow what the HF Mistral modules do in
 // the model dtype, so a bf16 run tracks the framework's bf16 run closely.
+#include <algorithm>
+
 #include "brk_common.cuh"
 
 namespace brk {
@@ -110,12 +112,12 @@ __global__ void __launch_bounds__(1024) rmsnorm_reg_kernel(const T* __restrict__
 }
 
 // ---- RoPE ---------------------------------------------------------------------
-// One thread per (row, 8 rotation pairs): the 8 angles are evaluated once and applied to every
-// query and key head of that row, with 16-byte loads and stores of both halves of each head.
+// One thread per (row, 8 rotation pairs, `per` heads): the 8 angles are evaluated once and applied to those
+// query and key heads of the row, with 16-byte loads and stores of both halves of each head.
 template <typename T>
 __global__ void __launch_bounds__(256) rope_kernel(T* __restrict__ q, int64_t q_rs, int N, T* __restrict__ k,
                                                    int64_t k_rs, int Nk, int D, const int32_t* __restrict__ pos,
-                                                   const float* __restrict__ inv_freq, int64_t T_rows) {
+                                                   const float* __restrict__ inv_freq, int64_t T_rows, int per) {
   const int half = D >> 1, chunks = half >> 3;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= T_rows * chunks) return;
@@ -129,7 +131,9 @@ __global__ void __launch_bounds__(256) rope_kernel(T* __restrict__ q, int64_t q_
     cs[i] = Elem<T>::round(cs[i]);
     sn[i] = Elem<T>::round(sn[i]);
   }
-  for (int h = 0; h < N + Nk; ++h) {
+  const int h_end = min(N + Nk, ((int)blockIdx.y + 1) * per);
+#pragma unroll 4
+  for (int h = blockIdx.y * per; h < h_end; ++h) {
     T* base = (h < N ? q + t * q_rs + (int64_t)h * D : k + t * k_rs + (int64_t)(h - N) * D) + i0;
     float x1[8], x2[8], o1[8], o2[8];
     load8(base, x1);
@@ -195,7 +199,37 @@ __global__ void __launch_bounds__(128) signal_rows_kernel(const uint4* __restric
   }
 }
 
+// What a ranking call returns to the host, in one block of memory: the logits, the indices of each prompt's k best
+// documents (by counting how many are better; equal ones in document order; NaN first, as torch.topk has it) and the status
+// word.  One CTA per prompt.
+__global__ void __launch_bounds__(256) rank_pack_kernel(const float* __restrict__ logits, int nd, int k, float* __restrict__ out,
+                                                        int64_t* __restrict__ top, const int32_t* __restrict__ status,
+                                                        int32_t* __restrict__ status_out) {
+  __shared__ float v[kRankPackDocs];
+  const int b = blockIdx.x;
+  for (int i = threadIdx.x; i < nd; i += blockDim.x) out[(int64_t)b * nd + i] = v[i] = logits[(int64_t)b * nd + i];
+  __syncthreads();
+  for (int i = threadIdx.x; i < nd; i += blockDim.x) {
+    const float x = v[i];
+    int better = 0;
+    for (int j = 0; j < nd; ++j) {
+      const float y = v[j];
+      const bool above = y > x || (isnan(y) && !isnan(x)), below = x > y || (isnan(x) && !isnan(y));
+      better += above || (!below && j < i);
+    }
+    if (better < k) top[(int64_t)b * k + better] = i;
+  }
+  if (b == 0 && threadIdx.x == 0) *status_out = *status;
+}
+
 }  // namespace
+
+int rank_pack_launch(const float* logits, int B, int nd, int k, float* out, int64_t* top, const int32_t* status,
+                     int32_t* status_out, cudaStream_t st) {
+  rank_pack_kernel<<<B, 256, 0, st>>>(logits, nd, k, out, top, status, status_out);
+  BRK_CUDA(cudaGetLastError());
+  return BRK_OK;
+}
 
 int signal_rows_launch(const void* x, int row_bytes, const int32_t* pos, const int32_t* rows, int B, int S, int R, void* x_out,
                        int32_t* pos_out, int32_t* local, int32_t* status, cudaStream_t st) {
@@ -244,13 +278,18 @@ int rmsnorm_launch(int dtype, const void* x, void* residual, const void* w, void
 int rope_launch(int dtype, void* q, int64_t q_rs, int N, void* k, int64_t k_rs, int Nk, int D, const int32_t* pos,
                 const float* inv_freq, int64_t T, cudaStream_t st) {
   const int64_t total = T * (D / 16);
-  const int threads = 256;
+  const int threads = 128, heads = N + Nk;
   const int64_t blocks = (total + threads - 1) / threads;
+  // Heads per thread: four loads of each half in flight are enough for a large call; a small one is cut until the blocks
+  // cover the SMs twice. 
+  int per = std::min(heads, 8);
+  while (per > 1 && blocks * ((heads + per - 1) / per) < 2 * 148) per = (per + 1) / 2;
+  const dim3 grid((unsigned)blocks, (unsigned)((heads + per - 1) / per));
   if (dtype == BRK_BF16)
-    rope_kernel<__nv_bfloat16><<<(unsigned)blocks, threads, 0, st>>>((__nv_bfloat16*)q, q_rs, N, (__nv_bfloat16*)k, k_rs,
-                                                                    Nk, D, pos, inv_freq, T);
+    rope_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>((__nv_bfloat16*)q, q_rs, N, (__nv_bfloat16*)k, k_rs, Nk, D, pos,
+                                                         inv_freq, T, per);
   else
-    rope_kernel<float><<<(unsigned)blocks, threads, 0, st>>>((float*)q, q_rs, N, (float*)k, k_rs, Nk, D, pos, inv_freq, T);
+    rope_kernel<float><<<grid, threads, 0, st>>>((float*)q, q_rs, N, (float*)k, k_rs, Nk, D, pos, inv_freq, T, per);
   BRK_CUDA(cudaGetLastError());
   return BRK_OK;
 }

@@ -6,6 +6,8 @@
 // same steps cost 40-60 us per attention call, more than its kernels take on a short prompt.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
+#include <ATen/ops/addmm_cuda_dispatch.h>
+#include <ATen/ops/mm_cuda_dispatch.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/extension.h>
@@ -417,7 +419,7 @@ struct NoAutograd {
 Tensor layer_qkv(const Tensor& h, const Tensor& ln1, const Tensor& wqkv, const Tensor& pos, const Tensor& inv_freq, int64_t N,
                  int64_t Nk, int64_t D, double eps) {
   NoAutograd guard;
-  Tensor qkv = at::mm(rmsnorm(h, ln1, eps, std::nullopt, std::nullopt), wqkv.t());
+  Tensor qkv = at::cuda::mm(rmsnorm(h, ln1, eps, std::nullopt, std::nullopt), wqkv.t());
   const int64_t T = qkv.size(0), row = qkv.stride(0), at0 = qkv.storage_offset();
   rope_(qkv.as_strided({T, N, D}, {row, D, 1}, at0), qkv.as_strided({T, Nk, D}, {row, D, 1}, at0 + N * D), pos, inv_freq);
   return qkv;
@@ -439,9 +441,9 @@ Tensor layer_attention(const Tensor& qkv, const Tensor& blk_start, const Tensor&
 void layer_rest(Tensor& h, const Tensor& attn, const Tensor& wo, const Tensor& ln2, const Tensor& wgu, const Tensor& wd,
                 double eps) {
   NoAutograd guard;
-  h.addmm_(attn.view({h.size(0), wo.size(1)}), wo.t());
+  at::cuda::addmm_(h, attn.view({h.size(0), wo.size(1)}), wo.t(), 1, 1);
   const Tensor x = rmsnorm(h, ln2, eps, std::nullopt, std::nullopt);
-  h.addmm_(silu_mul(at::mm(x, wgu.t()), std::nullopt), wd.t());
+  at::cuda::addmm_(h, silu_mul(at::cuda::mm(x, wgu.t()), std::nullopt), wd.t(), 1, 1);
 }
 
 // layers: {ln1, wqkv, wo, ln2, wgu, wd} of every layer in front of the scoring layer.  ids (B, S), pos int32 (B S,).
@@ -472,7 +474,7 @@ std::tuple<Tensor, Tensor, Tensor> score_qk(const Tensor& h, const Tensor& pos, 
             "signal_rows must be int32 (B, R) and positions contiguous int32");
   const int64_t B = signal_rows.size(0), R = signal_rows.size(1), T = h.size(0), S = T / B;
   const Tensor x = rmsnorm(h, ln1, eps, std::nullopt, std::nullopt), rows = signal_rows.contiguous();
-  Tensor k = at::mm(x, wk.t());
+  Tensor k = at::cuda::mm(x, wk.t());
   Tensor xs = at::empty({B * R, x.size(1)}, x.options()), ps = at::empty({B * R}, pos.options()), local = at::empty({B, R}, pos.options());
   check(brk_signal_rows(dtype_code(x), x.data_ptr(), (int32_t)x.size(1), (const int32_t*)pos.data_ptr(),
                         (const int32_t*)rows.data_ptr(), (int32_t)B, (int32_t)S, (int32_t)R, xs.data_ptr(),
@@ -480,56 +482,108 @@ std::tuple<Tensor, Tensor, Tensor> score_qk(const Tensor& h, const Tensor& pos, 
                         stream_of(x)),
         "brk_signal_rows");
   count(1);
-  Tensor q = at::mm(xs, wq.t());
+  Tensor q = at::cuda::mm(xs, wq.t());
   rope_(q.view({B * R, N, D}), std::nullopt, ps, inv_freq);
   rope_(std::nullopt, k.view({T, Nk, D}), pos, inv_freq);
   return {q.view({B, R, N, D}).permute({0, 2, 1, 3}), k.view({B, S, Nk, D}).permute({0, 2, 1, 3}), local};
 }
 
 // Host tensors of a batch -> device: (ids, positions int32, start, length, signal rows), and the longest query block.
+// They travel in one copy out of a pinned buffer (five copies and a conversion kernel were 40 us of a short request).
 std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, int64_t> upload(const Tensor& ids, const Tensor& pos, const Tensor& spans,
                                                                    const Tensor& rows, const c10::Device& device) {
   NoAutograd guard;
   BRK_VALUE(spans.dim() == 3 && spans.size(0) == 2 && spans.scalar_type() == at::kInt, "block_spans must be int32 (2, B, M)");
-  const Tensor d_ids = ids.to(device, ids.scalar_type(), true), d_pos = pos.to(device, pos.scalar_type(), true).to(at::kInt);
-  const Tensor d_spans = spans.to(device, spans.scalar_type(), true), d_rows = rows.to(device, rows.scalar_type(), true);
-  const Tensor q_len = spans.select(0, 1).select(1, spans.size(2) - 1);
-  int64_t longest = 0;
-  if (q_len.is_cpu()) {
-    for (int64_t b = 0; b < q_len.size(0); ++b)
-      longest = std::max<int64_t>(longest, static_cast<const int32_t*>(q_len.data_ptr())[b * q_len.stride(0)]);
-  } else {
-    longest = q_len.max().item().toLong();
+  const int64_t B = spans.size(1), M = spans.size(2);
+  bool packable = ids.scalar_type() == at::kLong && rows.scalar_type() == at::kInt &&
+                  (pos.scalar_type() == at::kLong || pos.scalar_type() == at::kInt);
+  for (const Tensor* t : {&ids, &pos, &spans, &rows}) packable = packable && t->is_cpu() && t->is_contiguous();
+  if (!packable) {
+    const Tensor d_ids = ids.to(device, ids.scalar_type(), true), d_pos = pos.to(device, pos.scalar_type(), true).to(at::kInt);
+    const Tensor d_spans = spans.to(device, spans.scalar_type(), true), d_rows = rows.to(device, at::kInt, true);
+    return {d_ids, d_pos, d_spans.select(0, 0), d_spans.select(0, 1), d_rows, spans.select(0, 1).select(1, M - 1).max().item().toLong()};
   }
-  return {d_ids, d_pos, d_spans.select(0, 0), d_spans.select(0, 1), d_rows, longest};
+  const int64_t n_ids = ids.numel(), n_pos = pos.numel(), n_spans = spans.numel(), n_rows = rows.numel();
+  Tensor stage = at::empty({8 * n_ids + 4 * (n_pos + n_spans + n_rows)}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
+  char* w = static_cast<char*>(stage.data_ptr());
+  memcpy(w, ids.data_ptr(), 8 * n_ids);
+  int32_t* p = reinterpret_cast<int32_t*>(w + 8 * n_ids);
+  if (pos.scalar_type() == at::kLong) {
+    const int64_t* src = static_cast<const int64_t*>(pos.data_ptr());
+    for (int64_t i = 0; i < n_pos; ++i) p[i] = (int32_t)src[i];
+  } else {
+    memcpy(p, pos.data_ptr(), 4 * n_pos);
+  }
+  memcpy(p + n_pos, spans.data_ptr(), 4 * n_spans);
+  memcpy(p + n_pos + n_spans, rows.data_ptr(), 4 * n_rows);
+  const Tensor d = stage.to(device, at::kByte, /*non_blocking=*/true);
+  const Tensor d32 = d.narrow(0, 8 * n_ids, 4 * (n_pos + n_spans + n_rows)).view(at::kInt);
+  auto part = [&](int64_t first, at::IntArrayRef sizes) {
+    int64_t n = 1;
+    for (int64_t x : sizes) n *= x;
+    return d32.narrow(0, first, n).view(sizes);
+  };
+  const int32_t* len = static_cast<const int32_t*>(spans.data_ptr()) + B * M;
+  int64_t longest = 0;
+  for (int64_t b = 0; b < B; ++b) longest = std::max<int64_t>(longest, len[b * M + M - 1]);
+  return {d.narrow(0, 0, 8 * n_ids).view(at::kLong).view(ids.sizes()), part(0, pos.sizes()), part(n_pos, {B, M}),
+          part(n_pos + B * M, {B, M}), part(n_pos + n_spans, rows.sizes()), longest};
 }
 
-// Scores and the indices of the k best documents -> host, with one synchronisation, after which a problem a kernel
-// reported is raised.
-std::tuple<Tensor, Tensor> download(const Tensor& logits_in, int64_t k) {
+// Scores and the indices of the k best documents -> host, with one copy and one synchronisation, after which a problem a
+// kernel reported is raised.
+std::tuple<Tensor, Tensor> download(const Tensor& logits_in, int64_t k_in) {
   NoAutograd guard;
   c10::cuda::CUDAGuard device(logits_in.device());
   const Tensor logits = logits_in.contiguous();
-  const Tensor top = std::get<1>(at::topk(logits, std::min(k, logits.size(-1)), -1));
+  const int64_t B = logits.size(0), nd = logits.size(1), k = std::min(k_in, nd);
   const Tensor word = status_word(logits.get_device());
   const auto stream = at::cuda::getCurrentCUDAStream(logits.get_device());
-  const size_t nl = logits.nbytes(), nt = top.nbytes(), at_top = (nl + 15) & ~(size_t)15, at_word = at_top + ((nt + 15) & ~(size_t)15);
-  Tensor stage = at::empty({(int64_t)(at_word + 16)}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
+  const size_t nl = logits.nbytes(), at_top = (nl + 15) & ~(size_t)15, nt = (size_t)B * k * 8, at_word = at_top + ((nt + 15) & ~(size_t)15);
+  const auto bytes = at::TensorOptions().dtype(at::kByte);
+  Tensor stage = at::empty({(int64_t)(at_word + 16)}, bytes.pinned_memory(true));
   char* const base = static_cast<char*>(stage.data_ptr());
-  C10_CUDA_CHECK(cudaMemcpyAsync(base, logits.data_ptr(), nl, cudaMemcpyDeviceToHost, stream));
-  C10_CUDA_CHECK(cudaMemcpyAsync(base + at_top, top.data_ptr(), nt, cudaMemcpyDeviceToHost, stream));
-  C10_CUDA_CHECK(cudaMemcpyAsync(base + at_word, word.data_ptr(), 4, cudaMemcpyDeviceToHost, stream));
+  Tensor dev;  // alive until the copy is complete
+  if (B > 0 && k > 0 && nd <= BRK_RANK_PACK_DOCS) {
+    dev = at::empty({(int64_t)(at_word + 16)}, bytes.device(logits.device()));
+    char* const d = static_cast<char*>(dev.data_ptr());
+    check(brk_rank_pack((const float*)logits.data_ptr(), (int32_t)B, (int32_t)nd, (int32_t)k, (float*)d, (int64_t*)(d + at_top),
+                        (const int32_t*)word.data_ptr(), (int32_t*)(d + at_word), stream.stream()),
+          "brk_rank_pack");
+    count(1);
+    C10_CUDA_CHECK(cudaMemcpyAsync(base, d, at_word + 4, cudaMemcpyDeviceToHost, stream));
+  } else {
+    dev = std::get<1>(at::topk(logits, k, -1));
+    C10_CUDA_CHECK(cudaMemcpyAsync(base, logits.data_ptr(), nl, cudaMemcpyDeviceToHost, stream));
+    C10_CUDA_CHECK(cudaMemcpyAsync(base + at_top, dev.data_ptr(), nt, cudaMemcpyDeviceToHost, stream));
+    C10_CUDA_CHECK(cudaMemcpyAsync(base + at_word, word.data_ptr(), 4, cudaMemcpyDeviceToHost, stream));
+  }
   {
     pybind11::gil_scoped_release release;
     C10_CUDA_CHECK(cudaStreamSynchronize(stream));
   }
-  Tensor h_logits = at::empty(logits.sizes(), logits.options().device(at::kCPU)), h_top = at::empty(top.sizes(), top.options().device(at::kCPU));
+  Tensor h_logits = at::empty(logits.sizes(), logits.options().device(at::kCPU));
+  Tensor h_top = at::empty({B, k}, at::TensorOptions().dtype(at::kLong));
   memcpy(h_logits.data_ptr(), base, nl);
   memcpy(h_top.data_ptr(), base + at_top, nt);
   int32_t code;
   memcpy(&code, base + at_word, 4);
   if (code != 0) check(brk_status_poll((int32_t*)word.data_ptr(), stream.stream()), "brk_status_poll");
   return {h_logits, h_top};
+}
+
+// A ranking request from host tensors to host results: what MistralPrefillRanker.rank_host does, in one call.
+// score_layer: {ln1, wq, wk} of the scoring layer.
+std::tuple<Tensor, Tensor> rank(const Tensor& embed, const std::vector<std::vector<Tensor>>& layers,
+                                const std::vector<Tensor>& score_layer, const Tensor& inv_freq, const Tensor& ids, const Tensor& pos,
+                                const Tensor& spans, const Tensor& rows, int64_t max_block_len, int64_t N, int64_t Nk, int64_t D,
+                                double eps, int64_t algo, double temperature, int64_t k) {
+  c10::cuda::CUDAGuard device(embed.device());
+  const auto [d_ids, d_pos, start, len, d_rows, longest] = upload(ids, pos, spans, rows, embed.device());
+  const Tensor flat = d_pos.reshape({-1});
+  const Tensor h = hidden_states(embed, d_ids, layers, flat, inv_freq, start, len, max_block_len, longest, N, Nk, D, eps, algo);
+  const auto [q, kk, local] = score_qk(h, flat, d_rows, score_layer.at(0), score_layer.at(1), score_layer.at(2), inv_freq, N, Nk, D, eps);
+  return download(std::get<1>(doc_scores(q, kk, start, len, local, 1.0 / std::sqrt((double)D), temperature)), k);
 }
 
 }  // namespace
@@ -574,4 +628,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("score_qk", &score_qk);
   m.def("upload", &upload);
   m.def("download", &download);
+  m.def("rank", &rank);
 }

@@ -145,7 +145,7 @@ class MistralPrefillRanker:
         pos = position_ids.reshape(B * S).to(torch.int32)
         if self.events is None:  # the layers in one native call
             return _lib.host().hidden_states(
-                self.embed, input_ids, [[L[n] for n in _LAYER_WEIGHTS] for L in self.layers[:c.score_layer]], pos, self.inv_freq,
+                self.embed, input_ids, self._full_layers(), pos, self.inv_freq,
                 blk_start, blk_len, max_block_len, max_query_len, c.num_attention_heads, c.num_key_value_heads, c.head_dim,
                 c.rms_norm_eps, self.algo)
         h = torch.embedding(self.embed, input_ids.reshape(B * S))
@@ -229,12 +229,22 @@ class MistralPrefillRanker:
         """End-to-end call on HOST tensors: ``batch`` holds pinned ``input_ids``/``position_ids`` (B, S) int64,
         ``block_spans`` int32 (2, B, M), ``signal_rows`` int32 (B, R) and ``max_block_len``.  Copies them to the
         device, scores, and returns (logits, top-k document indices) on the host."""
-        ids, pos, start, length, rows, max_query_len = _lib.host().upload(
-            batch["input_ids"], batch["position_ids"], batch["block_spans"], batch["signal_rows"], self.device)
+        c, host = self.cfg, _lib.host()
+        if not self.use_graphs and self.events is None:
+            last = self.layers[c.score_layer]
+            return host.rank(self.embed, self._full_layers(), [last["ln1"], last["wq"], last["wk"]], self.inv_freq,
+                             batch["input_ids"], batch["position_ids"], batch["block_spans"], batch["signal_rows"],
+                             int(batch["max_block_len"]), c.num_attention_heads, c.num_key_value_heads, c.head_dim,
+                             c.rms_norm_eps, self.algo, c.temperature, k)
+        ids, pos, start, length, rows, max_query_len = host.upload(
+            batch["input_ids"], batch["position_ids"], batch["block_spans"], batch["signal_rows"], self.embed.device)
         run = self.score_graphed if self.use_graphs else self.score
         logits, _ = run(ids, pos, start, length, int(batch["max_block_len"]), rows, max_query_len)
         # (raises if a kernel reported malformed spans or a wait that gave up)
-        return _lib.host().download(logits, k)
+        return host.download(logits, k)
+
+    def _full_layers(self):
+        return [[L[n] for n in _LAYER_WEIGHTS] for L in self.layers[:self.cfg.score_layer]]
 
     def weight_bytes(self) -> int:
         n = self.embed.numel() * self.embed.element_size()

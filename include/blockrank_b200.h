@@ -248,6 +248,11 @@ BRK_API int brk_rope(int32_t dtype, void* q, int64_t q_row_stride, int32_t N, vo
  * NULL; see brk_status_poll). */
 BRK_API int brk_signal_rows(int32_t dtype, const void* x, int32_t hidden, const int32_t* pos, const int32_t* rows, int32_t B,
                             int32_t S, int32_t R, void* x_out, int32_t* pos_out, int32_t* local, int32_t* status, void* stream);
+/* What a ranking call hands to its host: a copy of logits [B, nd], the indices of the k best documents of each prompt
+ * (top_out [B, k], best first; equal logits in document order, NaN first) and the status word.  nd <= BRK_RANK_PACK_DOCS. */
+#define BRK_RANK_PACK_DOCS 2048
+BRK_API int brk_rank_pack(const float* logits, int32_t B, int32_t nd, int32_t k, float* logits_out, int64_t* top_out,
+                          const int32_t* status, int32_t* status_out, void* stream);
 /* out[r, c] = silu(gate_up[r, c]) * gate_up[r, inter + c]. */
 BRK_API int brk_silu_mul(int32_t dtype, const void* gate_up, void* out, int64_t rows, int32_t inter, void* stream);
 
