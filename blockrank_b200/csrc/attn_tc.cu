@@ -43,6 +43,7 @@
 // a code in the caller's status word, stops waiting and runs to the normal exit.
 #include <cuda.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "attn_combine.cuh"
@@ -189,7 +190,7 @@ struct TcArgs {
   const int32_t* blk_start;
   const int32_t* blk_len;
   int32_t* status;
-  const int* hdr;   // workspace header: [0] work counter, [1] non-zero if the block spans are malformed
+  int* hdr;         // workspace header: [0] work counter, [1] non-zero if the block spans are malformed
   int B, N, Nk, S, M;
   int G, g_shift;   // query heads per KV head, log2
   float scale_log2;
@@ -437,6 +438,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       bad |= !span_ok(a.blk_start, a.blk_len, j, a.M, a.S, a.max_block_len, a.max_query_len);
     malformed = __syncthreads_or(bad);
     if (malformed && tid == 0 && a.status) atomicCAS(a.status, 0, kStatusBadSpans);
+    if (tid == 0) a.hdr[1] = malformed;  // for the merge kernel; every CTA writes the same
   } else {
     malformed = a.hdr[1] != 0;
   }
@@ -544,7 +546,15 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // ---- streamed pair: both chains walk the same 128-key tiles through a two-deep ring (slots 0-1, 2-3) ----
     auto run_pair = [&](int b, int g, int m, int chunk, int p, int start, int len, int s0, int l0, int s2, int l2) {
       Pair pr = decode_pair(a, b, g, m, chunk, p, start, len, s0, l0, s2, l2);
-      if (!pr.valid) return;
+      if (!pr.valid) {
+        if (a.one_wave && m == a.M - 1 && a.n_split > 1) {
+          // a chunk without keys: neutral statistics for its rows (the prologue kernel sets them otherwise)
+          const int t1 = min(len, pr.t0_0 + 2 * TOK);
+          for (int i = lane; i < (t1 - pr.t0_0) * G; i += 32)
+            a.part_ml[(((int64_t)b * a.N + g * G + i % G) * a.lq_max + pr.t0_0 + i / G) * a.n_split + chunk] = make_float2(-INFINITY, 0.f);
+        }
+        return;
+      }
       Job& it = pr.job;
       if (m == a.M - 1 && m > 0) {  // the query block's context may contain padding slots
         const int32_t* bl = a.blk_len + (size_t)b * a.M;
@@ -1226,12 +1236,18 @@ int attn_prologue_launch(const brk_attn_params& p, int* hdr, float2* ml, int64_t
 }
 
 // Key chunks for the query block.  Its context is every earlier token of the prompt (S is the only
-// bound known on the host), walked 128 keys per step per row tile; cutting it into chunks of about
-// 1024 keys keeps that serial chain short and spreads it over the SMs.
+// bound known on the host), walked 128 keys per step per row tile, 2.3 us each; cutting it into chunks of about
+// 1024 keys keeps that serial chain short and spreads it over the SMs.  A small call is cut further, down to 256 keys,
+// while its chunks find idle SMs: below 640 slots the chain is shorter than the merge.
 static int tc_splits(const brk_attn_params& p) {
   if (p.M < 2) return 1;
-  int n = (p.S + 1023) / 1024;
-  return n < 1 ? 1 : (n > 32 ? 32 : n);
+  int n = std::max(1, std::min(32, (p.S + 1023) / 1024));
+  if (p.S > 640) {
+    const int tok2 = 2 * BM / std::max(1, p.N / p.Nk);
+    const int64_t pairs = (int64_t)p.B * p.Nk * ((query_rows(p) + tok2 - 1) / tok2);
+    n = std::max(n, (int)std::min<int64_t>(std::min(32, (p.S + 255) / 256), sm_count() / std::max<int64_t>(1, pairs)));
+  }
+  return n;
 }
 
 size_t attn_tc_workspace(const brk_attn_params& p) {
@@ -1289,7 +1305,7 @@ static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cuda
   a.blk_start = p.blk_start;
   a.blk_len = p.blk_len;
   a.status = p.status;
-  a.hdr = reinterpret_cast<const int*>(ws);
+  a.hdr = reinterpret_cast<int*>(ws);
   a.B = p.B; a.N = p.N; a.Nk = p.Nk; a.S = p.S; a.M = p.M;
   a.G = G; a.g_shift = gs;
   a.scale_log2 = p.scale * 1.4426950408889634f;
@@ -1313,7 +1329,7 @@ static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cuda
   // themselves.  (One prompt of 5 documents: the prologue kernel and the gap behind it were 4 of 20 us.)
   a.max_block_len = p.max_block_len;
   a.max_query_len = p.max_query_len;
-  a.one_wave = ns == 1 && total_items <= sms[dev];
+  a.one_wave = total_items <= sms[dev];
   if (!a.one_wave && (rc = attn_prologue_launch(p, reinterpret_cast<int*>(ws), a.part_ml, ns > 1 ? (int64_t)rows : 0, st))) return rc;
   const int grid = (int)(total_items < sms[dev] ? total_items : sms[dev]);
   if ((rc = launch_dependent(attn_tc_kernel<HD>, dim3(grid), dim3(kThreads), Geo<HD>::kSmemBytes, st, tq, tk, tv, a))) return rc;
