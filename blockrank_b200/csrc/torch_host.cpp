@@ -9,6 +9,7 @@
 #include <ATen/ops/addmm_cuda_dispatch.h>
 #include <ATen/ops/mm_cuda_dispatch.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <cublas_v2.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/extension.h>
 
@@ -415,11 +416,37 @@ struct NoAutograd {
 };
 
 
+// out (+)= x w^T for row-major x (T, K), w (n, K): cuBLAS through PyTorch's handle (its stream, workspace and math mode), the
+// same product as torch.mm / addmm without their host path.
+void gemm_nt(Tensor& out, const Tensor& x, const Tensor& w, bool add) {
+  const int64_t T = x.size(0), K = x.size(1), n = w.size(0);
+  const bool plain = out.is_contiguous() && x.is_contiguous() && w.is_contiguous() && w.dim() == 2 && w.size(1) == K &&
+                     out.scalar_type() == x.scalar_type() && w.scalar_type() == x.scalar_type() && T > 0 && K > 0 && n > 0 &&
+                     std::max({T, K, n}) < (1ll << 31) &&
+                     (x.scalar_type() == at::kBFloat16 || x.scalar_type() == at::kFloat);
+  if (!plain) {
+    if (add) at::cuda::addmm_(out, x, w.t(), 1, 1);
+    else at::cuda::mm_out(out, x, w.t());
+    return;
+  }
+  const cudaDataType_t dt = x.scalar_type() == at::kBFloat16 ? CUDA_R_16BF : CUDA_R_32F;
+  const float one = 1.f, beta = add ? 1.f : 0.f;
+  const cublasStatus_t rc = cublasGemmEx(at::cuda::getCurrentCUDABlasHandle(), CUBLAS_OP_T, CUBLAS_OP_N, (int)n, (int)T, (int)K, &one,
+                                         w.data_ptr(), dt, (int)K, x.data_ptr(), dt, (int)K, &beta, out.data_ptr(), dt, (int)n,
+                                         CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT_TENSOR_OP);
+  TORCH_CHECK(rc == CUBLAS_STATUS_SUCCESS, "cublasGemmEx failed (", (int)rc, ")");
+}
+Tensor mm_nt(const Tensor& x, const Tensor& w) {
+  Tensor out = at::empty({x.size(0), w.size(0)}, x.options());
+  gemm_nt(out, x, w, false);
+  return out;
+}
+
 // input norm, fused QKV projection, RoPE on q and k in place: (T, (N + 2 Nk) D)
 Tensor layer_qkv(const Tensor& h, const Tensor& ln1, const Tensor& wqkv, const Tensor& pos, const Tensor& inv_freq, int64_t N,
                  int64_t Nk, int64_t D, double eps) {
   NoAutograd guard;
-  Tensor qkv = at::cuda::mm(rmsnorm(h, ln1, eps, std::nullopt, std::nullopt), wqkv.t());
+  Tensor qkv = mm_nt(rmsnorm(h, ln1, eps, std::nullopt, std::nullopt), wqkv);
   const int64_t T = qkv.size(0), row = qkv.stride(0), at0 = qkv.storage_offset();
   rope_(qkv.as_strided({T, N, D}, {row, D, 1}, at0), qkv.as_strided({T, Nk, D}, {row, D, 1}, at0 + N * D), pos, inv_freq);
   return qkv;
@@ -441,9 +468,9 @@ Tensor layer_attention(const Tensor& qkv, const Tensor& blk_start, const Tensor&
 void layer_rest(Tensor& h, const Tensor& attn, const Tensor& wo, const Tensor& ln2, const Tensor& wgu, const Tensor& wd,
                 double eps) {
   NoAutograd guard;
-  at::cuda::addmm_(h, attn.view({h.size(0), wo.size(1)}), wo.t(), 1, 1);
+  gemm_nt(h, attn.view({h.size(0), wo.size(1)}), wo, true);
   const Tensor x = rmsnorm(h, ln2, eps, std::nullopt, std::nullopt);
-  at::cuda::addmm_(h, silu_mul(at::cuda::mm(x, wgu.t()), std::nullopt), wd.t(), 1, 1);
+  gemm_nt(h, silu_mul(mm_nt(x, wgu), std::nullopt), wd, true);
 }
 
 // layers: {ln1, wqkv, wo, ln2, wgu, wd} of every layer in front of the scoring layer.  ids (B, S), pos int32 (B S,).
@@ -474,7 +501,7 @@ std::tuple<Tensor, Tensor, Tensor> score_qk(const Tensor& h, const Tensor& pos, 
             "signal_rows must be int32 (B, R) and positions contiguous int32");
   const int64_t B = signal_rows.size(0), R = signal_rows.size(1), T = h.size(0), S = T / B;
   const Tensor x = rmsnorm(h, ln1, eps, std::nullopt, std::nullopt), rows = signal_rows.contiguous();
-  Tensor k = at::cuda::mm(x, wk.t());
+  Tensor k = mm_nt(x, wk);
   Tensor xs = at::empty({B * R, x.size(1)}, x.options()), ps = at::empty({B * R}, pos.options()), local = at::empty({B, R}, pos.options());
   check(brk_signal_rows(dtype_code(x), x.data_ptr(), (int32_t)x.size(1), (const int32_t*)pos.data_ptr(),
                         (const int32_t*)rows.data_ptr(), (int32_t)B, (int32_t)S, (int32_t)R, xs.data_ptr(),
@@ -482,7 +509,7 @@ std::tuple<Tensor, Tensor, Tensor> score_qk(const Tensor& h, const Tensor& pos, 
                         stream_of(x)),
         "brk_signal_rows");
   count(1);
-  Tensor q = at::cuda::mm(xs, wq.t());
+  Tensor q = mm_nt(xs, wq);
   rope_(q.view({B * R, N, D}), std::nullopt, ps, inv_freq);
   rope_(std::nullopt, k.view({T, Nk, D}), pos, inv_freq);
   return {q.view({B, R, N, D}).permute({0, 2, 1, 3}), k.view({B, S, Nk, D}).permute({0, 2, 1, 3}), local};
