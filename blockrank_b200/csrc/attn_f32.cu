@@ -324,7 +324,7 @@ int attn_f32_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStr
   a.part_o = reinterpret_cast<float*>(static_cast<unsigned char*>(ws) + kWsHeader);
   a.part_ml = reinterpret_cast<float2*>(a.part_o + rows * p.D);
   // every (row, chunk) pair is written by the kernel, also of chunks without keys: nothing to reset
-  int rc = attn_prologue_launch(p, reinterpret_cast<int*>(ws), nullptr, 0, st);
+  int rc = attn_prologue_launch(p, reinterpret_cast<int*>(ws), nullptr, 0, nullptr, nullptr, 0, st);
   if (rc) return rc;
   if (p.D == 128) return launch<128>(p, a, st);
   if (p.D == 64) return launch<64>(p, a, st);

@@ -192,7 +192,7 @@ int launch_g(const brk_attn_params& p, const SimtArgs& a, cudaStream_t st) {
 int attn_simt_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStream_t st) {
   BRK_REQUIRE(ws != nullptr && ws_bytes >= kWsHeader && ((uintptr_t)ws & 15) == 0, BRK_E_WORKSPACE,
               "attention workspace: %zu bytes (16-byte aligned) needed, %zu given", kWsHeader, ws_bytes);
-  int rc = attn_prologue_launch(p, reinterpret_cast<int*>(ws), nullptr, 0, st);
+  int rc = attn_prologue_launch(p, reinterpret_cast<int*>(ws), nullptr, 0, nullptr, nullptr, 0, st);
   if (rc) return rc;
   SimtArgs a;
   a.hdr = reinterpret_cast<const int*>(ws);

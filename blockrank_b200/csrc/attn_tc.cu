@@ -207,6 +207,9 @@ struct TcArgs {
   int* work_counter;  // next unclaimed index of the work list (zeroed before the launch)
   float* part_o;    // [B, N, lq_max, n_split, 128] un-normalised partial outputs
   float2* part_ml;  // [B, N, lq_max, n_split] (running max in log2 units, sum)
+  const int4* win;    // [B, win_pitch] live 64-key windows of the query block's context, for prompts with padding inside it
+  const int* n_live;  // [B] how many, -1: no padding, every window is live (both null in a one-wave call)
+  int win_pitch;
 };
 
 // Is span j of the (B, M) arrays inside [0, S), no longer than allowed, and behind its predecessor?
@@ -220,7 +223,7 @@ __device__ __forceinline__ bool span_ok(const int32_t* blk_start, const int32_t*
 }
 
 // One row tile against a list of 64-key slots: what a chain works on.
-constexpr int kFSplit = 1, kFCtxCheck = 2, kFStop = 4, kFDoc = 8, kFFirst = 16, kFKeep = 32;
+constexpr int kFSplit = 1, kFCtxCheck = 2, kFStop = 4, kFDoc = 8, kFFirst = 16, kFKeep = 32, kFWindows = 64;
 struct Job {
   int b, g, m, chunk;
   int start, len;        // span of block m
@@ -285,6 +288,7 @@ struct ItemRaw {
   int start, len;      // span of block m + lane (kind 1) or of the query block (kind 0)
   int s0, l0;          // span of block 0 (the prefix)
   int s2, l2;          // span of block M-2 (end of the query block's context)
+  int live;            // kind 0: live windows of the context, -1: no list
 };
 
 // Work list: streamed pairs of the query block first (the longest items), then the groups of blocks 0 .. M-2.
@@ -322,6 +326,7 @@ __device__ __forceinline__ ItemRaw load_item(const TcArgs& a, int idx, int lane)
   r.l0 = bl[0];
   r.s2 = bs[m2];
   r.l2 = bl[m2];
+  r.live = r.kind == 0 && a.n_live ? a.n_live[r.b] : -1;
   return r;
 }
 
@@ -335,7 +340,7 @@ struct Pair {
 };
 
 __device__ __forceinline__ Pair decode_pair(const TcArgs& a, int b, int g, int m, int chunk, int p, int start, int len,
-                                            int s0, int l0, int s2, int l2) {
+                                            int s0, int l0, int s2, int l2, int live) {
   Pair pr;
   Job& it = pr.job;
   const int TOK = BM >> a.g_shift;
@@ -359,6 +364,11 @@ __device__ __forceinline__ Pair decode_pair(const TcArgs& a, int b, int g, int m
   const bool on1 = pr.t0_1 < len;
   it.own_n = min(len, (on1 ? pr.t0_1 : pr.t0_0) + TOK);
   it.n_ctx = (it.ctx_hi - it.ctx_lo + BN - 1) / BN;
+  if (live >= 0) {  // padding inside the context: its windows come from the list
+    it.n_ctx = live;
+    it.ctx_hi = it.ctx_lo + live * BN;  // (whole windows; their bits say which keys exist)
+    it.flags |= kFWindows | kFCtxCheck;
+  }
   const int own_slots = (it.own_n + BN - 1) / BN;
   int j1 = it.n_ctx + own_slots;
   if (split) {
@@ -544,8 +554,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     };
 
     // ---- streamed pair: both chains walk the same 128-key tiles through a two-deep ring (slots 0-1, 2-3) ----
-    auto run_pair = [&](int b, int g, int m, int chunk, int p, int start, int len, int s0, int l0, int s2, int l2) {
-      Pair pr = decode_pair(a, b, g, m, chunk, p, start, len, s0, l0, s2, l2);
+    auto run_pair = [&](int b, int g, int m, int chunk, int p, int start, int len, int s0, int l0, int s2, int l2, int live) {
+      Pair pr = decode_pair(a, b, g, m, chunk, p, start, len, s0, l0, s2, l2, live);
       if (!pr.valid) {
         if (a.one_wave && m == a.M - 1 && a.n_split > 1) {
           // a chunk without keys: neutral statistics for its rows (the prologue kernel sets them otherwise)
@@ -556,7 +566,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         return;
       }
       Job& it = pr.job;
-      if (m == a.M - 1 && m > 0) {  // the query block's context may contain padding slots
+      if (a.n_live == nullptr && m == a.M - 1 && m > 0) {  // the query block's context may contain padding slots
         const int32_t* bl = a.blk_len + (size_t)b * a.M;
         int part = 0;
         for (int i = lane; i < a.M - 1; i += 32) part += bl[i];
@@ -582,7 +592,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             ptx::mbar_expect_tx(bar(kKVFull + 2 * tb + v), (uint32_t)nslots * (kSlotBytes / 2));
             for (int h = 0; h < nslots; ++h) {
               int nk, own_off; bool own;
-              const int lo = tile_lo(it, 2 * t + h, nk, own, own_off);
+              int lo = tile_lo(it, 2 * t + h, nk, own, own_off);
+              if (!own && (it.flags & kFWindows)) lo = a.win[(size_t)b * a.win_pitch + it.j0 + 2 * t + h].x;
               load_slot(v, 2 * tb + h, 2 * tb + v, g, b, lo);
             }
           }
@@ -693,7 +704,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       const ItemRaw raw = raw_next;
       raw_next = load_item(a, idx_next, lane);  // in flight while this item is processed
       if (raw.kind == 0) {
-        run_pair(raw.b, raw.g, raw.m, raw.chunk, raw.p, raw.start, raw.len, raw.s0, raw.l0, raw.s2, raw.l2);
+        run_pair(raw.b, raw.g, raw.m, raw.chunk, raw.p, raw.start, raw.len, raw.s0, raw.l0, raw.s2, raw.l2, raw.live);
         continue;
       }
       auto fits = [&](int m, int len) {
@@ -713,7 +724,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         } else {
           const int pairs = (len + 2 * TOK - 1) / (2 * TOK);
           for (int p = 0; p < pairs; ++p)
-            run_pair(raw.b, raw.g, m, 0, p, start, len, raw.s0, raw.l0, raw.s2, raw.l2);
+            run_pair(raw.b, raw.g, m, 0, p, start, len, raw.s0, raw.l0, raw.s2, raw.l2, -1);
         }
       }
     }
@@ -971,13 +982,22 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           // A masked logit becomes -inf with one select per column, so that its P is exactly 0 and the
           // pass below stays one basic block: skipping the 8-column groups that no row of the warp sees
           // with warp-uniform branches measured 5 % slower over the whole kernel than exponentiating them.
-          const bool premasked = !own && ctx_check;  // padded context: columns masked one by one from the slot-validity ballots
+          const bool premasked = !own && ctx_check;  // padded context: columns masked one by one from the slots' validity bits
           if (nk < BN || (own && own_off + BN - 1 > it.t0) || premasked) {  // (warp-uniform)
             int lim = nk;
             if (own) lim = max(0, min(nk, tok - own_off + 1));
             if (premasked) {
-              const unsigned v0 = __ballot_sync(0xffffffffu, slot_valid(bs, bl, a.M, lo + lane));
-              const unsigned v1 = __ballot_sync(0xffffffffu, slot_valid(bs, bl, a.M, lo + 32 + lane));
+              // They come with the list of windows; a one-wave call has no list and searches the spans.  (Searching them in
+              // every slot, empty ones too, took a grid of 100 documents of 32..256 tokens from 155 to 190 us.)
+              unsigned v0, v1;
+              if (flags & kFWindows) {
+                const int4 w = a.win[(size_t)it.b * a.win_pitch + it.j0 + 2 * t + h];
+                v0 = (unsigned)w.y;
+                v1 = (unsigned)w.z;
+              } else {
+                v0 = __ballot_sync(0xffffffffu, slot_valid(bs, bl, a.M, lo + lane));
+                v1 = __ballot_sync(0xffffffffu, slot_valid(bs, bl, a.M, lo + 32 + lane));
+              }
 #pragma unroll
               for (int c = 0; c < 64; ++c) {
                 const bool ok = c < lim && (((c < 32 ? v0 : v1) >> (c & 31)) & 1u);
@@ -1203,10 +1223,73 @@ int selftest_wait_launch(int32_t* status, uint32_t budget, cudaStream_t st) {
 // Launched in front of either attention kernel.  Block 0 checks the block spans (inside [0, S), no longer than
 // max_block_len, ordered, not overlapping) and records the verdict in the workspace header -- a non-zero hdr[1]
 // makes the attention kernels return without touching memory, and the caller's status word (if any) gets
-// kStatusBadSpans.  All blocks reset the work counter and the query block's partial (max, sum) pairs to neutral.
-__global__ void attn_prologue_kernel(const int32_t* __restrict__ blk_start, const int32_t* __restrict__ blk_len, int B,
+// kStatusBadSpans.  All blocks reset the work counter and the query block's partial (max, sum) pairs to neutral.  With a
+// window list, the last B blocks write it, one prompt each: the 64-slot windows of the query block's context that hold
+// any key, {first slot, validity bits}, for prompts with padding between their blocks (a grid of ragged documents: 100
+// documents of 32..256 tokens fill 272 of 404 windows).
+__device__ void live_windows(const int32_t* bs, const int32_t* bl, int M, int4* win, int* n_live, int pitch) {
+  constexpr int kMaxSharedSpans = 2048;
+  __shared__ int s_span[2 * kMaxSharedSpans], s_cnt[8], s_sum;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) s_sum = 0;
+  __syncthreads();
+  int sum = 0;
+  for (int i = tid; i < M; i += 256) {
+    if (i < M - 1) sum += bl[i];
+    if (M <= kMaxSharedSpans) {
+      s_span[i] = bs[i];
+      s_span[M + i] = bl[i];
+    }
+  }
+  atomicAdd(&s_sum, sum);
+  __syncthreads();
+  if (M <= kMaxSharedSpans) {
+    bs = s_span;
+    bl = s_span + M;
+  }
+  const int lo0 = bs[0], hi = bs[M - 2] + bl[M - 2];
+  if (s_sum == hi - lo0) {
+    if (tid == 0) *n_live = -1;
+    return;
+  }
+  const int nw = max(0, min(pitch, (hi - lo0 + BN - 1) / BN));
+  int base = 0;
+  for (int w0 = 0; w0 < nw; w0 += 256) {
+    const int lo = lo0 + (w0 + tid) * BN;
+    unsigned long long bits = 0;
+    if (w0 + tid < nw) {
+      int l = 0, h = M;  // first block that starts behind lo
+      while (l < h) {
+        const int mid = (l + h) >> 1;
+        if (bs[mid] <= lo) l = mid + 1; else h = mid;
+      }
+      for (int m = max(0, l - 1); m < M - 1 && bs[m] < lo + BN; ++m) {
+        const int x0 = max(bs[m] - lo, 0), x1 = min(bs[m] + bl[m] - lo, BN);
+        if (x1 > x0) bits |= (~0ull >> (BN - (x1 - x0))) << x0;
+      }
+    }
+    const unsigned live = __ballot_sync(0xffffffffu, bits != 0);
+    if (lane == 0) s_cnt[warp] = __popc(live);
+    __syncthreads();
+    int at = base + __popc(live & ((1u << lane) - 1u));
+    for (int i = 0; i < 8; ++i) {
+      if (i < warp) at += s_cnt[i];
+      base += s_cnt[i];
+    }
+    if (bits != 0) win[at] = make_int4(lo, (int)(unsigned)bits, (int)(unsigned)(bits >> 32), 0);
+    __syncthreads();
+  }
+  if (tid == 0) *n_live = base;
+}
+
+__global__ void __launch_bounds__(256) attn_prologue_kernel(const int32_t* __restrict__ blk_start, const int32_t* __restrict__ blk_len, int B,
                                      int M, int S, int max_block_len, int max_query_len, int* hdr, int32_t* status,
-                                     float2* ml, int64_t n_ml) {
+                                     float2* ml, int64_t n_ml, int4* win, int* n_live, int win_pitch) {
+  if (win != nullptr && blockIdx.x >= gridDim.x - B) {
+    const int b = blockIdx.x - (gridDim.x - B);
+    live_windows(blk_start + (size_t)b * M, blk_len + (size_t)b * M, M, win + (size_t)b * win_pitch, n_live + b, win_pitch);
+    return;
+  }
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n_ml) ml[i] = make_float2(-INFINITY, 0.f);
   if (blockIdx.x != 0) return;
@@ -1227,10 +1310,11 @@ __global__ void attn_prologue_kernel(const int32_t* __restrict__ blk_start, cons
   }
 }
 
-int attn_prologue_launch(const brk_attn_params& p, int* hdr, float2* ml, int64_t n_ml, cudaStream_t st) {
-  const unsigned blocks = (unsigned)(n_ml > 0 ? (n_ml + 255) / 256 : 1);
+int attn_prologue_launch(const brk_attn_params& p, int* hdr, float2* ml, int64_t n_ml, int4* win, int* n_live, int win_pitch,
+                         cudaStream_t st) {
+  const unsigned blocks = (unsigned)(n_ml > 0 ? (n_ml + 255) / 256 : 1) + (win ? p.B : 0);
   attn_prologue_kernel<<<blocks, 256, 0, st>>>(p.blk_start, p.blk_len, p.B, p.M, p.S, p.max_block_len, p.max_query_len,
-                                               hdr, p.status, ml, n_ml);
+                                               hdr, p.status, ml, n_ml, win, n_live, win_pitch);
   BRK_CUDA(cudaGetLastError());
   return BRK_OK;
 }
@@ -1250,11 +1334,15 @@ static int tc_splits(const brk_attn_params& p) {
   return n;
 }
 
+// Header (work counter, span verdict), live windows of the query block's context, partials of its key chunks.
+static int win_pitch(const brk_attn_params& p) { return p.S / BN + 1; }
+static size_t window_bytes(const brk_attn_params& p) {
+  return ((size_t)p.B * (win_pitch(p) * sizeof(int4) + sizeof(int)) + 255) & ~(size_t)255;
+}
 size_t attn_tc_workspace(const brk_attn_params& p) {
   const int ns = tc_splits(p);
-  if (ns <= 1) return kWsHeader;  // work counter and span verdict
-  const size_t rows = (size_t)p.B * p.N * query_rows(p) * ns;
-  return kWsHeader + rows * p.D * sizeof(float) + rows * sizeof(float2);
+  const size_t rows = ns > 1 ? (size_t)p.B * p.N * query_rows(p) * ns : 0;
+  return kWsHeader + window_bytes(p) + rows * (p.D * sizeof(float) + sizeof(float2));
 }
 
 template <int HD>
@@ -1321,7 +1409,8 @@ static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cuda
   a.div_nbg = make_fastdiv((uint32_t)nbg);
   a.div_nk = make_fastdiv((uint32_t)p.Nk);
   const size_t rows = (size_t)p.B * p.N * lq * ns;
-  float* const part = reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + kWsHeader);
+  int4* const win = reinterpret_cast<int4*>(static_cast<uint8_t*>(ws) + kWsHeader);
+  float* const part = reinterpret_cast<float*>(static_cast<uint8_t*>(ws) + kWsHeader + window_bytes(p));
   a.work_counter = reinterpret_cast<int*>(ws);
   a.part_o = ns > 1 ? part : nullptr;
   a.part_ml = ns > 1 ? reinterpret_cast<float2*>(part + rows * HD) : nullptr;
@@ -1330,7 +1419,20 @@ static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cuda
   a.max_block_len = p.max_block_len;
   a.max_query_len = p.max_query_len;
   a.one_wave = total_items <= sms[dev];
-  if (!a.one_wave && (rc = attn_prologue_launch(p, reinterpret_cast<int*>(ws), a.part_ml, ns > 1 ? (int64_t)rows : 0, st))) return rc;
+  a.win = nullptr;
+  a.n_live = nullptr;
+  a.win_pitch = win_pitch(p);
+  if (!a.one_wave) {
+    int* const n_live = reinterpret_cast<int*>(win + (size_t)p.B * a.win_pitch);
+    const bool list = p.M > 2;  // (a single block has no gaps)
+    if (list) {
+      a.win = win;
+      a.n_live = n_live;
+    }
+    if ((rc = attn_prologue_launch(p, reinterpret_cast<int*>(ws), a.part_ml, ns > 1 ? (int64_t)rows : 0, list ? win : nullptr, n_live,
+                                   a.win_pitch, st)))
+      return rc;
+  }
   const int grid = (int)(total_items < sms[dev] ? total_items : sms[dev]);
   if ((rc = launch_dependent(attn_tc_kernel<HD>, dim3(grid), dim3(kThreads), Geo<HD>::kSmemBytes, st, tq, tk, tv, a))) return rc;
   if (ns > 1) {

@@ -126,7 +126,8 @@ constexpr int kStatusBadRows = 51;
 constexpr int kStatusSelfTest = 90;
 
 // kernel launchers implemented in the .cu files
-int attn_prologue_launch(const brk_attn_params& p, int* hdr, float2* ml, int64_t n_ml, cudaStream_t st);
+int attn_prologue_launch(const brk_attn_params& p, int* hdr, float2* ml, int64_t n_ml, int4* win, int* n_live, int win_pitch,
+                         cudaStream_t st);
 int attn_simt_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStream_t st);
 int selftest_wait_launch(int32_t* status, uint32_t budget, cudaStream_t st);
 int attn_tc_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStream_t st);

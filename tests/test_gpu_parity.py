@@ -131,6 +131,28 @@ def test_attention_tc_head_dim_64_vs_oracle(case):
     assert out.float().cpu()[~rows].abs().sum().item() == 0
 
 
+@pytest.mark.parametrize("M,H", [(40, 80), (41, 64), (60, 16), (220, 80)])  # the last: more than 256 windows of 64 slots
+def test_attention_tc_padded_query_context(M, H):
+    """The query block's context as live windows: no padding, stretches of empty documents, one-token documents."""
+    B, N, Nk, D = 3, 8, 2, 128
+    lens = H_.random_lens(B, M, H, 71)
+    lens[0] = [H] * M
+    lens[1][3:M - 4] = [0] * (M - 7)
+    lens[2][1:M - 1] = [1] * (M - 2)
+    mask = H_.ragged_mask(B, M, H, lens)
+    q, k, v = H_.qkv(B, N, Nk, M * H, D, 171, torch.bfloat16)
+    out, lse = _run_attn(q, k, v, mask, D ** -0.5, TC, lse=True)
+    if M * H <= 4096:
+        ref, ref_lse = orc.attention_dense(q, k, v, mask, D ** -0.5)
+    else:
+        ref, ref_lse = (t.cpu() for t in _run_attn(q, k, v, mask, D ** -0.5, SIMT, lse=True))
+    rows = mask.reshape(B, -1)
+    assert (out.float().cpu() - ref.float())[rows].abs().max().item() < 2e-2
+    lrows = rows[:, None, :].expand(B, N, M * H)
+    assert (lse.cpu() - ref_lse.float())[lrows].abs().max().item() < 2e-3
+    assert out.float().cpu()[~rows].abs().sum().item() == 0
+
+
 @pytest.mark.parametrize("algo", [SIMT, TC])
 def test_attention_large_logit_range(algo):
     """Logits spread over tens of units (queries scaled up): the running maximum jumps by more than the
