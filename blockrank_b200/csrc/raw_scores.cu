@@ -14,7 +14,7 @@
 // All four are bound by memory: per prompt of 100 documents (32/8 heads, 16 rows, 16,320 slots) the forward moves
 // 33 MB of keys and writes 17 MB of logits, the backward reads those and updates 33 MB of dk, for 2 and 4 GFLOP.
 // Measured there: forward 21.6 us (one thread per key row on CUDA cores: 230 us); 4 prompts of 20 documents (14,080
-// slots): forward 19 us (195), backward 47 us (fp32 matrix products, casts, fills and sums in PyTorch: about 500);
+// slots): forward 19 us (195), backward 29 us (fp32 matrix products, casts, fills and sums in PyTorch: about 500);
 // fp32 forward, 1 prompt of 20 documents: 21 us (81).
 #include <algorithm>
 
@@ -241,12 +241,18 @@ struct RawBwdArgs {
 // One CTA walks through 64-slot tiles of a (prompt, KV head).  q of 64 (head, row) pairs stays in shared memory; d_raw
 // [64 pairs x 64 slots] and k of a tile are staged, dk comes from 16 slots per warp, dq from 16 pairs per warp (held in
 // registers over all of the CTA's tiles).  More than 64 pairs: the passes over the pairs add into dk one after another.
+// d_raw, k and the dk to be added to arrive one tile ahead (two stages, two CTAs per SM): with three CTAs of one stage each,
+// 4 prompts of 20 documents took 48 us, most of it waiting for these loads; now 29.
+template <int D>
+struct RawBwdStage {
+  MmaTile<D> k, old;
+  MmaTile<kKeys> g;
+};
 template <int D>
 __global__ void __launch_bounds__(kThreads) raw_bwd_mma_kernel(RawBwdArgs a) {
   extern __shared__ __align__(16) unsigned char dyn[];
   MmaTile<D>& qt = *reinterpret_cast<MmaTile<D>*>(dyn);
-  MmaTile<D>& kt = *reinterpret_cast<MmaTile<D>*>(dyn + sizeof(MmaTile<D>));
-  MmaTile<kKeys>& gt = *reinterpret_cast<MmaTile<kKeys>*>(dyn + 2 * sizeof(MmaTile<D>));
+  RawBwdStage<D>* const stages = reinterpret_cast<RawBwdStage<D>*>(dyn + sizeof(MmaTile<D>));
   const ScoreArgs& s = a.s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
   const int G = s.N / s.Nk, GR = G * s.R;
@@ -268,27 +274,39 @@ __global__ void __launch_bounds__(kThreads) raw_bwd_mma_kernel(RawBwdArgs a) {
     float dq[D / 8][4];
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) dq[i][0] = dq[i][1] = dq[i][2] = dq[i][3] = 0.f;
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    const bool add = a.add || r0 > 0;
+    auto request = [&](int tile, RawBwdStage<D>& st) {
       const int s0 = tile * kKeys;
       for (int i = tid; i < kKeys * (D / 8); i += kThreads) {
-        const int row = i / (D / 8), c = i % (D / 8);
-        cp_async16_zfill(&kt.e[row][c * 8], kb + (int64_t)min(s0 + row, s.S - 1) * s.k.ss + c * 8, s0 + row < s.S);
+        const int row = i / (D / 8), c = i % (D / 8), sl = min(s0 + row, s.S - 1);
+        cp_async16_zfill(&st.k.e[row][c * 8], kb + (int64_t)sl * s.k.ss + c * 8, s0 + row < s.S);
+        if (add) cp_async16_zfill(&st.old.e[row][c * 8], dkb + (int64_t)sl * a.dk.ss + c * 8, s0 + row < s.S);
       }
       if (vec) {
         for (int i = tid; i < kRowsPass * (kKeys / 8); i += kThreads) {
           const int rr = i / (kKeys / 8), c = i % (kKeys / 8) * 8;
           const bool ok = rr < nrow && s0 + c < s.S;
-          cp_async16_zfill(&gt.e[rr][c], gb + (int64_t)(r0 + (ok ? rr : 0)) * s.S + (ok ? s0 + c : 0), ok);
+          cp_async16_zfill(&st.g.e[rr][c], gb + (int64_t)(r0 + (ok ? rr : 0)) * s.S + (ok ? s0 + c : 0), ok);
         }
       } else {
         for (int i = tid; i < kRowsPass * kKeys; i += kThreads) {
           const int rr = i / kKeys, c = i % kKeys;
-          gt.e[rr][c] = rr < nrow && s0 + c < s.S ? gb[(int64_t)(r0 + rr) * s.S + s0 + c] : __float2bfloat16_rn(0.f);
+          st.g.e[rr][c] = rr < nrow && s0 + c < s.S ? gb[(int64_t)(r0 + rr) * s.S + s0 + c] : __float2bfloat16_rn(0.f);
         }
       }
+    };
+    int tile = blockIdx.x, buf = 0;
+    if (tile < n_tiles) request(tile, stages[0]);
+    cp_async_commit();
+    for (; tile < n_tiles; tile += gridDim.x, buf ^= 1) {
+      const int s0 = tile * kKeys;
+      if (tile + (int)gridDim.x < n_tiles) request(tile + gridDim.x, stages[buf ^ 1]);
       cp_async_commit();
-      cp_async_wait<0>();
+      cp_async_wait<1>();
       __syncthreads();
+      MmaTile<D>& kt = stages[buf].k;
+      const MmaTile<D>& old = stages[buf].old;
+      const MmaTile<kKeys>& gt = stages[buf].g;
       // dq: pairs 16 warp .. + 15, contraction over the 64 slots
 #pragma unroll
       for (int c0 = 0; c0 < kKeys; c0 += 16) {
@@ -314,7 +332,6 @@ __global__ void __launch_bounds__(kThreads) raw_bwd_mma_kernel(RawBwdArgs a) {
         *reinterpret_cast<uint32_t*>(&kt.e[warp * 16 + gq + 8][col]) = pack_bf16(dk[nt][2] * s.scale, dk[nt][3] * s.scale);
       }
       __syncthreads();
-      const bool add = a.add || r0 > 0;
       for (int i = tid; i < kKeys * (D / 8); i += kThreads) {
         const int row = i / (D / 8), c = i % (D / 8);
         if (s0 + row >= s.S) continue;
@@ -323,7 +340,7 @@ __global__ void __launch_bounds__(kThreads) raw_bwd_mma_kernel(RawBwdArgs a) {
         if (add) {
           float v[8], o[8];
           load8(&kt.e[row][c * 8], v);
-          load8(p, o);
+          load8(&old.e[row][c * 8], o);
 #pragma unroll
           for (int j = 0; j < 8; ++j) v[j] += o[j];
           store8(p, v);
@@ -339,10 +356,7 @@ __global__ void __launch_bounds__(kThreads) raw_bwd_mma_kernel(RawBwdArgs a) {
       if (rr >= nrow) continue;
       float* d = a.dq32 + ((int64_t)(b * s.N + g * G) * s.R + r0 + rr) * D + 2 * tq;
 #pragma unroll
-      for (int nt = 0; nt < D / 8; ++nt) {
-        atomicAdd(d + nt * 8, dq[nt][2 * h]);
-        atomicAdd(d + nt * 8 + 1, dq[nt][2 * h + 1]);
-      }
+      for (int nt = 0; nt < D / 8; ++nt) atomicAdd(reinterpret_cast<float2*>(d + nt * 8), make_float2(dq[nt][2 * h], dq[nt][2 * h + 1]));
     }
   }
 }
@@ -510,15 +524,15 @@ int raw_scores_bwd_launch(const brk_score_params& p, const void* d_raw, const br
   const int64_t n4 = (int64_t)p.B * p.N * p.R * (p.D / 4);
   const unsigned rows_grid = (unsigned)((n4 + 255) / 256);
   if (p.dtype == BRK_BF16) {
-    const dim3 grid(tiles_grid(p.S, p.B * p.Nk, 3), p.B * p.Nk);
+    const dim3 grid(tiles_grid(p.S, p.B * p.Nk, 2), p.B * p.Nk);
     auto go = [&](auto kern, size_t sm) -> int {
       BRK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
       kern<<<grid, kThreads, sm, st>>>(a);
       BRK_CUDA(cudaGetLastError());
       return BRK_OK;
     };
-    rc = p.D == 128 ? go(raw_bwd_mma_kernel<128>, 2 * sizeof(MmaTile<128>) + sizeof(MmaTile<kKeys>))
-                    : go(raw_bwd_mma_kernel<64>, 2 * sizeof(MmaTile<64>) + sizeof(MmaTile<kKeys>));
+    rc = p.D == 128 ? go(raw_bwd_mma_kernel<128>, sizeof(MmaTile<128>) + 2 * sizeof(RawBwdStage<128>))
+                    : go(raw_bwd_mma_kernel<64>, sizeof(MmaTile<64>) + 2 * sizeof(RawBwdStage<64>));
     if (rc) return rc;
     raw_bwd_rows_kernel<__nv_bfloat16><<<rows_grid, 256, 0, st>>>(a, p.D);
   } else {
