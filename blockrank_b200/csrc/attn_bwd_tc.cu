@@ -691,12 +691,15 @@ __device__ __forceinline__ bool slot_in_block(const BwdTcArgs& a, int b, int s) 
   return s < start + len;
 }
 
-// delta = rowsum(dO * O): one warp per 32 slots of one (prompt, head), HD / 8 lanes per row.  The same warps write the
-// zeros of the slots outside every block; all threads clear the accumulators and the item counter.  Bound by memory:
-// reads O and dO once.  The last block orders the items.
+// delta = rowsum(dO * O): eight slots and all heads of a prompt per CTA, one token per warp, so that a warp's reads are
+// contiguous; the sums change places in shared memory, because delta is kept by head.  The same warps write the zeros of
+// the slots outside every block; all threads clear the accumulators and the item counter.  Bound by memory: reads O and
+// dO once.  The first block orders the items.  (By warps that owned 32 slots of one head, reads 8 KB apart, a grid of 100
+// documents of 32..256 tokens took 72 us, now 62; 16 slots per CTA: 70.)
+constexpr int kPrepTok = 8;
 template <int HD>
-__global__ void __launch_bounds__(256) attn_bwd_tc_prep_kernel(BwdTcArgs a, float4* zero, int64_t n_zero) {
-  if (a.order && blockIdx.x == gridDim.x - 1) {
+__global__ void __launch_bounds__(256, 4) attn_bwd_tc_prep_kernel(BwdTcArgs a, float4* zero, int64_t n_zero) {
+  if (a.order && blockIdx.x == 0) {
     // (prompt, block) pairs by length, longest first (counting sort, one bucket per 8 tokens up to 512)
     __shared__ int first[64];
     const int n = a.B * a.M;
@@ -721,53 +724,74 @@ __global__ void __launch_bounds__(256) attn_bwd_tc_prep_kernel(BwdTcArgs a, floa
     for (int i = threadIdx.x; i < n; i += 256) a.order[atomicAdd(&first[bucket(i)], 1)] = i;
     return;
   }
-  const int64_t gid = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  for (int64_t i = gid; i < n_zero; i += (int64_t)(gridDim.x - (a.order ? 1 : 0)) * 256) zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int skip = a.order ? 1 : 0, blk = blockIdx.x - skip;
+  const int64_t gid = (int64_t)blk * 256 + threadIdx.x;
+  for (int64_t i = gid; i < n_zero; i += (int64_t)(gridDim.x - skip) * 256) zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   if (gid == 0) *a.counter = 0;
-  const int lane = threadIdx.x & 31;
-  const int groups = (a.S + 31) / 32;
-  const int64_t w = gid >> 5;
-  if (w >= (int64_t)a.B * groups * a.N) return;
-  const int n = (int)(w % a.N), grp = (int)((w / a.N) % groups), b = (int)(w / ((int64_t)a.N * groups));
-  const __nv_bfloat16* gp = reinterpret_cast<const __nv_bfloat16*>(a.d_o.ptr) + (int64_t)b * a.d_o.sb + (int64_t)n * a.d_o.sh;
-  const __nv_bfloat16* op = reinterpret_cast<const __nv_bfloat16*>(a.o.ptr) + (int64_t)b * a.o.sb + (int64_t)n * a.o.sh;
-  constexpr int kLanes = HD / 8, kRows = 32 / kLanes;  // lanes per row, rows per pass
-  const int sub = lane / kLanes, c = (lane % kLanes) * 8;
-  const int own = grp * 32 + lane;
-  const unsigned live = __ballot_sync(0xffffffffu, own < a.S && slot_in_block(a, b, own));  // the others are not read
-  float mine = 0.f;
-#pragma unroll 4
-  for (int r = 0; r < 32; r += kRows) {
-    const int s = grp * 32 + r + sub;
-    float d = 0.f;
-    if ((live >> (r + sub)) & 1u) {
-      float x[8], y[8];
-      load8(gp + (int64_t)s * a.d_o.ss + c, x);
-      load8(op + (int64_t)s * a.o.ss + c, y);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) d = fmaf(x[i], y[i], d);
-    }
-#pragma unroll
-    for (int off = kLanes / 2; off > 0; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
-#pragma unroll
-    for (int k = 0; k < kRows; ++k) {
-      const float v = __shfl_sync(0xffffffffu, d, k * kLanes);
-      if (lane == r + k) mine = v;
-    }
+  constexpr int kLanes = HD / 8, kRows = 32 / kLanes;  // lanes per row, heads per access of a warp
+  constexpr int kHeads = 64;                            // heads per pass through shared memory
+  __shared__ float s_delta[kHeads][kPrepTok + 1];
+  __shared__ unsigned s_live;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int groups = (a.S + kPrepTok - 1) / kPrepTok;
+  const int b = blk / groups, t0 = (blk % groups) * kPrepTok;
+  if (warp == 0) {
+    const unsigned l = __ballot_sync(0xffffffffu, lane < kPrepTok && t0 + lane < a.S && slot_in_block(a, b, t0 + lane));
+    if (lane == 0) s_live = l;
   }
-  if (own < a.S) a.delta[((size_t)b * a.N + n) * a.S + own] = mine;
-  unsigned gap = ~live & __ballot_sync(0xffffffffu, own < a.S);
-  for (; gap; gap &= gap - 1) {
-    const int z = grp * 32 + __ffs((int)gap) - 1;
-    auto clear = [&](const View& t) {
-      __nv_bfloat16* p = reinterpret_cast<__nv_bfloat16*>(t.ptr) + (int64_t)b * t.sb + (int64_t)n * t.sh + (int64_t)z * t.ss;
-      if (lane < kLanes) *reinterpret_cast<uint4*>(p + lane * 8) = make_uint4(0, 0, 0, 0);
-    };
-    clear(a.dq);
-    if (n < a.Nk) {
-      clear(a.dk);
-      clear(a.dv);
+  __syncthreads();
+  const unsigned live = s_live;
+  const int sub = lane / kLanes, c = (lane % kLanes) * 8;
+  auto at = [&](const View& t, int s, int n) {
+    return reinterpret_cast<__nv_bfloat16*>(t.ptr) + (int64_t)b * t.sb + (int64_t)s * t.ss + (int64_t)n * t.sh + c;
+  };
+  auto clear = [&](const View& t, int s, int heads) {
+    for (int n = sub; n < heads; n += kRows) *reinterpret_cast<uint4*>(at(t, s, n)) = make_uint4(0, 0, 0, 0);
+  };
+  for (int n0 = 0; n0 < a.N; n0 += kHeads) {
+    const int nh = min(kHeads, a.N - n0);
+    for (int t = warp; t < kPrepTok; t += 8) {
+      const int s = t0 + t;
+      if (!((live >> t) & 1u)) {  // (not read)
+        if (s < a.S && n0 == 0) {
+          clear(a.dq, s, a.N);
+          clear(a.dk, s, a.Nk);
+          clear(a.dv, s, a.Nk);
+        }
+        for (int n = lane; n < nh; n += 32) s_delta[n][t] = 0.f;
+        continue;
+      }
+      const __nv_bfloat16 *const gp = at(a.d_o, s, n0 + sub), *const op = at(a.o, s, n0 + sub);
+#pragma unroll 1
+      for (int n1 = 0; n1 < nh; n1 += 4 * kRows) {
+        uint4 x[4], y[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int n = min(n1 + i * kRows, nh - 1 - sub);  // (past the last head: read again, not kept)
+          x[i] = *reinterpret_cast<const uint4*>(gp + (int64_t)n * a.d_o.sh);
+          y[i] = *reinterpret_cast<const uint4*>(op + (int64_t)n * a.o.sh);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float d = 0.f;
+          auto dot = [&](uint32_t u, uint32_t v) {
+            const float2 p = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u));
+            const float2 q = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&v));
+            d = fmaf(p.y, q.y, fmaf(p.x, q.x, d));
+          };
+          dot(x[i].x, y[i].x); dot(x[i].y, y[i].y); dot(x[i].z, y[i].z); dot(x[i].w, y[i].w);
+#pragma unroll
+          for (int off = kLanes / 2; off > 0; off >>= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
+          if (c == 0 && n1 + i * kRows + sub < nh) s_delta[n1 + i * kRows + sub][t] = d;
+        }
+      }
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < nh * kPrepTok; i += 256) {
+      const int n = i / kPrepTok, t = i % kPrepTok;
+      if (t0 + t < a.S) a.delta[((size_t)b * a.N + n0 + n) * a.S + t0 + t] = s_delta[n][t];
+    }
+    __syncthreads();
   }
 }
 
@@ -815,8 +839,8 @@ int launch(const brk_attn_bwd_params& p, BwdTcArgs a, float4* zero, int64_t n_ze
   if ((rc = make_tmap_f32(&t.dq32, a.dq32, HD, p.N, p.max_block_len, p.B, mbl * HD, HD, (int64_t)p.N * mbl * HD, a.G, tok_w))) return rc;
   t.pre = t.dq32;
   if (a.pre && (rc = make_tmap_f32(&t.pre, a.pre, HD, 2 * p.B * p.Nk, p.max_block_len, 1, mbl * HD, HD, 0, 1, 32))) return rc;
-  const int64_t warps = (int64_t)p.B * ((p.S + 31) / 32) * p.N;
-  attn_bwd_tc_prep_kernel<HD><<<(unsigned)((warps + 7) / 8 + (a.order ? 1 : 0)), 256, 0, st>>>(a, zero, n_zero);
+  const unsigned prep = (unsigned)p.B * ((p.S + kPrepTok - 1) / kPrepTok) + (a.order ? 1 : 0);
+  attn_bwd_tc_prep_kernel<HD><<<prep, 256, 0, st>>>(a, zero, n_zero);
   BRK_CUDA(cudaGetLastError());
   BRK_CUDA(cudaFuncSetAttribute(attn_bwd_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Geo<HD>::kSmem));
   const int sms = sm_count();

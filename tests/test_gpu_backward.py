@@ -136,6 +136,7 @@ TC_EDGES = [  # name, block lengths per prompt, H, N, Nk, D: tile edges of the t
     ("group_1", [[40, 129, 200, 5, 60]], 200, 2, 2, 64),
     ("two_long_blocks", [[200, 150]], 200, 4, 2, 128),
     ("longer_than_the_scratch", [[30, 600, 40]], 600, 4, 1, 64),  # more than 16 row tiles: the warp-level kernels
+    ("heads_beyond_a_pass", [[5, 12, 1, 7], [12, 0, 3, 9]], 13, 72, 9, 64),  # delta: 64 heads per pass, 52 slots in eights
 ]
 
 
@@ -205,6 +206,8 @@ def test_fused_doc_scores_refuse_autograd():
     (4, 2, 128, 7, 16, 16, torch.bfloat16),    # 32 pairs
     (16, 2, 64, 4, 32, 16, torch.bfloat16),    # 128 pairs: two passes
     (2, 1, 128, 3, 9, 5, torch.bfloat16),      # odd S (27), odd R
+    (32, 8, 64, 40, 80, 16, torch.bfloat16),   # several tiles per CTA
+    (32, 4, 128, 48, 70, 16, torch.bfloat16),  # the same with two passes
     (8, 2, 128, 5, 48, 16, torch.float32),
     (16, 2, 64, 3, 9, 9, torch.float32),       # 72 pairs, odd S
 ])
