@@ -1,16 +1,17 @@
 // BlockRank attention forward for fp32 models on CUDA cores (tensor cores would drop to tf32).
 //
-// A CTA of 128 threads owns 64 query rows (64 / G consecutive tokens x the G heads of a KV head) of one block and walks
+// A CTA of 256 threads owns 64 query rows (64 / G consecutive tokens x the G heads of a KV head) of one block and walks
 // through the list of keys those rows see -- the prefix block (documents) or every earlier slot (query block), then the
-// own keys -- 64 at a time.  Both products are register-tiled: thread (ty, tx) keeps rows ty + 8 i of the scores (8 x 4,
-// packed two head_dim elements per fma.rn.f32x2) and of the output (8 x D / 16).  The kernel is bound by the FMA pipe:
-// an inner step of 128 FMAs reads 12 16-byte pieces of shared memory, 16 wavefronts per warp.  Two CTAs share an SM
-// (101 KB each), so one computes while the other loads or exponentiates.
+// own keys -- 64 at a time.  Both products are register-tiled: thread (ty, tx) keeps rows ty + 16 i of the scores (4 x 4,
+// packed two head_dim elements per fma.rn.f32x2) and of the output (4 x D / 16).  The kernel is bound by the FMA pipe and
+// by the latency in front of it: an inner step of 64 FMAs reads 8 16-byte pieces of shared memory, 12 wavefronts per warp.
+// Two CTAs share an SM (101 KB each), so one computes while the other loads or exponentiates.  (Tiles of 8 x 4 need fewer
+// wavefronts per FMA but leave two warps per scheduler: 399 us where this takes 351.)
 //
 // The query block's context is cut into chunks of about 512 keys whose partial results attn_combine_kernel merges: its
 // rows see thousands of keys where a document's see a few hundred, and as single CTAs they were the tail of the launch.
 //
-// One prompt of 20 documents (32/8 heads, head_dim 128, 8.4 GFLOP visible): 405 us; one query row per four threads with
+// One prompt of 20 documents (32/8 heads, head_dim 128, 8.4 GFLOP visible): 351 us; one query row per four threads with
 // the keys re-read from shared memory for every row took 1,790 us.
 #include <algorithm>
 
@@ -23,7 +24,8 @@ namespace brk {
 
 namespace {
 
-constexpr int kThreads = 128;
+constexpr int kThreads = 256;
+constexpr int kRowStep = kThreads / 16, kR = 64 / kRowStep;  // a thread's rows: ty + kRowStep i, i < kR
 constexpr int kRows = 64;
 constexpr int kKeys = 64;
 constexpr int kChunkKeys = 512;  // context keys of one chunk of the query block, about
@@ -129,10 +131,10 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f32_kernel(F32Args a) {
                            (int64_t)(start + tok) * a.q.ss + d);
     store4(qs + r * kPitch + d, make_float4(x.x * a.scale_log2, x.y * a.scale_log2, x.z * a.scale_log2, x.w * a.scale_log2));
   }
-  float m_run[8], l_run[8];
-  ptx::f32x2 o[8][kE / 2];
+  float m_run[kR], l_run[kR];
+  ptx::f32x2 o[kR][kE / 2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < kR; ++i) {
     m_run[i] = -INFINITY;
     l_run[i] = 0.f;
 #pragma unroll
@@ -168,27 +170,27 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f32_kernel(F32Args a) {
     cp_async_wait<1>();
     __syncthreads();
     // scores: rows ty + 8 i, keys tx + 16 c
-    float s[8][4];
+    float s[kR][4];
     {
-      ptx::f32x2 acc[8][4];
+      ptx::f32x2 acc[kR][4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < kR; ++i)
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[i][c] = 0ull;
-#pragma unroll 2
+#pragma unroll 1
       for (int d = 0; d < D; d += 4) {
         ulonglong2 kk[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) kk[c] = *reinterpret_cast<const ulonglong2*>(ks + (tx + 16 * c) * kPitch + d);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(qs + (ty + 8 * i) * kPitch + d);
+        for (int i = 0; i < kR; ++i) {
+          const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(qs + (ty + kRowStep * i) * kPitch + d);
 #pragma unroll
           for (int c = 0; c < 4; ++c) acc[i][c] = ptx::fma2(qq.y, kk[c].y, ptx::fma2(qq.x, kk[c].x, acc[i][c]));
         }
       }
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < kR; ++i)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           float x, y;
@@ -201,12 +203,12 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f32_kernel(F32Args a) {
       const int key = tx + 16 * c, own = j0 + key - n_ctx;  // own > token: behind the diagonal
       const bool none = s_slot[key] < 0;
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (none || own > t0 + (ty + 8 * i) / G) s[i][c] = -INFINITY;
+      for (int i = 0; i < kR; ++i)
+        if (none || own > t0 + (ty + kRowStep * i) / G) s[i][c] = -INFINITY;
     }
     __syncthreads();  // every thread has read the keys: their place takes the probabilities
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < kR; ++i) {
       float mx = fmaxf(fmaxf(s[i][0], s[i][1]), fmaxf(s[i][2], s[i][3]));
 #pragma unroll
       for (int off = 8; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
@@ -218,7 +220,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f32_kernel(F32Args a) {
       for (int c = 0; c < 4; ++c) {
         const float p = exp2f(s[i][c] - ref);
         sum += p;
-        ks[(ty + 8 * i) * kPitchP + tx + 16 * c] = p;
+        ks[(ty + kRowStep * i) * kPitchP + tx + 16 * c] = p;
       }
       l_run[i] = l_run[i] * corr + sum;  // (this thread's keys only: added up over the row at the end)
       const ptx::f32x2 c2 = ptx::pack2(corr, corr);
@@ -230,16 +232,16 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f32_kernel(F32Args a) {
     const int n4 = (min(kKeys, j_hi - j0) + 3) >> 2;
 #pragma unroll 1
     for (int k4 = 0; k4 < n4; ++k4) {
-      float4 p[8];
+      float4 p[kR];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) p[i] = load4(ks + (ty + 8 * i) * kPitchP + k4 * 4);
+      for (int i = 0; i < kR; ++i) p[i] = load4(ks + (ty + kRowStep * i) * kPitchP + k4 * 4);
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
         ulonglong2 v[kE / 4];
 #pragma unroll
         for (int e = 0; e < kE / 4; ++e) v[e] = *reinterpret_cast<const ulonglong2*>(vs + (k4 * 4 + kk) * D + tx * 4 + e * 64);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < kR; ++i) {
           const float x = kk == 0 ? p[i].x : kk == 1 ? p[i].y : kk == 2 ? p[i].z : p[i].w;
           const ptx::f32x2 p2 = ptx::pack2(x, x);
 #pragma unroll
@@ -252,11 +254,11 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f32_kernel(F32Args a) {
     }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
+  for (int i = 0; i < kR; ++i) {
     float l = l_run[i];
 #pragma unroll
     for (int off = 8; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
-    const int r = ty + 8 * i, tok = t0 + r / G, n = g * G + r % G;
+    const int r = ty + kRowStep * i, tok = t0 + r / G, n = g * G + r % G;
     if (tok >= len) continue;
     const bool part = query && a.n_chunk > 1;
     const float inv = part ? 1.f : l > 0.f ? 1.f / l : 0.f;
