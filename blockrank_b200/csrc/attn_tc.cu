@@ -1321,11 +1321,14 @@ int attn_prologue_launch(const brk_attn_params& p, int* hdr, float2* ml, int64_t
 
 // Key chunks for the query block.  Its context is every earlier token of the prompt (S is the only
 // bound known on the host), walked 128 keys per step per row tile, 2.3 us each; cutting it into chunks of about
-// 1024 keys keeps that serial chain short and spreads it over the SMs.  A small call is cut further, down to 256 keys,
+// 1024 keys keeps that serial chain short and spreads it over the SMs.  Once there is a chunk for every SM, longer ones
+// are as good, because they are handed out first, and leave fewer partials to write and merge (4 prompts of 100 documents:
+// 5 chunks of each where 1024 keys make 16).  A small call is cut further, down to 256 keys,
 // while its chunks find idle SMs: below 640 slots the chain is shorter than the merge.
 static int tc_splits(const brk_attn_params& p) {
   if (p.M < 2) return 1;
-  int n = std::max(1, std::min(32, (p.S + 1023) / 1024));
+  const int bg = std::max(1, p.B * p.Nk);
+  int n = std::max(1, std::min({32, (p.S + 1023) / 1024, (sm_count() + bg - 1) / bg}));
   if (p.S > 640) {
     const int tok2 = 2 * BM / std::max(1, p.N / p.Nk);
     const int64_t pairs = (int64_t)p.B * p.Nk * ((query_rows(p) + tok2 - 1) / tok2);
