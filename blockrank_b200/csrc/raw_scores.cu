@@ -13,8 +13,8 @@
 //
 // All four are bound by memory: per prompt of 100 documents (32/8 heads, 16 rows, 16,320 slots) the forward moves
 // 33 MB of keys and writes 17 MB of logits, the backward reads those and updates 33 MB of dk, for 2 and 4 GFLOP.
-// Measured there: forward 21.6 us (one thread per key row on CUDA cores: 230 us); 4 prompts of 20 documents (14,080
-// slots): forward 19 us (195), backward 29 us (fp32 matrix products, casts, fills and sums in PyTorch: about 500);
+// Measured there: forward 18.6 us (one thread per key row on CUDA cores: 230 us); 4 prompts of 20 documents (14,080
+// slots): forward 17 us (195), backward 29 us (fp32 matrix products, casts, fills and sums in PyTorch: about 500);
 // fp32 forward, 1 prompt of 20 documents: 21 us (81).
 #include <algorithm>
 
@@ -54,12 +54,20 @@ __device__ __forceinline__ bool pair_ok(int qb, int qslot, int kblk, int s, int 
 // eight different bank groups.
 __device__ __forceinline__ int swz(int row, int piece) { return piece ^ ((((row >> 3) & 3) << 1 | (row & 1)) & 7); }
 
+// Bound by instruction issue (64 x 64 logits per tile, each with its visibility).  Nearly every tile lies in front of the
+// query block that holds all R rows: there a key is visible if it exists, so a thread's eight keys take eight bits of a
+// ballot, and where the prompt has no padding nothing is looked up at all.  (With every pair tested on its own a prompt of 100
+// documents took 22 us, 1,150 instructions per warp and tile; now 18.6.)
 template <int D>
-__global__ void __launch_bounds__(kThreads) raw_scores_mma_kernel(ScoreArgs a, __nv_bfloat16* __restrict__ out, float neg) {
+constexpr int kRawPerSm = D == 128 ? 4 : 5;  // CTAs per SM
+template <int D>
+__global__ void __launch_bounds__(kThreads, kRawPerSm<D>) raw_scores_mma_kernel(ScoreArgs a, __nv_bfloat16* __restrict__ out, float neg) {
   constexpr int kPieces = D / 8;
   __shared__ __align__(16) __nv_bfloat16 ktile[2][kKeys][D];
   __shared__ int s_kblk[2][kKeys];
   __shared__ int s_qblk[64];
+  __shared__ unsigned s_bits[2][kKeys / 32];  // which keys of the tile exist
+  __shared__ int s_sum[kThreads / 32];
   extern __shared__ int32_t s_spans[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, tq = lane & 3;
   const int G = a.N / a.Nk, GR = G * a.R;
@@ -67,27 +75,51 @@ __global__ void __launch_bounds__(kThreads) raw_scores_mma_kernel(ScoreArgs a, _
   const int32_t* bs = a.blk_start + (size_t)b * a.M;
   const int32_t* bl = a.blk_len + (size_t)b * a.M;
   ptx::grid_dependency_wait();  // (launched beside the end of the attention call's last kernel: 156.6 -> 154.2 us for both)
-  if (a.M <= kMaxSharedSpans) {
-    for (int i = tid; i < a.M; i += kThreads) {
-      s_spans[i] = bs[i];
-      s_spans[a.M + i] = bl[i];
+  int sum = 0;  // keys in front of the last block
+  for (int i = tid; i < a.M; i += kThreads) {
+    const int start = bs[i], len = bl[i];
+    if (i < a.M - 1) sum += len;
+    if (a.M <= kMaxSharedSpans) {
+      s_spans[i] = start;
+      s_spans[a.M + i] = len;
     }
-    __syncthreads();
+  }
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if (lane == 0) s_sum[warp] = sum;
+  __syncthreads();
+  if (a.M <= kMaxSharedSpans) {
     bs = s_spans;
     bl = s_spans + a.M;
   }
+  const int first = bs[0], own = bs[a.M - 1];
+  const bool all_query = a.S - a.R >= own && a.S <= own + bl[a.M - 1];  // all R rows belong to the last block
+  const bool no_gaps = s_sum[0] + s_sum[1] + s_sum[2] + s_sum[3] == own - first;
+  auto in_front = [&](int tile) { return all_query && (tile + 1) * kKeys <= own; };           // visible: every key that exists
+  auto solid = [&](int tile) { return no_gaps && in_front(tile) && tile * kKeys >= first; };  // every key exists
   if (tid < a.R) s_qblk[tid] = block_of(bs, bl, a.M, a.S - a.R + tid);
   const int n_tiles = (a.S + kKeys - 1) / kKeys;
   const __nv_bfloat16* kb = reinterpret_cast<const __nv_bfloat16*>(a.k.ptr) + (int64_t)b * a.k.sb + (int64_t)g * a.k.sh;
+  const int row0 = tid / kPieces, pc = tid % kPieces;
+  constexpr int kRowStep = kThreads / kPieces;
+  const int64_t step = kRowStep * a.k.ss;
   auto request = [&](int tile, int buf) {
+    const __nv_bfloat16* src = kb + (int64_t)(tile * kKeys + row0) * a.k.ss + pc * 8;
+    if ((tile + 1) * kKeys <= a.S) {
 #pragma unroll
-    for (int i = tid; i < kKeys * kPieces; i += kThreads) {
-      const int row = i / kPieces, pc = i % kPieces, s = tile * kKeys + row;
-      cp_async16_zfill(&ktile[buf][row][swz(row, pc) * 8], kb + (int64_t)min(s, a.S - 1) * a.k.ss + pc * 8, s < a.S);
+      for (int j = 0; j < kKeys / kRowStep; ++j, src += step)
+        cp_async16(&ktile[buf][row0 + j * kRowStep][swz(row0 + j * kRowStep, pc) * 8], src);
+    } else {
+#pragma unroll 1
+      for (int row = row0; row < kKeys; row += kRowStep, src += step) {
+        const bool ok = tile * kKeys + row < a.S;
+        cp_async16_zfill(&ktile[buf][row][swz(row, pc) * 8], ok ? src : kb, ok);
+      }
     }
-    if (tid < kKeys) {
-      const int s = tile * kKeys + tid;
-      s_kblk[buf][tid] = s < a.S ? block_of(bs, bl, a.M, s) : -1;
+    if (tid < kKeys && !solid(tile)) {
+      const int s = tile * kKeys + tid, kblk = s < a.S ? block_of(bs, bl, a.M, s) : -1;
+      s_kblk[buf][tid] = kblk;
+      const unsigned bits = __ballot_sync(0xffffffffu, kblk >= 0);
+      if (lane == 0) s_bits[buf][warp] = bits;
     }
   };
   for (int r0 = 0; r0 < GR; r0 += kRowsPass) {
@@ -148,15 +180,23 @@ __global__ void __launch_bounds__(kThreads) raw_scores_mma_kernel(ScoreArgs a, _
         }
         const int s0 = tile * kKeys + c0 + 8 * tq;
         if (s0 >= a.S) continue;
-        int kblk[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) kblk[i] = s_kblk[buf][c0 + 8 * tq + i];
+        const bool front = in_front(tile);
+        const unsigned exist = solid(tile) ? 0xffu : (s_bits[buf][c0 >> 5] >> (8 * tq)) & 0xffu;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           if (rows[h] >= GR) continue;
           float v[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = pair_ok(qb[h], qslot[h], kblk[i], s0 + i, a.M) ? c[i >> 1][2 * h + (i & 1)] : neg;
+          for (int i = 0; i < 8; ++i) v[i] = c[i >> 1][2 * h + (i & 1)];
+          if (!front) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              if (!pair_ok(qb[h], qslot[h], s_kblk[buf][c0 + 8 * tq + i], s0 + i, a.M)) v[i] = neg;
+          } else if (exist != 0xffu) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              if (!((exist >> i) & 1u)) v[i] = neg;
+          }
           __nv_bfloat16* o = out + orow[h] + s0;
           if ((a.S & 7) == 0) {
             store8(o, v);
@@ -481,7 +521,7 @@ int raw_scores_launch(const brk_score_params& p, void* out, cudaStream_t st) {
   // 0.7 * lowest finite value of the dtype, computed the way the reference does (python float -> dtype)
   if (p.dtype == BRK_BF16) {
     const float neg = 0.7f * -3.3895313892515355e38f;
-    const dim3 grid(tiles_grid(p.S, p.B * p.Nk, p.D == 128 ? 4 : 6), p.B * p.Nk);
+    const dim3 grid(tiles_grid(p.S, p.B * p.Nk, p.D == 128 ? kRawPerSm<128> : kRawPerSm<64>), p.B * p.Nk);
     const size_t sm = p.M <= kMaxSharedSpans ? (size_t)p.M * 8 : 0;
     return p.D == 128 ? launch_dependent(raw_scores_mma_kernel<128>, grid, dim3(kThreads), sm, st, a, (__nv_bfloat16*)out, neg)
                       : launch_dependent(raw_scores_mma_kernel<64>, grid, dim3(kThreads), sm, st, a, (__nv_bfloat16*)out, neg);

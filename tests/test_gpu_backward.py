@@ -238,3 +238,26 @@ def test_raw_scores_and_gradient(N, Nk, D, M, H, R, dtype):
         for got, r, base in ((dq, rq, dq0), (dk, rk, dk0)):
             r = r + base.double().cpu() if given else r
             assert (got.double().cpu() - r).norm() <= tol * r.norm()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("lens,H,R", [
+    ([[48] * 9, [48] * 9], 48, 16),                 # no padding, the query block starts on a tile edge (384)
+    ([[50] * 9, [50, 0, 50, 50, 50, 50, 50, 50, 50]], 50, 16),  # ... inside a tile; a prompt with an empty block
+    ([[3] + [40] * 8, [1] * 9], 40, 16),            # padding in front only; a key here and there
+    ([[33, 20, 40, 40, 5], [40, 40, 40, 40, 40]], 40, 40),  # R reaches into the query block's padding
+])
+def test_raw_scores_visibility_by_tile(lens, H, R, D):
+    """Tiles in front of the query block, with and without padding, and tiles that it starts in."""
+    from blockrank_b200 import ops
+    g = torch.Generator().manual_seed(D + H)
+    B, N, Nk, S, scale = 2, 8, 2, len(lens[0]) * H, D ** -0.5
+    mask = _mask(lens, H)
+    rb = lambda *s: torch.randn(*s, generator=g).bfloat16().cuda()
+    q, k = rb(B, N, S, D), rb(B, Nk, S, D)
+    raw = ops.raw_scores(q, k, *ops.spans_from_mask(mask.cuda()), scale, R).double().cpu()
+    kx = k.double().cpu().repeat_interleave(N // Nk, 1)
+    ref = (q[:, :, S - R:] * scale).double().cpu() @ kx.transpose(-1, -2)
+    ok = orc.allowed_pairs(mask)[:, None, S - R:].expand(B, N, R, S)
+    assert (raw[~ok] < -1e37).all()
+    assert (raw - ref)[ok].norm() <= 1e-2 * ref[ok].norm()
