@@ -164,7 +164,8 @@ std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Ten
   Tensor ws = scratch(nbytes, q);
   check(brk_attn_fwd(&p, ws.data_ptr(), nbytes, stream_of(q)), "brk_attn_fwd");
   // span check / reset kernel + main kernel [+ merge of the key-chunked query block on the tensor-core path]
-  count(nbytes > 256 ? 3 : 2);
+  // (partials of key chunks come on top of the header and the 16 bytes per 64 slots of the list of windows)
+  count(nbytes > 512 + (size_t)(B * (S / 64 + 2)) * 16 ? 3 : 2);
   return {out, lse};
 }
 
