@@ -57,9 +57,9 @@ __global__ void __launch_bounds__(128) attn_combine_kernel(CombineArgs a) {
     for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     const float ref = (mx == -INFINITY) ? 0.f : mx;
     const float wgt = ml.y > 0.f ? exp2f(ml.x - ref) : 0.f;  // chunks that saw no key carry no output
-    float l = ml.y * wgt;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+    float l = 0.f;  // (in the order of the chunks, as the rows below: the result does not depend on how the lanes are dealt)
+    for (int c = 0; c < a.n_split; ++c)
+      l = fmaf(__shfl_sync(0xffffffffu, ml.y, c), __shfl_sync(0xffffffffu, wgt, c), l);
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int c0 = 0; c0 < a.n_split; c0 += U * kSplit) {
       if (c0 > 0) fetch(c0);
