@@ -38,6 +38,14 @@
 // by more than 2^8).  P (bf16, two keys per 32-bit column) overwrites the first half of the S
 // tile it was computed from.
 //
+// Two forms of P (kFine).  Rounded to bf16 it is what head_dim 128 with four heads per KV head has always had here, and the
+// reference too.  Every other shape that BRK_ALGO_AUTO brings here has the CUDA-core kernel as its other route, which keeps P
+// in fp32; there P goes in as two bf16 parts, P = hi + lo, one product each, and fills the whole S tile ([hi | lo] per 64-key
+// slot): what is dropped is below 2^-17 of a probability.  Error of the output against 64 bits (2 heads per KV head, head_dim
+// 64, 20 documents of 120..160 tokens): 1.6462e-3 like the CUDA-core kernel, which is the rounding of the output alone; P in
+// bf16 2.17e-3.  4 prompts of 20 such documents: 8 heads on 8 58.8 us (P in bf16 53.9, CUDA cores 1,023), 8 heads on one
+// 52.6 us (44.0, 901).
+//
 // Shared memory 227 KB: Q 2x32 KB, K pool 80 KB, V pool 80 KB, barriers, job records, row statistics.
 // No cluster multicast anywhere.  Every mbarrier wait is bounded; on expiry the thread records
 // a code in the caller's status word, stops waiting and runs to the normal exit.
@@ -398,7 +406,13 @@ __device__ __forceinline__ Pair decode_pair(const TcArgs& a, int b, int g, int m
 // (tiles are dealt 0,1,1,0,0,1,1,0,...)
 __device__ __forceinline__ int deal_chain(int i) { return ((i & 3) == 0 || (i & 3) == 3) ? 0 : 1; }
 
-template <int HD>
+// bf16 pair of what bf16 rounding took off x and y; `hi` is their rounded pair (x in the low half)
+__device__ __forceinline__ uint32_t low_part(uint32_t hi, float x, float y) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(x - __uint_as_float(hi << 16), y - __uint_as_float(hi & 0xffff0000u));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+template <int HD, bool kFine>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                const __grid_constant__ CUtensorMap tmV, const TcArgs a) {
@@ -769,16 +783,19 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         if (last) ptx::mma_commit(bar(kQFree + x));  // last read of this chain's Q tile
       }
     };
-    // O (+)= P V over `keys` keys starting at pool slot `slot`; P sits over the first 64 columns of S
+    // O (+)= P V over `keys` keys starting at pool slot `slot`; P sits over the first 64 columns of S (kFine: over all 128)
     auto issue_pv = [&](int slot, int keys, bool first, bool last) {
       const uint32_t b_lo = (uint32_t)v_desc0 + (uint32_t)slot * (kSlotHalf >> 4), b_hi = (uint32_t)(v_desc0 >> 32);
       const int ksteps = (keys + 15) >> 4;
       if (ptx::elect_one()) {
 #pragma unroll 1
         for (int ks = 0; ks < BT / 16; ++ks)
-          if (ks < ksteps)
-            ptx::mma_ts_lohi(tm_o, tm_s + (uint32_t)ks * 8, b_lo + (uint32_t)ks * ((16 * 128) >> 4), b_hi, idesc_pv,
-                             (!first || ks > 0) ? 1u : 0u);
+          if (ks < ksteps) {
+            const uint32_t b_ks = b_lo + (uint32_t)ks * ((16 * 128) >> 4);
+            const uint32_t a_ks = tm_s + (kFine ? (uint32_t)(ks >> 2) * 64 + (uint32_t)(ks & 3) * 8 : (uint32_t)ks * 8);
+            ptx::mma_ts_lohi(tm_o, a_ks, b_ks, b_hi, idesc_pv, (!first || ks > 0) ? 1u : 0u);
+            if (kFine) ptx::mma_ts_lohi(tm_o, a_ks + 32, b_ks, b_hi, idesc_pv, 1u);
+          }
         ptx::mma_commit(bar(kPVDone + x));
         if (last) ptx::mma_commit(bar(kOFull + x));
       }
@@ -963,7 +980,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         __syncwarp();
         // One pass per 64-key slot: logits -> registers, mask, row maximum, running-max update,
         // p = 2^(s*scale - m) from the same registers, P (bf16) -> columns [32h, 32h+32) of the
-        // tile, which only covers logits that have already been consumed.
+        // tile (kFine: [64h, 64h+64)), which only covers logits that have already been consumed.
 #pragma unroll 1
         for (int h = 0; h < cnt; ++h) {
           int nk, own_off; bool own;
@@ -1025,7 +1042,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             // p with packed fp32x2 arithmetic; see kPolyOf8 for where the exponentials are evaluated
             const ptx::f32x2 sc2 = ptx::pack2(a.scale_log2, a.scale_log2), nr2 = ptx::pack2(neg_ref, neg_ref);
             ptx::f32x2 ps2[2] = {0ull, 0ull};
-            uint32_t pk[32];
+            uint32_t pk[32], pl[kFine ? 32 : 1];
 #pragma unroll
             {
               {
@@ -1056,10 +1073,15 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                   __nv_bfloat162 h0 = __floats2bfloat162_rn(p0, p1), h1 = __floats2bfloat162_rn(p2, p3);
                   pk[c >> 1] = *reinterpret_cast<uint32_t*>(&h0);
                   pk[(c >> 1) + 1] = *reinterpret_cast<uint32_t*>(&h1);
+                  if constexpr (kFine) {
+                    pl[c >> 1] = low_part(pk[c >> 1], p0, p1);
+                    pl[(c >> 1) + 1] = low_part(pk[(c >> 1) + 1], p2, p3);
+                  }
                 }
               }
             }
-            ptx::tmem_st32(tmem_lane + (uint32_t)h * 32, pk);
+            ptx::tmem_st32(tmem_lane + (uint32_t)h * (kFine ? 64 : 32), pk);
+            if constexpr (kFine) ptx::tmem_st32(tmem_lane + (uint32_t)h * 64 + 32, pl);
             if ((t > 0 || h > 0) && __any_sync(0xffffffffu, changed)) {
               // The reference moved by more than the lazy threshold (rare): bring what was accumulated
               // against the old one in line -- O of the earlier tiles, P of this tile's first slot.  (Behind the
@@ -1076,7 +1098,23 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                   ptx::tmem_st32(tmem_lane + kColO + (uint32_t)ch * 32, orow);
                 }
               }
-              if (h > 0) {
+              if (kFine && h > 0) {
+                uint32_t ph[32], pm[32];
+                ptx::tmem_ld32(tmem_lane, ph);
+                ptx::tmem_ld32(tmem_lane + 32, pm);
+                ptx::tmem_wait_ld(ph);
+                ptx::tmem_wait_ld(pm);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                  const float u = (__uint_as_float(ph[i] << 16) + __uint_as_float(pm[i] << 16)) * corr;
+                  const float v = (__uint_as_float(ph[i] & 0xffff0000u) + __uint_as_float(pm[i] & 0xffff0000u)) * corr;
+                  const __nv_bfloat162 w = __floats2bfloat162_rn(u, v);
+                  ph[i] = *reinterpret_cast<const uint32_t*>(&w);
+                  pm[i] = low_part(ph[i], u, v);
+                }
+                ptx::tmem_st32(tmem_lane, ph);
+                ptx::tmem_st32(tmem_lane + 32, pm);
+              } else if (h > 0) {
                 uint32_t p0[32];
                 ptx::tmem_ld32(tmem_lane, p0);
                 ptx::tmem_wait_ld(p0);
@@ -1349,7 +1387,7 @@ size_t attn_tc_workspace(const brk_attn_params& p) {
   return kWsHeader + window_bytes(p) + rows * (p.D * sizeof(float) + sizeof(float2));
 }
 
-template <int HD>
+template <int HD, bool kFine>
 static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStream_t st) {
   const int G = p.N / p.Nk;
   BRK_REQUIRE(G == 1 || G == 2 || G == 4 || G == 8, BRK_E_UNSUPPORTED, "tcgen05 attention needs N/Nk in {1,2,4,8}, got %d", G);
@@ -1375,7 +1413,7 @@ static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cuda
   BRK_CUDA(cudaGetDevice(&dev));
   BRK_REQUIRE(dev >= 0 && dev < 64, BRK_E_UNSUPPORTED, "device ordinal %d out of range", dev);
   if (!configured[dev]) {
-    BRK_CUDA(cudaFuncSetAttribute(attn_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    BRK_CUDA(cudaFuncSetAttribute(attn_tc_kernel<HD, kFine>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)Geo<HD>::kSmemBytes));
     sms[dev] = sm_count();
     BRK_REQUIRE(sms[dev] > 0, BRK_E_CUDA, "could not read the SM count");
@@ -1438,7 +1476,7 @@ static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cuda
       return rc;
   }
   const int grid = (int)(total_items < sms[dev] ? total_items : sms[dev]);
-  if ((rc = launch_dependent(attn_tc_kernel<HD>, dim3(grid), dim3(kThreads), Geo<HD>::kSmemBytes, st, tq, tk, tv, a))) return rc;
+  if ((rc = launch_dependent(attn_tc_kernel<HD, kFine>, dim3(grid), dim3(kThreads), Geo<HD>::kSmemBytes, st, tq, tk, tv, a))) return rc;
   if (ns > 1) {
     const CombineArgs c{a.o, a.lse, a.blk_start, a.blk_len, a.hdr, p.B, p.N, p.S, p.M, lq, ns, a.part_o, a.part_ml};
     return attn_combine_launch<__nv_bfloat16, HD>(c, st);
@@ -1449,7 +1487,10 @@ static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cuda
 int attn_tc_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStream_t st) {
   BRK_REQUIRE(p.dtype == BRK_BF16 && (p.D == 64 || p.D == 128), BRK_E_UNSUPPORTED,
               "tcgen05 attention needs bf16 and head_dim 64 or 128 (dtype %d, head_dim %d)", p.dtype, p.D);
-  return p.D == 128 ? attn_tc_run<128>(p, ws, ws_bytes, st) : attn_tc_run<64>(p, ws, ws_bytes, st);
+  // AUTO keeps the precision of the kernel it would choose otherwise; asked for by name, this kernel rounds P to bf16.
+  const bool fine = p.algo == BRK_ALGO_AUTO && !(p.D == 128 && p.Nk > 0 && p.N / p.Nk == 4);
+  if (p.D == 128) return fine ? attn_tc_run<128, true>(p, ws, ws_bytes, st) : attn_tc_run<128, false>(p, ws, ws_bytes, st);
+  return fine ? attn_tc_run<64, true>(p, ws, ws_bytes, st) : attn_tc_run<64, false>(p, ws, ws_bytes, st);
 }
 
 }  // namespace brk

@@ -56,9 +56,10 @@ enum { BRK_BF16 = 0, BRK_F32 = 1 };
 
 /* attention algorithm selector */
 enum {
-  BRK_ALGO_AUTO = 0,  /* tcgen05 kernel for bf16, otherwise SIMT */
+  BRK_ALGO_AUTO = 0,  /* tcgen05 kernel for bf16, otherwise SIMT; probabilities are rounded to bf16 at head_dim 128 with
+                         four heads per KV head and nowhere else */
   BRK_ALGO_SIMT = 1,  /* CUDA-core fp32-accumulate kernel: bf16 and fp32, head_dim 64 or 128 */
-  BRK_ALGO_TC = 2     /* tcgen05 + TMEM + TMA kernel: bf16, head_dim 64 or 128 */
+  BRK_ALGO_TC = 2     /* tcgen05 + TMEM + TMA kernel: bf16, head_dim 64 or 128, probabilities rounded to bf16 */
 };
 
 /* A (B, heads, S, D) tensor view; strides in elements, innermost stride 1. */

@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from oracle import blockrank_oracle as orc
 from tests import helpers as H_
 
 pytestmark = pytest.mark.gpu
@@ -29,3 +30,23 @@ def test_forward_of_a_prompt_does_not_depend_on_its_batch():
     alone = ops.attention(q[:1], k[:1], v[:1], spans[0][:1], spans[1][:1], 128 ** -0.5, spans.max_block_len,
                           max_query_len=spans.max_query_len)
     assert torch.equal(batch[:1], alone)
+
+
+@pytest.mark.parametrize("q_scale", [1, 32], ids=["", "rescaled"])  # 32: the running maximum jumps, also inside a 128-key tile
+@pytest.mark.parametrize("N,Nk,D,M,H", [
+    (16, 8, 64, 7, 160), (8, 1, 64, 5, 96), (4, 4, 64, 3, 130), (8, 2, 64, 1, 200),   # every group size, one block
+    (4, 2, 64, 30, 96), (4, 2, 64, 3, 700),          # key chunks of the query block; blocks too long to stay resident
+    (16, 8, 128, 7, 160), (8, 1, 128, 12, 64), (2, 2, 128, 2, 300)])
+def test_default_bf16_forward_rounds_the_output_only(N, Nk, D, M, H, q_scale):
+    """Off head_dim 128 with four heads per KV head, probabilities are not rounded to bf16: the error against 64 bits is that
+    of the rounded output (1 % for the sums in 32 bits; with P in bf16 it is 28 % more)."""
+    lens = H_.random_lens(2, M, H, 7 * M + D)
+    mask = H_.ragged_mask(2, M, H, lens)
+    q, k, v = H_.qkv(2, N, Nk, M * H, D, M, torch.bfloat16)
+    q = (q.float() * q_scale).bfloat16()
+    ref, _ = orc.attention_dense(q, k, v, mask, D ** -0.5)
+    start, ln = ops.spans_from_mask(mask.cuda())
+    out = ops.attention(*(H_.to_cuda_view(x) for x in (q, k, v)), start, ln, D ** -0.5, H)
+    rows = mask.reshape(2, -1)
+    ref = ref[rows]
+    assert (out.cpu()[rows].double() - ref).norm() <= 1.01 * (ref.bfloat16().double() - ref).norm()
