@@ -1359,18 +1359,22 @@ int attn_prologue_launch(const brk_attn_params& p, int* hdr, float2* ml, int64_t
 
 // Key chunks for the query block.  Its context is every earlier token of the prompt (S is the only
 // bound known on the host), walked 128 keys per step per row tile, 2.3 us each; cutting it into chunks of about
-// 1024 keys keeps that serial chain short and spreads it over the SMs.  A call whose chunks of 1024 keys leave more than half
-// of the SMs idle is cut further, down to 256 keys, while the chunks find idle SMs: below 640 slots the chain is shorter than
-// the merge.  The rule decides the order in which a row's keys are summed, so it does not chase the last chunk: batches cut
-// into one chunk per SM instead (4 prompts of 100 documents: 5 of each, not 16) differ in the last bit of a few outputs, which
-// 20 layers of the 7B ranker turn into 2.4e-3 of its logits, for 467 us where this takes 478.
+// 1024 keys keeps that serial chain short and spreads it over the SMs.  A call whose chunks of 1024 keys leave more than a
+// third of the SMs idle, with other blocks for no more than one and a half rounds of them, is cut further, down to 256 keys,
+// while the chunks find idle SMs (one prompt of 8 documents of 100 tokens 31.1 -> 20.6 us, of 20 documents of 160 tokens 51.7 ->
+// 41.3, 2 prompts of 8 documents of 500 tokens 182 -> 119; with more blocks the finer chunks cost: 2 prompts of 20 documents
+// 68.8 -> 75.8, one of 50 74.1 -> 78.7); below 640 slots the chain is shorter than the merge.
+// The rule decides the order in which a row's keys are summed, so it does not chase the last chunk: batches cut into one chunk
+// per SM instead (4 prompts of 100 documents: 5 of each, not 16) differ in the last bit of a few outputs, which 20 layers of
+// the 7B ranker turn into 2.4e-3 of its logits, for 467 us where this takes 478.
 static int tc_splits(const brk_attn_params& p) {
   if (p.M < 2) return 1;
   int n = std::max(1, std::min(32, (p.S + 1023) / 1024));
   if (p.S > 640) {
     const int tok2 = 2 * BM / std::max(1, p.N / p.Nk);
     const int64_t pairs = (int64_t)p.B * p.Nk * ((query_rows(p) + tok2 - 1) / tok2);
-    if (2 * pairs * n <= sm_count())
+    const int64_t blocks = (int64_t)p.B * p.Nk * (p.M - 1);
+    if (3 * pairs * n <= 2 * sm_count() && 2 * blocks <= 3 * sm_count())
       n = std::max(n, (int)std::min<int64_t>(std::min(32, (p.S + 255) / 256), sm_count() / std::max<int64_t>(1, pairs)));
   }
   return n;
