@@ -50,3 +50,18 @@ def test_default_bf16_forward_rounds_the_output_only(N, Nk, D, M, H, q_scale):
     rows = mask.reshape(2, -1)
     ref = ref[rows]
     assert (out.cpu()[rows].double() - ref).norm() <= 1.01 * (ref.bfloat16().double() - ref).norm()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("N,Nk,R", [(8, 2, 16), (5, 1, 13), (8, 1, 16), (16, 4, 64), (4, 1, 64)])  # 64, 65, 128, 256 pairs
+def test_raw_score_gradient_rounds_dk_once(N, Nk, R, D):
+    """dk of more (head, row) pairs than a pass holds is summed in fp32 over the passes: its error against 64 bits is that of
+    one rounding to bf16 (1.66e-3; 2.4e-3 and 3.1e-3 with a rounding after each of two and four passes)."""
+    g = torch.Generator().manual_seed(N + R)
+    B, S, scale = 2, 5 * 130, D ** -0.5
+    rb = lambda *s: torch.randn(*s, generator=g).bfloat16()
+    q, k, d_raw = rb(B, N, S, D), rb(B, Nk, S, D), rb(B, N, R, S)
+    start, ln = ops.spans_from_mask(torch.ones(B, 5, 130, dtype=torch.bool).cuda())
+    _, dk = ops.raw_scores_bwd(q.cuda(), k.cuda(), d_raw.cuda(), start, ln, scale)
+    rk = ((d_raw.double() * scale).transpose(-1, -2) @ q[:, :, S - R:].double()).view(B, Nk, N // Nk, S, D).sum(2)
+    assert (dk.cpu().double() - rk).norm() <= 1.01 * (rk.bfloat16().double() - rk).norm()
