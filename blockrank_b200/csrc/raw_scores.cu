@@ -61,7 +61,8 @@ __device__ __forceinline__ int swz(int row, int piece) { return piece ^ ((((row 
 template <int D>
 constexpr int kRawPerSm = D == 128 ? 4 : 5;  // CTAs per SM
 template <int D>
-__global__ void __launch_bounds__(kThreads, kRawPerSm<D>) raw_scores_mma_kernel(ScoreArgs a, __nv_bfloat16* __restrict__ out, float neg) {
+__global__ void __launch_bounds__(kThreads, kRawPerSm<D>) raw_scores_mma_kernel(ScoreArgs a, __nv_bfloat16* __restrict__ out, float neg,
+                                                                              int wide) {
   constexpr int kPieces = D / 8;
   __shared__ __align__(16) __nv_bfloat16 ktile[2][kKeys][D];
   __shared__ int s_kblk[2][kKeys];
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, kRawPerSm<D>) raw_scores_mma_kernel(
               if (!((exist >> i) & 1u)) v[i] = neg;
           }
           __nv_bfloat16* o = out + orow[h] + s0;
-          if ((a.S & 7) == 0) {
+          if (wide) {
             store8(o, v);
           } else {
 #pragma unroll
@@ -545,8 +546,9 @@ int raw_scores_launch(const brk_score_params& p, void* out, cudaStream_t st) {
     const float neg = 0.7f * -3.3895313892515355e38f;
     const dim3 grid(tiles_grid(p.S, p.B * p.Nk, p.D == 128 ? kRawPerSm<128> : kRawPerSm<64>), p.B * p.Nk);
     const size_t sm = p.M <= kMaxSharedSpans ? (size_t)p.M * 8 : 0;
-    return p.D == 128 ? launch_dependent(raw_scores_mma_kernel<128>, grid, dim3(kThreads), sm, st, a, (__nv_bfloat16*)out, neg)
-                      : launch_dependent(raw_scores_mma_kernel<64>, grid, dim3(kThreads), sm, st, a, (__nv_bfloat16*)out, neg);
+    const int wide = ((uintptr_t)out & 15) == 0 && p.S % 8 == 0;  // eight logits per store; `out` may have any alignment
+    return p.D == 128 ? launch_dependent(raw_scores_mma_kernel<128>, grid, dim3(kThreads), sm, st, a, (__nv_bfloat16*)out, neg, wide)
+                      : launch_dependent(raw_scores_mma_kernel<64>, grid, dim3(kThreads), sm, st, a, (__nv_bfloat16*)out, neg, wide);
   } else {
     const float neg = (float)(0.7 * -3.4028234663852886e38);
     const dim3 grid((p.S + kKeys - 1) / kKeys, p.B * p.Nk);

@@ -65,3 +65,22 @@ def test_raw_score_gradient_rounds_dk_once(N, Nk, R, D):
     _, dk = ops.raw_scores_bwd(q.cuda(), k.cuda(), d_raw.cuda(), start, ln, scale)
     rk = ((d_raw.double() * scale).transpose(-1, -2) @ q[:, :, S - R:].double()).view(B, Nk, N // Nk, S, D).sum(2)
     assert (dk.cpu().double() - rk).norm() <= 1.01 * (rk.bfloat16().double() - rk).norm()
+
+
+@pytest.mark.parametrize("shift", [1, 4, 8])
+def test_raw_scores_into_a_buffer_of_any_alignment(shift):
+    """The C entry takes any `out` that is aligned for its elements, also where a row is whole 16-byte pieces."""
+    import ctypes as C
+    spans, q, k, _ = packed([[9, 30, 41, 24]], 4, 2, 128, torch.bfloat16, seed=3)
+    B, N, S, D, R = 1, 4, q.shape[2], 128, 16
+    assert S % 8 == 0
+    ref = ops.raw_scores(q, k, spans[0], spans[1], D ** -0.5, R)
+    start, ln = spans[0].contiguous(), spans[1].contiguous()
+    p = _lib.ScoreParams()
+    p.dtype, p.B, p.N, p.Nk, p.D, p.S, p.M, p.R, p.scale, p.temperature = _lib.BRK_BF16, B, N, 2, D, S, 4, R, D ** -0.5, 1.0
+    p.q, p.k, p.blk_start, p.blk_len = ops._view(q), ops._view(k), start.data_ptr(), ln.data_ptr()
+    buf = torch.full((ref.numel() + 16,), 7.0, dtype=torch.bfloat16, device="cuda")
+    rc = _lib.lib().brk_raw_scores(C.byref(p), buf.data_ptr() + 2 * shift, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0, _lib.lib().brk_last_error()
+    assert torch.equal(buf[shift:shift + ref.numel()], ref.flatten())
+    assert (buf[:shift] == 7).all() and (buf[shift + ref.numel():] == 7).all()
