@@ -417,7 +417,7 @@ struct NoAutograd {
 };
 
 
-// out (+)= x w^T for row-major x (T, K), w (n, K): cuBLAS through PyTorch's handle (its stream, workspace and math mode), the
+// out (+)= x w^T for row-major x (T, K), w (n, K) on the current device: cuBLAS through PyTorch's handle (its stream, workspace and math mode), the
 // same product as torch.mm / addmm without their host path.
 void gemm_nt(Tensor& out, const Tensor& x, const Tensor& w, bool add) {
   const int64_t T = x.size(0), K = x.size(1), n = w.size(0);
@@ -447,6 +447,7 @@ Tensor mm_nt(const Tensor& x, const Tensor& w) {
 Tensor layer_qkv(const Tensor& h, const Tensor& ln1, const Tensor& wqkv, const Tensor& pos, const Tensor& inv_freq, int64_t N,
                  int64_t Nk, int64_t D, double eps) {
   NoAutograd guard;
+  c10::cuda::CUDAGuard device(h.device());
   Tensor qkv = mm_nt(rmsnorm(h, ln1, eps, std::nullopt, std::nullopt), wqkv);
   const int64_t T = qkv.size(0), row = qkv.stride(0), at0 = qkv.storage_offset();
   rope_(qkv.as_strided({T, N, D}, {row, D, 1}, at0), qkv.as_strided({T, Nk, D}, {row, D, 1}, at0 + N * D), pos, inv_freq);
@@ -469,6 +470,7 @@ Tensor layer_attention(const Tensor& qkv, const Tensor& blk_start, const Tensor&
 void layer_rest(Tensor& h, const Tensor& attn, const Tensor& wo, const Tensor& ln2, const Tensor& wgu, const Tensor& wd,
                 double eps) {
   NoAutograd guard;
+  c10::cuda::CUDAGuard device(h.device());
   gemm_nt(h, attn.view({h.size(0), wo.size(1)}), wo, true);
   const Tensor x = rmsnorm(h, ln2, eps, std::nullopt, std::nullopt);
   gemm_nt(h, silu_mul(mm_nt(x, wgu), std::nullopt), wd, true);

@@ -84,3 +84,19 @@ def test_raw_scores_into_a_buffer_of_any_alignment(shift):
     assert rc == 0, _lib.lib().brk_last_error()
     assert torch.equal(buf[shift:shift + ref.numel()], ref.flatten())
     assert (buf[:shift] == 7).all() and (buf[shift + ref.numel():] == 7).all()
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs a device that is not the current one")
+def test_ranker_layers_run_on_their_own_device():
+    """decoder_layer, and the whole forward when launches are timed, on a device that is not the current one."""
+    from blockrank_b200 import packed_block_collate_fn
+    from blockrank_b200.runner import MistralPrefillRanker, RankerConfig
+    cfg = RankerConfig.tiny()
+    bl = [30, 40, 50, 20, 4]
+    items = [{"input_ids": torch.arange(3, 3 + sum(bl)), "block_lengths": bl}]
+    batch = packed_block_collate_fn(items)
+    ref = MistralPrefillRanker(cfg, "cuda:0").init_random(seed=1).rank_host(batch)[0]
+    other = MistralPrefillRanker(cfg, "cuda:1").init_random(seed=1)
+    other.events = {"attn": [], "score": []}
+    with torch.cuda.device(0):
+        assert torch.equal(other.rank_host(batch)[0], ref)
