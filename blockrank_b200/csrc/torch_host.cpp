@@ -6,6 +6,7 @@
 // same steps cost 40-60 us per attention call, more than its kernels take on a short prompt.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
+#include <ATen/cuda/tunable/Tunable.h>
 #include <ATen/ops/addmm_cuda_dispatch.h>
 #include <ATen/ops/mm_cuda_dispatch.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -417,24 +418,31 @@ struct NoAutograd {
 };
 
 
-// out (+)= x w^T for row-major x (T, K), w (n, K) on the current device: cuBLAS through PyTorch's handle (its stream, workspace and math mode), the
-// same product as torch.mm / addmm without their host path.
+// Are PyTorch's switches for bf16 products where they start out?  The call below knows none of them.
+bool default_products() {
+  auto& ctx = at::globalContext();
+  const auto blas = ctx.blasPreferredBackend();
+  return ctx.allowBF16ReductionCuBLAS() == at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK &&
+         (blas == at::BlasBackend::Default || blas == at::BlasBackend::Cublas) && !ctx.deterministicAlgorithms() &&
+         !at::cuda::tunable::getTuningContext()->IsTunableOpEnabled();
+}
+
+// out (+)= x w^T for row-major x (T, K), w (n, K) on the current device: for bf16, and while nobody has set a switch, cuBLAS on
+// PyTorch's handle (its stream and workspace), the call that torch.mm / addmm end in without their host path.
 void gemm_nt(Tensor& out, const Tensor& x, const Tensor& w, bool add) {
   const int64_t T = x.size(0), K = x.size(1), n = w.size(0);
   const bool plain = out.is_contiguous() && x.is_contiguous() && w.is_contiguous() && w.dim() == 2 && w.size(1) == K &&
-                     out.scalar_type() == x.scalar_type() && w.scalar_type() == x.scalar_type() && T > 0 && K > 0 && n > 0 &&
-                     std::max({T, K, n}) < (1ll << 31) &&
-                     (x.scalar_type() == at::kBFloat16 || x.scalar_type() == at::kFloat);
+                     out.scalar_type() == at::kBFloat16 && x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
+                     T > 0 && K > 0 && n > 0 && std::max({T, K, n}) < (1ll << 31) && default_products();
   if (!plain) {
     if (add) at::cuda::addmm_(out, x, w.t(), 1, 1);
     else at::cuda::mm_out(out, x, w.t());
     return;
   }
-  const cudaDataType_t dt = x.scalar_type() == at::kBFloat16 ? CUDA_R_16BF : CUDA_R_32F;
   const float one = 1.f, beta = add ? 1.f : 0.f;
   const cublasStatus_t rc = cublasGemmEx(at::cuda::getCurrentCUDABlasHandle(), CUBLAS_OP_T, CUBLAS_OP_N, (int)n, (int)T, (int)K, &one,
-                                         w.data_ptr(), dt, (int)K, x.data_ptr(), dt, (int)K, &beta, out.data_ptr(), dt, (int)n,
-                                         CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT_TENSOR_OP);
+                                         w.data_ptr(), CUDA_R_16BF, (int)K, x.data_ptr(), CUDA_R_16BF, (int)K, &beta, out.data_ptr(),
+                                         CUDA_R_16BF, (int)n, CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT_TENSOR_OP);
   TORCH_CHECK(rc == CUBLAS_STATUS_SUCCESS, "cublasGemmEx failed (", (int)rc, ")");
 }
 Tensor mm_nt(const Tensor& x, const Tensor& w) {

@@ -100,3 +100,28 @@ def test_ranker_layers_run_on_their_own_device():
     other.events = {"attn": [], "score": []}
     with torch.cuda.device(0):
         assert torch.equal(other.rank_host(batch)[0], ref)
+
+
+@pytest.mark.parametrize("switch", ["none", "bf16_reduction", "cublaslt", "deterministic"])
+def test_ranker_products_follow_pytorchs_switches(switch, monkeypatch):
+    """The products of a layer are torch.addmm's, bit for bit, whatever PyTorch's switches say."""
+    monkeypatch.setenv("CUBLAS_WORKSPACE_CONFIG", ":4096:8")
+    matmul, blas = torch.backends.cuda.matmul, torch.backends.cuda.preferred_blas_library()
+    monkeypatch.setattr(matmul, "allow_bf16_reduced_precision_reduction", switch != "bf16_reduction")
+    if switch == "cublaslt":
+        torch.backends.cuda.preferred_blas_library("cublaslt")
+    torch.use_deterministic_algorithms(switch == "deterministic")
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(2)
+        for dtype in (torch.bfloat16, torch.float32):
+            for T, K, n in [(16, 14336, 4096), (64, 4096, 1024), (2, 4096, 4096), (40, 8192, 256)]:
+                x = torch.randn(T, K, generator=gen, device="cuda").to(dtype)
+                w = (torch.randn(n, K, generator=gen, device="cuda") / K ** 0.5).to(dtype)
+                h = torch.randn(T, n, generator=gen, device="cuda").to(dtype)
+                ref = h.clone().addmm_(x, w.t())
+                zero = lambda *s: torch.zeros(*s, dtype=dtype, device="cuda")
+                _lib.host().layer_rest(h, x, w, zero(n), zero(16, n), zero(n, 8), 1e-5)  # (an MLP that adds nothing)
+                assert torch.equal(h, ref), (dtype, T, K, n)
+    finally:
+        torch.use_deterministic_algorithms(False)
+        torch.backends.cuda.preferred_blas_library(blas)
