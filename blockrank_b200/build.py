@@ -67,7 +67,11 @@ def _link_host(proc: subprocess.Popen) -> None:
         raise RuntimeError("building _host.so failed:\n" + out)
     import torch
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    link = [os.environ.get("CXX", "g++"), "-shared", "-o", HOST_LIB + ".tmp", HOST_SOURCE[:-4] + ".o", LIB, f"-L{lib}", "-lc10",
+    # libstdc++.so.6 by name: the one that PyTorch has loaded.  A compiler whose own libstdc++ is only there as an archive would
+    # link that in, and a second copy of the library in one process does not work: the first number written into an error
+    # message went through the wrong locale facet and ended the process.
+    link = [os.environ.get("CXX", "g++"), "-shared", "-o", HOST_LIB + ".tmp", HOST_SOURCE[:-4] + ".o", "-l:libstdc++.so.6", LIB,
+            f"-L{lib}", "-lc10",
             "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-L/usr/local/cuda/lib64", "-lcudart",
             "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{lib}"]
     r = subprocess.run(link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
@@ -77,7 +81,7 @@ def _link_host(proc: subprocess.Popen) -> None:
 
 
 def needs_host_build() -> bool:
-    return not os.path.exists(HOST_LIB) or any(os.path.getmtime(d) > os.path.getmtime(HOST_LIB) for d in (HOST_SOURCE, HEADER))
+    return not os.path.exists(HOST_LIB) or any(os.path.getmtime(d) > os.path.getmtime(HOST_LIB) for d in (HOST_SOURCE, HEADER, os.path.abspath(__file__)))
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

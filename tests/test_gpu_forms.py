@@ -125,3 +125,9 @@ def test_ranker_products_follow_pytorchs_switches(switch, monkeypatch):
     finally:
         torch.use_deterministic_algorithms(False)
         torch.backends.cuda.preferred_blas_library(blas)
+
+
+def test_error_messages_carry_their_numbers():
+    spans, q, k, v = packed([[9, 30, 41, 24]], 4, 2, 64, torch.bfloat16)
+    with pytest.raises(ValueError, match=r"shape mismatch q\[1, 4, 104, 64\]"):
+        ops.attention(q, k[:, :, :-8], v, spans[0], spans[1], 0.125, spans.max_block_len)

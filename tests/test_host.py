@@ -217,3 +217,14 @@ def test_gather_detects_missing_prompt():
     outs = _run_world("drop", 29613)
     for r, o in enumerate(outs):
         assert f"RESULT {r} error" in o and "no rank delivered" in o, o
+
+
+def test_host_module_shares_the_process_c_plus_plus_library():
+    """_host.so uses the libstdc++ that PyTorch has loaded (with a copy of its own, an error message with a number in it ends
+    the process)."""
+    import shutil
+    if shutil.which("readelf") is None:
+        pytest.skip("readelf is not installed")
+    path = os.path.join(os.path.dirname(_lib.LIB_PATH), "_host.so")
+    dynamic = subprocess.run(["readelf", "-d", path], capture_output=True, text=True, check=True).stdout
+    assert "[libstdc++.so.6]" in dynamic
