@@ -501,7 +501,8 @@ Tensor hidden_states(const Tensor& embed, const Tensor& ids, const std::vector<s
 }
 
 // The scoring layer up to the score epilogue: keys of every token, queries of the signal rows, both rotated; and the
-// index of each query row inside q.  Returns (q (B,N,R,D), k (B,Nk,S,D), rows int32 (B,R)).
+// index of each query row inside q.  pos (B, S); signal_rows (B, R), or (1, R): the same rows of every prompt.
+// Returns (q (B,N,R,D), k (B,Nk,S,D), rows int32 (B,R)).
 std::tuple<Tensor, Tensor, Tensor> score_qk(const Tensor& h, const Tensor& pos, const Tensor& signal_rows, const Tensor& ln1,
                                             const Tensor& wq, const Tensor& wk, const Tensor& inv_freq, int64_t N, int64_t Nk,
                                             int64_t D, double eps) {
@@ -510,8 +511,12 @@ std::tuple<Tensor, Tensor, Tensor> score_qk(const Tensor& h, const Tensor& pos, 
   need_cuda({&h, &pos, &signal_rows});
   BRK_VALUE(signal_rows.scalar_type() == at::kInt && signal_rows.dim() == 2 && pos.scalar_type() == at::kInt && pos.is_contiguous(),
             "signal_rows must be int32 (B, R) and positions contiguous int32");
-  const int64_t B = signal_rows.size(0), R = signal_rows.size(1), T = h.size(0), S = T / B;
-  const Tensor x = rmsnorm(h, ln1, eps, std::nullopt, std::nullopt), rows = signal_rows.contiguous();
+  BRK_VALUE(pos.dim() == 2 && h.dim() == 2 && h.size(0) == pos.numel(), "positions must be (B, S) for hidden states (B S, hidden), got ",
+            pos.sizes(), " and ", h.sizes());
+  const int64_t B = pos.size(0), R = signal_rows.size(1), T = h.size(0), S = pos.size(1);
+  BRK_VALUE(signal_rows.size(0) == B || signal_rows.size(0) == 1, "signal_rows must be (B, R) or (1, R), got ", signal_rows.sizes(),
+            " for ", B, " prompts");
+  const Tensor x = rmsnorm(h, ln1, eps, std::nullopt, std::nullopt), rows = signal_rows.expand({B, R}).contiguous();
   Tensor k = mm_nt(x, wk);
   Tensor xs = at::empty({B * R, x.size(1)}, x.options()), ps = at::empty({B * R}, pos.options()), local = at::empty({B, R}, pos.options());
   check(brk_signal_rows(dtype_code(x), x.data_ptr(), (int32_t)x.size(1), (const int32_t*)pos.data_ptr(),
@@ -522,7 +527,7 @@ std::tuple<Tensor, Tensor, Tensor> score_qk(const Tensor& h, const Tensor& pos, 
   count(1);
   Tensor q = mm_nt(xs, wq);
   rope_(q.view({B * R, N, D}), std::nullopt, ps, inv_freq);
-  rope_(std::nullopt, k.view({T, Nk, D}), pos, inv_freq);
+  rope_(std::nullopt, k.view({T, Nk, D}), pos, inv_freq);  // (pos: T of them, contiguous)
   return {q.view({B, R, N, D}).permute({0, 2, 1, 3}), k.view({B, S, Nk, D}).permute({0, 2, 1, 3}), local};
 }
 
@@ -618,9 +623,10 @@ std::tuple<Tensor, Tensor> rank(const Tensor& embed, const std::vector<std::vect
                                 double eps, int64_t algo, double temperature, int64_t k) {
   c10::cuda::CUDAGuard device(embed.device());
   const auto [d_ids, d_pos, start, len, d_rows, longest] = upload(ids, pos, spans, rows, embed.device());
-  const Tensor flat = d_pos.reshape({-1});
-  const Tensor h = hidden_states(embed, d_ids, layers, flat, inv_freq, start, len, max_block_len, longest, N, Nk, D, eps, algo);
-  const auto [q, kk, local] = score_qk(h, flat, d_rows, score_layer.at(0), score_layer.at(1), score_layer.at(2), inv_freq, N, Nk, D, eps);
+  BRK_VALUE(d_ids.dim() == 2 && d_pos.sizes() == d_ids.sizes(), "input_ids and position_ids must be (B, S), got ", d_ids.sizes(), " and ",
+            d_pos.sizes());
+  const Tensor h = hidden_states(embed, d_ids, layers, d_pos.reshape({-1}), inv_freq, start, len, max_block_len, longest, N, Nk, D, eps, algo);
+  const auto [q, kk, local] = score_qk(h, d_pos.contiguous(), d_rows, score_layer.at(0), score_layer.at(1), score_layer.at(2), inv_freq, N, Nk, D, eps);
   return download(std::get<1>(doc_scores(q, kk, start, len, local, 1.0 / std::sqrt((double)D), temperature)), k);
 }
 

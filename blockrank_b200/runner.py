@@ -155,7 +155,8 @@ class MistralPrefillRanker:
 
     @torch.no_grad()
     def score(self, input_ids, position_ids, blk_start, blk_len, max_block_len, signal_rows, max_query_len=0):
-        """input_ids/position_ids (B, S) on the device, spans int32 (B, M), signal_rows int32 (B, R);
+        """input_ids/position_ids (B, S) on the device, spans int32 (B, M), signal_rows int32 (B, R), or (1, R) for
+        the same rows of every prompt;
         ``max_query_len`` (optional) bounds the query block's length (smaller attention scratch).
 
         Returns (logits (B, num_docs) fp32, doc_mass (B, N, R, num_docs) fp32).  Device-side problems
@@ -171,7 +172,7 @@ class MistralPrefillRanker:
         input RMSNorm, ``k_proj`` of every token, ``q_proj`` of the signal rows, RoPE, fused score epilogue."""
         c = self.cfg
         L = self.layers[c.score_layer]
-        pos = position_ids.reshape(-1).to(torch.int32)
+        pos = position_ids.to(torch.int32).contiguous()
         q, k, rows = _lib.host().score_qk(h, pos, signal_rows.to(torch.int32), L["ln1"], L["wq"], L["wk"], self.inv_freq,
                                           c.num_attention_heads, c.num_key_value_heads, c.head_dim, c.rms_norm_eps)
         ev = self._tick("score")

@@ -127,6 +127,37 @@ def test_ranker_products_follow_pytorchs_switches(switch, monkeypatch):
         torch.backends.cuda.preferred_blas_library(blas)
 
 
+def _requests(n, lens, dtype=torch.bfloat16):
+    """(ranker, batch) of n prompts of the same block lengths on the tiny model."""
+    from blockrank_b200 import packed_block_collate_fn
+    from blockrank_b200.runner import MistralPrefillRanker, RankerConfig
+    cfg = RankerConfig.tiny()
+    g = torch.Generator().manual_seed(n)
+    items = [{"input_ids": torch.randint(3, cfg.vocab_size, (sum(lens),), generator=g), "block_lengths": lens} for _ in range(n)]
+    return MistralPrefillRanker(cfg, "cuda", dtype).init_random(seed=1), packed_block_collate_fn(items)
+
+
+def test_one_set_of_signal_rows_serves_every_prompt():
+    """signal_rows of shape (1, R) are the rows of every prompt: host request, device call, captured graph."""
+    rk, batch = _requests(3, [30, 40, 50, 60, 20, 4])
+    full = rk.rank_host(batch)[0]
+    one = dict(batch, signal_rows=batch["signal_rows"][:1])
+    assert torch.equal(rk.rank_host(one)[0], full)
+    spans = batch["block_spans"].cuda()
+    args = (batch["input_ids"].cuda(), batch["position_ids"].cuda(), spans[0], spans[1], int(batch["max_block_len"]))
+    assert torch.equal(rk.score(*args, one["signal_rows"].cuda())[0].cpu(), full)
+    rk.use_graphs = True
+    assert torch.equal(rk.rank_host(one)[0], full)
+
+
+def test_request_shapes_that_do_not_belong_together_are_refused():
+    rk, batch = _requests(3, [30, 40, 50, 20, 4])
+    for bad in (dict(batch, signal_rows=batch["signal_rows"][:2]), dict(batch, position_ids=batch["position_ids"].flatten()),
+                dict(batch, position_ids=batch["position_ids"][:, :-1].contiguous())):
+        with pytest.raises((ValueError, RuntimeError)):
+            rk.rank_host(bad)
+
+
 def test_error_messages_carry_their_numbers():
     spans, q, k, v = packed([[9, 30, 41, 24]], 4, 2, 64, torch.bfloat16)
     with pytest.raises(ValueError, match=r"shape mismatch q\[1, 4, 104, 64\]"):
