@@ -40,7 +40,11 @@ class BlockSpans(torch.Tensor):
     layout)."""
 
     def __getitem__(self, item):
-        """Plain tensors: the halves are read on every call, and subclass dispatch would cost more than the slice."""
+        """A half (``spans[0]``, ``spans[1]``) is a plain tensor: they are read on every call, and subclass dispatch would
+        cost more than the slice.  Anything else stays a BlockSpans, but one without a ``max_block_len``: the attention
+        refuses it, where a plain tensor would be taken for a block mask."""
+        if type(item) is not int:
+            return super().__getitem__(item)
         with torch._C.DisableTorchFunctionSubclass():
             return super().__getitem__(item)
 

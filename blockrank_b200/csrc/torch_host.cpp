@@ -76,6 +76,13 @@ int dtype_code(const Tensor& t) {
 }
 void* stream_of(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 
+// starts and lengths of every block of B prompts: the kernels read B * M of each
+void need_spans(const Tensor& start, const Tensor& length, int64_t B) {
+  BRK_VALUE(start.scalar_type() == at::kInt && length.scalar_type() == at::kInt && start.sizes() == length.sizes() && start.dim() >= 1,
+            "blk_start / blk_len must be int32 tensors of the same (B, M) shape");
+  BRK_VALUE(start.numel() >= B * start.size(-1), "block spans of ", start.sizes(), " are too few for ", B, " prompts");
+}
+
 // (B, heads, S, D) tensor (any strides, innermost contiguous) -> brk_view
 brk_view view_of(const Tensor& t) {
   BRK_VALUE(t.dim() == 4 && t.stride(3) == 1, "expected a (B, heads, S, D) tensor with contiguous head_dim");
@@ -139,8 +146,7 @@ std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Ten
   BRK_VALUE(k.size(0) == B && k.size(2) == S && k.size(3) == D && v.sizes() == k.sizes(), "shape mismatch q", q.sizes(), " k",
             k.sizes(), " v", v.sizes());
   BRK_VALUE(k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(), "q, k, v must share a dtype");
-  BRK_VALUE(blk_start.scalar_type() == at::kInt && blk_len.scalar_type() == at::kInt && blk_start.sizes() == blk_len.sizes(),
-            "blk_start / blk_len must be int32 tensors of the same (B, M) shape");
+  need_spans(blk_start, blk_len, B);
   c10::cuda::CUDAGuard guard(q.device());
   Tensor out = out_in.has_value() ? *out_in : empty_bshd(q, B, S, N, D);
   Tensor lse = lse_in.has_value() ? *lse_in
@@ -182,6 +188,7 @@ std::tuple<Tensor, Tensor, Tensor> attention_bwd(const Tensor& q, const Tensor& 
             "lse must be the forward's fp32 (B, N, S) tensor");
   for (const Tensor* t : {&k, &v, &out, &d_out_in})
     BRK_VALUE(t->scalar_type() == q.scalar_type(), "q, k, v, out, d_out must share a dtype");
+  need_spans(blk_start, blk_len, B);
   c10::cuda::CUDAGuard guard(q.device());
   const Tensor d_out = d_out_in.contiguous(), lse = lse_in.contiguous();  // (autograd may hand over expanded or transposed gradients)
   Tensor dq = empty_bshd(q, B, S, N, D).permute({0, 2, 1, 3});
@@ -211,6 +218,7 @@ std::tuple<Tensor, Tensor, Tensor> attention_bwd(const Tensor& q, const Tensor& 
 // ---- scores -----------------------------------------------------------------------------------
 brk_score_params score_params(const Tensor& q, const Tensor& k, const Tensor& bs, const Tensor& bl, double scale, int64_t R,
                               double temperature) {
+  need_spans(bs, bl, q.size(0));
   brk_score_params p{};
   p.dtype = dtype_code(q);
   p.B = (int32_t)q.size(0); p.N = (int32_t)q.size(1); p.Nk = (int32_t)k.size(1); p.D = (int32_t)q.size(3);
@@ -340,11 +348,11 @@ struct AttentionFn : torch::autograd::Function<AttentionFn> {
   }
 };
 
-// num_last < 0: no raw logits.  spans: int32 (2, B, M) [starts; lengths].  Returns (out, raw or None).
+// num_last < 0: no raw logits.  spans: int32 (2, B, M) [starts; lengths], (2, M) for one prompt.  Returns (out, raw or None).
 std::tuple<Tensor, OptTensor> attention_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& spans,
                                                 double scale, int64_t max_block_len, int64_t max_query_len, int64_t algo,
                                                 int64_t num_last, int64_t grid_h) {
-  BRK_VALUE(spans.dim() == 3 && spans.size(0) == 2, "block spans must be an int32 (2, B, M) tensor");
+  BRK_VALUE(spans.dim() >= 2 && spans.size(0) >= 2, "block spans must be an int32 (2, B, M) tensor, or (2, M) for one prompt");
   const Tensor start = spans.select(0, 0), length = spans.select(0, 1);
   if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) {
     auto res = AttentionFn::apply(q, k, v, start, length, scale, max_block_len, max_query_len, algo, num_last, grid_h);

@@ -162,3 +162,18 @@ def test_error_messages_carry_their_numbers():
     spans, q, k, v = packed([[9, 30, 41, 24]], 4, 2, 64, torch.bfloat16)
     with pytest.raises(ValueError, match=r"shape mismatch q\[1, 4, 104, 64\]"):
         ops.attention(q, k[:, :, :-8], v, spans[0], spans[1], 0.125, spans.max_block_len)
+
+
+def test_spans_of_one_prompt_and_parts_of_spans():
+    """(2, M) spans serve one prompt; a slice of spans is refused, not read as a block mask; too few spans are refused."""
+    spans, q, k, v = packed([[9, 30, 41, 24]] * 2, 4, 2, 64, torch.bfloat16)
+    run = lambda n, sp: cuda_blockrank_attention_forward(Layer(), q[:n], k[:n], v[:n], sp, 0.125)[0]
+    full = run(2, spans)
+    assert torch.equal(run(1, BlockSpans.make(spans[0][0], spans[1][0], spans.max_block_len)), full[:1])
+    with pytest.raises(AttributeError):
+        run(1, spans[:, :1])
+    for call in (lambda: run(2, BlockSpans.make(spans[0][0], spans[1][0], spans.max_block_len)),
+                 lambda: ops.raw_scores(q, k, spans[0][:1], spans[1][:1], 0.125),
+                 lambda: ops.doc_scores(q, k, spans[0][:1], spans[1][:1], torch.zeros(2, 2, dtype=torch.int32, device="cuda"), 0.125)):
+        with pytest.raises(ValueError, match="too few"):
+            call()
