@@ -12,6 +12,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <cublas_v2.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
 
 #include <atomic>
@@ -305,43 +307,65 @@ std::tuple<Tensor, Tensor> raw_scores_bwd(const Tensor& q, const Tensor& k, cons
   throw err;
 }
 
-// BlockRank attention with its backward (brk_attn_bwd).  With num_last >= 0 it also returns the raw logits of the last R
-// slots, (B,N,R,S) = scale * q[:, :, S-R:] k^T + a constant mask addend (std:219-233, 256-262): the addend is constant,
-// so their gradient flows to q and k at every position (brk_raw_scores_bwd, which adds into the gradients of the
-// attention output instead of leaving two pairs of tensors for autograd to sum).
-struct AttentionFn : torch::autograd::Function<AttentionFn> {
-  using Ctx = torch::autograd::AutogradContext;
-  using List = torch::autograd::variable_list;
+// Gradient of the raw logits in PyTorch operations, for a backward that is differentiated itself (create_graph).
+std::tuple<Tensor, Tensor> raw_grad_graph(const Tensor& q, const Tensor& k, const Tensor& d_raw, double scale) {
+  const int64_t B = q.size(0), N = q.size(1), S = q.size(2), D = q.size(3), Nk = k.size(1), R = d_raw.size(2);
+  const Tensor g = (d_raw.to(at::kFloat) * scale).reshape({B, Nk, N / Nk, R, S});
+  const Tensor q_last = q.narrow(2, S - R, R).to(at::kFloat).reshape({B, Nk, N / Nk, R, D});
+  const Tensor dq = at::einsum("bkgrs,bksd->bkgrd", {g, k.to(at::kFloat)}).reshape({B, N, R, D}).to(q.scalar_type());
+  return {at::constant_pad_nd(dq, {0, 0, S - R, 0}), at::einsum("bkgrs,bkgrd->bksd", {g, q_last}).to(k.scalar_type())};
+}
 
-  static List forward(Ctx* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& start, const Tensor& length,
-                      double scale, int64_t max_block_len, int64_t max_query_len, int64_t algo, int64_t num_last,
-                      int64_t grid_h) {
-    ctx->set_materialize_grads(false);
-    auto [out, lse] = attention(q, k, v, start, length, scale, max_block_len, std::nullopt, true, algo, max_query_len,
-                                std::nullopt);
-    ctx->save_for_backward({q, k, v, out, lse, start, length});
-    ctx->saved_data["scale"] = scale;
-    ctx->saved_data["max_block_len"] = max_block_len;
-    if (num_last < 0) return {out};
-    return {out, raw_scores(q, k, start, length, scale, num_last, grid_h)};
+// Backward of the attention output (brk_attn_bwd) and, where they were asked for, of the raw logits of the last R slots,
+// (B,N,R,S) = scale * q[:, :, S-R:] k^T + a mask addend (std:219-233, 256-262): the addend is constant, so their gradient
+// flows to q and k at every position (brk_raw_scores_bwd).  One node for both outputs: a pass that brings both gradients adds
+// the second into the first instead of leaving two pairs of tensors for autograd to sum.  What an output saved is given back
+// on its own, behind the pass that used it, so that the two can be differentiated in passes of their own.
+struct AttentionNode : torch::autograd::Node {
+  using List = torch::autograd::variable_list;
+  using Saved = torch::autograd::SavedVariable;
+
+  Saved q, k, v, out, lse, start, length;
+  double scale = 0;
+  int64_t max_block_len = 0;
+  bool spent[2] = {false, true};  // output 0: attention, 1: raw logits (none: nothing saved for them)
+  bool used[2] = {false, false};  // by the latest pass
+
+  std::string name() const override { return "BlockRankAttentionBackward"; }
+
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (int i = 0; i < 2; ++i) spent[i] |= used[i];
+    if (spent[0])
+      for (Saved* t : {&v, &out, &lse}) t->reset_data();
+    if (spent[0] && spent[1])
+      for (Saved* t : {&q, &k, &start, &length}) t->reset_data();
   }
 
-  static List backward(Ctx* ctx, List grads) {
+  List apply(List&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
     try {
-      const auto saved = ctx->get_saved_variables();
-      const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &out = saved[3], &lse = saved[4], &start = saved[5],
-                   &length = saved[6];
-      const double scale = ctx->saved_data["scale"].toDouble();
-      const int64_t max_block_len = ctx->saved_data["max_block_len"].toInt();
+      used[0] = grads[0].defined();
+      used[1] = grads.size() > 1 && grads[1].defined();
+      for (int i = 0; i < 2; ++i) TORCH_CHECK(!(used[i] && spent[i]), torch::autograd::ERR_BACKWARD_TWICE);
       Tensor dq, dk, dv;
-      if (grads[0].defined())
-        std::tie(dq, dk, dv) = attention_bwd(q, k, v, out, grads[0].to(out.scalar_type()), lse, start, length, scale, max_block_len);
-      if (grads.size() > 1 && grads[1].defined()) {
-        const bool add = dq.defined();
-        std::tie(dq, dk) = raw_scores_bwd(q, k, grads[1].to(q.scalar_type()), start, length, scale,
-                                          add ? OptTensor(dq) : std::nullopt, add ? OptTensor(dk) : std::nullopt);
+      if (!used[0] && !used[1]) return {dq, dk, dv};
+      const Tensor sq = q.unpack(), sk = k.unpack(), ss = start.unpack(), sl = length.unpack();
+      const bool graph = at::GradMode::is_enabled();
+      if (used[0]) {
+        const Tensor so = out.unpack(shared_from_this()), sv = v.unpack(), slse = lse.unpack();
+        at::NoGradGuard no_grad;
+        std::tie(dq, dk, dv) = attention_bwd(sq, sk, sv, so, grads[0].to(so.scalar_type()), slse, ss, sl, scale, max_block_len);
       }
-      return {dq, dk, dv, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+      if (used[1] && graph) {
+        const auto [rq, rk] = raw_grad_graph(sq, sk, grads[1], scale);
+        dq = used[0] ? dq + rq : rq;
+        dk = used[0] ? dk + rk : rk;
+      } else if (used[1]) {
+        std::tie(dq, dk) = raw_scores_bwd(sq, sk, grads[1].to(sq.scalar_type()), ss, sl, scale,
+                                          used[0] ? OptTensor(dq) : std::nullopt, used[0] ? OptTensor(dk) : std::nullopt);
+      }
+      return {dq, dk, dv};
     } catch (const LibError& e) {
       rethrow_as_python(e);
     }
@@ -354,14 +378,35 @@ std::tuple<Tensor, OptTensor> attention_forward(const Tensor& q, const Tensor& k
                                                 int64_t num_last, int64_t grid_h) {
   BRK_VALUE(spans.dim() >= 2 && spans.size(0) >= 2, "block spans must be an int32 (2, B, M) tensor, or (2, M) for one prompt");
   const Tensor start = spans.select(0, 0), length = spans.select(0, 1);
-  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) {
-    auto res = AttentionFn::apply(q, k, v, start, length, scale, max_block_len, max_query_len, algo, num_last, grid_h);
-    return {res[0], num_last < 0 ? OptTensor() : OptTensor(res[1])};
+  const bool train = torch::autograd::compute_requires_grad(q, k, v);
+  if (train)
+    for (const Tensor* t : {&q, &k, &v})
+      TORCH_CHECK_NOT_IMPLEMENTED(!t->_fw_grad(/*level=*/0).defined(), "BlockRank attention has no forward-mode derivative");
+  Tensor out, lse, raw;
+  {
+    at::AutoGradMode no_grad(false);
+    std::tie(out, lse) = attention(q, k, v, start, length, scale, max_block_len, std::nullopt, train, algo, max_query_len, std::nullopt);
+    if (num_last >= 0) raw = raw_scores(q, k, start, length, scale, num_last, grid_h);
   }
-  Tensor out = std::get<0>(attention(q, k, v, start, length, scale, max_block_len, std::nullopt, false, algo, max_query_len,
-                                     std::nullopt));
-  if (num_last < 0) return {out, std::nullopt};
-  return {out, raw_scores(q, k, start, length, scale, num_last, grid_h)};
+  if (train) {
+    std::shared_ptr<AttentionNode> node(new AttentionNode(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
+    node->q = AttentionNode::Saved(q, false);
+    node->k = AttentionNode::Saved(k, false);
+    node->v = AttentionNode::Saved(v, false);
+    node->lse = AttentionNode::Saved(lse, false);
+    node->start = AttentionNode::Saved(start, false);
+    node->length = AttentionNode::Saved(length, false);
+    node->scale = scale;
+    node->max_block_len = max_block_len;
+    torch::autograd::set_history(out, node);
+    if (raw.defined()) {
+      node->spent[1] = false;
+      torch::autograd::set_history(raw, node);
+    }
+    node->out = AttentionNode::Saved(out, true);
+  }
+  return {out, raw.defined() ? OptTensor(raw) : std::nullopt};
 }
 
 // ---- runner helpers ---------------------------------------------------------------------------
@@ -651,6 +696,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       PyErr_SetString(g_oom_error, e.what_without_backtrace());
     } catch (const c10::ValueError& e) {
       PyErr_SetString(PyExc_ValueError, e.what_without_backtrace());
+    } catch (const c10::NotImplementedError& e) {
+      PyErr_SetString(PyExc_NotImplementedError, e.what_without_backtrace());
     } catch (const c10::IndexError& e) {
       PyErr_SetString(PyExc_IndexError, e.what_without_backtrace());
     } catch (const c10::Error& e) {

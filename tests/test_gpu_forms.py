@@ -177,3 +177,78 @@ def test_spans_of_one_prompt_and_parts_of_spans():
                  lambda: ops.doc_scores(q, k, spans[0][:1], spans[1][:1], torch.zeros(2, 2, dtype=torch.int32, device="cuda"), 0.125)):
         with pytest.raises(ValueError, match="too few"):
             call()
+
+
+def _train(dtype, lens=((20, 30, 40, 24),) * 2, N=4, Nk=2, D=64):
+    """(leaves, call): call() is a forward with raw logits under autograd on fresh graph nodes."""
+    spans, q, k, v = packed([list(x) for x in lens], N, Nk, D, dtype, seed=5)
+    leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    return leaves, lambda: cuda_blockrank_attention_forward(Layer(), *leaves, spans, D ** -0.5, layers_to_return_scores=[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_outputs_can_be_differentiated_in_passes_of_their_own(dtype):
+    """The attention output and the raw logits, in one pass, in two passes of either order, and no output twice."""
+    leaves, call = _train(dtype)
+    out, raw = call()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    go, gr = (torch.randn(t.shape, generator=g, device="cuda").to(dtype) for t in (out, raw))
+    both = torch.autograd.grad([out, raw], leaves, [go, gr], retain_graph=True)
+    a = torch.autograd.grad(out, leaves, go)
+    r = torch.autograd.grad(raw, leaves, gr, allow_unused=True)
+    assert r[2] is None
+    tol = 1e-2 if dtype == torch.bfloat16 else 1e-5
+    for x, y, z in zip(both[:2], a, r):
+        assert (x.double() - (y.double() + z.double())).norm() <= tol * x.double().norm()
+    out, raw = call()  # the other order
+    r2 = torch.autograd.grad(raw, leaves[:2], gr)
+    a2 = torch.autograd.grad(out, leaves, go)
+    for x, y in zip((*a, *r[:2]), (*a2, *r2)):
+        assert (x.double() - y.double()).norm() <= 1e-4 * x.double().norm()  # (sums of the prefix in another order)
+    for t, gt in ((out, go), (raw, gr)):
+        with pytest.raises(RuntimeError, match="second time"):
+            torch.autograd.grad(t, leaves[:2], gt)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_raw_logits_can_be_differentiated_twice(dtype):
+    """A penalty on the gradient of the raw logits: its gradient against 64 bits."""
+    leaves, call = _train(dtype)
+    _, raw = call()
+    g = torch.randn(raw.shape, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda").to(dtype) * 0.1
+    dq, dk = torch.autograd.grad(raw, leaves[:2], g, create_graph=True)
+    got = torch.autograd.grad(dq.float().square().sum() + dk.float().square().sum(), leaves[:2])
+    q, k = (t.detach().double().requires_grad_(True) for t in leaves[:2])
+    R, S = raw.shape[2:]
+    ref = (q[:, :, S - R:] * 0.125) @ k.repeat_interleave(2, 1).transpose(-1, -2)
+    rq, rk = torch.autograd.grad(ref, (q, k), g.double(), create_graph=True)
+    want = torch.autograd.grad(rq.square().sum() + rk.square().sum(), (q, k))
+    for x, y in zip(got, want):
+        assert (x.double() - y).norm() <= (1e-2 if dtype == torch.bfloat16 else 1e-5) * y.norm()
+
+
+def test_autograd_forms_that_are_refused_or_hooked():
+    leaves, call = _train(torch.bfloat16)
+    kept = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: kept.append(t) or t.cpu(), lambda t: t.cuda()):
+        out, raw = call()
+    assert len(kept) == 7
+    hooked = torch.autograd.grad([out, raw], leaves, [torch.ones_like(out), torch.ones_like(raw)])
+    out, raw = call()
+    plain = torch.autograd.grad([out, raw], leaves, [torch.ones_like(out), torch.ones_like(raw)])
+    for x, y in zip(hooked, plain):
+        assert (x.double() - y.double()).norm() <= 1e-4 * y.double().norm()
+    spans, q, k, v = packed([[20, 30, 40, 24]], 4, 2, 64, torch.bfloat16)
+    y = q.clone().requires_grad_(True) * 1
+    out, _ = cuda_blockrank_attention_forward(Layer(), y, k, v, spans, 0.125)
+    with torch.no_grad():
+        y.add_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.float().sum().backward()
+    import torch.autograd.forward_ad as fa
+    with fa.dual_level(), pytest.raises(NotImplementedError):
+        dual = fa.make_dual(q.clone().requires_grad_(True), torch.ones_like(q))
+        cuda_blockrank_attention_forward(Layer(), dual, k, v, spans, 0.125)
+    for transform in (lambda f: torch.func.grad(lambda x: f(x).float().sum())(q), lambda f: torch.vmap(f)(torch.stack([q, q]))):
+        with pytest.raises(RuntimeError):
+            transform(lambda x: cuda_blockrank_attention_forward(Layer(), x, k, v, spans, 0.125)[0])
