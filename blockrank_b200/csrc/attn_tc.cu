@@ -52,6 +52,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "attn_combine.cuh"
@@ -62,15 +63,15 @@ namespace brk {
 
 // ---- host: tensor maps -----------------------------------------------------------------
 EncodeTiledFn get_encode_tiled() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn) return fn;
+  static std::atomic<EncodeTiledFn> fn{nullptr};
+  if (EncodeTiledFn f = fn.load(std::memory_order_acquire)) return f;
   void* p = nullptr;
   cudaDriverEntryPointQueryResult qres;
   if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres) != cudaSuccess ||
       qres != cudaDriverEntryPointSuccess || p == nullptr)
     return nullptr;
-  fn = reinterpret_cast<EncodeTiledFn>(p);
-  return fn;
+  fn.store(reinterpret_cast<EncodeTiledFn>(p), std::memory_order_release);
+  return reinterpret_cast<EncodeTiledFn>(p);
 }
 
 static int make_tmap(CUtensorMap* out, CUtensorMapDataType type, int bytes, const void* ptr, int D, int heads, int S, int B,
@@ -1411,23 +1412,23 @@ static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cuda
   if ((rc = make_tmap_bf16(&tq, p.q.ptr, HD, p.N, p.S, p.B, p.q.stride_h, p.q.stride_s, p.q.stride_b, G, TOK))) return rc;
   if ((rc = make_tmap_bf16(&tk, p.k.ptr, HD, p.Nk, p.S, p.B, p.k.stride_h, p.k.stride_s, p.k.stride_b, 1, BN))) return rc;
   if ((rc = make_tmap_bf16(&tv, p.v.ptr, HD, p.Nk, p.S, p.B, p.v.stride_h, p.v.stride_s, p.v.stride_b, 1, BN))) return rc;
-  static bool configured[64] = {};
-  static int sms[64] = {};
+  static std::atomic<int> sms[64] = {};  // SMs of a device whose kernel is configured (by any thread: the steps can be repeated)
   int dev = 0;
   BRK_CUDA(cudaGetDevice(&dev));
   BRK_REQUIRE(dev >= 0 && dev < 64, BRK_E_UNSUPPORTED, "device ordinal %d out of range", dev);
-  if (!configured[dev]) {
+  int n_sm = sms[dev].load(std::memory_order_acquire);
+  if (n_sm == 0) {
     BRK_CUDA(cudaFuncSetAttribute(attn_tc_kernel<HD, kFine>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)Geo<HD>::kSmemBytes));
-    sms[dev] = sm_count();
-    BRK_REQUIRE(sms[dev] > 0, BRK_E_CUDA, "could not read the SM count");
-    configured[dev] = true;
+    n_sm = sm_count();
+    BRK_REQUIRE(n_sm > 0, BRK_E_CUDA, "could not read the SM count");
+    sms[dev].store(n_sm, std::memory_order_release);
   }
   // Blocks are handed out in groups of consecutive blocks of one (prompt, KV head), so that the prefix's K/V
   // stays in shared memory from one block to the next.  Balance matters more than that reuse (measured: single
   // blocks 0.560 ms, groups of three 0.572 ms on 4 prompts of 100 documents), so groups only form when every SM
   // still gets two dozen of them.
-  int group = (int)((nbg * (p.M > 1 ? p.M - 1 : 0)) / (24 * (int64_t)sms[dev]));
+  int group = (int)((nbg * (p.M > 1 ? p.M - 1 : 0)) / (24 * (int64_t)n_sm));
   group = group < 1 ? 1 : (group > kMaxGroup ? kMaxGroup : group);
   const int n_groups = p.M > 1 ? (p.M - 1 + group - 1) / group : 0;
   const int64_t sec1 = nbg * ns * pairs_q;
@@ -1464,7 +1465,7 @@ static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cuda
   // themselves.  (One prompt of 5 documents: the prologue kernel and the gap behind it were 4 of 20 us.)
   a.max_block_len = p.max_block_len;
   a.max_query_len = p.max_query_len;
-  a.one_wave = total_items <= sms[dev];
+  a.one_wave = total_items <= n_sm;
   a.win = nullptr;
   a.n_live = nullptr;
   a.win_pitch = win_pitch(p);
@@ -1479,7 +1480,7 @@ static int attn_tc_run(const brk_attn_params& p, void* ws, size_t ws_bytes, cuda
                                    a.win_pitch, st)))
       return rc;
   }
-  const int grid = (int)(total_items < sms[dev] ? total_items : sms[dev]);
+  const int grid = (int)(total_items < n_sm ? total_items : n_sm);
   if ((rc = launch_dependent(attn_tc_kernel<HD, kFine>, dim3(grid), dim3(kThreads), Geo<HD>::kSmemBytes, st, tq, tk, tv, a))) return rc;
   if (ns > 1) {
     const CombineArgs c{a.o, a.lse, a.blk_start, a.blk_len, a.hdr, p.B, p.N, p.S, p.M, lq, ns, a.part_o, a.part_ml};

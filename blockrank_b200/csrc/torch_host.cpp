@@ -654,10 +654,7 @@ std::tuple<Tensor, Tensor> download(const Tensor& logits_in, int64_t k_in) {
     C10_CUDA_CHECK(cudaMemcpyAsync(base + at_top, dev.data_ptr(), nt, cudaMemcpyDeviceToHost, stream));
     C10_CUDA_CHECK(cudaMemcpyAsync(base + at_word, word.data_ptr(), 4, cudaMemcpyDeviceToHost, stream));
   }
-  {
-    pybind11::gil_scoped_release release;
-    C10_CUDA_CHECK(cudaStreamSynchronize(stream));
-  }
+  C10_CUDA_CHECK(cudaStreamSynchronize(stream));
   Tensor h_logits = at::empty(logits.sizes(), logits.options().device(at::kCPU));
   Tensor h_top = at::empty({B, k}, at::TensorOptions().dtype(at::kLong));
   memcpy(h_logits.data_ptr(), base, nl);
@@ -709,23 +706,26 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     g_oom_error = oom.release().ptr();
   });
   m.def("launch_count", [] { return g_launches.load(); });
-  m.def("status_word", &status_word);
-  m.def("spans_from_mask", &spans_from_mask);
-  m.def("attention", &attention);
-  m.def("attention_bwd", &attention_bwd);
-  m.def("attention_forward", &attention_forward);
-  m.def("doc_scores", &doc_scores);
-  m.def("raw_scores", &raw_scores);
-  m.def("raw_scores_bwd", &raw_scores_bwd);
-  m.def("rmsnorm", &rmsnorm);
-  m.def("rope_", &rope_);
-  m.def("silu_mul", &silu_mul);
-  m.def("layer_qkv", &layer_qkv);
-  m.def("layer_attention", &layer_attention);
-  m.def("layer_rest", &layer_rest);
-  m.def("hidden_states", &hidden_states);
-  m.def("score_qk", &score_qk);
-  m.def("upload", &upload);
-  m.def("download", &download);
-  m.def("rank", &rank);
+  // Other Python threads run meanwhile: a launch blocks once the device's queue is full, and a ranking request waits for its
+  // results.
+  auto def = [&m](const char* name, auto f) { m.def(name, f, py::call_guard<py::gil_scoped_release>()); };
+  def("status_word", &status_word);
+  def("spans_from_mask", &spans_from_mask);
+  def("attention", &attention);
+  def("attention_bwd", &attention_bwd);
+  def("attention_forward", &attention_forward);
+  def("doc_scores", &doc_scores);
+  def("raw_scores", &raw_scores);
+  def("raw_scores_bwd", &raw_scores_bwd);
+  def("rmsnorm", &rmsnorm);
+  def("rope_", &rope_);
+  def("silu_mul", &silu_mul);
+  def("layer_qkv", &layer_qkv);
+  def("layer_attention", &layer_attention);
+  def("layer_rest", &layer_rest);
+  def("hidden_states", &hidden_states);
+  def("score_qk", &score_qk);
+  def("upload", &upload);
+  def("download", &download);
+  def("rank", &rank);
 }

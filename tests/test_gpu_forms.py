@@ -252,3 +252,52 @@ def test_autograd_forms_that_are_refused_or_hooked():
     for transform in (lambda f: torch.func.grad(lambda x: f(x).float().sum())(q), lambda f: torch.vmap(f)(torch.stack([q, q]))):
         with pytest.raises(RuntimeError):
             transform(lambda x: cuda_blockrank_attention_forward(Layer(), x, k, v, spans, 0.125)[0])
+
+
+def test_other_threads_run_while_calls_are_enqueued():
+    """A call that blocks on the full queue of a busy device does not hold Python's lock."""
+    import threading
+    import time
+    spans, q, k, v = packed([[64] + [100] * 10 + [48]], 32, 8, 128, torch.bfloat16)
+    call = lambda: cuda_blockrank_attention_forward(Layer(), q, k, v, spans, 0.1)
+    call()
+    torch.cuda.synchronize()
+    gap, stop = [0.0], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gap[0], last = max(gap[0], now - last), now
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    torch.cuda._sleep(1_500_000_000)  # about 0.8 s of an idle kernel; the queue holds about a thousand launches
+    for _ in range(1200):
+        call()
+    torch.cuda.synchronize()
+    stop.set()
+    thread.join()
+    assert gap[0] < 0.3
+
+
+def test_calls_of_several_threads_on_streams_of_their_own():
+    import threading
+    spans, q, k, v = packed([[30, 90, 70, 50, 24]] * 2, 8, 2, 128, torch.bfloat16)
+    ref, raw = cuda_blockrank_attention_forward(Layer(), q, k, v, spans, 0.1, layers_to_return_scores=[0])
+    torch.cuda.synchronize()
+    bad = []
+
+    def work():
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(50):
+                o, r = cuda_blockrank_attention_forward(Layer(), q, k, v, spans, 0.1, layers_to_return_scores=[0])
+                bad.append(not (torch.equal(o, ref) and torch.equal(r, raw)))
+
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(bad) == 200 and not any(bad)
