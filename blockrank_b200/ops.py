@@ -62,7 +62,8 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, blk_start: torc
     tensor-core path.  Device-side problems (malformed spans, a wait that gave
     up) surface at the next :func:`check_status`.
     """
-    res = _lib.host().attention(q, k, v, blk_start, blk_len, scale, max_block_len, out, return_lse, algo, max_query_len, lse)
+    res = _lib.host().attention(q, k, v, blk_start, blk_len, scale, int(max_block_len), out, return_lse, algo,
+                                int(max_query_len), lse)
     return res if (return_lse or lse is not None) else res[0]
 
 
@@ -74,7 +75,7 @@ def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.
     q (B,N,S,D), k/v (B,Nk,S,D) as given to the forward; out / d_out (B,S,N,D); lse (B,N,S) fp32 from the
     forward.  Returns (dq (B,N,S,D), dk, dv (B,Nk,S,D)) in the input dtype; slots outside every block get zeros.
     """
-    return _lib.host().attention_bwd(q, k, v, out, d_out, lse, blk_start, blk_len, scale, max_block_len)
+    return _lib.host().attention_bwd(q, k, v, out, d_out, lse, blk_start, blk_len, scale, int(max_block_len))
 
 
 def doc_scores(q: torch.Tensor, k: torch.Tensor, blk_start: torch.Tensor, blk_len: torch.Tensor, rows: torch.Tensor,

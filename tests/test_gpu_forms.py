@@ -301,3 +301,10 @@ def test_calls_of_several_threads_on_streams_of_their_own():
     for t in threads:
         t.join()
     assert len(bad) == 200 and not any(bad)
+
+
+def test_sizes_may_be_any_number():
+    spans, q, k, v = packed([[9, 30, 41, 24]], 4, 2, 64, torch.bfloat16)
+    ref = ops.attention(q, k, v, spans[0], spans[1], 0.125, spans.max_block_len)
+    for size in (float(spans.max_block_len), torch.tensor(spans.max_block_len)):
+        assert torch.equal(ops.attention(q, k, v, spans[0], spans[1], torch.tensor(0.125), size), ref)
