@@ -47,6 +47,7 @@ class RankerConfig:
                             num_attention_heads=4, num_key_value_heads=2, head_dim=64, score_layer=score_layer)
 
 
+_STEPS = ("decoder_layer", "hidden_before_score_layer", "score", "score_from_hidden")  # methods that rank_host stands on
 _LAYER_WEIGHTS = ("ln1", "wqkv", "wo", "ln2", "wgu", "wd")  # of a full layer
 
 
@@ -143,7 +144,7 @@ class MistralPrefillRanker:
         B, S = input_ids.shape
         c = self.cfg
         pos = position_ids.reshape(B * S).to(torch.int32)
-        if self.events is None:  # the layers in one native call
+        if self.events is None and not self._overridden("decoder_layer"):  # the layers in one native call
             return _lib.host().hidden_states(
                 self.embed, input_ids, self._full_layers(), pos, self.inv_freq,
                 blk_start, blk_len, max_block_len, max_query_len, c.num_attention_heads, c.num_key_value_heads, c.head_dim,
@@ -231,7 +232,7 @@ class MistralPrefillRanker:
         ``block_spans`` int32 (2, B, M), ``signal_rows`` int32 (B, R) and ``max_block_len``.  Copies them to the
         device, scores, and returns (logits, top-k document indices) on the host."""
         c, host = self.cfg, _lib.host()
-        if not self.use_graphs and self.events is None:
+        if not self.use_graphs and self.events is None and not self._overridden(*_STEPS):
             last = self.layers[c.score_layer]
             return host.rank(self.embed, self._full_layers(), [last["ln1"], last["wq"], last["wk"]], self.inv_freq,
                              batch["input_ids"], batch["position_ids"], batch["block_spans"], batch["signal_rows"],
@@ -243,6 +244,10 @@ class MistralPrefillRanker:
         logits, _ = run(ids, pos, start, length, int(batch["max_block_len"]), rows, max_query_len)
         # (raises if a kernel reported malformed spans or a wait that gave up)
         return host.download(logits, k)
+
+    def _overridden(self, *steps) -> bool:
+        """Has a subclass, or somebody on this object, put another method in the place of one of ``steps``?"""
+        return any(s in self.__dict__ or getattr(type(self), s) is not getattr(MistralPrefillRanker, s) for s in steps)
 
     def _full_layers(self):
         return [[L[n] for n in _LAYER_WEIGHTS] for L in self.layers[:self.cfg.score_layer]]

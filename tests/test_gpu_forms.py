@@ -308,3 +308,20 @@ def test_sizes_may_be_any_number():
     ref = ops.attention(q, k, v, spans[0], spans[1], 0.125, spans.max_block_len)
     for size in (float(spans.max_block_len), torch.tensor(spans.max_block_len)):
         assert torch.equal(ops.attention(q, k, v, spans[0], spans[1], torch.tensor(0.125), size), ref)
+
+
+def test_overridden_steps_of_the_ranker_are_used():
+    from blockrank_b200.runner import MistralPrefillRanker
+    rk, batch = _requests(2, [30, 40, 50, 20, 4])
+    full = rk.rank_host(batch)[0]
+
+    class Halved(MistralPrefillRanker):
+        def decoder_layer(self, i, h, *args, **kwargs):
+            self.seen = getattr(self, "seen", 0) + 1
+            return super().decoder_layer(i, h, *args, **kwargs)
+
+    sub = Halved(rk.cfg, "cuda").init_random(seed=1)
+    assert torch.equal(sub.rank_host(batch)[0], full) and sub.seen == rk.cfg.score_layer
+    score = rk.score_from_hidden
+    rk.score_from_hidden = lambda *a, **kw: (score(*a, **kw)[0] + 1, None)
+    assert torch.equal(rk.rank_host(batch)[0], full + 1)
