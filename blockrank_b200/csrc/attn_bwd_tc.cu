@@ -817,7 +817,7 @@ __global__ void __launch_bounds__(256) attn_bwd_tc_finish_kernel(BwdTcArgs a) {
   }
 }
 
-int row_tiles(const brk_attn_bwd_params& p) { return (p.max_block_len * (p.N / p.Nk) + kTile - 1) / kTile; }
+int row_tiles(const brk_attn_bwd_params& p) { return (int)(((int64_t)p.max_block_len * (p.N / p.Nk) + kTile - 1) / kTile); }
 // Rows whose keys can span several key tiles need the fp32 dQ scratch.
 bool needs_part(const brk_attn_bwd_params& p) { return (int64_t)(p.M > 2 ? 2 : 1) * p.max_block_len > kTile; }
 size_t part_bytes(const brk_attn_bwd_params& p) {

@@ -1370,9 +1370,10 @@ int attn_prologue_launch(const brk_attn_params& p, int* hdr, float2* ml, int64_t
 // the 7B ranker turn into 2.4e-3 of its logits, for 467 us where this takes 478.
 static int tc_splits(const brk_attn_params& p) {
   if (p.M < 2) return 1;
+  const int G = std::max(1, p.N / std::max(1, p.Nk));
   int n = std::max(1, std::min(32, (p.S + 1023) / 1024));
   if (p.S > 640) {
-    const int tok2 = 2 * BM / std::max(1, p.N / p.Nk);
+    const int tok2 = std::max(1, 2 * BM / G);
     const int64_t pairs = (int64_t)p.B * p.Nk * ((query_rows(p) + tok2 - 1) / tok2);
     const int64_t blocks = (int64_t)p.B * p.Nk * (p.M - 1);
     if (3 * pairs * n <= 2 * sm_count() && 2 * blocks <= 3 * sm_count())

@@ -33,7 +33,7 @@ static int check_view(const brk_view& v, int dtype, const char* name) {
   return BRK_OK;
 }
 
-static int check_attn(const brk_attn_params* p) {
+static int check_attn_sizes(const brk_attn_params* p) {
   BRK_REQUIRE(p != nullptr, BRK_E_ARG, "params is null");
   BRK_REQUIRE(p->dtype == BRK_BF16 || p->dtype == BRK_F32, BRK_E_UNSUPPORTED, "dtype %d not supported", p->dtype);
   BRK_REQUIRE(p->B > 0 && p->N > 0 && p->Nk > 0 && p->S > 0 && p->M > 0, BRK_E_ARG,
@@ -42,10 +42,15 @@ static int check_attn(const brk_attn_params* p) {
   BRK_REQUIRE(p->D == 64 || p->D == 128, BRK_E_UNSUPPORTED, "head_dim %d not supported (64 or 128)", p->D);
   BRK_REQUIRE(p->max_block_len > 0 && p->max_block_len <= p->S, BRK_E_ARG, "max_block_len=%d out of range (S=%d)",
               p->max_block_len, p->S);
-  BRK_REQUIRE(p->blk_start && p->blk_len, BRK_E_ARG, "block spans are null");
   BRK_REQUIRE(p->max_query_len >= 0 && p->max_query_len <= p->S, BRK_E_ARG, "max_query_len=%d out of range (S=%d)",
               p->max_query_len, p->S);
-  int rc;
+  return BRK_OK;
+}
+
+static int check_attn(const brk_attn_params* p) {
+  int rc = check_attn_sizes(p);
+  if (rc) return rc;
+  BRK_REQUIRE(p->blk_start && p->blk_len, BRK_E_ARG, "block spans are null");
   if ((rc = check_view(p->q, p->dtype, "q"))) return rc;
   if ((rc = check_view(p->k, p->dtype, "k"))) return rc;
   if ((rc = check_view(p->v, p->dtype, "v"))) return rc;
@@ -90,6 +95,7 @@ int brk_spans_from_mask(const uint8_t* mask, int32_t B, int32_t M, int32_t H, in
 
 size_t brk_attn_fwd_workspace_bytes(const brk_attn_params* p) {
   if (p == nullptr) return 0;
+  if (check_attn_sizes(p) != BRK_OK) return kWsHeader;  // (the call refuses them: nothing is computed from such sizes)
   if (resolve_algo(p) == BRK_ALGO_TC) return attn_tc_workspace(*p);
   return p->dtype == BRK_F32 ? attn_f32_workspace(*p) : kWsHeader;
 }

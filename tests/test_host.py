@@ -228,3 +228,22 @@ def test_host_module_shares_the_process_c_plus_plus_library():
     path = os.path.join(os.path.dirname(_lib.LIB_PATH), "_host.so")
     dynamic = subprocess.run(["readelf", "-d", path], capture_output=True, text=True, check=True).stdout
     assert "[libstdc++.so.6]" in dynamic
+
+
+def test_forward_workspace_sizes():
+    """Sizes that the call refuses ask for no scratch (and divide nothing by zero)."""
+    L = _lib.lib()
+
+    def size(dtype, algo, B, N, Nk, D, S, M, longest):
+        p = _lib.AttnParams()
+        p.dtype, p.algo, p.B, p.N, p.Nk, p.D, p.S, p.M, p.max_block_len, p.scale = dtype, algo, B, N, Nk, D, S, M, longest, 0.1
+        return L.brk_attn_fwd_workspace_bytes(ctypes.byref(p))
+
+    for dtype in (_lib.BRK_BF16, _lib.BRK_F32):
+        for longest in (-5, 0, 4097, 10**9):
+            assert size(dtype, 0, 1, 8, 8, 64, 4096, 3, longest) == 256
+        assert size(dtype, 0, 1, 8, 0, 64, 4096, 3, 100) == 256
+        assert size(dtype, 0, 0, 8, 8, 64, 4096, 3, 100) == 256
+    assert size(_lib.BRK_BF16, _lib.ALGO_TC, 1, 512, 1, 64, 1024, 3, 512) > 0      # a group of 512 heads: refused by the call
+    # 20 documents of up to 160 tokens, fp32: header + 7 chunks of every row's output, max and sum
+    assert size(_lib.BRK_F32, 0, 1, 32, 8, 128, 22 * 160, 22, 160) == 256 + 32 * 160 * 7 * (128 * 4 + 8)
