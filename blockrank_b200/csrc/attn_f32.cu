@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f32_kernel(F32Args a) {
 }
 
 int chunks(const brk_attn_params& p) {
-  return p.M < 2 ? 1 : std::max(1, std::min(kMaxChunks, (p.S + kChunkKeys - 1) / kChunkKeys));
+  return p.M < 2 ? 1 : capped_chunks(p, std::max(1, std::min(kMaxChunks, (p.S + kChunkKeys - 1) / kChunkKeys)));
 }
 
 template <int D>

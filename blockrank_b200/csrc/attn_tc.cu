@@ -1379,7 +1379,7 @@ static int tc_splits(const brk_attn_params& p) {
     if (3 * pairs * n <= 2 * sm_count() && 2 * blocks <= 3 * sm_count())
       n = std::max(n, (int)std::min<int64_t>(std::min(32, (p.S + 255) / 256), sm_count() / std::max<int64_t>(1, pairs)));
   }
-  return n;
+  return p.D == 128 && G == 4 ? n : capped_chunks(p, n);  // (there the chunks are never fewer: see above)
 }
 
 // Header (work counter, span verdict), live windows of the query block's context, partials of its key chunks.

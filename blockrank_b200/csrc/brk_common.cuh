@@ -137,6 +137,12 @@ int attn_f32_launch(const brk_attn_params& p, void* ws, size_t ws_bytes, cudaStr
 inline int query_rows(const brk_attn_params& p) {
   return (p.max_query_len > 0 && p.max_query_len < p.max_block_len) ? p.max_query_len : p.max_block_len;
 }
+// Key chunks whose partial results (fp32 rows of the output, max and sum) stay within 512 MB: a query block long enough to exceed
+// that has row tiles for every SM without being cut (two blocks of 32,768 slots, fp32: 17 GB of partials in 32 chunks).
+inline int capped_chunks(const brk_attn_params& p, int n) {
+  const size_t chunk = (size_t)p.B * p.N * query_rows(p) * (p.D * sizeof(float) + sizeof(float2));
+  return n > 1 && chunk * n > (512u << 20) ? (int)((512u << 20) / chunk > 1 ? (512u << 20) / chunk : 1) : n;
+}
 size_t attn_tc_workspace(const brk_attn_params& p);
 size_t attn_bwd_workspace(const brk_attn_bwd_params& p);
 int attn_bwd_launch(const brk_attn_bwd_params& p, void* ws, size_t ws_bytes, cudaStream_t st);

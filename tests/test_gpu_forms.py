@@ -325,3 +325,17 @@ def test_overridden_steps_of_the_ranker_are_used():
     score = rk.score_from_hidden
     rk.score_from_hidden = lambda *a, **kw: (score(*a, **kw)[0] + 1, None)
     assert torch.equal(rk.rank_host(batch)[0], full + 1)
+
+
+@pytest.mark.parametrize("dtype,D,lens", [(torch.float32, 128, [512, 4096]), (torch.bfloat16, 64, [512, 8192])])
+def test_long_query_block_within_the_scratch_limit(dtype, D, lens):
+    """Partials of all chunks would exceed the limit: fewer chunks, the same result (heads of three KV heads against 64 bits)."""
+    N, Nk = 32, 8
+    spans, q, k, v = packed([lens], N, Nk, D, dtype)
+    out, lse = ops.attention(q, k, v, spans[0], spans[1], D ** -0.5, spans.max_block_len, return_lse=True)
+    for n in (0, 13, 31):
+        s = (q[0, n].double() @ k[0, n // 4].double().t()) * D ** -0.5
+        s = s.masked_fill(torch.ones_like(s, dtype=torch.bool).triu(1), float("-inf"))
+        ref = s.softmax(-1) @ v[0, n // 4].double()
+        assert (out[0, :, n].double() - ref).norm() <= (1e-6 if dtype == torch.float32 else 1.7e-3) * ref.norm()
+        assert (lse[0, n].double() - s.logsumexp(-1)).abs().max() < 1e-5

@@ -231,7 +231,8 @@ def test_host_module_shares_the_process_c_plus_plus_library():
 
 
 def test_forward_workspace_sizes():
-    """Sizes that the call refuses ask for no scratch (and divide nothing by zero)."""
+    """Sizes that the call refuses ask for no scratch (and divide nothing by zero); partials of key chunks stay bounded where
+    the call had needed none before."""
     L = _lib.lib()
 
     def size(dtype, algo, B, N, Nk, D, S, M, longest):
@@ -245,5 +246,7 @@ def test_forward_workspace_sizes():
         assert size(dtype, 0, 1, 8, 0, 64, 4096, 3, 100) == 256
         assert size(dtype, 0, 0, 8, 8, 64, 4096, 3, 100) == 256
     assert size(_lib.BRK_BF16, _lib.ALGO_TC, 1, 512, 1, 64, 1024, 3, 512) > 0      # a group of 512 heads: refused by the call
+    for dtype, N, Nk, D in ((_lib.BRK_F32, 32, 8, 128), (_lib.BRK_F32, 16, 8, 64), (_lib.BRK_BF16, 16, 8, 64), (_lib.BRK_BF16, 16, 2, 128)):
+        assert size(dtype, 0, 4, N, Nk, D, 65536, 2, 65536) <= (512 << 20) + (1 << 20)
     # 20 documents of up to 160 tokens, fp32: header + 7 chunks of every row's output, max and sum
     assert size(_lib.BRK_F32, 0, 1, 32, 8, 128, 22 * 160, 22, 160) == 256 + 32 * 160 * 7 * (128 * 4 + 8)
