@@ -64,8 +64,12 @@ static int resolve_algo(const brk_attn_params* p) {
   // its running maximum is taken before the scaling).  It carries the probabilities at the CUDA-core kernel's precision where
   // that kernel is the alternative (attn_tc_launch).  Against it: 1,023 -> 59 us and 901 -> 53 us per call on 4 prompts of 20
   // documents, head_dim 64, 8 heads on 8 and on one.
+  // A scale that is not positive goes to the CUDA cores, except in the one shape that has always been this kernel's, which
+  // refuses it as it did.
   const int G = p->Nk > 0 ? p->N / p->Nk : 0;
-  return (p->dtype == BRK_BF16 && (G == 1 || G == 2 || G == 4 || G == 8) && p->scale > 0.f) ? BRK_ALGO_TC : BRK_ALGO_SIMT;
+  return (p->dtype == BRK_BF16 && (G == 1 || G == 2 || G == 4 || G == 8) && (p->scale > 0.f || (p->D == 128 && G == 4)))
+             ? BRK_ALGO_TC
+             : BRK_ALGO_SIMT;
 }
 
 }  // namespace brk

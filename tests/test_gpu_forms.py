@@ -339,3 +339,16 @@ def test_long_query_block_within_the_scratch_limit(dtype, D, lens):
         ref = s.softmax(-1) @ v[0, n // 4].double()
         assert (out[0, :, n].double() - ref).norm() <= (1e-6 if dtype == torch.float32 else 1.7e-3) * ref.norm()
         assert (lse[0, n].double() - s.logsumexp(-1)).abs().max() < 1e-5
+
+
+def test_scales_that_are_not_positive():
+    """Refused where the tcgen05 kernel alone serves a shape, computed on CUDA cores elsewhere."""
+    for N, Nk, D, dtype, refused in ((8, 2, 128, torch.bfloat16, True), (8, 2, 64, torch.bfloat16, False), (8, 2, 128, torch.float32, False)):
+        spans, q, k, v = packed([[9, 30, 41, 24]], N, Nk, D, dtype)
+        call = lambda s: ops.attention(q, k, v, spans[0], spans[1], s, spans.max_block_len)
+        if refused:
+            with pytest.raises(ValueError, match="scale must be positive"):
+                call(-0.1)
+        else:  # the same logits with the sign on the queries
+            ref = ops.attention(-q, k, v, spans[0], spans[1], 0.1, spans.max_block_len)
+            assert (call(-0.1).double() - ref.double()).norm() <= 1e-3 * ref.double().norm()
