@@ -19,6 +19,7 @@ ERRORS = {-1: "BRK_E_ARG", -2: "BRK_E_UNSUPPORTED", -3: "BRK_E_WORKSPACE", -4: "
 
 EXPORTS = ("brk_version", "brk_last_error", "brk_device_check", "brk_spans_from_mask",
            "brk_attn_fwd_workspace_bytes", "brk_attn_fwd", "brk_attn_bwd_workspace_bytes", "brk_attn_bwd",
+           "brk_attn_bwd_reporting",
            "brk_status_poll", "brk_selftest_bounded_wait",
            "brk_doc_scores_workspace_bytes",
            "brk_doc_scores", "brk_doc_scores_static", "brk_raw_scores",
@@ -42,8 +43,7 @@ class AttnBwdParams(C.Structure):
     _fields_ = [("dtype", C.c_int32), ("B", C.c_int32), ("N", C.c_int32), ("Nk", C.c_int32), ("D", C.c_int32),
                 ("S", C.c_int32), ("M", C.c_int32), ("max_block_len", C.c_int32), ("scale", C.c_float),
                 ("q", View), ("k", View), ("v", View), ("o", View), ("d_o", View), ("lse", C.c_void_p),
-                ("blk_start", C.c_void_p), ("blk_len", C.c_void_p), ("dq", View), ("dk", View), ("dv", View),
-                ("status", C.c_void_p)]
+                ("blk_start", C.c_void_p), ("blk_len", C.c_void_p), ("dq", View), ("dk", View), ("dv", View)]
 
 
 class ScoreParams(C.Structure):
@@ -84,6 +84,8 @@ def lib() -> C.CDLL:
     L.brk_attn_bwd_workspace_bytes.argtypes = [C.POINTER(AttnBwdParams)]
     L.brk_attn_bwd.restype = C.c_int
     L.brk_attn_bwd.argtypes = [C.POINTER(AttnBwdParams), C.c_void_p, C.c_size_t, C.c_void_p]
+    L.brk_attn_bwd_reporting.restype = C.c_int
+    L.brk_attn_bwd_reporting.argtypes = [C.POINTER(AttnBwdParams), C.c_void_p, C.c_size_t, C.c_void_p, C.c_void_p]
     L.brk_status_poll.restype = C.c_int
     L.brk_status_poll.argtypes = [C.c_void_p, C.c_void_p]
     L.brk_selftest_bounded_wait.restype = C.c_int

@@ -30,7 +30,7 @@ size_t attn_bwd_workspace(const brk_attn_bwd_params& p) {
   return delta_bytes(p) + 2 * acc_bytes(p) + dq_last_bytes(p) + (attn_bwd_tc_supported(p) ? attn_bwd_tc_extra_bytes(p) : 0);
 }
 
-int attn_bwd_launch(const brk_attn_bwd_params& p, void* ws, size_t ws_bytes, cudaStream_t st) {
+int attn_bwd_launch(const brk_attn_bwd_params& p, void* ws, size_t ws_bytes, int32_t* status, cudaStream_t st) {
   BRK_REQUIRE(ws != nullptr && ws_bytes >= attn_bwd_workspace(p) && ((uintptr_t)ws & 15) == 0, BRK_E_WORKSPACE,
               "workspace %zu < %zu bytes (or not 16-byte aligned)", ws_bytes, attn_bwd_workspace(p));
   unsigned char* const w = static_cast<unsigned char*>(ws);
@@ -39,7 +39,7 @@ int attn_bwd_launch(const brk_attn_bwd_params& p, void* ws, size_t ws_bytes, cud
   float* const acc = reinterpret_cast<float*>(w + delta_bytes(p));
   unsigned char* const dq32 = w + delta_bytes(p) + 2 * acc_bytes(p);
   if (attn_bwd_tc_supported(p))
-    return attn_bwd_tc_launch(p, delta, acc, reinterpret_cast<float*>(dq32), dq32 + dq_last_bytes(p), st);
+    return attn_bwd_tc_launch(p, delta, acc, reinterpret_cast<float*>(dq32), dq32 + dq_last_bytes(p), status, st);
   BRK_CUDA(cudaMemsetAsync(acc, 0, 2 * acc_bytes(p) + dq_last_bytes(p), st));
   return attn_bwd_mma_launch(p, delta, acc, acc + acc_bytes(p) / sizeof(float), reinterpret_cast<float*>(dq32), st);
 }

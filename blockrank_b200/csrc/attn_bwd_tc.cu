@@ -869,14 +869,15 @@ size_t attn_bwd_tc_extra_bytes(const brk_attn_bwd_params& p) { return p.M > 2 ||
 
 // ws32: the two [B, Nk, S, D] accumulators of the warp-level kernels (used for the prefix sums here), then dq32; extra: the
 // bytes of attn_bwd_tc_extra_bytes (the item counter goes into the unused accumulators when there are none)
-int attn_bwd_tc_launch(const brk_attn_bwd_params& p, float* delta, float* ws32, float* dq32, void* extra, cudaStream_t st) {
+int attn_bwd_tc_launch(const brk_attn_bwd_params& p, float* delta, float* ws32, float* dq32, void* extra, int32_t* status,
+                       cudaStream_t st) {
   BwdTcArgs a{};
   a.q = make_view(p.q); a.k = make_view(p.k); a.v = make_view(p.v); a.o = make_view(p.o); a.d_o = make_view(p.d_o);
   a.dq = make_view(p.dq); a.dk = make_view(p.dk); a.dv = make_view(p.dv);
   a.lse = p.lse;
   a.delta = delta;
   a.blk_start = p.blk_start; a.blk_len = p.blk_len;
-  a.status = p.status;
+  a.status = status;
   a.B = p.B; a.N = p.N; a.Nk = p.Nk; a.S = p.S; a.M = p.M; a.G = p.N / p.Nk; a.max_block_len = p.max_block_len;
   while ((1 << a.g_shift) < a.G) ++a.g_shift;
   a.row_tiles = row_tiles(p);

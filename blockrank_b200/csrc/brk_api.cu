@@ -142,10 +142,14 @@ size_t brk_attn_bwd_workspace_bytes(const brk_attn_bwd_params* p) {
   return attn_bwd_workspace(*p);
 }
 
-int brk_attn_bwd(const brk_attn_bwd_params* p, void* workspace, size_t workspace_bytes, void* stream) {
+int brk_attn_bwd_reporting(const brk_attn_bwd_params* p, void* workspace, size_t workspace_bytes, int32_t* status, void* stream) {
   int rc = check_attn_bwd(p);
   if (rc) return rc;
-  return attn_bwd_launch(*p, workspace, workspace_bytes, (cudaStream_t)stream);
+  return attn_bwd_launch(*p, workspace, workspace_bytes, status, (cudaStream_t)stream);
+}
+
+int brk_attn_bwd(const brk_attn_bwd_params* p, void* workspace, size_t workspace_bytes, void* stream) {
+  return brk_attn_bwd_reporting(p, workspace, workspace_bytes, nullptr, stream);
 }
 
 int brk_status_poll(int32_t* status, void* stream) {

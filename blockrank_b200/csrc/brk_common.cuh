@@ -145,11 +145,12 @@ inline int capped_chunks(const brk_attn_params& p, int n) {
 }
 size_t attn_tc_workspace(const brk_attn_params& p);
 size_t attn_bwd_workspace(const brk_attn_bwd_params& p);
-int attn_bwd_launch(const brk_attn_bwd_params& p, void* ws, size_t ws_bytes, cudaStream_t st);
+int attn_bwd_launch(const brk_attn_bwd_params& p, void* ws, size_t ws_bytes, int32_t* status, cudaStream_t st);
 int attn_bwd_f32_launch(const brk_attn_bwd_params& p, float* delta, cudaStream_t st);
 bool attn_bwd_tc_supported(const brk_attn_bwd_params& p);
 size_t attn_bwd_tc_extra_bytes(const brk_attn_bwd_params& p);
-int attn_bwd_tc_launch(const brk_attn_bwd_params& p, float* delta, float* ws32, float* dq32, void* extra, cudaStream_t st);
+int attn_bwd_tc_launch(const brk_attn_bwd_params& p, float* delta, float* ws32, float* dq32, void* extra, int32_t* status,
+                       cudaStream_t st);
 int attn_bwd_mma_launch(const brk_attn_bwd_params& p, float* delta, float* dk32, float* dv32, float* dq32, cudaStream_t st);
 int sm_count();
 

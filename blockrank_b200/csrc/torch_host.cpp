@@ -209,10 +209,10 @@ std::tuple<Tensor, Tensor, Tensor> attention_bwd(const Tensor& q, const Tensor& 
   p.blk_start = (const int32_t*)bs.data_ptr();
   p.blk_len = (const int32_t*)bl.data_ptr();
   p.dq = view_of(dq); p.dk = view_of(dk); p.dv = view_of(dv);
-  p.status = (int32_t*)status_word(q.get_device()).data_ptr();
   const size_t nbytes = brk_attn_bwd_workspace_bytes(&p);
   Tensor ws = scratch(nbytes, q);
-  check(brk_attn_bwd(&p, ws.data_ptr(), nbytes, stream_of(q)), "brk_attn_bwd");
+  check(brk_attn_bwd_reporting(&p, ws.data_ptr(), nbytes, (int32_t*)status_word(q.get_device()).data_ptr(), stream_of(q)),
+        "brk_attn_bwd");
   count(3);  // dq (+ delta), dk/dv accumulation, conversion of the accumulators
   return {dq, dk, dv};
 }

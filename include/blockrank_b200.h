@@ -34,7 +34,7 @@
 extern "C" {
 #endif
 
-#define BRK_VERSION 102
+#define BRK_VERSION 103
 
 #if defined(__GNUC__)
 #define BRK_API __attribute__((visibility("default")))
@@ -139,12 +139,15 @@ typedef struct brk_attn_bwd_params {
   const int32_t* blk_start;
   const int32_t* blk_len;
   brk_view dq, dk, dv;    /* written through their strides; dk, dv: (B, Nk, S, D) views */
-  int32_t* status;        /* optional device word (bf16: a bounded wait that gave up); see brk_status_poll */
 } brk_attn_bwd_params;
 
 /* fp32 scratch: the rows' dot(d_o, o), the dk / dv accumulators and (bf16) the last block's dq; cleared by the call */
 BRK_API size_t brk_attn_bwd_workspace_bytes(const brk_attn_bwd_params* p);
 BRK_API int brk_attn_bwd(const brk_attn_bwd_params* p, void* workspace, size_t workspace_bytes, void* stream);
+/* The same with a status word as the forward has it (a device word or NULL; bf16: a bounded wait that gave up, see
+ * brk_status_poll).  The structures of this header do not change from one version to the next. */
+BRK_API int brk_attn_bwd_reporting(const brk_attn_bwd_params* p, void* workspace, size_t workspace_bytes, int32_t* status,
+                                   void* stream);
 
 /* Device-side status.  The kernels never trap: a bounded wait that gives up, or malformed block spans, set
  * the caller's status word (brk_attn_params.status; first event wins) and the kernel returns normally.

@@ -250,3 +250,18 @@ def test_forward_workspace_sizes():
         assert size(dtype, 0, 4, N, Nk, D, 65536, 2, 65536) <= (512 << 20) + (1 << 20)
     # 20 documents of up to 160 tokens, fp32: header + 7 chunks of every row's output, max and sum
     assert size(_lib.BRK_F32, 0, 1, 32, 8, 128, 22 * 160, 22, 160) == 256 + 32 * 160 * 7 * (128 * 4 + 8)
+
+
+def test_structures_of_the_c_abi_keep_their_size(tmp_path):
+    """A caller compiled against an earlier header passes structures of these sizes."""
+    import shutil
+    sizes = {"brk_view": 32, "brk_attn_params": 208, "brk_attn_bwd_params": 320, "brk_score_params": 144}
+    python = {"brk_view": _lib.View, "brk_attn_params": _lib.AttnParams, "brk_attn_bwd_params": _lib.AttnBwdParams,
+              "brk_score_params": _lib.ScoreParams}
+    assert {n: ctypes.sizeof(t) for n, t in python.items()} == sizes
+    cc = shutil.which("cc") or shutil.which("gcc")
+    if cc is None:
+        pytest.skip("no C compiler")
+    src = tmp_path / "sizes.c"
+    src.write_text('#include "blockrank_b200.h"\n' + "".join(f"_Static_assert(sizeof({n}) == {v}, \"{n}\");\n" for n, v in sizes.items()))
+    subprocess.run([cc, "-fsyntax-only", "-I", os.path.join(ROOT, "include"), str(src)], check=True)
