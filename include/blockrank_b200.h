@@ -128,7 +128,9 @@ BRK_API int brk_attn_fwd(const brk_attn_params* p, void* workspace, size_t works
  * Inputs are the forward's q, k, v, its output o and its lse ([B, N, S], natural log) and the gradient d_o of o
  * (same layout as o).  Outputs dq (like q), dk and dv (like k, v; summed over the query heads of each KV group);
  * slots outside every block get zero gradients.  bf16: tcgen05 (fp32 accumulation; warp-level MMA for blocks of more than 16 row tiles of 128 / (N / Nk) tokens);
- * fp32: CUDA cores (there N / Nk must divide 64). */
+ * fp32: CUDA cores (there N / Nk must divide 64).
+ * Sums that several thread blocks contribute to -- the prefix block's dk and dv, dq of the last block and, in fp32, dq of
+ * rows that see more than 128 keys -- are added up in no fixed order: they can differ in the last bits from call to call. */
 typedef struct brk_attn_bwd_params {
   int32_t dtype;          /* BRK_BF16 or BRK_F32 (q, k, v, o, d_o, dq, dk, dv share it) */
   int32_t B, N, Nk, D;    /* D = 64 or 128 */

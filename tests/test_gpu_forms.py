@@ -352,3 +352,29 @@ def test_scales_that_are_not_positive():
         else:  # the same logits with the sign on the queries
             ref = ops.attention(-q, k, v, spans[0], spans[1], 0.1, spans.max_block_len)
             assert (call(-0.1).double() - ref.double()).norm() <= 1e-3 * ref.double().norm()
+
+
+@pytest.mark.parametrize("N,Nk,D,lens", [(8, 1, 64, [[64] + [140] * 20 + [48]]), (8, 2, 128, [[64, 700, 650, 48]]), (8, 8, 128, [[64, 30, 35, 28, 48]] * 2)])
+def test_fp32_gradients_stay_close_to_64_bits(N, Nk, D, lens):
+    """Sums of hundreds of rows in fp32, each product rounded once: errors of the gradients, and of the output, against fp64
+    autograd.  Bounds: 10 % above those of sums taken in parts of D / 4 and of 64 rows (one long sum: up to 1.4e-6)."""
+    spans, q, k, v = packed(lens, N, Nk, D, torch.float32, seed=5)
+    leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    out, _ = cuda_blockrank_attention_forward(Layer(), *leaves, spans, D ** -0.5)
+    go = torch.randn(out.shape, generator=torch.Generator(device="cuda").manual_seed(9), device="cuda")
+    exact = [t.detach().double().requires_grad_(True) for t in leaves]
+    start, ln = spans[0].tolist(), spans[1].tolist()
+    S, M = q.shape[2], len(lens[0])
+    ok = torch.zeros(len(lens), S, S, dtype=torch.bool, device="cuda")
+    for b in range(len(lens)):
+        for m in range(M):
+            s, e = start[b][m], start[b][m] + ln[b][m]
+            ok[b, s:e, s:e] = torch.ones(e - s, e - s, dtype=torch.bool, device="cuda").tril()
+            if m > 0:
+                ok[b, s:e, :ln[b][0] if m < M - 1 else s] = True
+    logits = (exact[0] @ exact[1].repeat_interleave(N // Nk, 1).transpose(-1, -2)) * D ** -0.5
+    p = logits.masked_fill(~ok[:, None], float("-inf")).softmax(-1).nan_to_num(0.0)
+    ref = (p @ exact[2].repeat_interleave(N // Nk, 1)).transpose(1, 2)
+    assert (out.detach().double() - ref.detach()).norm() <= 3.4e-7 * ref.detach().norm()
+    for got, want, bound in zip(torch.autograd.grad(out, leaves, go), torch.autograd.grad(ref, exact, go.double()), (3.95e-7, 4.05e-7, 3.8e-7)):
+        assert (got.double() - want).norm() <= bound * want.norm()
