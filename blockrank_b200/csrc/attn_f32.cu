@@ -6,12 +6,12 @@
 // packed two head_dim elements per fma.rn.f32x2) and of the output (4 x D / 16).  The kernel is bound by the FMA pipe and
 // by the latency in front of it: an inner step of 64 FMAs reads 8 16-byte pieces of shared memory, 12 wavefronts per warp.
 // Two CTAs share an SM (101 KB each), so one computes while the other loads or exponentiates.  (Tiles of 8 x 4 need fewer
-// wavefronts per FMA but leave two warps per scheduler: 399 us where this takes 351.)
+// wavefronts per FMA but leave two warps per scheduler: 399 us where this took 351.)
 //
 // The query block's context is cut into chunks of about 512 keys whose partial results attn_combine_kernel merges: its
 // rows see thousands of keys where a document's see a few hundred, and as single CTAs they were the tail of the launch.
 //
-// One prompt of 20 documents (32/8 heads, head_dim 128, 8.4 GFLOP visible): 351 us; one query row per four threads with
+// One prompt of 20 documents (32/8 heads, head_dim 128, 8.4 GFLOP visible): 360 us (351 with one sum over head_dim); one query row per four threads with
 // the keys re-read from shared memory for every row took 1,790 us.
 #include <algorithm>
 
@@ -169,16 +169,19 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f32_kernel(F32Args a) {
     }
     cp_async_wait<1>();
     __syncthreads();
-    // scores: rows ty + 8 i, keys tx + 16 c
+    // scores: rows ty + 16 i, keys tx + 16 c, in sums of 32 products (of 64 at head_dim 128, the output of short prompts was 5 %
+    // further from 64 bits than the kernel before this one's)
+    constexpr int kParts = D / 64;
     float s[kR][4];
-    {
+#pragma unroll
+    for (int h = 0; h < kParts; ++h) {
       ptx::f32x2 acc[kR][4];
 #pragma unroll
       for (int i = 0; i < kR; ++i)
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[i][c] = 0ull;
 #pragma unroll 1
-      for (int d = 0; d < D; d += 4) {
+      for (int d = h * 64; d < (h + 1) * 64; d += 4) {
         ulonglong2 kk[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) kk[c] = *reinterpret_cast<const ulonglong2*>(ks + (tx + 16 * c) * kPitch + d);
@@ -195,7 +198,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f32_kernel(F32Args a) {
         for (int c = 0; c < 4; ++c) {
           float x, y;
           ptx::unpack2(acc[i][c], x, y);
-          s[i][c] = x + y;
+          s[i][c] = h ? s[i][c] + (x + y) : x + y;
         }
     }
 #pragma unroll

@@ -375,6 +375,6 @@ def test_fp32_gradients_stay_close_to_64_bits(N, Nk, D, lens):
     logits = (exact[0] @ exact[1].repeat_interleave(N // Nk, 1).transpose(-1, -2)) * D ** -0.5
     p = logits.masked_fill(~ok[:, None], float("-inf")).softmax(-1).nan_to_num(0.0)
     ref = (p @ exact[2].repeat_interleave(N // Nk, 1)).transpose(1, 2)
-    assert (out.detach().double() - ref.detach()).norm() <= 3.4e-7 * ref.detach().norm()
+    assert (out.detach().double() - ref.detach()).norm() <= 3e-7 * ref.detach().norm()
     for got, want, bound in zip(torch.autograd.grad(out, leaves, go), torch.autograd.grad(ref, exact, go.double()), (3.95e-7, 4.05e-7, 3.8e-7)):
         assert (got.double() - want).norm() <= bound * want.norm()
