@@ -17,7 +17,7 @@ ALGO_AUTO, ALGO_SIMT, ALGO_TC = 0, 1, 2
 ERRORS = {-1: "BRK_E_ARG", -2: "BRK_E_UNSUPPORTED", -3: "BRK_E_WORKSPACE", -4: "BRK_E_CUDA",
           -5: "BRK_E_DEVICE", -6: "BRK_E_TIMEOUT"}
 
-EXPORTS = ("brk_version", "brk_last_error", "brk_device_check", "brk_spans_from_mask",
+EXPORTS = ("brk_version", "brk_last_error", "brk_launch_count", "brk_device_check", "brk_spans_from_mask",
            "brk_attn_fwd_workspace_bytes", "brk_attn_fwd", "brk_attn_bwd_workspace_bytes", "brk_attn_bwd",
            "brk_attn_bwd_reporting",
            "brk_status_poll", "brk_selftest_bounded_wait",
@@ -73,6 +73,7 @@ def lib() -> C.CDLL:
     L = C.CDLL(LIB_PATH)
     L.brk_version.restype = C.c_int
     L.brk_last_error.restype = C.c_char_p
+    L.brk_launch_count.restype = C.c_int64
     L.brk_device_check.restype = C.c_int
     L.brk_spans_from_mask.restype = C.c_int
     L.brk_spans_from_mask.argtypes = [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]

@@ -285,7 +285,7 @@ int launch(const BwdF32Args& a, cudaStream_t st) {
   constexpr int smem = (4 * kTile * (D + 4) + 2 * kTile * kPitchS) * (int)sizeof(float);
   BRK_CUDA(cudaFuncSetAttribute(attn_bwd_f32_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   attn_bwd_f32_kernel<D><<<dim3((unsigned)(a.key_tiles * a.M), (unsigned)(a.B * a.Nk)), kThreads, smem, st>>>(a);
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return BRK_OK;
 }
 
@@ -307,7 +307,7 @@ int attn_bwd_f32_launch(const brk_attn_bwd_params& p, float* delta, cudaStream_t
   BRK_REQUIRE(p.B * p.Nk <= 65535 && (int64_t)a.key_tiles * p.M < (1ll << 31) && (rows + 7) / 8 < (1ll << 31), BRK_E_UNSUPPORTED,
               "grid too large: B*Nk=%d M=%d", p.B * p.Nk, p.M);
   attn_bwd_f32_prep_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(a, p.D);
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return p.D == 128 ? launch<128>(a, st) : launch<64>(a, st);
 }
 

@@ -488,16 +488,16 @@ int launch_mma(BwdMmaArgs a, cudaStream_t st) {
   // the last block first: its CTAs are the long ones
   a.ksplit = std::max(1, std::min(32, (a.S / kT) / 8));
   attn_bwd_dq_mma_kernel<D, true><<<dim3(tiles, a.ksplit, a.B * a.N), kThreadsM, smem_dq, st>>>(a);
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   if (a.M > 1) {
     attn_bwd_dq_mma_kernel<D, false><<<dim3(tiles, a.M - 1, a.B * a.N), kThreadsM, smem_dq, st>>>(a);
-    BRK_CUDA(cudaGetLastError());
+    BRK_LAUNCHED();
   }
   {
     const int64_t n8 = (int64_t)a.B * a.N * a.max_block_len * (D / 8);
     const int blocks = (int)std::min<int64_t>((n8 + 255) / 256, 148 * 8);
     attn_bwd_store_dq_last_kernel<D><<<std::max(blocks, 1), 256, 0, st>>>(a);
-    BRK_CUDA(cudaGetLastError());
+    BRK_LAUNCHED();
   }
   const int smem = (2 + 2 * kRowBufs) * (int)sizeof(MmaTile<D>) + 2 * kRowBufs * kT * (int)sizeof(float);
   BRK_CUDA(cudaFuncSetAttribute(attn_bwd_dkv_mma_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -505,16 +505,16 @@ int launch_mma(BwdMmaArgs a, cudaStream_t st) {
   a.m_base = 0;
   a.nsplit = a.M > 2 ? std::min(a.M, 64) : 1;
   attn_bwd_dkv_mma_kernel<D><<<dim3(tiles, 1, a.B * a.Nk * a.nsplit), kThreadsM, smem, st>>>(a);
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   if (a.M > 1) {
     a.m_base = 1;
     a.nsplit = 2;
     attn_bwd_dkv_mma_kernel<D><<<dim3(tiles, a.M - 1, a.B * a.Nk * a.nsplit), kThreadsM, smem, st>>>(a);
-    BRK_CUDA(cudaGetLastError());
+    BRK_LAUNCHED();
   }
   const int64_t n4 = (int64_t)a.B * a.Nk * a.S * (D / 4);
   attn_bwd_store_kernel<<<(unsigned)std::min<int64_t>((n4 + 255) / 256, 148 * 16), 256, 0, st>>>(a, D);
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return BRK_OK;
 }
 

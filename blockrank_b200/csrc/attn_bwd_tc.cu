@@ -841,16 +841,16 @@ int launch(const brk_attn_bwd_params& p, BwdTcArgs a, float4* zero, int64_t n_ze
   if (a.pre && (rc = make_tmap_f32(&t.pre, a.pre, HD, 2 * p.B * p.Nk, p.max_block_len, 1, mbl * HD, HD, 0, 1, 32))) return rc;
   const unsigned prep = (unsigned)p.B * ((p.S + kPrepTok - 1) / kPrepTok) + (a.order ? 1 : 0);
   attn_bwd_tc_prep_kernel<HD><<<prep, 256, 0, st>>>(a, zero, n_zero);
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   BRK_CUDA(cudaFuncSetAttribute(attn_bwd_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Geo<HD>::kSmem));
   const int sms = sm_count();
   BRK_REQUIRE(sms > 0, BRK_E_CUDA, "could not read the SM count");
   attn_bwd_tc_kernel<HD><<<std::min(sms, a.total_items), kThreads, Geo<HD>::kSmem, st>>>(t, a);
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   if (p.M > 1) {
     const int64_t n = (int64_t)p.B * (p.N + (a.pre ? 2 * p.Nk : 0)) * p.max_block_len * (HD / 8);
     attn_bwd_tc_finish_kernel<HD><<<(unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8), 256, 0, st>>>(a);
-    BRK_CUDA(cudaGetLastError());
+    BRK_LAUNCHED();
   }
   return BRK_OK;
 }

@@ -183,7 +183,7 @@ int launch_g(const brk_attn_params& p, const SimtArgs& a, cudaStream_t st) {
       set_error("SIMT attention supports N/Nk in {1,2,4,8}, got %d", G);
       return BRK_E_UNSUPPORTED;
   }
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return BRK_OK;
 }
 

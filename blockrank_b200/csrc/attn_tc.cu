@@ -1255,7 +1255,7 @@ __global__ void selftest_wait_kernel(int32_t* status, uint32_t budget) {
 
 int selftest_wait_launch(int32_t* status, uint32_t budget, cudaStream_t st) {
   selftest_wait_kernel<<<1, 1, 0, st>>>(status, budget);
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return BRK_OK;
 }
 
@@ -1354,7 +1354,7 @@ int attn_prologue_launch(const brk_attn_params& p, int* hdr, float2* ml, int64_t
   const unsigned blocks = (unsigned)(n_ml > 0 ? (n_ml + 255) / 256 : 1) + (win ? p.B : 0);
   attn_prologue_kernel<<<blocks, 256, 0, st>>>(p.blk_start, p.blk_len, p.B, p.M, p.S, p.max_block_len, p.max_query_len,
                                                hdr, p.status, ml, n_ml, win, n_live, win_pitch);
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return BRK_OK;
 }
 

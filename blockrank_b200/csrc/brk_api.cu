@@ -7,6 +7,7 @@
 
 namespace brk {
 
+std::atomic<int64_t> g_launches{0};
 static thread_local char g_err[512] = "";
 
 void set_error(const char* fmt, ...) {
@@ -81,6 +82,8 @@ extern "C" {
 int brk_version(void) { return BRK_VERSION; }
 
 const char* brk_last_error(void) { return g_err; }
+
+int64_t brk_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 
 int brk_device_check(void) {
   int dev = 0, major = 0;

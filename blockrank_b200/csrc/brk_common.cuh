@@ -5,6 +5,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #include "../../include/blockrank_b200.h"
 
 namespace brk {
@@ -26,6 +28,15 @@ void set_error(const char* fmt, ...);
       ::brk::set_error("%s failed: %s", #expr, cudaGetErrorString(e_));            \
       return BRK_E_CUDA;                                                           \
     }                                                                              \
+  } while (0)
+
+// Kernels enqueued by this process; every launch below counts itself.
+extern std::atomic<int64_t> g_launches;
+// behind a <<<>>> launch
+#define BRK_LAUNCHED()                                                             \
+  do {                                                                             \
+    BRK_CUDA(cudaGetLastError());                                                  \
+    ::brk::g_launches.fetch_add(1, std::memory_order_relaxed);                     \
   } while (0)
 
 // ---- element access helpers -------------------------------------------------
@@ -106,6 +117,7 @@ int launch_dependent(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t 
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   BRK_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  g_launches.fetch_add(1, std::memory_order_relaxed);
   return BRK_OK;
 }
 

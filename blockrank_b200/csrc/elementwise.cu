@@ -227,14 +227,14 @@ __global__ void __launch_bounds__(256) rank_pack_kernel(const float* __restrict_
 int rank_pack_launch(const float* logits, int B, int nd, int k, float* out, int64_t* top, const int32_t* status,
                      int32_t* status_out, cudaStream_t st) {
   rank_pack_kernel<<<B, 256, 0, st>>>(logits, nd, k, out, top, status, status_out);
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return BRK_OK;
 }
 
 int signal_rows_launch(const void* x, int row_bytes, const int32_t* pos, const int32_t* rows, int B, int S, int R, void* x_out,
                        int32_t* pos_out, int32_t* local, int32_t* status, cudaStream_t st) {
   signal_rows_kernel<<<B * R, 128, 0, st>>>((const uint4*)x, row_bytes / 16, pos, rows, S, R, (uint4*)x_out, pos_out, local, status);
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return BRK_OK;
 }
 
@@ -242,7 +242,7 @@ int spans_launch(const uint8_t* mask, int B, int M, int H, int32_t* start, int32
   const int total = B * M;
   const int warps = 8;
   spans_kernel<<<(total + warps - 1) / warps, warps * 32, 0, st>>>(mask, total, M, H, start, len);
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return BRK_OK;
 }
 
@@ -256,7 +256,7 @@ int rmsnorm_launch(int dtype, const void* x, void* residual, const void* w, void
     else
       rmsnorm_reg_kernel<float><<<(unsigned)rows, threads, 0, st>>>((const float*)x, (float*)residual, (const float*)w,
                                                                   (float*)out, hidden, eps);
-    BRK_CUDA(cudaGetLastError());
+    BRK_LAUNCHED();
     return BRK_OK;
   }
   const size_t sm = (size_t)hidden * 4;
@@ -271,7 +271,7 @@ int rmsnorm_launch(int dtype, const void* x, void* residual, const void* w, void
     rmsnorm_kernel<float><<<(unsigned)rows, 256, sm, st>>>((const float*)x, (float*)residual, (const float*)w,
                                                           (float*)out, hidden, eps);
   }
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return BRK_OK;
 }
 
@@ -290,7 +290,7 @@ int rope_launch(int dtype, void* q, int64_t q_rs, int N, void* k, int64_t k_rs, 
                                                          inv_freq, T, per);
   else
     rope_kernel<float><<<grid, threads, 0, st>>>((float*)q, q_rs, N, (float*)k, k_rs, Nk, D, pos, inv_freq, T, per);
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return BRK_OK;
 }
 
@@ -308,7 +308,7 @@ int silu_mul_launch(int dtype, const void* gu, void* out, int64_t rows, int inte
     if (vec == 16) silu_mul_kernel<float, 16><<<blocks, threads, 0, st>>>((const float*)gu, (float*)out, rows, inter);
     else silu_mul_kernel<float, 8><<<blocks, threads, 0, st>>>((const float*)gu, (float*)out, rows, inter);
   }
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return BRK_OK;
 }
 

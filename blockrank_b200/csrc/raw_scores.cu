@@ -560,7 +560,7 @@ int raw_scores_launch(const brk_score_params& p, void* out, cudaStream_t st) {
       raw_scores_f32_kernel<64><<<grid, kThreadsF, sm, st>>>(a, (float*)out, neg);
     }
   }
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return BRK_OK;
 }
 
@@ -600,7 +600,7 @@ int raw_scores_bwd_launch(const brk_score_params& p, const void* d_raw, const br
     auto go = [&](auto kern, size_t sm) -> int {
       BRK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
       kern<<<grid, kThreads, sm, st>>>(a);
-      BRK_CUDA(cudaGetLastError());
+      BRK_LAUNCHED();
       return BRK_OK;
     };
     rc = p.D == 128 ? go(raw_bwd_mma_kernel<128>, sizeof(MmaTile<128>) + 2 * sizeof(RawBwdStage<128>))
@@ -613,14 +613,14 @@ int raw_scores_bwd_launch(const brk_score_params& p, const void* d_raw, const br
     auto go = [&](auto kern) -> int {
       BRK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
       kern<<<grid, kThreadsF, sm, st>>>(a);
-      BRK_CUDA(cudaGetLastError());
+      BRK_LAUNCHED();
       return BRK_OK;
     };
     rc = p.D == 128 ? go(raw_bwd_f32_kernel<128>) : go(raw_bwd_f32_kernel<64>);
     if (rc) return rc;
     raw_bwd_rows_kernel<float><<<rows_grid, 256, 0, st>>>(a, p.D);
   }
-  BRK_CUDA(cudaGetLastError());
+  BRK_LAUNCHED();
   return BRK_OK;
 }
 

@@ -439,7 +439,7 @@ static int doc_scores_run(const brk_score_params& p, void* ws, size_t ws_bytes, 
     // (the kernels also hold a few KB of static shared memory, which counts against the same 48 KB default)
     if (sm + 8192 > 48 * 1024) BRK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     kern<<<grid, kThreads, sm, st>>>(a);
-    BRK_CUDA(cudaGetLastError());
+    BRK_LAUNCHED();
     return BRK_OK;
   };
   if (p.dtype == BRK_BF16) {
@@ -459,7 +459,7 @@ static int doc_scores_run(const brk_score_params& p, void* ws, size_t ws_bytes, 
                                     (int)cudaSharedmemCarveoutMaxShared));
       doc_partial_mma_kernel<64><<<grid_docs, kThreads, 0, st>>>(a);
     }
-    BRK_CUDA(cudaGetLastError());
+    BRK_LAUNCHED();
     return BRK_OK;
   }
   return p.D == 128 ? launch(doc_partial_kernel<float, 128>) : launch(doc_partial_kernel<float, 64>);

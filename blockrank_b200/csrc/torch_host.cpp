@@ -16,7 +16,6 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
 
-#include <atomic>
 #include <mutex>
 #include <optional>
 #include <string>
@@ -66,9 +65,6 @@ void need_cuda(std::initializer_list<const Tensor*> ts) {
       TORCH_CHECK(t->is_cuda(), "blockrank_b200 kernels run on CUDA tensors only (there is no CPU path)");
 }
 const Tensor* opt(const OptTensor& t) { return t.has_value() ? &*t : nullptr; }
-
-std::atomic<int64_t> g_launches{0};  // kernels launched through this module
-void count(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
 // ---- parameter building -----------------------------------------------------------------------
 int dtype_code(const Tensor& t) {
@@ -134,7 +130,6 @@ std::tuple<Tensor, Tensor> spans_from_mask(const Tensor& mask) {
   check(brk_spans_from_mask((const uint8_t*)m8.data_ptr(), (int)m8.size(0), (int)m8.size(1), (int)m8.size(2),
                             (int32_t*)start.data_ptr(), (int32_t*)len.data_ptr(), stream_of(m8)),
         "brk_spans_from_mask");
-  count(1);
   return {start, len};
 }
 
@@ -172,9 +167,6 @@ std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Ten
   const size_t nbytes = brk_attn_fwd_workspace_bytes(&p);
   Tensor ws = scratch(nbytes, q);
   check(brk_attn_fwd(&p, ws.data_ptr(), nbytes, stream_of(q)), "brk_attn_fwd");
-  // span check / reset kernel + main kernel [+ merge of the key-chunked query block on the tensor-core path]
-  // (partials of key chunks come on top of the header and the 16 bytes per 64 slots of the list of windows)
-  count(nbytes > 512 + (size_t)(B * (S / 64 + 2)) * 16 ? 3 : 2);
   return {out, lse};
 }
 
@@ -213,7 +205,6 @@ std::tuple<Tensor, Tensor, Tensor> attention_bwd(const Tensor& q, const Tensor& 
   Tensor ws = scratch(nbytes, q);
   check(brk_attn_bwd_reporting(&p, ws.data_ptr(), nbytes, (int32_t*)status_word(q.get_device()).data_ptr(), stream_of(q)),
         "brk_attn_bwd");
-  count(3);  // dq (+ delta), dk/dv accumulation, conversion of the accumulators
   return {dq, dk, dv};
 }
 
@@ -254,7 +245,6 @@ std::tuple<Tensor, Tensor> doc_scores(const Tensor& q, const Tensor& k, const Te
   const size_t nbytes = brk_doc_scores_workspace_bytes(&p);
   Tensor ws = scratch(nbytes > 8 ? nbytes : 8, q);
   check(brk_doc_scores(&p, ws.data_ptr(), nbytes, stream_of(q)), "brk_doc_scores");
-  count(1);  // per-document partials; the CTA that completes a prompt also writes its masses and logits
   return {mass, logits};
 }
 
@@ -270,7 +260,6 @@ Tensor raw_scores(const Tensor& q, const Tensor& k, const Tensor& blk_start, con
   brk_score_params p = score_params(q, k, bs, bl, scale, R, 0.05);
   Tensor out = at::empty({B, N, R, S}, q.options().requires_grad(false));
   check(brk_raw_scores(&p, out.data_ptr(), stream_of(q)), "brk_raw_scores");
-  count(1);
   return out;
 }
 
@@ -293,7 +282,6 @@ std::tuple<Tensor, Tensor> raw_scores_bwd(const Tensor& q, const Tensor& k, cons
   Tensor ws = scratch(nbytes, q);
   check(brk_raw_scores_bwd(&p, d_raw.data_ptr(), &vq, &vk, add ? 1 : 0, ws.data_ptr(), nbytes, stream_of(q)),
         "brk_raw_scores_bwd");
-  count(2);
   return {dq, dk};
 }
 
@@ -419,7 +407,6 @@ Tensor rmsnorm(const Tensor& x, const Tensor& weight, double eps, const OptTenso
   check(brk_rmsnorm(dtype_code(x), x.data_ptr(), residual.has_value() ? residual->data_ptr() : nullptr, weight.data_ptr(),
                     out.data_ptr(), rows, (int32_t)hidden, (float)eps, stream_of(x)),
         "brk_rmsnorm");
-  count(1);
   return out;
 }
 
@@ -441,7 +428,6 @@ void rope_(const OptTensor& q, const OptTensor& k, const Tensor& pos, const Tens
                  k.has_value() ? k->stride(0) : 0, k.has_value() ? (int32_t)k->size(1) : 0, (int32_t)D,
                  (const int32_t*)pos.data_ptr(), (const float*)inv_freq.data_ptr(), T, stream_of(ref)),
         "brk_rope");
-  count(1);
 }
 
 Tensor silu_mul(const Tensor& gate_up, const OptTensor& out_in) {
@@ -459,7 +445,6 @@ Tensor silu_mul(const Tensor& gate_up, const OptTensor& out_in) {
   }
   check(brk_silu_mul(dtype_code(gate_up), gate_up.data_ptr(), out.data_ptr(), rows, (int32_t)inter, stream_of(gate_up)),
         "brk_silu_mul");
-  count(1);
   return out;
 }
 
@@ -577,7 +562,6 @@ std::tuple<Tensor, Tensor, Tensor> score_qk(const Tensor& h, const Tensor& pos, 
                         (int32_t*)ps.data_ptr(), (int32_t*)local.data_ptr(), (int32_t*)status_word(x.get_device()).data_ptr(),
                         stream_of(x)),
         "brk_signal_rows");
-  count(1);
   Tensor q = mm_nt(xs, wq);
   rope_(q.view({B * R, N, D}), std::nullopt, ps, inv_freq);
   rope_(std::nullopt, k.view({T, Nk, D}), pos, inv_freq);  // (pos: T of them, contiguous)
@@ -646,7 +630,6 @@ std::tuple<Tensor, Tensor> download(const Tensor& logits_in, int64_t k_in) {
     check(brk_rank_pack((const float*)logits.data_ptr(), (int32_t)B, (int32_t)nd, (int32_t)k, (float*)d, (int64_t*)(d + at_top),
                         (const int32_t*)word.data_ptr(), (int32_t*)(d + at_word), stream.stream()),
           "brk_rank_pack");
-    count(1);
     C10_CUDA_CHECK(cudaMemcpyAsync(base, d, at_word + 4, cudaMemcpyDeviceToHost, stream));
   } else {
     dev = std::get<1>(at::topk(logits, k, -1));
@@ -705,7 +688,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     g_lib_error = lib.release().ptr();
     g_oom_error = oom.release().ptr();
   });
-  m.def("launch_count", [] { return g_launches.load(); });
+  m.def("launch_count", &brk_launch_count);
   // Other Python threads run meanwhile: a launch blocks once the device's queue is full, and a ranking request waits for its
   // results.
   auto def = [&m](const char* name, auto f) { m.def(name, f, py::call_guard<py::gil_scoped_release>()); };

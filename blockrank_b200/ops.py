@@ -14,7 +14,7 @@ from . import _lib
 
 
 def __getattr__(name: str):
-    if name == "launch_count":  # kernels launched through this module since import (each call adds what it enqueues)
+    if name == "launch_count":  # kernels of the library enqueued in this process so far
         return _lib.host().launch_count()
     raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 

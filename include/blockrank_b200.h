@@ -103,6 +103,8 @@ typedef struct brk_attn_params {
 
 BRK_API int brk_version(void);
 BRK_API const char* brk_last_error(void);
+/* Kernels that the library has enqueued in this process so far (a replayed CUDA graph adds none). */
+BRK_API int64_t brk_launch_count(void);
 /* 0 if the current device is sm_100, BRK_E_DEVICE otherwise. */
 BRK_API int brk_device_check(void);
 

@@ -378,3 +378,29 @@ def test_fp32_gradients_stay_close_to_64_bits(N, Nk, D, lens):
     assert (out.detach().double() - ref.detach()).norm() <= 3e-7 * ref.detach().norm()
     for got, want, bound in zip(torch.autograd.grad(out, leaves, go), torch.autograd.grad(ref, exact, go.double()), (3.95e-7, 4.05e-7, 3.8e-7)):
         assert (got.double() - want).norm() <= bound * want.norm()
+
+
+def test_launches_are_counted_where_they_happen():
+    """One prompt of five short documents is one kernel; a call of more than one wave has a kernel in front, chunks one behind."""
+    def count(call):
+        before = ops.launch_count
+        call()
+        return ops.launch_count - before
+
+    def attend(lens, N, Nk, D, dtype, raw=False, **kw):
+        spans, q, k, v = packed(lens, N, Nk, D, dtype)
+        return lambda: cuda_blockrank_attention_forward(Layer(), q, k, v, spans, 0.1, layers_to_return_scores=[0] if raw else [], **kw)
+
+    short, long = [[27] + [60] * 5 + [19]], [[64] + [160] * 20 + [48]] * 4
+    assert count(attend(short, 32, 8, 128, torch.bfloat16)) == 1
+    assert count(attend(short, 32, 8, 128, torch.bfloat16, raw=True)) == 2
+    assert count(attend(long, 32, 8, 128, torch.bfloat16)) == 3
+    assert count(attend(short, 32, 8, 128, torch.float32)) == 2
+    assert count(attend(long, 32, 8, 128, torch.float32)) == 3
+    assert count(attend(short, 32, 8, 128, torch.bfloat16, blockrank_algo=_lib.ALGO_SIMT)) == 2
+    for dtype, one, two in ((torch.bfloat16, 2, 3), (torch.float32, 2, 2)):  # backward of one block, of several
+        for lens, n in (([[100]], one), (short, two)):
+            spans, q, k, v = packed(lens, 32, 8, 128, dtype)
+            leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+            out, _ = cuda_blockrank_attention_forward(Layer(), *leaves, spans, 0.1)
+            assert count(lambda: torch.autograd.grad(out, leaves, torch.ones_like(out))) == n
