@@ -17,17 +17,23 @@
 
 namespace brk {
 
-// scratch: delta [B, N, S]; bf16 only: fp32 dk, dv [B, Nk, S, D]; fp32 dq of the last block's rows [B, N, max_block_len, D];
-// what the tcgen05 kernel needs beyond that
+// scratch: delta [B, N, S]; bf16 only: fp32 dk, dv, of every slot ([B, Nk, S, D] each) for the warp-level kernels, of the prefix
+// block ([B, Nk, max_block_len, D]) for the tcgen05 kernel of three blocks or more; fp32 dq of the last block's rows [B, N,
+// max_block_len, D]; what the tcgen05 kernel needs beyond that
 static size_t delta_bytes(const brk_attn_bwd_params& p) {
   return (((size_t)p.B * p.N * p.S * sizeof(float)) + 255) & ~(size_t)255;
 }
 static size_t acc_bytes(const brk_attn_bwd_params& p) { return (size_t)p.B * p.Nk * p.S * p.D * sizeof(float); }
 static size_t dq_last_bytes(const brk_attn_bwd_params& p) { return (size_t)p.B * p.N * p.max_block_len * p.D * sizeof(float); }
 
+static size_t sums_bytes(const brk_attn_bwd_params& p) {
+  const bool prefix = attn_bwd_tc_supported(p) && p.M > 2;
+  return 2 * (prefix ? (size_t)p.B * p.Nk * p.max_block_len * p.D * sizeof(float) : acc_bytes(p));
+}
+
 size_t attn_bwd_workspace(const brk_attn_bwd_params& p) {
   if (p.dtype == BRK_F32) return delta_bytes(p);
-  return delta_bytes(p) + 2 * acc_bytes(p) + dq_last_bytes(p) + (attn_bwd_tc_supported(p) ? attn_bwd_tc_extra_bytes(p) : 0);
+  return delta_bytes(p) + sums_bytes(p) + dq_last_bytes(p) + (attn_bwd_tc_supported(p) ? attn_bwd_tc_extra_bytes(p) : 0);
 }
 
 int attn_bwd_launch(const brk_attn_bwd_params& p, void* ws, size_t ws_bytes, int32_t* status, cudaStream_t st) {
@@ -37,7 +43,7 @@ int attn_bwd_launch(const brk_attn_bwd_params& p, void* ws, size_t ws_bytes, int
   float* const delta = reinterpret_cast<float*>(w);
   if (p.dtype == BRK_F32) return attn_bwd_f32_launch(p, delta, st);
   float* const acc = reinterpret_cast<float*>(w + delta_bytes(p));
-  unsigned char* const dq32 = w + delta_bytes(p) + 2 * acc_bytes(p);
+  unsigned char* const dq32 = w + delta_bytes(p) + sums_bytes(p);
   if (attn_bwd_tc_supported(p))
     return attn_bwd_tc_launch(p, delta, acc, reinterpret_cast<float*>(dq32), dq32 + dq_last_bytes(p), status, st);
   BRK_CUDA(cudaMemsetAsync(acc, 0, 2 * acc_bytes(p) + dq_last_bytes(p), st));

@@ -867,8 +867,8 @@ bool attn_bwd_tc_supported(const brk_attn_bwd_params& p) {
 static size_t head_bytes(const brk_attn_bwd_params& p) { return (256 + (size_t)p.B * p.M * sizeof(int) + 255) & ~(size_t)255; }
 size_t attn_bwd_tc_extra_bytes(const brk_attn_bwd_params& p) { return p.M > 2 || part_bytes(p) > 0 ? head_bytes(p) + part_bytes(p) : 0; }
 
-// ws32: the two [B, Nk, S, D] accumulators of the warp-level kernels (used for the prefix sums here), then dq32; extra: the
-// bytes of attn_bwd_tc_extra_bytes (the item counter goes into the unused accumulators when there are none)
+// ws32: the prefix sums, right in front of dq32 (two blocks or fewer: accumulators of which only the item counter is used);
+// extra: the bytes of attn_bwd_tc_extra_bytes
 int attn_bwd_tc_launch(const brk_attn_bwd_params& p, float* delta, float* ws32, float* dq32, void* extra, int32_t* status,
                        cudaStream_t st) {
   BwdTcArgs a{};
@@ -887,7 +887,7 @@ int attn_bwd_tc_launch(const brk_attn_bwd_params& p, float* delta, float* ws32, 
   a.scale_log2 = p.scale * 1.4426950408889634f;
   // With two blocks or fewer no document adds to the prefix's dK / dV: block 0's own item stores them.
   const int64_t n_pre = p.M > 2 ? 2ll * p.B * p.Nk * p.max_block_len * p.D : 0, n_q = p.M > 1 ? (int64_t)p.B * p.N * p.max_block_len * p.D : 0;
-  // The prefix sums sit at the end of the accumulators, directly in front of dq32: one range to clear.
+  // The prefix sums sit directly in front of dq32: one range to clear.
   a.pre = n_pre ? dq32 - n_pre : nullptr;
   a.dq32 = dq32;
   unsigned char* const x = static_cast<unsigned char*>(extra);

@@ -265,3 +265,16 @@ def test_structures_of_the_c_abi_keep_their_size(tmp_path):
     src = tmp_path / "sizes.c"
     src.write_text('#include "blockrank_b200.h"\n' + "".join(f"_Static_assert(sizeof({n}) == {v}, \"{n}\");\n" for n, v in sizes.items()))
     subprocess.run([cc, "-fsyntax-only", "-I", os.path.join(ROOT, "include"), str(src)], check=True)
+
+
+def test_backward_scratch_holds_what_its_kernel_uses():
+    """bf16 with blocks that fit the tcgen05 kernel: fp32 sums of the prefix block and of the last block's dq, not of every slot."""
+    L = _lib.lib()
+    p = _lib.AttnBwdParams()
+    p.dtype, p.B, p.N, p.Nk, p.D, p.S, p.M, p.max_block_len, p.scale = 0, 1, 32, 8, 128, 26112, 102, 256, 0.1
+    delta, prefix, dq = 32 * 26112 * 4, 2 * 8 * 256 * 128 * 4, 32 * 256 * 128 * 4
+    head, part = 256 + 512, 8 * 128 * 128 * 4  # item counter and order; the partial dQ of a thread block, one per SM
+    blocks = (L.brk_attn_bwd_workspace_bytes(ctypes.byref(p)) - delta - prefix - dq - head) / part
+    assert blocks == int(blocks) and 1 <= blocks <= 148  # (1 without a device)
+    p.max_block_len = 2000  # too long for it: the warp-level kernels sum dk and dv of every slot
+    assert L.brk_attn_bwd_workspace_bytes(ctypes.byref(p)) == delta + 2 * 8 * 26112 * 128 * 4 + 32 * 2000 * 128 * 4
