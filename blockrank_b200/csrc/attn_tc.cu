@@ -1099,6 +1099,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
                   ptx::tmem_st32(tmem_lane + kColO + (uint32_t)ch * 32, orow);
                 }
               }
+              if (h > 0) ptx::tmem_wait_st();  // the first slot's P was stored by this thread: complete before it is read back
               if (kFine && h > 0) {
                 uint32_t ph[32], pm[32];
                 ptx::tmem_ld32(tmem_lane, ph);
