@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(256) attn_bwd_store_kernel(BwdMmaArgs a, int D
 
 template <int D>
 int launch_mma(BwdMmaArgs a, cudaStream_t st) {
-  const int tiles = (a.max_block_len + kT - 1) / kT;
+  const int tiles = (a.max_block_len + kT - 1) / kT, sms = std::max(1, sm_count());
   const int smem_dq = 4 * (int)sizeof(MmaTile<D>);
   BRK_CUDA(cudaFuncSetAttribute(attn_bwd_dq_mma_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dq));
   BRK_CUDA(cudaFuncSetAttribute(attn_bwd_dq_mma_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_dq));
@@ -495,7 +495,7 @@ int launch_mma(BwdMmaArgs a, cudaStream_t st) {
   }
   {
     const int64_t n8 = (int64_t)a.B * a.N * a.max_block_len * (D / 8);
-    const int blocks = (int)std::min<int64_t>((n8 + 255) / 256, 148 * 8);
+    const int blocks = (int)std::min<int64_t>((n8 + 255) / 256, sms * 8);
     attn_bwd_store_dq_last_kernel<D><<<std::max(blocks, 1), 256, 0, st>>>(a);
     BRK_LAUNCHED();
   }
@@ -513,7 +513,7 @@ int launch_mma(BwdMmaArgs a, cudaStream_t st) {
     BRK_LAUNCHED();
   }
   const int64_t n4 = (int64_t)a.B * a.Nk * a.S * (D / 4);
-  attn_bwd_store_kernel<<<(unsigned)std::min<int64_t>((n4 + 255) / 256, 148 * 16), 256, 0, st>>>(a, D);
+  attn_bwd_store_kernel<<<(unsigned)std::min<int64_t>((n4 + 255) / 256, sms * 16), 256, 0, st>>>(a, D);
   BRK_LAUNCHED();
   return BRK_OK;
 }

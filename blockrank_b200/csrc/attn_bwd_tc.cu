@@ -203,10 +203,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
   const uint32_t tmem = *tmem_slot;
   bool failed = false;
   auto wait = [&](int i, uint32_t parity, int code) {
-    if (failed) return;
-    // (inlined: 64 probabilities are live across some of these waits)
-    for (uint32_t n = 0; n < kWaitBudget; ++n)
-      if (ptx::mbar_try(bar(i), parity & 1u)) return;
+    if (failed || ptx::mbar_wait(bar(i), parity & 1u, kWaitBudget)) return;
     failed = true;
     if (a.status) atomicCAS(a.status, 0, code);
   };
@@ -849,7 +846,7 @@ int launch(const brk_attn_bwd_params& p, BwdTcArgs a, float4* zero, int64_t n_ze
   BRK_LAUNCHED();
   if (p.M > 1) {
     const int64_t n = (int64_t)p.B * (p.N + (a.pre ? 2 * p.Nk : 0)) * p.max_block_len * (HD / 8);
-    attn_bwd_tc_finish_kernel<HD><<<(unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8), 256, 0, st>>>(a);
+    attn_bwd_tc_finish_kernel<HD><<<(unsigned)std::min<int64_t>((n + 255) / 256, sms * 8), 256, 0, st>>>(a);
     BRK_LAUNCHED();
   }
   return BRK_OK;

@@ -143,13 +143,6 @@ constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kChainCols = 256;  // per chain: S [0,128) (P over its first 64 columns), then O [128,256)
 constexpr uint32_t kColO = 128;
 constexpr float kLazy = 8.f;
-// Exponentials per 8 evaluated as a Cody-Waite polynomial on the FMA pipe instead of the special-function unit:
-// 0, 2 or 4.  Measured on the 100-document workload (4 prompts per launch): 0 -> 0.58 ms, 4 -> 0.64 ms; the
-// softmax warps are bound by instruction issue, not by the special-function unit, so the default is 0.
-#ifndef BRK_POLY_OF_8
-#define BRK_POLY_OF_8 0
-#endif
-constexpr int kPolyOf8 = BRK_POLY_OF_8;
 constexpr uint32_t kWaitBudget = 1u << 18;
 constexpr int kTileFixedCost = 136;  // cost of a row tile beyond its keys (output drain), in keys
 
@@ -473,10 +466,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   }
 
   auto wait = [&](int i, uint32_t parity, int code) {
-    if (failed) return;
-#pragma unroll 1
-    for (uint32_t n = 0; n < kWaitBudget; ++n)
-      if (ptx::mbar_try(bar(i), parity & 1u)) return;
+    if (failed || ptx::mbar_wait(bar(i), parity & 1u, kWaitBudget)) return;
     failed = true;
     if (a.status) atomicCAS(a.status, 0, code);
   };
@@ -1040,45 +1030,27 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
             const bool changed = m_new != m_run;
             m_run = m_new;
 
-            // p with packed fp32x2 arithmetic; see kPolyOf8 for where the exponentials are evaluated
+            // p with packed fp32x2 arithmetic (the warps are bound by instruction issue, not by the special-function unit)
             const ptx::f32x2 sc2 = ptx::pack2(a.scale_log2, a.scale_log2), nr2 = ptx::pack2(neg_ref, neg_ref);
             ptx::f32x2 ps2[2] = {0ull, 0ull};
             uint32_t pk[32], pl[kFine ? 32 : 1];
 #pragma unroll
-            {
-              {
-#pragma unroll
-                for (int c = 0; c < 64; c += 4) {
-                  const ptx::f32x2 t01 = ptx::fma2(ptx::pack2(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), sc2, nr2);
-                  const ptx::f32x2 t23 = ptx::fma2(ptx::pack2(__uint_as_float(sr[c + 2]), __uint_as_float(sr[c + 3])), sc2, nr2);
-                  float t0, t1, p2, p3;
-                  ptx::unpack2(t01, t0, t1);
-                  const float p0 = ptx::ex2(t0), p1 = ptx::ex2(t1);
-                  // kPolyOf8 of every 8 exponentials go to the FMA pipe as a polynomial, the rest to the
-                  // special-function unit (a -inf logit gives exactly 0 there)
-                  if ((kPolyOf8 == 4) || (kPolyOf8 == 2 && (c & 4))) {
-                    const ptx::f32x2 p23 = ptx::ex2_poly2(t23);
-                    ptx::unpack2(p23, p2, p3);
-                    // a masked column must contribute exactly nothing: the polynomial maps -inf to 2^-126,
-                    // which times a huge (finite) value in a padding slot of V would still be visible
-                    p2 = sr[c + 2] == 0xff800000u ? 0.f : p2;
-                    p3 = sr[c + 3] == 0xff800000u ? 0.f : p3;
-                  } else {
-                    float t2, t3;
-                    ptx::unpack2(t23, t2, t3);
-                    p2 = ptx::ex2(t2);
-                    p3 = ptx::ex2(t3);
-                  }
-                  ps2[1] = ptx::add2(ps2[1], ptx::pack2(p2, p3));
-                  ps2[0] = ptx::add2(ps2[0], ptx::pack2(p0, p1));
-                  __nv_bfloat162 h0 = __floats2bfloat162_rn(p0, p1), h1 = __floats2bfloat162_rn(p2, p3);
-                  pk[c >> 1] = *reinterpret_cast<uint32_t*>(&h0);
-                  pk[(c >> 1) + 1] = *reinterpret_cast<uint32_t*>(&h1);
-                  if constexpr (kFine) {
-                    pl[c >> 1] = low_part(pk[c >> 1], p0, p1);
-                    pl[(c >> 1) + 1] = low_part(pk[(c >> 1) + 1], p2, p3);
-                  }
-                }
+            for (int c = 0; c < 64; c += 4) {
+              const ptx::f32x2 t01 = ptx::fma2(ptx::pack2(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), sc2, nr2);
+              const ptx::f32x2 t23 = ptx::fma2(ptx::pack2(__uint_as_float(sr[c + 2]), __uint_as_float(sr[c + 3])), sc2, nr2);
+              float t0, t1, t2, t3;
+              ptx::unpack2(t01, t0, t1);
+              const float p0 = ptx::ex2(t0), p1 = ptx::ex2(t1);
+              ptx::unpack2(t23, t2, t3);
+              const float p2 = ptx::ex2(t2), p3 = ptx::ex2(t3);  // (a -inf logit gives exactly 0)
+              ps2[1] = ptx::add2(ps2[1], ptx::pack2(p2, p3));
+              ps2[0] = ptx::add2(ps2[0], ptx::pack2(p0, p1));
+              __nv_bfloat162 h0 = __floats2bfloat162_rn(p0, p1), h1 = __floats2bfloat162_rn(p2, p3);
+              pk[c >> 1] = *reinterpret_cast<uint32_t*>(&h0);
+              pk[(c >> 1) + 1] = *reinterpret_cast<uint32_t*>(&h1);
+              if constexpr (kFine) {
+                pl[c >> 1] = low_part(pk[c >> 1], p0, p1);
+                pl[(c >> 1) + 1] = low_part(pk[(c >> 1) + 1], p2, p3);
               }
             }
             ptx::tmem_st32(tmem_lane + (uint32_t)h * (kFine ? 64 : 32), pk);

@@ -278,12 +278,12 @@ int rmsnorm_launch(int dtype, const void* x, void* residual, const void* w, void
 int rope_launch(int dtype, void* q, int64_t q_rs, int N, void* k, int64_t k_rs, int Nk, int D, const int32_t* pos,
                 const float* inv_freq, int64_t T, cudaStream_t st) {
   const int64_t total = T * (D / 16);
-  const int threads = 128, heads = N + Nk;
+  const int threads = 128, heads = N + Nk, sms = sm_count();
   const int64_t blocks = (total + threads - 1) / threads;
   // Heads per thread: four loads of each half in flight are enough for a large call; a small one is cut until the blocks
-  // cover the SMs twice. 
+  // cover the SMs twice.
   int per = std::min(heads, 8);
-  while (per > 1 && blocks * ((heads + per - 1) / per) < 2 * 148) per = (per + 1) / 2;
+  while (per > 1 && blocks * ((heads + per - 1) / per) < 2 * sms) per = (per + 1) / 2;
   const dim3 grid((unsigned)blocks, (unsigned)((heads + per - 1) / per));
   if (dtype == BRK_BF16)
     rope_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>((__nv_bfloat16*)q, q_rs, N, (__nv_bfloat16*)k, k_rs, Nk, D, pos,

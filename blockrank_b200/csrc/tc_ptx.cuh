@@ -30,24 +30,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Bounded wait on a phase parity. Returns false if the budget ran out.  Out of line: the kernels wait in
-// dozens of places and an inlined copy of the loop at each of them is pure instruction-cache pressure.
-static __device__ __noinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t budget = (1u << 22)) {
-  for (uint32_t it = 0; it < budget; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
-// One suspending attempt (the hardware bounds it), for waits written in line.
+// One suspending attempt (the hardware bounds it).
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -58,6 +41,15 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
       : "r"(bar), "r"(parity)
       : "memory");
   return ok != 0;
+}
+
+// Bounded wait on a phase parity: false if `budget` attempts ran out.  In line: values are live in registers across many of
+// the kernels' waits.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t budget) {
+#pragma unroll 1
+  for (uint32_t n = 0; n < budget; ++n)
+    if (mbar_try(bar, parity)) return true;
+  return false;
 }
 
 // Non-blocking test of a phase parity.
@@ -109,29 +101,6 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
-}
-
-// 2^x for two values on the FMA/ALU pipes (no special-function unit): Cody-Waite split
-// x = n + f with f in [-0.5, 0.5], a minimax cubic for 2^f (relative error 7.5e-5, far below bf16
-// resolution), and n added into the exponent field.  Inputs below -126 (including -inf) give
-// 2^-126, i.e. zero for every purpose here.
-__device__ __forceinline__ f32x2 ex2_poly2(f32x2 x2) {
-  float x0, x1;
-  unpack2(x2, x0, x1);
-  x2 = pack2(fmaxf(x0, -126.f), fmaxf(x1, -126.f));
-  const f32x2 magic = pack2(12582912.f, 12582912.f);      // 1.5 * 2^23: adding it rounds to nearest integer
-  const f32x2 neg_magic = pack2(-12582912.f, -12582912.f);
-  const f32x2 neg_one = pack2(-1.f, -1.f);
-  const f32x2 r = add2(x2, magic);
-  const f32x2 f = fma2(add2(r, neg_magic), neg_one, x2);  // x - round(x)
-  f32x2 p = fma2(f, pack2(0.05517148599f, 0.05517148599f), pack2(0.24261091650f, 0.24261091650f));
-  p = fma2(p, f, pack2(0.69326096773f, 0.69326096773f));
-  p = fma2(p, f, pack2(0.99992805719f, 0.99992805719f));
-  float p0, p1, r0, r1;
-  unpack2(p, p0, p1);
-  unpack2(r, r0, r1);
-  return pack2(__int_as_float(__float_as_int(p0) + (__float_as_int(r0) << 23)),
-               __int_as_float(__float_as_int(p1) + (__float_as_int(r1) << 23)));
 }
 
 // 32-byte global store (eight 32-bit words); the address must be 32-byte aligned.
@@ -186,8 +155,7 @@ __device__ __forceinline__ void tma_add_4d(const CUtensorMap* m, uint32_t src, i
                : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// every committed bulk operation of this thread has read its shared memory / is complete
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+// all but the newest committed bulk operation of this thread have read their shared memory / every one is complete
 __device__ __forceinline__ void bulk_wait_read_but_one() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
@@ -227,32 +195,11 @@ __device__ __forceinline__ uint32_t idesc_bf16(uint32_t M, uint32_t N, uint32_t 
 }
 
 // ---- MMA (issued by a single thread) ------------------------------------------------
-// D[tmem] (+)= A[smem] * B[smem]; accumulate = 0 overwrites D.
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                       uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]: the A operand (M x K, bf16) lives in tensor memory, one row per
-// lane, two consecutive K elements packed per 32-bit column.
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                       uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same two instructions with the shared-memory descriptors passed as 32-bit halves.  Stepping a
-// descriptor along K or to another buffer only changes the 14-bit start-address field in the low
-// word, so the issuing thread spends one 32-bit add per operand and MMA instead of 64-bit
-// arithmetic: that thread's instruction stream, not the tensor pipe, is what bounds a sequence of
-// short MMAs.
+// D[tmem] (+)= A B, accumulate = 0 overwrites D; B in shared memory, A in shared memory (ss) or in tensor memory (ts: M x K bf16,
+// one row per lane, two consecutive K elements per 32-bit column).  The shared-memory descriptors are passed as 32-bit halves:
+// stepping one along K or to another buffer only changes the 14-bit start-address field in the low word, so the issuing thread
+// spends one 32-bit add per operand and MMA instead of 64-bit arithmetic; that thread's instruction stream, not the tensor
+// pipe, is what bounds a sequence of short MMAs.
 __device__ __forceinline__ void mma_ss_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                             uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -303,7 +250,6 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
         "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // Wait for outstanding tcgen05.ld, then tie the destination registers to the wait: the loaded
 // values are only defined after wait::ld, but to the compiler the wait has no data dependence on
 // them, so arithmetic on the registers could legally be scheduled above it.  Passing every
