@@ -404,3 +404,64 @@ def test_launches_are_counted_where_they_happen():
             leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
             out, _ = cuda_blockrank_attention_forward(Layer(), *leaves, spans, 0.1)
             assert count(lambda: torch.autograd.grad(out, leaves, torch.ones_like(out))) == n
+
+
+@pytest.mark.parametrize("N,Nk,D", [(8, 2, 128), (8, 1, 64), (4, 4, 64)])
+def test_fp32_chunked_query_block_on_a_padded_grid(N, Nk, D):
+    """fp32 with a query block in several key chunks: padding between documents, a run of empty documents longer than a chunk,
+    a prompt with one document only; output, lse and gradients against fp64 autograd."""
+    M, H = 30, 48                                     # 1,440 slots: three chunks of 512
+    lens = H_.random_lens(3, M, H, 9)
+    lens[0][3:16] = [0] * 13                          # 624 empty slots
+    lens[1] = [0] + [0] * (M - 3) + [40, H]           # empty prefix, everything in the last chunk
+    mask = H_.ragged_mask(3, M, H, lens)
+    q, k, v = H_.qkv(3, N, Nk, M * H, D, 5, torch.float32)
+    start, ln = ops.spans_from_mask(mask.cuda())
+    qd, kd, vd = (H_.to_cuda_view(t) for t in (q, k, v))
+    out, lse = ops.attention(qd, kd, vd, start, ln, D ** -0.5, H, return_lse=True)
+    exact = [t.double().requires_grad_(True) for t in (q, k, v)]
+    ref, ref_lse = orc.attention_dense(*exact, mask, D ** -0.5)
+    rows = mask.reshape(3, -1)
+    assert (out.cpu().double() - ref.detach())[rows].norm() <= 1e-6 * ref.detach()[rows].norm()
+    assert out.cpu()[~rows].abs().max() == 0
+    live = rows[:, None].expand(3, N, M * H)
+    assert (lse.cpu().double() - ref_lse.detach())[live].abs().max() < 1e-5
+    g = torch.randn(ref.shape, generator=torch.Generator().manual_seed(1)) * rows[..., None, None]
+    grads = ops.attention_bwd(qd, kd, vd, out, g.cuda(), lse, start, ln, D ** -0.5, H)
+    for got, want in zip(grads, torch.autograd.grad(ref[rows], exact, g.double()[rows])):
+        assert (got.cpu().double() - want).norm() <= 2e-6 * want.norm()
+
+
+@pytest.mark.parametrize("nd,k", [(1, 1), (5, 5), (300, 10), (2048, 2048), (2048, 7), (2049, 12)])  # 2,049: the general path
+def test_best_documents_with_ties_and_nan(nd, k):
+    """Indices of the k best: best first, NaN in front, equal scores in document order (up to 2,048 documents)."""
+    g = torch.Generator().manual_seed(nd)
+    logits = torch.randint(-3, 4, (3, nd), generator=g).float() if nd <= 2048 else torch.randperm(3 * nd, generator=g).view(3, nd).float()
+    logits[0, nd // 2] = float("nan")
+    logits[1, 0], logits[1, -1] = float("-inf"), float("inf")
+    got, top = _lib.host().download(logits.cuda(), k)
+    assert torch.equal(got.nan_to_num(9.0), logits.nan_to_num(9.0)) and top.shape == (3, k) and top.dtype == torch.int64
+    for b in range(3):
+        key = [(0, 0.0) if x != x else (1, -x) for x in logits[b].tolist()]
+        assert top[b].tolist() == sorted(range(nd), key=lambda i: (key[i], i))[:k]
+
+
+def test_requests_of_other_types_and_layouts():
+    """Tensors that cannot travel in one packed copy give the same scores: other integer types, strides, device tensors."""
+    rk, batch = _requests(3, [30, 40, 50, 20, 4])
+    full, order = rk.rank_host(batch, k=2)
+    for name, f in (("input_ids", lambda t: t.int()), ("input_ids", lambda t: t.t().contiguous().t()), ("position_ids", lambda t: t.int()),
+                    ("position_ids", lambda t: t.float()), ("signal_rows", lambda t: t.long()), ("signal_rows", lambda t: t.cuda()),
+                    ("block_spans", lambda t: t.cuda())):
+        logits, top = rk.rank_host(dict(batch, **{name: f(batch[name])}), k=2)
+        assert torch.equal(logits, full) and torch.equal(top, order)
+
+
+@pytest.mark.parametrize("row", [-1, "S"])
+def test_signal_row_outside_the_prompt_is_reported(row):
+    rk, batch = _requests(2, [30, 40, 50, 20, 4])
+    rows = batch["signal_rows"].clone()
+    rows[1, 0] = batch["input_ids"].shape[1] if row == "S" else row
+    with pytest.raises(ValueError, match="signal row"):
+        rk.rank_host(dict(batch, signal_rows=rows))
+    assert torch.isfinite(rk.rank_host(batch)[0]).all()  # (the word is clear again)
