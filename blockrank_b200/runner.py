@@ -8,7 +8,7 @@ scores with the minimal work: layers 0..l*-1 in full, and at layer ``l*`` only
 the input RMSNorm, ``k_proj`` for every token, ``q_proj`` for the signal rows,
 RoPE and the fused score epilogue.
 
-Dense projections are cuBLAS GEMMs through torch.matmul; RMSNorm, RoPE,
+Dense projections are cuBLAS GEMMs on PyTorch's handle; RMSNorm, RoPE,
 SiLU*up, the block-sparse attention and the scorer are this package's CUDA
 kernels.  Weights use the HF parameter names, so a real checkpoint's state
 dict loads directly.
@@ -127,7 +127,7 @@ class MistralPrefillRanker:
         """One full decoder layer ``i < score_layer`` applied in place to the residual stream ``h`` (B*S, hidden).
 
         Both residual additions happen in the epilogue of the GEMM that produces the branch
-        (``h.addmm_``: C = C + A·B, added in fp32 before the rounding), so the branch output is never
+        (C = C + A·B, added in fp32 before the rounding), so the branch output is never
         written to memory and the RMSNorm that follows reads one tensor instead of two."""
         c, L, host = self.cfg, self.layers[i], _lib.host()
         N, Nk, D = c.num_attention_heads, c.num_key_value_heads, c.head_dim

@@ -97,7 +97,8 @@ typedef struct brk_attn_params {
  *    slots behind the end of any block (tiles are loaded 64 keys at a time; slots past S are never read).  Keys
  *    outside a row's visible set get a probability of exactly zero, but 0 x Inf or 0 x NaN in V would still
  *    poison the row.  Zero-filled or token-filled padding (what a model produces) is fine.
- * What IS checked, on the device, by a small kernel in front of every attention call: every block lies inside
+ * What IS checked, on the device, in front of every attention call (by a small kernel, or by the attention kernel itself
+ * where all of its work starts at once): every block lies inside
  * [0, S), is no longer than max_block_len (the last one: max_query_len, if given), and starts at or after the end
  * of its predecessor.  If not, the call writes nothing and the status word (if given) is set. */
 
@@ -117,8 +118,8 @@ BRK_API int brk_spans_from_mask(const uint8_t* mask, int32_t B, int32_t M, int32
 
 /* Device scratch the call needs (16-byte aligned; contents need not be initialised or
  * preserved between calls, but two calls in flight must not share it).  Every path needs at
- * least a 256-byte header (work counter, verdict of the span check); the tensor-core path adds
- * the partial results of the query block's key chunks for long prompts. */
+ * least a 256-byte header (work counter, verdict of the span check); the tensor-core path adds a list of the query block's
+ * context windows, and it and the fp32 path the partial results of the query block's key chunks for long prompts. */
 BRK_API size_t brk_attn_fwd_workspace_bytes(const brk_attn_params* p);
 BRK_API int brk_attn_fwd(const brk_attn_params* p, void* workspace, size_t workspace_bytes, void* stream);
 

@@ -266,7 +266,7 @@ def model_bench(a, ops, ref_loader, mask, H, S, prompts, bl):
 
 
 def backward_bench(a, ops, ref_loader, q, k, v, mask, start, ln, scale, H, S, prompts, bl, flops, valid):
-    """Forward + backward of the attention op under autograd: this library (tcgen05 forward, CUDA-core backward)
+    """Forward + backward of the attention op under autograd: this library (tcgen05 forward and backward)
     beside autograd over the reference's eager and SDPA functions, same tensors, gradients compared."""
     from blockrank_b200 import BlockSpans, cuda_blockrank_attention_forward
     spans = BlockSpans.make(start, ln, H)
