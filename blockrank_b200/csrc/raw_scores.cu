@@ -447,9 +447,10 @@ __global__ void __launch_bounds__(kThreadsF) raw_bwd_f32_kernel(RawBwdArgs a) {
     __syncthreads();
     for (int i = tid; i < 64 * (D / 4); i += kThreadsF) {
       const int rr = i / (D / 4), d = i % (D / 4) * 4, row = min(r0 + rr, GR - 1);
-      *reinterpret_cast<float4*>(qt + rr * D + d) =
-          load4(reinterpret_cast<const float*>(s.q.ptr) + (int64_t)b * s.q.sb + (int64_t)(g * G + row / s.R) * s.q.sh +
-                (int64_t)(s.S - s.R + row % s.R) * s.q.ss + d);
+      const float4 x = load4(reinterpret_cast<const float*>(s.q.ptr) + (int64_t)b * s.q.sb + (int64_t)(g * G + row / s.R) * s.q.sh +
+                             (int64_t)(s.S - s.R + row % s.R) * s.q.ss + d);
+      // (zeros behind the last pair and the last slot: their weights are zero, but an infinity would make NaN of it)
+      *reinterpret_cast<float4*>(qt + rr * D + d) = rr < nrow ? x : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     float dq[4][E] = {};
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
@@ -457,7 +458,8 @@ __global__ void __launch_bounds__(kThreadsF) raw_bwd_f32_kernel(RawBwdArgs a) {
       __syncthreads();
       for (int i = tid; i < kKeys * (D / 4); i += kThreadsF) {
         const int row = i / (D / 4), d = i % (D / 4) * 4;
-        *reinterpret_cast<float4*>(kt + row * D + d) = load4(kb + (int64_t)min(s0 + row, s.S - 1) * s.k.ss + d);
+        const float4 x = load4(kb + (int64_t)min(s0 + row, s.S - 1) * s.k.ss + d);
+        *reinterpret_cast<float4*>(kt + row * D + d) = s0 + row < s.S ? x : make_float4(0.f, 0.f, 0.f, 0.f);
       }
       for (int i = tid; i < 64 * kKeys; i += kThreadsF) {
         const int rr = i / kKeys, c = i % kKeys;

@@ -465,3 +465,22 @@ def test_signal_row_outside_the_prompt_is_reported(row):
     with pytest.raises(ValueError, match="signal row"):
         rk.rank_host(dict(batch, signal_rows=rows))
     assert torch.isfinite(rk.rank_host(batch)[0]).all()  # (the word is clear again)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_raw_score_gradient_with_infinite_keys_and_queries(dtype):
+    """An infinity in the last slot's key or the last pair's query reaches what it multiplies, as an infinity."""
+    g = torch.Generator().manual_seed(6)
+    B, N, Nk, S, D, R = 1, 5, 1, 3 * 30, 64, 13          # 65 pairs and 90 slots: remainders of both tiles
+    rb = lambda *s: (torch.rand(*s, generator=g) + 0.5).to(dtype)
+    q, k, d_raw = rb(B, N, S, D), rb(B, Nk, S, D), rb(B, N, R, S)
+    k[0, 0, S - 1, 3] = float("inf")
+    q[0, N - 1, S - 1, 5] = float("inf")
+    start, ln = ops.spans_from_mask(torch.ones(B, 3, 30, dtype=torch.bool).cuda())
+    dq, dk = ops.raw_scores_bwd(q.cuda(), k.cuda(), d_raw.cuda(), start, ln, 0.5)
+    want_q = torch.zeros(B, N, S, D)
+    want_q[0, :, S - R:, 3] = float("inf")
+    want_k = torch.zeros(B, Nk, S, D)
+    want_k[..., 5] = float("inf")
+    for got, want in ((dq, want_q), (dk, want_k)):
+        assert not got.isnan().any() and torch.equal(got.float().cpu().isinf(), want.isinf()) and (got >= 0).all()
