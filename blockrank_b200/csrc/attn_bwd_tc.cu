@@ -201,15 +201,21 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  bool failed = false;
+  uint32_t budget = kWaitBudget;  // tries of a wait; a thread whose wait gave up keeps that wait's code here instead
+  // What a wait does when it runs out stays out of its loop: with an atomic to the status word there, and the arrivals below in
+  // a branch of lane 0, a backward of 100 documents of 32..256 tokens took 562 us with its forward, now 545.
   auto wait = [&](int i, uint32_t parity, int code) {
-    if (failed || ptx::mbar_wait(bar(i), parity & 1u, kWaitBudget)) return;
-    failed = true;
-    if (a.status) atomicCAS(a.status, 0, code);
+    uint32_t n = 0;
+#pragma unroll 1
+    while (!ptx::mbar_try(bar(i), parity & 1u))
+      if (++n >= budget) {
+        if (budget == kWaitBudget) budget = (uint32_t)code;
+        break;
+      }
   };
   auto arrive = [&](int i) {
     __syncwarp();
-    if (lane == 0) ptx::mbar_arrive(bar(i));
+    ptx::mbar_arrive_warp(bar(i));
   };
   uint32_t n_items = 0;
   // next item of this CTA, or -1 (every warp but the loader)
@@ -217,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
     const uint32_t slot = n_items & 1u;
     wait(kItemFull + slot, n_items >> 1, 60);
     int idx = item_slot[slot];
-    if (__any_sync(0xffffffffu, failed)) idx = -1;
+    if (__any_sync(0xffffffffu, budget != kWaitBudget)) idx = -1;
     arrive(kItemFree + slot);
     ++n_items;
     return idx;
@@ -241,7 +247,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
           ptx::mbar_arrive(bar(kItemFull + (pub & 1u)));
         }
         ++pub;
-        if (idx < 0 || __any_sync(0xffffffffu, failed)) break;
+        if (idx < 0 || __any_sync(0xffffffffu, budget != kWaitBudget)) break;
         const Item it = decode(a, idx);
         for (int kt = 0; kt < it.n_kt; ++kt) {
           const RowList rows = rows_of(a, it, kt);
@@ -671,6 +677,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
       }
     }
   }
+  if (budget != kWaitBudget && a.status) atomicCAS(a.status, 0, (int)budget);
   ptx::tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) ptx::tmem_dealloc(tmem, 512);
