@@ -10,8 +10,6 @@ struct ScoreArgs {
   const int32_t* blk_start;
   const int32_t* blk_len;
   float2* partial;  // [B, N, R, nd]
-  unsigned* done_bg;  // [B, Nk] document CTAs of the (prompt, KV head) that have published their partials
-  unsigned* done_b;   // [B] KV-head groups of the prompt whose masses are written; both wrap to 0 by themselves
   float* mass;      // [B, N, R, nd] out
   float* logits;    // [B, nd] out, optional
   float inv_count_temp;  // 1 / (N * R * temperature)
@@ -27,8 +25,6 @@ inline ScoreArgs make_score_args(const brk_score_params& p) {
   a.blk_start = p.blk_start;
   a.blk_len = p.blk_len;
   a.partial = nullptr;
-  a.done_bg = nullptr;
-  a.done_b = nullptr;
   a.mass = nullptr;
   a.logits = nullptr;
   a.inv_count_temp = 0.f;

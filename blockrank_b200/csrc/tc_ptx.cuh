@@ -15,6 +15,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 
 // Programmatic dependent launch: everything the preceding kernel of the stream wrote is visible behind this.  A kernel
 // launched by launch_dependent() may be running its set-up while that kernel still does.
+// Its counterpart in that preceding kernel: the dependent one may be brought up once every block has passed here.
+__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- mbarrier -----------------------------------------------------------------

@@ -178,8 +178,8 @@ BRK_API int brk_selftest_bounded_wait(int32_t* status, uint32_t budget, void* st
  *   doc_mass  device [B, N, R, M-2] fp32 out: per head / row normalised mass per document
  *   logits    device [B, M-2] fp32 out, optional: mean over heads and rows / temperature
  * workspace: brk_doc_scores_workspace_bytes() bytes of device scratch, 8-byte aligned, contents
- * need not be initialised.  One kernel launch (plus a memset of B counters): the CTA that finishes
- * a prompt last merges its per-document partials and writes doc_mass and logits. */
+ * need not be initialised.  Two kernel launches: per-document partials, then their merge, which
+ * writes doc_mass and logits. */
 typedef struct brk_score_params {
   int32_t dtype;
   int32_t B, N, Nk, D, S, M, R;
@@ -215,10 +215,8 @@ BRK_API int brk_doc_scores(const brk_score_params* p, void* workspace, size_t wo
  *  - The first call on a device looks up the array's device address; make that first call
  *    outside any stream capture.
  *  - All calls on a device share the one array.  Nothing needs clearing between calls (every
- *    (max, sum) pair is rewritten before it is read, and the per-prompt completion counters count
- *    back to zero by the end of a call), but two calls that can run at the same time on the
- *    GPU -- different streams, or different host threads -- race on it: serialise them.  A call
- *    that was aborted half-way (device reset, a fault elsewhere) leaves the counters undefined.
+ *    (max, sum) pair is rewritten before it is read), but two calls that can run at the same time on
+ *    the GPU -- different streams, or different host threads -- race on it: serialise them.
  *  - `stream` must belong to the device that is current when the call is made.
  *  - No cudaMalloc / cudaFree / allocating library routine is called. */
 #define BRK_STATIC_SCRATCH_BYTES (4u << 20)
