@@ -17,9 +17,10 @@
 //                        latency to a kernel that has no tensor-rate problem.
 //   doc_merge_kernel     one CTA per prompt, launched beside the partial kernel's end: merges the per-document pairs into
 //                        the softmax over all document tokens, emits the per-document probability mass and then the mean
-//                        over heads and rows / temperature.  (As the job of the last CTA of a prompt, found by counters that
-//                        a memset cleared in front: 4 prompts of 100 documents 38.8 us, now 31.1; the partial kernel alone 24.5, the K read at
-//                        5.4 TB/s.)
+//                        over heads and rows / temperature.  As the job of the last CTA of a prompt, found by counters that
+//                        a memset cleared in front, with a fence and an atomic in every CTA: 4 prompts of 100 documents
+//                        38.0 us, now 29.1 (the K read at 5.4 TB/s), one prompt of 100 20.5, now 13.6.  A call of a few
+//                        short documents: alone 24.5, now 23.0; in a row, bound by the host, 12.0 and 12.9.
 #include <algorithm>
 #include <atomic>
 
@@ -159,6 +160,7 @@ __global__ void __launch_bounds__(kThreads) doc_partial_kernel(ScoreArgs a) {
   constexpr int kRowBytes = D * (int)sizeof(T);
   constexpr int kPitch = kRowBytes + 16;
   constexpr int kChunks = kRowBytes / 16;  // 16-byte pieces per key row
+  ptx::grid_dependency_wait();    // (a call's launch overlaps the end of what is in front of it, the merge of the call before for one)
   ptx::grid_dependency_launch();  // the merge kernel may be brought up once every CTA is at work
   extern __shared__ __align__(16) float smem[];
   const int G = a.N / a.Nk;
@@ -257,6 +259,7 @@ __global__ void __launch_bounds__(kThreads, 4) doc_partial_mma_kernel(ScoreArgs 
   __shared__ float2 red[2][kThreads / 32][16];
   __shared__ int s_start[kDocsPerCta], s_len[kDocsPerCta];
   __shared__ uint4 ring[kKeyStages][kSteps][kThreads];  // every lane copies into and reads back its own 16-byte cells
+  ptx::grid_dependency_wait();    // (a call's launch overlaps the end of what is in front of it, the merge of the call before for one)
   ptx::grid_dependency_launch();  // the merge kernel may be brought up once every CTA is at work
   const int G = a.N / a.Nk;
   const int GR = G * a.R;
@@ -404,8 +407,7 @@ static int doc_scores_run(const brk_score_params& p, void* ws, size_t ws_bytes, 
   auto launch = [&](auto kern) -> int {
     // (the kernels also hold a few KB of static shared memory, which counts against the same 48 KB default)
     if (sm + 8192 > 48 * 1024) BRK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    kern<<<grid, kThreads, sm, st>>>(a);
-    BRK_LAUNCHED();
+    if ((rc = launch_dependent(kern, grid, dim3(kThreads), sm, st, a))) return rc;
     return launch_dependent(doc_merge_kernel, dim3(p.B), dim3(kMergeThreads), 0, st, a);
   };
   if (p.dtype == BRK_BF16) {
@@ -415,17 +417,19 @@ static int doc_scores_run(const brk_score_params& p, void* ws, size_t ws_bytes, 
     int per_bg = std::max(1, slots / (p.B * p.Nk));
     per_bg = std::min(nd, std::max(per_bg, (nd + kDocsPerCta - 1) / kDocsPerCta));
     dim3 grid_docs(per_bg, p.B * p.Nk);
-    // (four CTAs with their key rings need 170 KB of shared memory per SM: ask for the large carve-out)
-    if (p.D == 128) {
-      BRK_CUDA(cudaFuncSetAttribute(doc_partial_mma_kernel<128>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                    (int)cudaSharedmemCarveoutMaxShared));
-      doc_partial_mma_kernel<128><<<grid_docs, kThreads, 0, st>>>(a);
-    } else {
-      BRK_CUDA(cudaFuncSetAttribute(doc_partial_mma_kernel<64>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                    (int)cudaSharedmemCarveoutMaxShared));
-      doc_partial_mma_kernel<64><<<grid_docs, kThreads, 0, st>>>(a);
-    }
-    BRK_LAUNCHED();
+    auto run = [&](auto kern, std::atomic<bool>* configured) -> int {
+      // Four CTAs with their key rings need 170 KB of shared memory per SM: ask for the large carve-out, once per device.
+      int dev = 0;
+      BRK_CUDA(cudaGetDevice(&dev));
+      if (dev < 0 || dev >= 64 || !configured[dev].load(std::memory_order_acquire)) {
+        BRK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+        if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
+      }
+      return launch_dependent(kern, grid_docs, dim3(kThreads), 0, st, a);
+    };
+    static std::atomic<bool> done128[64] = {}, done64[64] = {};
+    rc = p.D == 128 ? run(doc_partial_mma_kernel<128>, done128) : run(doc_partial_mma_kernel<64>, done64);
+    if (rc) return rc;
     return launch_dependent(doc_merge_kernel, dim3(p.B), dim3(kMergeThreads), 0, st, a);
   }
   return p.D == 128 ? launch(doc_partial_kernel<float, 128>) : launch(doc_partial_kernel<float, 64>);
