@@ -484,3 +484,27 @@ def test_raw_score_gradient_with_infinite_keys_and_queries(dtype):
     want_k[..., 5] = float("inf")
     for got, want in ((dq, want_q), (dk, want_k)):
         assert not got.isnan().any() and torch.equal(got.float().cpu().isinf(), want.isinf()) and (got >= 0).all()
+
+
+@pytest.mark.parametrize("B,N,Nk,R,docs", [(1, 4, 4, 1, 1), (2, 8, 2, 3, 40), (1, 40, 40, 2, 33), (1, 8, 2, 5, 257), (2, 32, 8, 2, 300)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_document_scores_merge(B, N, Nk, R, docs, dtype):
+    """One document, rows that do not fill a warp's turn, more documents than a lane holds, more (document, group) pairs than
+    threads: masses and logits against fp64.  Products of bf16 (and sums of 64 fp32 products) are good to 1e-6; the exponentials
+    of logits up to 10 in magnitude take that to 1e-5."""
+    gen = torch.Generator().manual_seed(N + docs)
+    lens = torch.randint(1, 12, (B, docs + 2), generator=gen, dtype=torch.int32)
+    start = torch.zeros_like(lens)
+    start[:, 1:] = lens.cumsum(1)[:, :-1]
+    S, D = int(lens.sum(1).max()), 64
+    q, k = (torch.randn(B, s, h, D, generator=gen).to(dtype).cuda().transpose(1, 2) for s, h in ((R, N), (S, Nk)))
+    rows = torch.arange(R, dtype=torch.int32).expand(B, R).contiguous()
+    mass, logits = ops.doc_scores(q, k, start.cuda(), lens.cuda(), rows.cuda(), D ** -0.5)
+    z = (q.double() @ k.double().repeat_interleave(N // Nk, 1).transpose(2, 3) * D ** -0.5).cpu()
+    for b in range(B):
+        lo, hi = int(start[b, 1]), int(start[b, -1])
+        p = torch.softmax(z[b, :, :, lo:hi], -1)
+        want = torch.stack([p[..., s - lo:s - lo + n].sum(-1) for s, n in zip(start[b, 1:-1].tolist(), lens[b, 1:-1].tolist())], -1)
+        assert (mass[b].cpu().double() - want).norm() <= 1e-5 * want.norm()
+        mean = want.mean((0, 1))
+        assert (logits[b].cpu().double() * 0.05 - mean).norm() <= 1e-5 * mean.norm()  # (the default temperature)
