@@ -47,7 +47,7 @@ namespace {
 constexpr int kTile = 128;  // keys per key tile, rows per row tile
 constexpr int kThreads = 512;
 constexpr uint32_t kChunk = kTile * 128;  // 128 rows of 64 bf16: one 64-wide chunk of a tile
-constexpr uint32_t kWaitBudget = 1u << 18;
+constexpr int kWaitBudget = 1 << 18;
 constexpr int kMaxRowTiles = 16;  // per block: bounds the dQ scratch of a CTA (64 KB per tile at head_dim 128)
 
 template <int HD>
@@ -87,7 +87,8 @@ enum {
   kItemFree = 20,  // +slot (15 consuming warps)
   kNumBars = 22
 };
-static_assert(kNumBars * 8 + 16 <= 256, "barrier area");  // + TMEM base, two item slots
+constexpr uint32_t kGaveUp = kNumBars * 8 + 12;  // behind the barriers: TMEM base, two item slots, code of the first wait that gave up
+static_assert(kGaveUp + 4 <= 256, "barrier area");
 
 struct BwdTcArgs {
   View q, k, v, o, d_o, dq, dk, dv;
@@ -188,6 +189,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
       if (i >= kItemFree) cnt = 15u;
       ptx::mbar_init(bar(i), cnt);
     }
+    *reinterpret_cast<int*>(smem + L::kOffBar + kGaveUp) = 0;
     ptx::fence_barrier_init();
     ptx::prefetch_tmap(&maps.q);
     ptx::prefetch_tmap(&maps.g);
@@ -201,18 +203,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  uint32_t budget = kWaitBudget;  // tries of a wait; a thread whose wait gave up keeps that wait's code here instead
-  // What a wait does when it runs out stays out of its loop: with an atomic to the status word there, and the arrivals below in
-  // a branch of lane 0, a backward of 100 documents of 32..256 tokens took 562 us with its forward, now 545.
-  auto wait = [&](int i, uint32_t parity, int code) {
-    uint32_t n = 0;
-#pragma unroll 1
-    while (!ptx::mbar_try(bar(i), parity & 1u))
-      if (++n >= budget) {
-        if (budget == kWaitBudget) budget = (uint32_t)code;
-        break;
-      }
-  };
+  ptx::BoundedWaits waits(kWaitBudget, sbase + L::kOffBar + kGaveUp);
+  auto wait = [&](int i, uint32_t parity, int code) { waits(bar(i), parity & 1u, code); };
   auto arrive = [&](int i) {
     __syncwarp();
     ptx::mbar_arrive_warp(bar(i));
@@ -223,7 +215,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
     const uint32_t slot = n_items & 1u;
     wait(kItemFull + slot, n_items >> 1, 60);
     int idx = item_slot[slot];
-    if (__any_sync(0xffffffffu, budget != kWaitBudget)) idx = -1;
+    if (__any_sync(0xffffffffu, waits.gave_up())) idx = -1;
     arrive(kItemFree + slot);
     ++n_items;
     return idx;
@@ -247,7 +239,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
           ptx::mbar_arrive(bar(kItemFull + (pub & 1u)));
         }
         ++pub;
-        if (idx < 0 || __any_sync(0xffffffffu, budget != kWaitBudget)) break;
+        if (idx < 0 || __any_sync(0xffffffffu, waits.gave_up())) break;
         const Item it = decode(a, idx);
         for (int kt = 0; kt < it.n_kt; ++kt) {
           const RowList rows = rows_of(a, it, kt);
@@ -677,9 +669,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
       }
     }
   }
-  if (budget != kWaitBudget && a.status) atomicCAS(a.status, 0, (int)budget);
   ptx::tc_fence_before_sync();
-  __syncthreads();
+  ptx::end_of_waits(waits, a.status);
   if (warp == 0) ptx::tmem_dealloc(tmem, 512);
 }
 

@@ -54,8 +54,8 @@
 // 146, of 500 documents of 32..256 tokens 586 -> 580 (calls with their merge).
 //
 // Shared memory 227 KB: Q 2x32 KB, K pool 80 KB, V pool 80 KB, barriers, job records, row statistics.
-// No cluster multicast anywhere.  Every mbarrier wait is bounded; on expiry the thread records
-// a code in the caller's status word, stops waiting and runs to the normal exit.
+// No cluster multicast anywhere.  Every mbarrier wait is bounded (ptx::BoundedWaits); on expiry the thread leaves a code for the
+// caller's status word, tries once in every later wait and runs to the normal exit.
 #include <cuda.h>
 
 #include <algorithm>
@@ -150,7 +150,7 @@ constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kChainCols = 256;  // per chain: S [0,128) (P over its first 64 columns), then O [128,256)
 constexpr uint32_t kColO = 128;
 constexpr float kLazy = 8.f;
-constexpr uint32_t kWaitBudget = 1u << 18;
+constexpr int kWaitBudget = 1 << 18;
 constexpr int kTileFixedCost = 136;  // cost of a row tile beyond its keys (output drain), in keys
 
 enum {
@@ -170,7 +170,8 @@ enum {
   kStat = kOFull + 2,                     // +chain  softmax -> output: row statistics written (4 warp arrivals)
   kNumBars = kStat + 2
 };
-static_assert(kNumBars * 8 + 8 <= 512, "barrier area");  // + the TMEM base address
+constexpr uint32_t kGaveUp = kNumBars * 8 + 4;  // behind the barriers: TMEM base, code of the first wait that gave up
+static_assert(kGaveUp + 4 <= 512, "barrier area");
 
 // Division by a run-time constant with a host-computed reciprocal (round-up method, exact for every
 // 32-bit numerator): q = umulhi(n, mul); n / d = (((n - q) >> 1) + q) >> shift.
@@ -432,8 +433,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffBar + kNumBars * 8);
   auto bar = [&](int i) { return sBar + (uint32_t)i * 8u; };
 
-  bool failed = false;
-  uint32_t budget = kWaitBudget;  // tries of a wait; one when one has given up
   if (tid == 0) {
     for (int i = 0; i < kNumBars; ++i) {
       uint32_t cnt = 1u;
@@ -442,6 +441,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       if (i >= kJobFree && i < kOFull) cnt = 9u;                                          // MMA, softmax, output warps
       ptx::mbar_init(bar(i), cnt);
     }
+    *reinterpret_cast<int*>(smem + kOffBar + kGaveUp) = 0;
     ptx::fence_barrier_init();
     ptx::prefetch_tmap(&tmQ);
     ptx::prefetch_tmap(&tmK);
@@ -473,28 +473,17 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     return;
   }
 
-  // The loop keeps next to nothing for the case that it runs out: an atomic with a code per wait on the spot made the whole
-  // kernel 2 % slower, a code per wait kept in a register 6 %.
-  auto wait = [&](int i, uint32_t parity) {
-    uint32_t n = 0;
-#pragma unroll 1
-    while (!ptx::mbar_try(bar(i), parity & 1u)) {
-      if (++n >= budget) {
-        budget = 1;
-        failed = true;
-        break;
-      }
-    }
-  };
+  ptx::BoundedWaits waits(kWaitBudget, sBar + kGaveUp);
+  auto wait = [&](int i, uint32_t parity, int code) { waits(bar(i), parity & 1u, code); };
 
   int* const job_ring = reinterpret_cast<int*>(smem + kOffJobs);
   const int tok_shift = 7 - a.g_shift, TOK = 1 << tok_shift;  // query tokens of a row tile
   // consumer side of chain x's job ring: copy record number i, release its slot
   auto next_job = [&](int x, uint32_t i) {
     const uint32_t slot = i % kJobRing;
-    wait(kJobFull + x * kJobRing + slot, i / kJobRing);
+    wait(kJobFull + x * kJobRing + slot, i / kJobRing, 40 + x);
     Job it = read_record(job_ring + (x * kJobRing + slot) * 16);
-    if (__any_sync(0xffffffffu, failed)) it.flags |= kFStop;  // a wait gave up: the whole warp stops here
+    if (__any_sync(0xffffffffu, waits.gave_up())) it.flags |= kFStop;  // a wait gave up: the whole warp stops here
     __syncwarp();
     ptx::mbar_arrive_warp(bar(kJobFree + x * kJobRing + slot));
     return it;
@@ -546,7 +535,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     auto publish = [&](int x, const Job& it) {
       const uint32_t np = x ? n_pub1 : n_pub0;
       const uint32_t slot = np % kJobRing;
-      if (np >= kJobRing) wait(kJobFree + x * kJobRing + slot, np / kJobRing - 1);
+      if (np >= kJobRing) wait(kJobFree + x * kJobRing + slot, np / kJobRing - 1, 14 + x);
       if (leader) {
         if (it.n > 0) {  // its Q tile on its way into L2: the MMA warp requests it when the chain's buffer is free
           ptx::tma_prefetch_4d(&tmQ, 0, it.g * G, it.start + it.t0, it.b);
@@ -560,7 +549,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // wait until both MMA warps have handed back the load last signalled on barrier s
     auto drain = [&](int s) {
       if ((out_mask >> s) & 1u) {
-        wait(kKVFree + s, (free_par >> s) & 1u);
+        wait(kKVFree + s, (free_par >> s) & 1u, 12);
         free_par ^= 1u << s;
         out_mask &= ~(1u << s);
       }
@@ -780,7 +769,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     const uint64_t v_desc0 = ptx::smem_desc_sw128(sbase + kOffV, kPoolHalf, 1024);
     const uint32_t tm_s = tmem + (uint32_t)x * kChainCols, tm_o = tm_s + kColO;
     auto wait_full = [&](int s) {
-      wait(kKVFull + s, (full_par >> s) & 1u);
+      wait(kKVFull + s, (full_par >> s) & 1u, 22 + x);
       full_par ^= 1u << s;
     };
     // S = Q K^T against `keys` keys starting at pool slot `slot`
@@ -832,7 +821,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // has been published, otherwise at the start of that job.
     uint32_t q_issued = 0;
     auto request_q = [&](const Job& jb) {
-      if (q_issued > 0) wait(kQFree + x, q_issued - 1);  // every Q K^T of the previous job has read the buffer
+      if (q_issued > 0) wait(kQFree + x, q_issued - 1, 28 + x);  // every Q K^T of the previous job has read the buffer
       if (ptx::elect_one()) {
         const uint32_t dst = sbase + kOffQ + (uint32_t)x * kQBytes;
         ptx::mbar_expect_tx(bar(kQFull + x), kQBytes);
@@ -860,7 +849,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       // a phase further, and a parity wait must never fall two phases behind)
       if (T > 0 && !pre_qk) {
         if (q_issued == q_uses) request_q(it);  // not requested ahead
-        wait(kQFull + x, q_uses);
+        wait(kQFull + x, q_uses, 20 + x);
         ++q_uses;
       }
       if (T == 1 && pre_qk) request_next_q(job_no);  // its only Q K^T went out with the previous job's last P V
@@ -881,9 +870,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           pre_qk = false;
           for (int t = 0; t < T; ++t) {
             if (t + 1 < T) ensure(min(n, 2 * t + 4));
-            wait(kPFull + x, p_seen);
+            wait(kPFull + x, p_seen, 24 + x);
             ++p_seen;
-            if (t == 0 && jobs_done > 0) wait(kOFree + x, jobs_done - 1);
+            if (t == 0 && jobs_done > 0) wait(kOFree + x, jobs_done - 1, 26 + x);
             // After the job's last tile the chain's next row tile of the same block can start at once if its
             // record and its Q tile are already here (its first key tile is resident): its first Q K^T then
             // rides behind this P V, and its S tile is waiting when the softmax warps have drained O.
@@ -943,9 +932,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           // tile has landed)
           wait_full(pos(t) + 1);
           if (t + 1 < T) wait_full(pos(t + 1));
-          wait(kPFull + x, p_seen);
+          wait(kPFull + x, p_seen, 24 + x);
           ++p_seen;
-          if (t == 0 && jobs_done > 0) wait(kOFree + x, jobs_done - 1);
+          if (t == 0 && jobs_done > 0) wait(kOFree + x, jobs_done - 1, 26 + x);
           ptx::tc_fence_after_sync();
           issue_pv(pos(t), keys_of(t), t == 0, t + 1 == T);
           free_kv(pos(t) + 1);
@@ -974,7 +963,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     for (uint32_t job_no = 0;; ++job_no) {
       const Job it = next_job(x, job_no);
       const int flags = it.flags;
-      if (flags & kFStop) break;
+      if (flags & kFStop) {
+        if (waits.gave_up()) waits.record(36 + x);  // the wait at the end of a job, if no other: recorded there it made the role spill
+        break;
+      }
       if (it.n == 0) continue;
       const int32_t* bs = a.blk_start + (size_t)it.b * a.M;
       const int32_t* bl = a.blk_len + (size_t)it.b * a.M;
@@ -986,13 +978,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
       for (int t = 0; t < t_mine; ++t) {
         const int cnt = min(2, n_mine - 2 * t);  // slots of this tile the chain sees
-        wait(kSFull + x, s_seen);
+        wait(kSFull + x, s_seen, 30 + x);
         ++s_seen;
         if (t > 0) {
           // The previous tile's P V was issued before this tile's Q K^T, so it has completed too: O is stable
           // and the P columns (first half of S) may be overwritten.  Consuming that phase here keeps the pass
           // below free of calls (64 logits are live across its middle).
-          wait(kPVDone + x, pv_seen);
+          wait(kPVDone + x, pv_seen, 32 + x);
           ++pv_seen;
         }
         ptx::tc_fence_after_sync();
@@ -1136,7 +1128,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       }
 
       ++pv_seen;  // (the output warps wait for the job's last P V)
-      if (tiles_done > 0) wait(kOFree + x, tiles_done - 1);  // the previous tile's statistics have been read
+      if (tiles_done > 0) wait(kOFree + x, tiles_done - 1, 0);  // the previous tile's statistics have been read
       ++tiles_done;
       stat[r] = make_float2(m_run, l_run);
       __syncwarp();
@@ -1159,10 +1151,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       const int n = it.g * G + (r & (G - 1));
       const bool active = tok < it.len;
       const bool split = (it.flags & kFSplit) != 0;
-      wait(kStat + x, done);
+      wait(kStat + x, done, 38 + x);
       const float2 ml = stat[r];
       const float m_run = ml.x, l_run = ml.y;
-      wait(kOFull + x, done);
+      wait(kOFull + x, done, 34 + x);
       ++done;
       ptx::tc_fence_after_sync();
       auto chunk = [&](int ch, uint32_t (&orow)[32]) {
@@ -1229,27 +1221,40 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   }
 
   // ---- teardown ---------------------------------------------------------------------------------
-  if (failed && a.status) atomicCAS(a.status, 0, warp < 8 ? 30 : warp < 16 ? 34 : warp == 16 ? 12 : 20);  // (by role)
   ptx::tc_fence_before_sync();
-  __syncthreads();
+  ptx::end_of_waits(waits, a.status);
   if (warp == 0) ptx::tmem_dealloc(tmem, kTmemCols);
 }
 
 }  // namespace
 
-// The give-up path of the kernels' bounded waits, exercised without a fault: one thread waits, with a small
-// budget, on an mbarrier that nothing ever arrives at; the wait runs out, the thread records kStatusSelfTest in
-// the caller's status word exactly as attn_tc_kernel's waits do, and the kernel returns normally.
-__global__ void selftest_wait_kernel(int32_t* status, uint32_t budget) {
-  __shared__ __align__(8) uint64_t mbar;
-  const uint32_t b = ptx::smem_u32(&mbar);
-  ptx::mbar_init(b, 1);
+// The kernels' bounded waits (ptx::BoundedWaits) running out, without a fault: one thread waits with a small budget on an
+// mbarrier that nothing arrives at, then on another one, which may take one try and must not replace the first one's code,
+// then on one whose phase is complete, and leaves as the kernels do.  Anything else than expected is reported as the code
+// behind kStatusSelfTest.
+__global__ void selftest_wait_kernel(int32_t* status, int budget) {
+  __shared__ __align__(8) uint64_t mbar[3];
+  __shared__ int word;
+  uint32_t b[3];
+  for (int i = 0; i < 3; ++i) {
+    b[i] = ptx::smem_u32(&mbar[i]);
+    ptx::mbar_init(b[i], 1);
+  }
+  word = 0;
   ptx::fence_barrier_init();
-  if (!ptx::mbar_wait(b, 0, budget)) atomicCAS(status, 0, kStatusSelfTest);
+  ptx::mbar_arrive(b[2]);
+  ptx::BoundedWaits waits(budget, ptx::smem_u32(&word));
+  waits(b[2], 0, kStatusSelfTest + 2);
+  bool ok = !waits.gave_up();
+  ok &= waits(b[0], 0, kStatusSelfTest) == budget && waits.gave_up();
+  ok &= waits(b[1], 0, kStatusSelfTest + 2) == 1;
+  ok &= waits(b[2], 0, kStatusSelfTest + 2) == 0;
+  if (!ok) atomicCAS(status, 0, kStatusSelfTest + 1);
+  ptx::end_of_waits(waits, status);
 }
 
 int selftest_wait_launch(int32_t* status, uint32_t budget, cudaStream_t st) {
-  selftest_wait_kernel<<<1, 1, 0, st>>>(status, budget);
+  selftest_wait_kernel<<<1, 1, 0, st>>>(status, (int)budget);
   BRK_LAUNCHED();
   return BRK_OK;
 }

@@ -108,8 +108,8 @@ Tensor scratch(size_t bytes, const Tensor& like) {
   return at::empty({(int64_t)bytes}, like.options().dtype(at::kByte).requires_grad(false));
 }
 
-// One int32 status word per device, zeroed when created.  Every attention call passes it; the kernels set it (first
-// event wins) when a bounded wait gives up or the block spans are malformed.
+// One int32 status word per device, zeroed when created.  Every attention call passes it; the kernels set it (the first
+// code written stays) when a bounded wait gives up or the block spans are malformed.
 Tensor status_word(int device) {
   static std::mutex mu;
   static auto* words = new std::vector<Tensor>();  // (never destroyed: the CUDA context may be gone at exit)

@@ -33,7 +33,7 @@ def spans_from_mask(mask_bmh: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]
 
 def status_word(device) -> torch.Tensor:
     """The device's int32 status word, zeroed when created.  Every attention call passes it; the kernels set
-    it (first event wins) when a bounded wait gives up or the block spans are malformed, and check_status()
+    it (the first code written stays) when a bounded wait gives up or the block spans are malformed, and check_status()
     turns it into an exception at the caller's next synchronisation point."""
     device = torch.device(device)
     return _lib.host().status_word(device.index if device.index is not None else torch.cuda.current_device())

@@ -155,7 +155,8 @@ BRK_API int brk_attn_bwd_reporting(const brk_attn_bwd_params* p, void* workspace
                                    void* stream);
 
 /* Device-side status.  The kernels never trap: a bounded wait that gives up, or malformed block spans, set
- * the caller's status word (brk_attn_params.status; first event wins) and the kernel returns normally.
+ * the caller's status word (brk_attn_params.status) and the kernel returns normally.  The word keeps the first code
+ * written to it; a kernel's CTAs write theirs, the wait that gave up first in each, as they leave.
  * brk_status_poll synchronises `stream`, reads the word and clears it: BRK_OK if it was zero,
  * BRK_E_TIMEOUT after a wait gave up (the outputs of that call are incomplete), BRK_E_ARG after malformed
  * spans (nothing was written); brk_last_error() names the event.  Call it where the host synchronises
@@ -163,7 +164,8 @@ BRK_API int brk_attn_bwd_reporting(const brk_attn_bwd_params* p, void* workspace
  * error reporting. */
 BRK_API int brk_status_poll(int32_t* status, void* stream);
 /* Self-test of that give-up path: one thread waits `budget` (1..65536) polls on a barrier nothing arrives
- * at, then records its code in *status and returns; a following brk_status_poll returns BRK_E_TIMEOUT.
+ * at (the attention kernels' own wait), then records its code in *status and returns; a following brk_status_poll
+ * returns BRK_E_TIMEOUT.
  * Nothing faults or hangs. */
 BRK_API int brk_selftest_bounded_wait(int32_t* status, uint32_t budget, void* stream);
 

@@ -294,14 +294,16 @@ def test_7b_architecture_prompt_vs_fp32_oracle():
     same_order(top16, err16, "bf16 runner, end to end")
 
 
-def test_bounded_wait_gives_up_and_is_reported():
+@pytest.mark.parametrize("budget", [1, 1024])
+def test_bounded_wait_gives_up_and_is_reported(budget):
     """A wait that runs out sets the status word and the kernel returns; the host sees BRK_E_TIMEOUT at its next
     poll, the word is cleared, and the next attention call is unaffected."""
     L = _lib.lib()
     ops.check_status()
     w = ops.status_word("cuda")
-    rc = L.brk_selftest_bounded_wait(w.data_ptr(), 1024, torch.cuda.current_stream().cuda_stream)
+    rc = L.brk_selftest_bounded_wait(w.data_ptr(), budget, torch.cuda.current_stream().cuda_stream)
     assert rc == 0, L.brk_last_error()
+    assert int(w.item()) == 90  # the first wait's code; 91: a wait behind it took more than one try, or replaced the code
     with pytest.raises(_lib.BlockRankLibraryError, match="BRK_E_TIMEOUT"):
         ops.check_status()
     assert int(w.item()) == 0

@@ -267,6 +267,18 @@ def test_structures_of_the_c_abi_keep_their_size(tmp_path):
     subprocess.run([cc, "-fsyntax-only", "-I", os.path.join(ROOT, "include"), str(src)], check=True)
 
 
+def test_every_wait_of_the_kernels_is_the_one_that_the_self_test_runs():
+    """Tries on an mbarrier stand in ptx::BoundedWaits alone, which the attention kernels and brk_selftest_bounded_wait construct,
+    and every kernel that waits reports at its end."""
+    csrc = os.path.join(ROOT, "blockrank_b200", "csrc")
+    text = {n: open(os.path.join(csrc, n)).read() for n in os.listdir(csrc) if n.endswith((".cu", ".cuh"))}
+    assert {n for n, t in text.items() if re.search(r"mbar_try\(|try_wait", t)} == {"tc_ptx.cuh"}
+    assert text["tc_ptx.cuh"].count("mbar_try(") == 2  # its definition and the loop
+    for name, kernels in (("attn_tc.cu", 2), ("attn_bwd_tc.cu", 1)):
+        assert len(re.findall(r"ptx::BoundedWaits waits\(", text[name])) == kernels
+        assert len(re.findall(r"ptx::end_of_waits\(waits, (?:a\.)?status\);", text[name])) == kernels
+
+
 def test_backward_scratch_holds_what_its_kernel_uses():
     """bf16 with blocks that fit the tcgen05 kernel: fp32 sums of the prefix block and of the last block's dq, not of every slot."""
     L = _lib.lib()
