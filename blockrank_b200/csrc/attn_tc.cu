@@ -536,7 +536,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       const uint32_t np = x ? n_pub1 : n_pub0;
       const uint32_t slot = np % kJobRing;
       if (np >= kJobRing) wait(kJobFree + x * kJobRing + slot, np / kJobRing - 1, 14 + x);
-      if (leader) {
+      if (leader && !waits.gave_up()) {  // (behind a wait that gave up the record may still be read)
         if (it.n > 0) {  // its Q tile on its way into L2: the MMA warp requests it when the chain's buffer is free
           ptx::tma_prefetch_4d(&tmQ, 0, it.g * G, it.start + it.t0, it.b);
           if (HD == 128) ptx::tma_prefetch_4d(&tmQ, 64, it.g * G, it.start + it.t0, it.b);
@@ -709,8 +709,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // atomic nor the loads are waited for.
     auto claim = [&]() {
       if (a.one_wave) return a.total_items;
-      int v = 0;
-      if (leader) v = atomicAdd(a.work_counter, 1);
+      int v = a.total_items;  // (a wait gave up: no more items)
+      if (leader && !waits.gave_up()) v = atomicAdd(a.work_counter, 1);
       return (int)gridDim.x + __shfl_sync(0xffffffffu, v, 0);
     };
     int idx = -1, idx_next = blockIdx.x;  // the first item needs no counter: its 0 is item gridDim.x
