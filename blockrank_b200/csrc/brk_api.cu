@@ -172,7 +172,8 @@ int brk_status_poll(int32_t* status, void* stream) {
     return BRK_E_ARG;
   }
   set_error("a bounded device-side wait gave up (code %d: %s); the outputs of that call are incomplete", v,
-            v == kStatusSelfTest ? "self-test" : v < 20 ? "TMA warp" : v < 30 ? "MMA warp" : v < 40 ? "softmax warp" : v < 60 ? "job ring" : "backward");
+            v >= kStatusSelfTest ? "self-test" : v < 20 ? "TMA warp" : v < 30 ? "MMA warp"
+            : v == 34 || v == 35 || v == 38 || v == 39 ? "output warp" : v < 40 ? "softmax warp" : v < 60 ? "job ring" : "backward");
   return BRK_E_TIMEOUT;
 }
 

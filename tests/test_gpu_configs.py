@@ -312,6 +312,16 @@ def test_bounded_wait_gives_up_and_is_reported(budget):
     _check_against_oracle(c)
 
 
+@pytest.mark.parametrize("code,role", [(12, "TMA"), (15, "TMA"), (20, "MMA"), (29, "MMA"), (30, "softmax"), (33, "softmax"), (37, "softmax"),
+                                       (34, "output"), (35, "output"), (38, "output"), (39, "output"), (40, "job ring"), (60, "backward"),
+                                       (80, "backward"), (90, "self-test"), (91, "self-test")])
+def test_status_codes_name_the_role(code, role):
+    w = torch.tensor([code], dtype=torch.int32, device="cuda")
+    L = _lib.lib()
+    assert L.brk_status_poll(w.data_ptr(), torch.cuda.current_stream().cuda_stream) == -6
+    assert f"code {code}: {role}".encode() in L.brk_last_error() and int(w.item()) == 0
+
+
 @pytest.mark.parametrize("algo", [SIMT, TC])
 def test_malformed_spans_write_nothing_and_are_reported(algo):
     bl = [64, 100, 48]
