@@ -87,8 +87,7 @@ enum {
   kItemFree = 20,  // +slot (15 consuming warps)
   kNumBars = 22
 };
-constexpr uint32_t kGaveUp = kNumBars * 8 + 12;  // behind the barriers: TMEM base, two item slots, code of the first wait that gave up
-static_assert(kGaveUp + 4 <= 256, "barrier area");
+static_assert(kNumBars * 8 + 16 <= 256, "barrier area");  // + TMEM base, two item slots
 
 struct BwdTcArgs {
   View q, k, v, o, d_o, dq, dk, dv;
@@ -189,7 +188,6 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
       if (i >= kItemFree) cnt = 15u;
       ptx::mbar_init(bar(i), cnt);
     }
-    *reinterpret_cast<int*>(smem + L::kOffBar + kGaveUp) = 0;
     ptx::fence_barrier_init();
     ptx::prefetch_tmap(&maps.q);
     ptx::prefetch_tmap(&maps.g);
@@ -203,7 +201,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  ptx::BoundedWaits waits(kWaitBudget, sbase + L::kOffBar + kGaveUp);
+  ptx::BoundedWaits waits(kWaitBudget);
   auto wait = [&](int i, uint32_t parity, int code) { waits(bar(i), parity & 1u, code); };
   auto arrive = [&](int i) {
     __syncwarp();
@@ -670,7 +668,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_bwd_tc_kernel(const __grid_c
     }
   }
   ptx::tc_fence_before_sync();
-  ptx::end_of_waits(waits, a.status);
+  ptx::end_of_waits(waits, [](int mark) { return mark; }, a.status);
   if (warp == 0) ptx::tmem_dealloc(tmem, 512);
 }
 

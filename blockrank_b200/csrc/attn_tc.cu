@@ -170,8 +170,23 @@ enum {
   kStat = kOFull + 2,                     // +chain  softmax -> output: row statistics written (4 warp arrivals)
   kNumBars = kStat + 2
 };
-constexpr uint32_t kGaveUp = kNumBars * 8 + 4;  // behind the barriers: TMEM base, code of the first wait that gave up
-static_assert(kGaveUp + 4 <= 512, "barrier area");
+static_assert(kNumBars * 8 + 8 <= 512, "barrier area");  // + the TMEM base address
+
+// Code for the status word of warp `warp`'s wait on barrier i.
+__device__ __forceinline__ int wait_code(int i, int warp) {
+  const int x = i & 1;  // (the chain, of the barriers that come in pairs)
+  if (i < kQFree) return 20 + x;
+  if (i < kSFull) return 28 + x;
+  if (i < kPFull) return 30 + x;
+  if (i < kPVDone) return 24 + x;
+  if (i < kOFree) return 32 + x;
+  if (i < kKVFull) return (warp < 8 ? 36 : 26) + x;
+  if (i < kKVFree) return 22 + (warp - 17);
+  if (i < kJobFull) return 12;
+  if (i < kJobFree) return 40 + (i - kJobFull) / kJobRing;
+  if (i < kOFull) return 14 + (i - kJobFree) / kJobRing;
+  return (i < kStat ? 34 : 38) + x;
+}
 
 // Division by a run-time constant with a host-computed reciprocal (round-up method, exact for every
 // 32-bit numerator): q = umulhi(n, mul); n / d = (((n - q) >> 1) + q) >> shift.
@@ -441,7 +456,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       if (i >= kJobFree && i < kOFull) cnt = 9u;                                          // MMA, softmax, output warps
       ptx::mbar_init(bar(i), cnt);
     }
-    *reinterpret_cast<int*>(smem + kOffBar + kGaveUp) = 0;
     ptx::fence_barrier_init();
     ptx::prefetch_tmap(&tmQ);
     ptx::prefetch_tmap(&tmK);
@@ -473,15 +487,15 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     return;
   }
 
-  ptx::BoundedWaits waits(kWaitBudget, sBar + kGaveUp);
-  auto wait = [&](int i, uint32_t parity, int code) { waits(bar(i), parity & 1u, code); };
+  ptx::BoundedWaits waits(kWaitBudget);  // (a wait's mark is its barrier's address: it is in a register there)
+  auto wait = [&](int i, uint32_t parity) { waits(bar(i), parity & 1u, (int)bar(i)); };
 
   int* const job_ring = reinterpret_cast<int*>(smem + kOffJobs);
   const int tok_shift = 7 - a.g_shift, TOK = 1 << tok_shift;  // query tokens of a row tile
   // consumer side of chain x's job ring: copy record number i, release its slot
   auto next_job = [&](int x, uint32_t i) {
     const uint32_t slot = i % kJobRing;
-    wait(kJobFull + x * kJobRing + slot, i / kJobRing, 40 + x);
+    wait(kJobFull + x * kJobRing + slot, i / kJobRing);
     Job it = read_record(job_ring + (x * kJobRing + slot) * 16);
     if (__any_sync(0xffffffffu, waits.gave_up())) it.flags |= kFStop;  // a wait gave up: the whole warp stops here
     __syncwarp();
@@ -535,7 +549,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     auto publish = [&](int x, const Job& it) {
       const uint32_t np = x ? n_pub1 : n_pub0;
       const uint32_t slot = np % kJobRing;
-      if (np >= kJobRing) wait(kJobFree + x * kJobRing + slot, np / kJobRing - 1, 14 + x);
+      if (np >= kJobRing) wait(kJobFree + x * kJobRing + slot, np / kJobRing - 1);
       if (leader && !waits.gave_up()) {  // (behind a wait that gave up the record may still be read)
         if (it.n > 0) {  // its Q tile on its way into L2: the MMA warp requests it when the chain's buffer is free
           ptx::tma_prefetch_4d(&tmQ, 0, it.g * G, it.start + it.t0, it.b);
@@ -549,7 +563,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // wait until both MMA warps have handed back the load last signalled on barrier s
     auto drain = [&](int s) {
       if ((out_mask >> s) & 1u) {
-        wait(kKVFree + s, (free_par >> s) & 1u, 12);
+        wait(kKVFree + s, (free_par >> s) & 1u);
         free_par ^= 1u << s;
         out_mask &= ~(1u << s);
       }
@@ -769,7 +783,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     const uint64_t v_desc0 = ptx::smem_desc_sw128(sbase + kOffV, kPoolHalf, 1024);
     const uint32_t tm_s = tmem + (uint32_t)x * kChainCols, tm_o = tm_s + kColO;
     auto wait_full = [&](int s) {
-      wait(kKVFull + s, (full_par >> s) & 1u, 22 + x);
+      wait(kKVFull + s, (full_par >> s) & 1u);
       full_par ^= 1u << s;
     };
     // S = Q K^T against `keys` keys starting at pool slot `slot`
@@ -821,7 +835,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     // has been published, otherwise at the start of that job.
     uint32_t q_issued = 0;
     auto request_q = [&](const Job& jb) {
-      if (q_issued > 0) wait(kQFree + x, q_issued - 1, 28 + x);  // every Q K^T of the previous job has read the buffer
+      if (q_issued > 0) wait(kQFree + x, q_issued - 1);  // every Q K^T of the previous job has read the buffer
       if (ptx::elect_one()) {
         const uint32_t dst = sbase + kOffQ + (uint32_t)x * kQBytes;
         ptx::mbar_expect_tx(bar(kQFull + x), kQBytes);
@@ -849,7 +863,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       // a phase further, and a parity wait must never fall two phases behind)
       if (T > 0 && !pre_qk) {
         if (q_issued == q_uses) request_q(it);  // not requested ahead
-        wait(kQFull + x, q_uses, 20 + x);
+        wait(kQFull + x, q_uses);
         ++q_uses;
       }
       if (T == 1 && pre_qk) request_next_q(job_no);  // its only Q K^T went out with the previous job's last P V
@@ -870,9 +884,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           pre_qk = false;
           for (int t = 0; t < T; ++t) {
             if (t + 1 < T) ensure(min(n, 2 * t + 4));
-            wait(kPFull + x, p_seen, 24 + x);
+            wait(kPFull + x, p_seen);
             ++p_seen;
-            if (t == 0 && jobs_done > 0) wait(kOFree + x, jobs_done - 1, 26 + x);
+            if (t == 0 && jobs_done > 0) wait(kOFree + x, jobs_done - 1);
             // After the job's last tile the chain's next row tile of the same block can start at once if its
             // record and its Q tile are already here (its first key tile is resident): its first Q K^T then
             // rides behind this P V, and its S tile is waiting when the softmax warps have drained O.
@@ -932,9 +946,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
           // tile has landed)
           wait_full(pos(t) + 1);
           if (t + 1 < T) wait_full(pos(t + 1));
-          wait(kPFull + x, p_seen, 24 + x);
+          wait(kPFull + x, p_seen);
           ++p_seen;
-          if (t == 0 && jobs_done > 0) wait(kOFree + x, jobs_done - 1, 26 + x);
+          if (t == 0 && jobs_done > 0) wait(kOFree + x, jobs_done - 1);
           ptx::tc_fence_after_sync();
           issue_pv(pos(t), keys_of(t), t == 0, t + 1 == T);
           free_kv(pos(t) + 1);
@@ -963,10 +977,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     for (uint32_t job_no = 0;; ++job_no) {
       const Job it = next_job(x, job_no);
       const int flags = it.flags;
-      if (flags & kFStop) {
-        if (waits.gave_up()) waits.record(36 + x);  // the wait at the end of a job, if no other: recorded there it made the role spill
-        break;
-      }
+      if (flags & kFStop) break;
       if (it.n == 0) continue;
       const int32_t* bs = a.blk_start + (size_t)it.b * a.M;
       const int32_t* bl = a.blk_len + (size_t)it.b * a.M;
@@ -978,13 +989,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
       for (int t = 0; t < t_mine; ++t) {
         const int cnt = min(2, n_mine - 2 * t);  // slots of this tile the chain sees
-        wait(kSFull + x, s_seen, 30 + x);
+        wait(kSFull + x, s_seen);
         ++s_seen;
         if (t > 0) {
           // The previous tile's P V was issued before this tile's Q K^T, so it has completed too: O is stable
           // and the P columns (first half of S) may be overwritten.  Consuming that phase here keeps the pass
           // below free of calls (64 logits are live across its middle).
-          wait(kPVDone + x, pv_seen, 32 + x);
+          wait(kPVDone + x, pv_seen);
           ++pv_seen;
         }
         ptx::tc_fence_after_sync();
@@ -1128,7 +1139,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       }
 
       ++pv_seen;  // (the output warps wait for the job's last P V)
-      if (tiles_done > 0) wait(kOFree + x, tiles_done - 1, 0);  // the previous tile's statistics have been read
+      if (tiles_done > 0) waits.unless_given_up(bar(kOFree + x), (tiles_done - 1) & 1u, (int)bar(kOFree + x));  // the previous tile's statistics have been read
       ++tiles_done;
       stat[r] = make_float2(m_run, l_run);
       __syncwarp();
@@ -1151,10 +1162,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
       const int n = it.g * G + (r & (G - 1));
       const bool active = tok < it.len;
       const bool split = (it.flags & kFSplit) != 0;
-      wait(kStat + x, done, 38 + x);
+      wait(kStat + x, done);
       const float2 ml = stat[r];
       const float m_run = ml.x, l_run = ml.y;
-      wait(kOFull + x, done, 34 + x);
+      wait(kOFull + x, done);
       ++done;
       ptx::tc_fence_after_sync();
       auto chunk = [&](int ch, uint32_t (&orow)[32]) {
@@ -1222,7 +1233,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
   // ---- teardown ---------------------------------------------------------------------------------
   ptx::tc_fence_before_sync();
-  ptx::end_of_waits(waits, a.status);
+  ptx::end_of_waits(waits, [&](int mark) { return wait_code((mark - (int)sBar) >> 3, warp); }, a.status);
   if (warp == 0) ptx::tmem_dealloc(tmem, kTmemCols);
 }
 
@@ -1234,23 +1245,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 // behind kStatusSelfTest.
 __global__ void selftest_wait_kernel(int32_t* status, int budget) {
   __shared__ __align__(8) uint64_t mbar[3];
-  __shared__ int word;
   uint32_t b[3];
   for (int i = 0; i < 3; ++i) {
     b[i] = ptx::smem_u32(&mbar[i]);
     ptx::mbar_init(b[i], 1);
   }
-  word = 0;
   ptx::fence_barrier_init();
   ptx::mbar_arrive(b[2]);
-  ptx::BoundedWaits waits(budget, ptx::smem_u32(&word));
+  ptx::BoundedWaits waits(budget);
   waits(b[2], 0, kStatusSelfTest + 2);
   bool ok = !waits.gave_up();
   ok &= waits(b[0], 0, kStatusSelfTest) == budget && waits.gave_up();
   ok &= waits(b[1], 0, kStatusSelfTest + 2) == 1;
-  ok &= waits(b[2], 0, kStatusSelfTest + 2) == 0;
+  ok &= waits(b[2], 0, kStatusSelfTest + 2) == 0 && waits.unless_given_up(b[1], 0, kStatusSelfTest + 2) == 0;
   if (!ok) atomicCAS(status, 0, kStatusSelfTest + 1);
-  ptx::end_of_waits(waits, status);
+  ptx::end_of_waits(waits, [](int mark) { return mark; }, status);
 }
 
 int selftest_wait_launch(int32_t* status, uint32_t budget, cudaStream_t st) {

@@ -130,9 +130,9 @@ inline View make_view(const brk_view& v) { return View{(char*)v.ptr, v.stride_b,
 // Every attention call gets a 256-byte header at the start of its workspace: [0] the work counter of the
 // tensor-core kernel, [1] the verdict of the span check (non-zero: malformed, the kernels write nothing).
 constexpr size_t kWsHeader = 256;
-// Values of the caller's status word: 10..49 (forward) and 60..80 (backward) name the bounded wait that gave up first in its CTA
-// (10..19 TMA warp, 20..29 MMA warps, 34, 35, 38, 39 output warps, other 30..39 softmax warps, 40, 41 any of these at the job
-// ring; even numbers chain 0, odd ones chain 1), 50 malformed block spans, 51 a signal row outside the prompt, 90 the
+// Values of the caller's status word: 10..49 (forward) and 60..80 (backward) name the bounded wait that gave up first in its thread
+// (10..19 TMA warp, 20..29 MMA warps, 34, 35, 38, 39 output warps, other 30..39 softmax warps, 40, 41 one of the last three at
+// the job ring; even numbers chain 0, odd ones chain 1), 50 malformed block spans, 51 a signal row outside the prompt, 90 the
 // self-test's wait, 91 a self-test that found something else.
 constexpr int kStatusBadSpans = 50;
 constexpr int kStatusBadRows = 51;

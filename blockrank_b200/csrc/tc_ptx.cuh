@@ -55,42 +55,47 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// The bounded waits of one thread.  The first one in the CTA to give up leaves its code in a word of shared memory (`word`, zero
-// at the start), which report() puts into the caller's status word when the kernel is left; a thread whose wait gave up tries
-// once in every later wait.  In line, because values are live in registers across many of the kernels' waits, and with next to
-// nothing for the case that they run out: with the atomic on the status word itself at each site the attention forward was 2 %
-// slower and a training step 7 %, with the code kept in a register the forward spilled and was 6 % slower.
+// The bounded waits of one thread.  The first one that gives up leaves its mark behind, negative, where the number of tries was:
+// every later wait of the thread tries once.  In line, because values are live in registers across many of the kernels' waits,
+// and with next to nothing for the case that they run out, because each instruction there is fetched with the loop: with an
+// atomic on the status word at each site the attention forward was 2 % slower and a training step 7 %, with one on a word of
+// shared memory a call of 5 documents 2 %.
 struct BoundedWaits {
   int tries;
-  uint32_t word;
-  __device__ __forceinline__ BoundedWaits(int budget, uint32_t smem_word) : tries(budget), word(smem_word) {}
-  __device__ __forceinline__ void record(int code) const {
-    asm volatile("{\n\t.reg .b32 r;\n\tatom.shared::cta.cas.b32 r, [%0], 0, %1;\n\t}" ::"r"(word), "r"(code) : "memory");
+  __device__ __forceinline__ explicit BoundedWaits(int budget) : tries(budget) {}
+  // `mark` is positive.  Returns how many tries failed (the kernels drop it).
+  __device__ __forceinline__ int operator()(uint32_t bar, uint32_t parity, int mark) {
+    return loop<false>(bar, parity, mark);
   }
-  // Number of tries that failed (the kernels drop it).  Code 0: recorded by the caller later.
-  __device__ __forceinline__ int operator()(uint32_t bar, uint32_t parity, int code) {
+  // The same, with no try at all in a thread that has given up (at one site of the attention forward the compiler spills 41
+  // registers unless it knows that the mark needs no keeping).
+  __device__ __forceinline__ int unless_given_up(uint32_t bar, uint32_t parity, int mark) {
+    return gave_up() ? 0 : loop<true>(bar, parity, mark);
+  }
+  __device__ __forceinline__ bool gave_up() const { return tries < 0; }
+  __device__ __forceinline__ int mark() const { return -tries; }
+
+ private:
+  template <bool kFirst>
+  __device__ __forceinline__ int loop(uint32_t bar, uint32_t parity, int mark) {
     int n = 0;
 #pragma unroll 1
     while (!mbar_try(bar, parity))
       if (++n >= tries) {
-        tries = 0;
-        if (code != 0) record(code);
+        if (kFirst || tries > 0) tries = -mark;
         break;
       }
     return n;
   }
-  __device__ __forceinline__ bool gave_up() const { return tries == 0; }
 };
 
-// The end of a kernel that waits, called by all threads (with a barrier inside): reports, and when a wait has given up lets a
-// millisecond pass, far more than copies and products take that nothing has waited for and that may still be under way.
-__device__ __forceinline__ void end_of_waits(const BoundedWaits& w, int32_t* status) {
+// The end of a kernel that waits, called by all threads, with a barrier in it: puts the code that `code_of` makes of a thread's
+// mark into the status word, and when a wait of any thread has given up lets a millisecond pass, far more than copies and
+// products take that nothing has waited for and that may still be under way.
+template <typename F>
+__device__ __forceinline__ void end_of_waits(const BoundedWaits& w, F code_of, int32_t* status) {
   if (__syncthreads_or(w.gave_up())) {
-    if (w.gave_up() && status) {
-      int code;
-      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(code) : "r"(w.word) : "memory");
-      atomicCAS(status, 0, code);
-    }
+    if (w.gave_up() && status) atomicCAS(status, 0, code_of(w.mark()));
 #pragma unroll 1
     for (int i = 0; i < 100; ++i) __nanosleep(10000);
   }

@@ -156,7 +156,7 @@ BRK_API int brk_attn_bwd_reporting(const brk_attn_bwd_params* p, void* workspace
 
 /* Device-side status.  The kernels never trap: a bounded wait that gives up, or malformed block spans, set
  * the caller's status word (brk_attn_params.status) and the kernel returns normally.  The word keeps the first code
- * written to it; a kernel's CTAs write theirs, the wait that gave up first in each, as they leave.
+ * written to it; that of a wait is written when its thread leaves the kernel.
  * brk_status_poll synchronises `stream`, reads the word and clears it: BRK_OK if it was zero,
  * BRK_E_TIMEOUT after a wait gave up (the outputs of that call are incomplete), BRK_E_ARG after malformed
  * spans (nothing was written); brk_last_error() names the event.  Call it where the host synchronises
