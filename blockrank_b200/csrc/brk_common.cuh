@@ -104,21 +104,29 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&v)[8]) {
 
 // Launch that may start before the preceding kernel of the stream has finished (its blocks become resident while that one
 // drains); the kernel must execute ptx::grid_dependency_wait() before it touches memory.
+// `cluster` neighbouring blocks (in x, a divisor of the grid) form a cluster.
 template <typename K, typename... A>
-int launch_dependent(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+int launch_dependent_clusters(int cluster, K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at = {};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute at[2] = {};
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   BRK_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return BRK_OK;
+}
+template <typename K, typename... A>
+int launch_dependent(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+  return launch_dependent_clusters(1, kernel, grid, block, smem, st, args...);
 }
 
 struct View {

@@ -15,12 +15,13 @@
 //                        a tcgen05 tile (M >= 64, operands staged in shared
 //                        memory, result through tensor memory) would add
 //                        latency to a kernel that has no tensor-rate problem.
-//   doc_merge_kernel     one CTA per prompt, launched beside the partial kernel's end: merges the per-document pairs into
-//                        the softmax over all document tokens, emits the per-document probability mass and then the mean
-//                        over heads and rows / temperature.  As the job of the last CTA of a prompt, found by counters that
-//                        a memset cleared in front, with a fence and an atomic in every CTA: 4 prompts of 100 documents
-//                        38.0 us, now 29.1 (the K read at 5.4 TB/s), one prompt of 100 20.5, now 13.6.  A call of a few
-//                        short documents: alone 24.5, now 23.0; in a row, bound by the host, 12.0 and 12.9.
+//   doc_merge_kernel     one CTA per prompt, or a cluster of up to eight for many pairs, brought up as the partial kernel's
+//                        CTAs leave the SMs: merges the per-document pairs into the softmax over all document tokens, emits
+//                        the per-document probability mass and then the mean over heads and rows / temperature.  As the job
+//                        of the last CTA of a prompt, found by counters that a memset cleared in front, with a fence and an
+//                        atomic in every CTA: 4 prompts of 100 documents 37.4 us, now 29.1 (the K read at 5.4 TB/s), one
+//                        prompt of 100 20.5, now 13.7.  A call of a few short documents: alone 20.5, now 19.2; in a row,
+//                        bound by the host, 12.3 and 9.2.
 #include <algorithm>
 #include <atomic>
 
@@ -53,18 +54,28 @@ __device__ __forceinline__ void merge_pair(float& m, float& l, float x0, float x
   m = mn;
 }
 
-// One CTA per prompt.  A warp takes two (head, signal row) pairs at a time, so that their statistics travel together; then
-// the masses are summed per document, group by group of heads, in a fixed order.  Bound by latency: a read of the pairs, a
-// write and a read of the masses.
-constexpr int kMergeThreads = 1024;
-__global__ void __launch_bounds__(kMergeThreads) doc_merge_kernel(ScoreArgs a) {
+// One CTA per prompt, or a cluster of them (kCluster: grid.x) that share its KV heads.  A warp takes two (head, signal row)
+// pairs at a time, so that their statistics travel together; then the masses are summed per document, group by group of heads,
+// in a fixed order, the same for any number of CTAs.  Bound by latency: a read of the pairs, a write and a read of the masses.
+// (Clusters of 512 threads at 64 registers, so that two CTAs share an SM: at 78 registers 32 prompts of 300 documents took 196
+// us, now 185; one row at a time, no spill, 2,000 documents with 16 rows 277, now 248.)
+template <bool kCluster>
+constexpr int merge_threads = kCluster ? 512 : 1024;
+template <bool kCluster>
+__global__ void __launch_bounds__(merge_threads<kCluster>, kCluster ? 2 : 1) doc_merge_kernel(ScoreArgs a) {
+  constexpr int kMergeThreads = merge_threads<kCluster>;
   constexpr int kHeld = 8;  // pairs per lane kept in registers: one round trip per row up to 256 documents
   constexpr int kWarps = kMergeThreads / 32, kRows = 2;
   __shared__ float s_group[kMergeThreads];
   ptx::grid_dependency_wait();  // the partial kernel's pairs
-  const int nd = a.M - 2, b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int G = a.N / a.Nk, GR = G * a.R, W = a.N * a.R;
-  const size_t w0 = (size_t)b * W;
+  const int nd = a.M - 2, b = kCluster ? blockIdx.y : blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // KV heads of this CTA: g_lo .. g_lo + n_g - 1, of `per` in all but the last ones (a.Nk spelled out below where there is one
+  // CTA: kept in a variable from here on, it made the kernel spill)
+  const int n_cta = kCluster ? (int)gridDim.x : 1, rank = kCluster ? (int)blockIdx.x : 0;
+  const int per = kCluster ? (a.Nk + n_cta - 1) / n_cta : 0;
+  const int g_lo = min(a.Nk, rank * per), n_g = kCluster ? min(a.Nk, g_lo + per) - g_lo : 0;
+  const int G = a.N / a.Nk, GR = G * a.R, W = kCluster ? n_g * GR : a.N * a.R;
+  const size_t w0 = kCluster ? ((size_t)b * a.Nk + g_lo) * GR : (size_t)b * W;
   for (int first = warp; first < W; first += kRows * kWarps) {
     float2 held[kRows][kHeld];
     float mx[kRows], z[kRows];
@@ -104,28 +115,35 @@ __global__ void __launch_bounds__(kMergeThreads) doc_merge_kernel(ScoreArgs a) {
     }
   }
   if (a.logits == nullptr) return;
-  __syncthreads();  // every mass of the prompt has been written
-  // A thread sums a group's rows for one document, then one thread per document the groups.
-  const int tile = max(1, kMergeThreads / a.Nk);  // documents at a time
+  __syncthreads();  // every mass of these heads has been written
+  // A thread sums a group's rows for one document, then one thread per document the groups of all CTAs, in order.
+  const int tile = max(1, kMergeThreads / (kCluster ? per : a.Nk));  // documents at a time
   for (int d0 = 0; d0 < nd; d0 += tile) {
     const int n = min(tile, nd - d0);
-    float total = 0.f;  // (more groups than threads: in rounds)
-    for (int g0 = 0; g0 < a.Nk; g0 += kMergeThreads) {
-      const int ng = min(a.Nk - g0, kMergeThreads);
+    float total = 0.f;
+    for (int g0 = 0; g0 < (kCluster ? per : a.Nk); g0 += kMergeThreads) {  // (more groups than threads: in rounds)
+      const int ng = min((kCluster ? per : a.Nk) - g0, kMergeThreads);
       const int g = tid / n, d = tid % n;
-      if (g < ng) {
+      if (g < (kCluster ? min(ng, n_g - g0) : ng)) {
         const float* const m = a.mass + (w0 + (size_t)(g0 + g) * GR) * nd + d0 + d;
         float acc = 0.f;
 #pragma unroll 8
         for (int row = 0; row < GR; ++row) acc += m[(size_t)row * nd];
         s_group[g * n + d] = acc;
       }
-      __syncthreads();
-      if (tid < n)
+      if (kCluster) ptx::cluster_sync(); else __syncthreads();
+      if (kCluster) {
+        if (tid < n && tid % n_cta == rank)
+          for (int c = 0; c < n_cta; ++c) {
+            const int left = min(ng, a.Nk - c * per - g0);  // of CTA c's groups in this round
+            for (int i = 0; i < left; ++i) total += ptx::ld_cluster_f32(ptx::smem_u32(s_group + i * n + tid), c);
+          }
+      } else if (tid < n) {
         for (int i = 0; i < ng; ++i) total += s_group[i * n + tid];
-      __syncthreads();
+      }
+      if (kCluster) ptx::cluster_sync(); else __syncthreads();
     }
-    if (tid < n) a.logits[(size_t)b * nd + d0 + tid] = total * a.inv_count_temp;
+    if (tid < n && (!kCluster || tid % n_cta == rank)) a.logits[(size_t)b * nd + d0 + tid] = total * a.inv_count_temp;
   }
 }
 
@@ -154,7 +172,8 @@ __device__ __forceinline__ void key_dots(const T* __restrict__ kp, const float* 
 // One CTA per (document, prompt, KV head).  Each warp stages 32 key rows at a time in shared memory
 // with fully coalesced 16-byte loads (all in flight together), then every lane owns one key: its
 // dot products against the G*R staged query rows read the key from shared memory (row stride padded
-// by 16 bytes, conflict-free for 16-byte accesses) and the query rows as broadcasts.
+// by 16 bytes, conflict-free for 16-byte accesses) and the query rows as broadcasts.  (head_dim 64 spills 16 bytes at the 96
+// registers that it is given; with 128 and next to no spill, but fewer CTAs per SM, 4 prompts of 100 documents take 81 us, not 62.)
 template <typename T, int D>
 __global__ void __launch_bounds__(kThreads) doc_partial_kernel(ScoreArgs a) {
   constexpr int kRowBytes = D * (int)sizeof(T);
@@ -404,11 +423,22 @@ static int doc_scores_run(const brk_score_params& p, void* ws, size_t ws_bytes, 
   dim3 grid(nd, p.B * p.Nk);
   const size_t pitch = (size_t)p.D * (p.dtype == BRK_BF16 ? 2 : 4) + 16;
   const size_t sm = (size_t)G * p.R * p.D * 4 + (kThreads / 32) * kRowBatch * sizeof(float2) + (kThreads / 32) * 32 * pitch;
+  // The merge of one prompt: up to 16,384 pairs on one SM, more on up to eight.  One prompt of 300 documents (19,200 pairs) 31.1
+  // us on one, 28.4 on eight, of 500 with 16 signal rows 220 and 133, of 2,000 with 16 rows 600 and 248; 16 prompts of 250
+  // (16,000 pairs each) 101 and 104, 4 of 100 (6,400) 29.3 and 30.0.  (With every prompt on one, more than 100,000 pairs took
+  // longer than when the CTA of each KV head that finished last merged its rows: 206 us for 500 with 16 rows, 411 for 2,000.)
+  int merge_ctas = 1;
+  if ((int64_t)p.N * p.R * nd > 16384)
+    while (2 * merge_ctas <= std::min(p.Nk, 8)) merge_ctas *= 2;
+  auto merge = [&]() -> int {
+    if (merge_ctas == 1) return launch_dependent(doc_merge_kernel<false>, dim3(p.B), dim3(merge_threads<false>), 0, st, a);
+    return launch_dependent_clusters(merge_ctas, doc_merge_kernel<true>, dim3(merge_ctas, p.B), dim3(merge_threads<true>), 0, st, a);
+  };
   auto launch = [&](auto kern) -> int {
     // (the kernels also hold a few KB of static shared memory, which counts against the same 48 KB default)
     if (sm + 8192 > 48 * 1024) BRK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     if ((rc = launch_dependent(kern, grid, dim3(kThreads), sm, st, a))) return rc;
-    return launch_dependent(doc_merge_kernel, dim3(p.B), dim3(kMergeThreads), 0, st, a);
+    return merge();
   };
   if (p.dtype == BRK_BF16) {
     // A CTA walks through several documents so that its key loads overlap across document boundaries; the
@@ -430,7 +460,7 @@ static int doc_scores_run(const brk_score_params& p, void* ws, size_t ws_bytes, 
     static std::atomic<bool> done128[64] = {}, done64[64] = {};
     rc = p.D == 128 ? run(doc_partial_mma_kernel<128>, done128) : run(doc_partial_mma_kernel<64>, done64);
     if (rc) return rc;
-    return launch_dependent(doc_merge_kernel, dim3(p.B), dim3(kMergeThreads), 0, st, a);
+    return merge();
   }
   return p.D == 128 ? launch(doc_partial_kernel<float, 128>) : launch(doc_partial_kernel<float, 64>);
 }

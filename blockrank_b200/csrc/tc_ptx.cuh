@@ -20,6 +20,22 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 // has been written: only the wait does.
 __device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// ---- thread-block clusters ----
+// Barrier of all threads of the cluster (of the CTA, if launched without one); what was written before is visible behind it.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The shared-memory word at this CTA's address `addr`, of CTA `rank` of the cluster.
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t rank) {
+  float v;
+  asm volatile(
+      "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}"
+      : "=f"(v)
+      : "r"(addr), "r"(rank)
+      : "memory");
+  return v;
+}
+
 // ---- mbarrier -----------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
