@@ -474,7 +474,9 @@ int doc_scores_launch(const brk_score_params& p, void* ws, size_t ws_bytes, cuda
 // array instead of a caller-provided workspace.  It is part of the library image, so every device that
 // loads the library holds these bytes until the process exits.
 static __device__ __align__(256) unsigned char g_static_scratch[BRK_STATIC_SCRATCH_BYTES];
-constexpr size_t kStaticReserve = 16384;  // of the array, and with it the 4096 (prompt, KV head) pairs it served: the call's limits
+// The call's limits are those that it had when the array began with 4096 counters: nothing uses these bytes, and what was refused
+// stays refused.
+constexpr size_t kStaticReserve = 16384;
 
 int doc_scores_static_launch(const brk_score_params& p, cudaStream_t st) {
   int rc = check_score_params(p);  // argument errors are reported as such, before the size test

@@ -74,7 +74,7 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 // The bounded waits of one thread.  The first one that gives up leaves its mark behind, negative, where the number of tries was:
 // every later wait of the thread tries once.  In line, because values are live in registers across many of the kernels' waits,
 // and with next to nothing for the case that they run out, because each instruction there is fetched with the loop: with an
-// atomic on the status word at each site the attention forward was 2 % slower and a training step 7 %, with one on a word of
+// atomic on the status word at each site the attention forward was 2 % slower and the backward 3-5 %, with one on a word of
 // shared memory a call of 5 documents 2 %.
 struct BoundedWaits {
   int tries;
